@@ -343,7 +343,7 @@ mma_attention_kernel(const __grid_constant__ KernelArgs a, const int use_evict_f
     float o[C::NT_O][4];
     float m_a = -INFINITY, m_b = -INFINITY, l_a = 0.f, l_b = 0.f;
     uint32_t qf[C::KSTEPS][4];
-    int lim_a = 0, lim_b = 0, wlim = 0;      // wlim: the largest limit of any row of this warp
+    int lim_a = 0, lim_b = 0, vlen = 0;      // vlen: rows of the current fragment that hold keys and values
     RowId id_a = {0, 0, 0}, id_b = {0, 0, 0};
     bool valid_a = false, valid_b = false;
     uint32_t cphase = 0;
@@ -395,6 +395,7 @@ mma_attention_kernel(const __grid_constant__ KernelArgs a, const int use_evict_f
             // every load independent: one memory round trip), round them to the storage type and
             // stage them in shared memory; each warp then pulls its MMA A-fragments with ldmatrix.
             const int vf = visible_length(a, f, vis);
+            vlen = vf;
             const unsigned char* qsrc = qtile;
             if (C::Q2BYTES != 0 && pre_u == cur_u && pre_f == f) {
                 // staged at kernel start: nothing to load (the tile has been complete since the second
@@ -482,9 +483,6 @@ mma_attention_kernel(const __grid_constant__ KernelArgs a, const int use_evict_f
                 lim_a = valid_a ? min(loc_a, vf - 1) + 1 : vf;
                 lim_b = valid_b ? min(loc_b, vf - 1) + 1 : vf;
             }
-            wlim = max(lim_a, lim_b);
-#pragma unroll
-            for (int sh = 16; sh > 0; sh >>= 1) wlim = max(wlim, __shfl_xor_sync(0xffffffffu, wlim, sh));
             {
                 const uint32_t qaddr = smem_u32(qsrc) + (mt * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * C::QPITCH + (lane >> 4) * 16;
 #pragma unroll
@@ -523,11 +521,11 @@ mma_attention_kernel(const __grid_constant__ KernelArgs a, const int use_evict_f
 #endif
 
         const int i0 = slice * C::NT_S;      // first in-group position of this warp's slice
-        // Keys from `nvalid` on are masked for every row of this warp: their probabilities are exactly zero, but
-        // 0 * NaN would poison the sums, and their V rows may hold anything -- past the end of a short tile the
-        // copy wrote nothing, and under a host plan rows between a fragment's true length and the host's bound
-        // are fetched as they are.  Make those V rows (of this warp's own slice) finite.
-        const int nvalid = min(ntok, wlim - tok0);
+        // V rows from `nvalid` on are nobody's: past the end of a short tile the copy wrote nothing, and under a host
+        // plan rows between a fragment's true length and the host's bound are fetched as they are.  Their
+        // probabilities are exactly zero, but 0 * NaN would poison the sums: make them finite.  (Warps of different
+        // m-tiles share a slice's rows, so what is cleared must not depend on what a warp's own query rows see.)
+        const int nvalid = min(ntok, vlen - tok0);
         if (nvalid < C::TILE) {
             unsigned char* vgen = stages + (size_t)stage * C::STAGE_BYTES + C::KV_BYTES;
 #pragma unroll 1
