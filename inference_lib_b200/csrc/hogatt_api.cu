@@ -207,22 +207,56 @@ int resolve(const hogatt_problem* p, Resolved* r) {
 }
 
 struct WorkspaceLayout {
-    size_t header, o, m, l, rq, total;
+    size_t header, pre, cost, vis, start, merge, rec, o, m, l, rq, total;     // pre ... rec: the plan of the tcgen05 kernel
     int parts;
 };
 
+// Query tiles per kv head of a fragment call on the tcgen05 kernel: whole workers, or 128-row pieces of one worker.
+void dense_geometry(int W, int64_t gs, int* tiles, int* span) {
+    if (gs > kDenseRows) {
+        *span = (int)((gs + kDenseRows - 1) / kDenseRows);
+        *tiles = W * *span;
+    } else {
+        *span = kDenseRows / (int)gs;
+        *tiles = ceil_div(W, *span);
+    }
+}
+
+// Workspace of the tcgen05 kernel: the plan, then one slot of 256 rows per (CTA, unit) pair that can meet.
+void carve_dense(WorkspaceLayout* w, int64_t blocks, int Hkv, int F, int grid, bool paged) {
+    const size_t slots = (size_t)grid + (size_t)blocks * Hkv;
+    w->parts = 0;
+    w->header = 0;
+    w->pre = 256;
+    w->cost = w->pre + align_up((size_t)(blocks + 1) * sizeof(long long), 256);
+    w->vis = w->cost + align_up((size_t)(blocks + 1) * sizeof(long long), 256);
+    w->start = w->vis + align_up((size_t)blocks * 2 * F * sizeof(int), 256);
+    w->merge = w->start + align_up((size_t)grid * sizeof(int4), 256);
+    w->rec = w->merge + align_up((size_t)blocks * Hkv * sizeof(int4), 256);
+    w->o = w->rec + (paged ? align_up((size_t)blocks * sizeof(int4), 256) : 0);
+    w->m = w->o + slots * kDenseBlock * 128 * sizeof(float);
+    w->l = w->m + align_up(slots * kDenseBlock * sizeof(float), 256);
+    w->rq = w->l + align_up(slots * kDenseBlock * sizeof(float), 256);
+    w->total = w->rq;
+}
+
 WorkspaceLayout carve(const hogatt_problem* p, const Resolved& r, int grid) {
-    WorkspaceLayout w;
+    WorkspaceLayout w = {};
+    if (r.kernel == HOGATT_KERNEL_DENSE) {
+        int tiles, span;
+        dense_geometry(p->W, (int64_t)(p->Hq / p->Hkv) * p->S, &tiles, &span);
+        carve_dense(&w, (tiles + 1) / 2, p->Hkv, p->F, grid, false);
+        // the tcgen05 kernel reads rotated queries from memory: room for them in case the caller does not want them back
+        w.total += align_up((size_t)p->F * p->W * p->Hq * p->S * p->E * dtype_size(p->dtype), 256);
+        return w;
+    }
     w.parts = max_parts_per_unit(r.units, grid);
     const size_t slots = (size_t)r.units * w.parts * r.rows_per_block;
     w.header = 0;
     w.o = 256;
     w.m = w.o + align_up(slots * p->Ev * sizeof(float), 256);
     w.l = w.m + align_up(slots * sizeof(float), 256);
-    w.rq = w.l + align_up(slots * sizeof(float), 256);
-    // the tcgen05 kernel reads rotated queries from memory: room for them in case the caller does not want them back
-    w.total = w.rq + (r.kernel == HOGATT_KERNEL_DENSE
-                          ? align_up((size_t)p->F * p->W * p->Hq * p->S * p->E * dtype_size(p->dtype), 256) : 0);
+    w.total = w.l + align_up(slots * sizeof(float), 256);
     return w;
 }
 
@@ -576,40 +610,135 @@ int fragment_map(const void* ptr, int rows, int Hkv, int dtype, CUtensorMap* out
     return HOGATT_OK;
 }
 
-template <class T>
-int launch_dense(const KernelArgs& args, const void* q_rot, int dtype, int dev, int smem_optin, int grid, cudaStream_t stream) {
+bool aligned16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
+
+// `beside_predecessor`: the stream's preceding kernel is one of ours that writes nothing this one reads and lets it start
+// early; the rotation kernels end only after it (programmatic launch, waited for at the end).
+int rope_launch(void* rq, const void* queries, const float* cosines, const float* sines, int F, int W, int Hq, int S, int E,
+                int rotary_dim, int dtype, cudaStream_t stream, bool beside_predecessor = false) {
+    const int64_t rows = (int64_t)F * W * Hq * S;
+    if (rows > (1 << 30) || rows * std::max(E, 8) >= ((int64_t)1 << 31)) return HOGATT_ERR_TOO_LARGE;   // 32-bit element counts
+    cudaError_t rc = cudaSuccess;
+    auto go = [&](auto kernel, dim3 grid, auto... args) {
+        if (beside_predecessor) return launch_kernel(kernel, grid, dim3(128), 0, stream, args...);
+        kernel<<<grid, 128, 0, stream>>>(args...);
+        return cudaGetLastError();
+    };
+    const int64_t work = rows * ((dtype != HOGATT_F32 && E % 8 == 0) ? E / 8 : E);      // chunks or channels
+    if (dtype != HOGATT_F32 && rotary_dim == E && E % 16 == 0 && aligned16(cosines) && aligned16(sines) && aligned16(queries) &&
+        aligned16(rq)) {
+        // whole head rotated: a thread per pair of partner chunks, tables kept in registers over kRopeHeads heads
+        const int64_t items = (int64_t)F * W * S * (E / 16);
+        const dim3 grid((unsigned)((items + 127) / 128), (unsigned)ceil_div(Hq, kRopeHeads));
+        if (dtype == HOGATT_F16)
+            rc = go(rope_pairs_kernel<__half>, grid, (__half*)rq, (const __half*)queries, cosines, sines, F, W, Hq, S, E);
+        else
+            rc = go(rope_pairs_kernel<__nv_bfloat16>, grid, (__nv_bfloat16*)rq, (const __nv_bfloat16*)queries, cosines, sines, F, W, Hq, S, E);
+        HOGATT_CUDA_OK(rc);
+        return HOGATT_OK;
+    }
+    // one pass of four chunks per thread where there is enough work: 16 CTAs of 128 threads per SM
+    int dev = 0, sms = 0, smem_optin = 0;
+    if (const int bad = current_device_info(&dev, &sms, &smem_optin)) return bad;
+    const unsigned blocks = (unsigned)std::min<int64_t>((work + 127) / 128, (int64_t)sms * 16);
+    switch (dtype) {
+        case HOGATT_F32:
+            rc = go(rope_kernel<float>, dim3(blocks), (float*)rq, (const float*)queries, cosines, sines, F, W, Hq, S, E, rotary_dim);
+            break;
+        case HOGATT_F16:
+            rc = go(rope_kernel<__half>, dim3(blocks), (__half*)rq, (const __half*)queries, cosines, sines, F, W, Hq, S, E, rotary_dim);
+            break;
+        case HOGATT_BF16:
+            rc = go(rope_kernel<__nv_bfloat16>, dim3(blocks), (__nv_bfloat16*)rq, (const __nv_bfloat16*)queries, cosines, sines, F, W, Hq, S, E, rotary_dim);
+            break;
+        default: return HOGATT_ERR_UNSUPPORTED_DTYPE;
+    }
+    HOGATT_CUDA_OK(rc);
+    return HOGATT_OK;
+}
+
+// Plan, (rotation,) attention and merge of a call on the tcgen05 kernel.  `maps` is complete but for what is per call.
+template <class T, bool PAGED>
+int launch_dense_kernels(const DenseArgs& d, const DenseMaps& maps, int dev, int smem_optin, cudaStream_t stream) {
     static std::atomic<size_t> granted[kMaxDevices];
-    const size_t smem = dense_smem_bytes(args.F);
-    if (smem > (size_t)smem_optin) return HOGATT_ERR_TOO_MANY_FRAGMENTS;
-    int rc = ensure_smem_limit(dense_attention_kernel<T>, dev, smem, granted);
+    if (kDenseSmemBytes > (size_t)smem_optin) return HOGATT_ERR_CUDA;
+    const int rc = ensure_smem_limit(dense_attention_kernel<T, PAGED>, dev, kDenseSmemBytes, granted);
     if (rc != HOGATT_OK) return rc;
+    dense_attention_kernel<T, PAGED><<<dim3(d.ctas), dim3(kDenseThreads), kDenseSmemBytes, stream>>>(d, maps);
+    HOGATT_CUDA_OK(cudaGetLastError());
+    // at most ctas - 1 units are split; more on the list are blocks of one tile or blind ones (the kernel walks the list)
+    const dim3 grid((unsigned)std::min<int64_t>((int64_t)d.blocks * d.Hkv, 2 * (int64_t)d.ctas), kDenseBlock / 32, 128 / (16 * kDenseMergeWarps));
+    HOGATT_CUDA_OK(launch_kernel(dense_merge_kernel<T, PAGED>, grid, dim3(kDenseMergeWarps * 32), 0, stream, d));
+    return HOGATT_OK;
+}
+
+void dense_workspace(DenseArgs* d, unsigned char* ws, const WorkspaceLayout& w) {
+    d->nmerge = reinterpret_cast<int*>(ws + w.header);
+    d->start = reinterpret_cast<int4*>(ws + w.start);
+    d->merge = reinterpret_cast<int4*>(ws + w.merge);
+    d->pre = reinterpret_cast<long long*>(ws + w.pre);
+    d->cost = reinterpret_cast<long long*>(ws + w.cost);
+    d->vis = reinterpret_cast<int*>(ws + w.vis);
+    d->rec = reinterpret_cast<int4*>(ws + w.rec);
+    d->ws_o = reinterpret_cast<float4*>(ws + w.o);
+    d->ws_m = reinterpret_cast<float*>(ws + w.m);
+    d->ws_l = reinterpret_cast<float*>(ws + w.l);
+}
+
+// A fragment call on the tcgen05 kernel.  It takes its queries already rotated, from memory: the rotated-query output
+// of the call (or room in the workspace when the caller does not want it) is written by the stand-alone rotation kernel
+// first, which runs beside the one-CTA plan kernel.
+template <class T>
+int launch_dense(const hogatt_problem* p, const KernelArgs& args, const WorkspaceLayout& w, bool fused, int dev, int smem_optin,
+                 int grid, cudaStream_t stream) {
+    unsigned char* ws = static_cast<unsigned char*>(p->workspace);
+    DenseArgs d;
+    memset(&d, 0, sizeof(d));
+    d.F = args.F; d.W = args.W; d.Hq = args.Hq; d.Hkv = args.Hkv; d.G = args.G; d.S = args.S;
+    const int gs = args.G * args.S;
+    dense_geometry(args.W, gs, &d.tiles, &d.tile_span);
+    d.blocks = (d.tiles + 1) / 2;
+    d.l2scale = args.l2scale;
+    for (int f = 0; f < args.F; ++f) d.cap[f] = args.host_plan ? args.ft.e[f].vis : args.ft.e[f].rows;
+    d.loc = args.loc;
+    d.flen = args.flen;
+    dense_workspace(&d, ws, w);
+    d.ctas = std::min(grid, kDenseMaxCtas);
+    d.status = args.status;
+    d.out = args.out;
+    d.world = args.world;
+    d.rank = args.rank;
+    for (int i = 0; i < args.world; ++i) d.peer_out[i] = args.peer_out[i];
+
+    const void* q_rot = p->queries;
+    if (fused) q_rot = p->rq ? p->rq : static_cast<void*>(ws + w.rq);
     DenseMaps maps;
     memset(&maps, 0, sizeof(maps));
     for (int f = 0; f < args.F; ++f) {
         if (args.ft.e[f].rows == 0) continue;             // never addressed: no tile lies in an empty fragment
-        rc = fragment_map(args.ft.e[f].k, args.ft.e[f].rows, args.Hkv, dtype, &maps.k[f]);
-        if (rc == HOGATT_OK) rc = fragment_map(args.ft.e[f].v, args.ft.e[f].rows, args.Hkv, dtype, &maps.v[f]);
+        int rc = fragment_map(args.ft.e[f].k, args.ft.e[f].rows, args.Hkv, p->dtype, &maps.k[f]);
+        if (rc == HOGATT_OK) rc = fragment_map(args.ft.e[f].v, args.ft.e[f].rows, args.Hkv, p->dtype, &maps.v[f]);
         if (rc != HOGATT_OK) return rc;
     }
-    {   // rotated queries [F, W, Hq, S, E] seen as [F, W, Hkv, G*S, E]; a 128-row block is one box
-        const int gs = args.G * args.S;
+    {   // rotated queries [F, W, Hq, S, E] seen as [F, W, Hkv, G*S, E]; a tile is one box
         const cuuint64_t dims[5] = {128, (cuuint64_t)gs, (cuuint64_t)args.Hkv, (cuuint64_t)args.W, (cuuint64_t)args.F};
-        const cuuint32_t box[5] = {64, (cuuint32_t)std::min(gs, kDenseRows), 1, (cuuint32_t)(gs < kDenseRows ? kDenseRows / gs : 1), 1};
-        rc = encode_map(&maps.q, q_rot, dtype, 5, dims, box);
+        const cuuint32_t box[5] = {64, (cuuint32_t)std::min(gs, kDenseRows), 1, (cuuint32_t)(gs > kDenseRows ? 1 : d.tile_span), 1};
+        const int rc = encode_map(&maps.q, q_rot, p->dtype, 5, dims, box);
         if (rc != HOGATT_OK) return rc;
     }
-    dense_attention_kernel<T><<<dim3(grid), dim3(kDenseThreads), smem, stream>>>(args, maps);
-    HOGATT_CUDA_OK(cudaGetLastError());
-    return HOGATT_OK;
+    HOGATT_CUDA_OK(launch_kernel(dense_plan_kernel<false>, dim3(1), dim3(kDensePlanThreads), 0, stream, d));
+    if (fused) {
+        const int rc = rope_launch(const_cast<void*>(q_rot), p->queries, p->cosines, p->sines, p->F, p->W, p->Hq, p->S, p->E,
+                                   p->rotary_dim, p->dtype, stream, /*beside_predecessor=*/true);
+        if (rc != HOGATT_OK) return rc;
+    }
+    return launch_dense_kernels<T, false>(d, maps, dev, smem_optin, stream);
 }
 
 template <class T>
-int launch_all(const KernelArgs& args, const Resolved& r, int dev, int smem_optin, int grid, cudaStream_t stream,
-               const void* q_rot = nullptr) {
+int launch_all(const KernelArgs& args, const Resolved& r, int dev, int smem_optin, int grid, cudaStream_t stream) {
     int rc;
-    if (r.kernel == HOGATT_KERNEL_DENSE) {
-        rc = launch_dense<T>(args, q_rot, std::is_same<T, __half>::value ? HOGATT_F16 : HOGATT_BF16, dev, smem_optin, grid, stream);
-    } else if (r.kernel == HOGATT_KERNEL_MMA) {
+    if (r.kernel == HOGATT_KERNEL_MMA) {
         bool ef = r.row_blocks == 1;             // every K/V byte is read once: do not let it displace L2 contents
 #ifdef HOGATT_EXPERIMENT
         if (getenv("HOGATT_STREAM_ONLY")) return launch_mma_dims<T>(args, args.F, args.E, r.mt, dev, smem_optin,
@@ -629,50 +758,10 @@ int launch_all(const KernelArgs& args, const Resolved& r, int dev, int smem_opti
 }
 
 template <>
-int launch_all<float>(const KernelArgs& args, const Resolved& r, int dev, int smem_optin, int grid, cudaStream_t stream,
-                      const void*) {
+int launch_all<float>(const KernelArgs& args, const Resolved& r, int dev, int smem_optin, int grid, cudaStream_t stream) {
     int rc = launch_fma_dims<float>(args, dev, smem_optin, grid, stream);
     if (rc != HOGATT_OK) return rc;
     return launch_merge<float>(args, r, stream);
-}
-
-bool aligned16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
-
-int rope_launch(void* rq, const void* queries, const float* cosines, const float* sines, int F, int W, int Hq, int S, int E,
-                int rotary_dim, int dtype, cudaStream_t stream) {
-    const int64_t rows = (int64_t)F * W * Hq * S;
-    if (rows > (1 << 30) || rows * std::max(E, 8) >= ((int64_t)1 << 31)) return HOGATT_ERR_TOO_LARGE;   // 32-bit element counts
-    const int64_t work = rows * ((dtype != HOGATT_F32 && E % 8 == 0) ? E / 8 : E);      // chunks or channels
-    if (dtype != HOGATT_F32 && rotary_dim == E && E % 16 == 0 && aligned16(cosines) && aligned16(sines) && aligned16(queries) &&
-        aligned16(rq)) {
-        // whole head rotated: a thread per pair of partner chunks, tables kept in registers over kRopeHeads heads
-        const int64_t items = (int64_t)F * W * S * (E / 16);
-        const dim3 grid((unsigned)((items + 127) / 128), (unsigned)ceil_div(Hq, kRopeHeads));
-        if (dtype == HOGATT_F16)
-            rope_pairs_kernel<__half><<<grid, 128, 0, stream>>>((__half*)rq, (const __half*)queries, cosines, sines, F, W, Hq, S, E);
-        else
-            rope_pairs_kernel<__nv_bfloat16><<<grid, 128, 0, stream>>>((__nv_bfloat16*)rq, (const __nv_bfloat16*)queries, cosines, sines, F, W, Hq, S, E);
-        HOGATT_CUDA_OK(cudaGetLastError());
-        return HOGATT_OK;
-    }
-    // one pass of four chunks per thread where there is enough work: 16 CTAs of 128 threads per SM
-    int dev = 0, sms = 0, smem_optin = 0;
-    if (const int rc = current_device_info(&dev, &sms, &smem_optin)) return rc;
-    const unsigned blocks = (unsigned)std::min<int64_t>((work + 127) / 128, (int64_t)sms * 16);
-    switch (dtype) {
-        case HOGATT_F32:
-            rope_kernel<float><<<blocks, 128, 0, stream>>>((float*)rq, (const float*)queries, cosines, sines, F, W, Hq, S, E, rotary_dim);
-            break;
-        case HOGATT_F16:
-            rope_kernel<__half><<<blocks, 128, 0, stream>>>((__half*)rq, (const __half*)queries, cosines, sines, F, W, Hq, S, E, rotary_dim);
-            break;
-        case HOGATT_BF16:
-            rope_kernel<__nv_bfloat16><<<blocks, 128, 0, stream>>>((__nv_bfloat16*)rq, (const __nv_bfloat16*)queries, cosines, sines, F, W, Hq, S, E, rotary_dim);
-            break;
-        default: return HOGATT_ERR_UNSUPPORTED_DTYPE;
-    }
-    HOGATT_CUDA_OK(cudaGetLastError());
-    return HOGATT_OK;
 }
 
 int attention_launch(const hogatt_problem* p, bool fused, cudaStream_t stream, const hogatt_peers* peers = nullptr) {
@@ -775,19 +864,17 @@ int attention_launch(const hogatt_problem* p, bool fused, cudaStream_t stream, c
         args.stable_fragments = pdl_enabled() ? std::max(0, std::min(p->F, p->stable_fragments)) : 0;
     }
 
-    // The tcgen05 kernel takes its queries already rotated, from memory: the rotated-query output of the call (or
-    // room in the workspace when the caller does not want it) is written by the stand-alone rotation kernel first.
-    const void* q_rot = p->queries;
-    if (r.kernel == HOGATT_KERNEL_DENSE && fused) {
-        void* dst = p->rq ? p->rq : static_cast<void*>(ws + w.rq);
-        rc = rope_launch(dst, p->queries, p->cosines, p->sines, p->F, p->W, p->Hq, p->S, p->E, p->rotary_dim, p->dtype, stream);
-        if (rc != HOGATT_OK) return rc;
-        q_rot = dst;
-    }
+    const bool dense = r.kernel == HOGATT_KERNEL_DENSE;
     switch (p->dtype) {
-        case HOGATT_F32: rc = launch_all<float>(args, r, dev, smem_optin, grid, stream, nullptr); break;
-        case HOGATT_F16: rc = launch_all<__half>(args, r, dev, smem_optin, grid, stream, q_rot); break;
-        case HOGATT_BF16: rc = launch_all<__nv_bfloat16>(args, r, dev, smem_optin, grid, stream, q_rot); break;
+        case HOGATT_F32: rc = launch_all<float>(args, r, dev, smem_optin, grid, stream); break;
+        case HOGATT_F16:
+            rc = dense ? launch_dense<__half>(p, args, w, fused, dev, smem_optin, grid, stream)
+                       : launch_all<__half>(args, r, dev, smem_optin, grid, stream);
+            break;
+        case HOGATT_BF16:
+            rc = dense ? launch_dense<__nv_bfloat16>(p, args, w, fused, dev, smem_optin, grid, stream)
+                       : launch_all<__nv_bfloat16>(args, r, dev, smem_optin, grid, stream);
+            break;
         default: return HOGATT_ERR_UNSUPPORTED_DTYPE;
     }
     if (rc != HOGATT_OK || !peers) return rc;
@@ -985,11 +1072,21 @@ int hogatt_fused_launch_static(const hogatt_problem* p, hogatt_stream_t stream) 
         const int rc = resolve(p, &r);
         return rc != HOGATT_OK ? rc : HOGATT_ERR_CUDA;
     }
-    if (need > (size_t)HOGATT_STATIC_SCRATCH_BYTES) return HOGATT_ERR_EXCEEDS_STATIC_SCRATCH;
+    hogatt_problem q = *p;
+    if (need > (size_t)HOGATT_STATIC_SCRATCH_BYTES) {
+        // the tcgen05 kernel needs a slot per CTA: with up to half of the CTAs it may fit
+        Resolved r;
+        int dev, sms, smem_optin;
+        if (resolve(p, &r) != HOGATT_OK || r.kernel != HOGATT_KERNEL_DENSE) return HOGATT_ERR_EXCEEDS_STATIC_SCRATCH;
+        if (current_device_info(&dev, &sms, &smem_optin) != HOGATT_OK) return HOGATT_ERR_CUDA;
+        const int grid = grid_size(p, sms);
+        q.max_ctas = grid;
+        while (2 * q.max_ctas > grid && carve(&q, r, q.max_ctas).total > (size_t)HOGATT_STATIC_SCRATCH_BYTES) --q.max_ctas;
+        if (q.max_ctas < 1 || 2 * q.max_ctas <= grid) return HOGATT_ERR_EXCEEDS_STATIC_SCRATCH;
+    }
     void* scratch = nullptr;
     const int rc = static_scratch_for_current_device(&scratch);
     if (rc != HOGATT_OK) return rc;
-    hogatt_problem q = *p;
     q.workspace = scratch;
     q.workspace_bytes = HOGATT_STATIC_SCRATCH_BYTES;
     return attention_launch(&q, /*fused=*/true, reinterpret_cast<cudaStream_t>(stream));

@@ -1,84 +1,113 @@
-// Dense fragment attention on the 5th-generation tensor cores (tcgen05): the path for calls with many query
-// rows per kv head -- W workers x G grouped heads x S-token chunks >= 128 rows -- where the op is bound by the
-// tensor pipe instead of HBM (16-token causal chunks of 8 workers with GQA 8 are 1,024 rows per kv head: about
-// 1,000 flop per K/V byte).
+// Dense attention on the 5th-generation tensor cores (tcgen05): calls with many query rows per kv head -- prompts,
+// causal chunks -- where the op is bound by the tensor pipe and the exponentials instead of HBM (16-token chunks of 8
+// workers with GQA 8 are 1,024 rows per kv head: about 1,000 flop per K/V byte).  One kernel for fragment tensors
+// and (PAGED) for packed queries over a paged cache.
 //
-// Same decomposition, workspace format and merge step as the other attention kernels (hogatt_plan.h): a unit is
-// (block of 128 query rows, kv head), its visible keys are tiles of 128 keys that never straddle a fragment, a
-// persistent grid of one CTA per SM walks balanced contiguous tile ranges and leaves unnormalised partial
-// results, merge_kernel folds them.  What differs is how a tile is computed:
+// Decomposition.  Query rows are cut into tiles of 128 (the MMA's M).  A block is two tiles that read the same keys, a
+// unit is (block, kv head).  dense_plan_kernel finds, per tile and fragment, how many keys any of its rows sees; a
+// block walks only those, 128 keys per step -- of a causal prompt just over half (4,000 tokens: 543 us per call when
+// every block walked every key, see below) -- and the steps of all units are one list that a persistent grid of one
+// CTA per SM cuts into balanced contiguous ranges.  A unit that lies inside one range is normalised and stored by
+// its CTA; the others leave unnormalised partials for dense_merge_kernel.
 //
-//   * Queries arrive ALREADY ROTATED as [F, W, Hq, S, E] (the rotated-query output of the fused op, written by
-//     rope_kernel just before; or the caller's own for the pre-rotated entry point).  A 128-row query tile of one
-//     fragment and kv head is one 5-D TMA box of that tensor.
-//   * K, V and Q tiles are fetched by TMA (cp.async.bulk.tensor, one tensor map per fragment, encoded on the
-//     host) into shared memory in the 128-byte-swizzled layout the tensor core reads directly.
-//   * S = Q K^T (128 x 128 x 128) and O += P V (128 x 128 x 128) are tcgen05.mma instructions issued by one
-//     thread; S (two buffers), P and O live in tensor memory.  The softmax warps pull S out of tensor memory
-//     (tcgen05.ld), mask, exponentiate, write P as bf16/f16 back into tensor memory (tcgen05.st) -- the second MMA
-//     takes its A operand from there: no trip of P through shared memory, no proxy fence, and room for deeper K / V
-//     rings (measured 166 -> 157 us per 1,024-row group) -- and keep the running max and sum in registers.  (Measured
-//     and not kept: the query tile as a tensor-memory operand too, 176 us; two query buffers with a segment-ahead fetch
-//     at the price of a two-stage K ring, +4 us; two softmax groups taking the tiles in turn, one thread per row,
-//     +20 us; programmatic dependent launch behind the rotation kernel, +3 us; half of a tile's exponentials as a cubic on
-//     the FMA pipe instead of the special-function unit, +7 us: the softmax threads are bound by issue slots and
-//     latency, not by ex2 throughput.)  O is rescaled in tensor memory only when a row's
-//     max has grown by more than 2^8 since the scale it is stored at (then exp2 arguments stay below 8 and
-//     nothing overflows); the stored scale travels with the partial result, so the merge is exact.
+// A step.  Both tiles of the block use the K and V tile (64 KiB of copies per 16.8 MFLOP; each tile alone would be at
+// the SM's L2 bandwidth).  Where a block has only one tile, the second softmax group takes every other key tile
+// of the same queries instead, and the two halves are two partials.
+//   warp 8   K copies (TMA, ring of 3 tiles)         warp 11  V copies (ring of 2)
+//   warp 9   query copies and S = Q K^T: one S buffer in tensor memory, used by the two groups in turn
+//   warp 10  O_g += P_g V, P as the tensor-memory A operand
+//   warps 0-3 / 4-7  softmax of group 0 / 1: one thread per query row.  The 128 scores go to registers at once, which
+//            frees the S buffer for the other group's product; row maximum, exponentials and sums need no
+//            exchange between threads.  The groups run half a step apart: one's tensor-memory round trips and waits lie
+//            under the other's exponentials (128 x 128 per tile = 1,024 cycles of the special-function unit, as
+//            long as the two products of the tile take the tensor pipe).
+// Tensor memory, all 512 columns: O_0, O_1 (128 each), S (128), P_0, P_1 (64 each: two 16-bit probabilities a column).
+// Issuing one tcgen05.mma costs the issuing thread 60-70 cycles, hence two issuing threads.  O is rescaled in tensor
+// memory only when a row's maximum has grown by more than 2^8 since the scale it is stored at (then exp2 arguments
+// stay below 8); the stored scale travels with the partial, so the merge is exact.
 //
-// Warp roles (352 threads): warps 0-7 softmax, warp 8 issues the K/V copies, warp 9 allocates tensor memory, issues
-// the Q copies and the S MMAs, warp 10 issues the PV MMAs.  Softmax warps w and w + 4 share the 32 query rows of tensor-memory lanes
-// 32 (w % 4) ... + 31 and split the 128 columns of S (keys) and of O between them: two warps per scheduler hide each
-// other's latencies, and a thread keeps 64 scores in registers.  Both derive the same row maximum -- each also
-// reads the other half's scores for that, which costs two more tensor-memory loads and no synchronisation -- so
-// the probabilities of a row share one scale.  Every wait is bounded.
-//
-// The reference has no counterpart: its kernel gives every (kv head, worker, token) its own CTAs and re-reads the
-// KV once per (worker, token) on CUDA cores (src/kernels/kernel_v21.cuh:62-66,957-964).
+// Every wait is bounded.  The reference has no counterpart: its kernel gives every (kv head, worker, token) its own
+// CTAs and re-reads the KV once per (worker, token) on CUDA cores (src/kernels/kernel_v21.cuh:62-66,957-964).
 #pragma once
 #include <cuda.h>
+#include <limits.h>
 
 #include "hogatt_device.cuh"
+#include "hogatt_merge.cuh"
 
 namespace hogatt {
 
 constexpr int kDenseMaxFragments = 16;      // tensor maps travel in the kernel arguments
-constexpr int kDenseRows = 128;             // query rows per CTA (MMA M)
+constexpr int kDenseRows = 128;             // query rows per tile (MMA M)
 constexpr int kDenseTile = 128;             // keys per tile (MMA N of S, K of PV)
-// Softmax warps per 32-row group: each takes 128 / SPLIT columns of every row.  (Measured on the 1,024-row shape: two
-// beat four -- every warp re-reads the whole row for the maximum, so four warps issue 1.7 times the instructions.)
-constexpr int kDenseSplit = 2;
-constexpr int kDenseSoftmaxWarps = 4 * kDenseSplit;
-constexpr int kDenseThreads = (kDenseSoftmaxWarps + 3) * 32;
+constexpr int kDenseBlock = 2 * kDenseRows;
+constexpr int kDenseSoftmaxWarps = 16;      // two groups of eight: one group per query tile, two threads per row
+constexpr int kDenseThreads = (kDenseSoftmaxWarps + 4) * 32;
+constexpr int kDensePlanThreads = 1024;
+constexpr int kDenseMaxCtas = 256;
+constexpr int kDenseUnitSteps = 2;          // what starting and finishing a unit costs, in steps
+constexpr int kDenseMergeWarps = 4;         // warps per CTA of the merge step
 
 struct alignas(64) DenseMaps {
-    CUtensorMap q;                          // [F, W, Hkv, G*S, E] view of the rotated queries
-    CUtensorMap k[kDenseMaxFragments];      // [Hkv, rows, E] per fragment
-    CUtensorMap v[kDenseMaxFragments];      // [Hkv, rows, Ev]
+    CUtensorMap q;                          // fragments: [F, W, Hkv, G*S, E] view of the rotated queries; paged: [F, total_q, Hkv, G, E]
+    CUtensorMap k[kDenseMaxFragments];      // fragments: [Hkv, rows, E] each; paged: k[0] = [blocks, Hkv, block_size, E]
+    CUtensorMap v[kDenseMaxFragments];
+};
+
+struct DenseArgs {
+    int F, W, Hq, Hkv, G, S;
+    int tiles;             // query tiles per kv head (paged: upper bound)
+    int blocks;            // blocks per kv head: pairs of tiles (paged: upper bound)
+    int tile_span;         // fragments: workers per tile (G*S <= 128) or tiles per worker; paged: query tokens per tile
+    int total_q;           // paged: packed query tokens
+    int block_size, max_blocks;
+    float l2scale;         // scale * log2(e)
+    int cap[kDenseMaxFragments];     // rows of the fragment tensors (or the host's bound); unused when paged
+    const int* loc;        // [F, W, S] or [F, total_q]
+    const int* flen;       // [F] (may be null) or [F, W]
+    const int* cu;         // paged: [W + 1]
+    const int* block_table;
+    // the plan, written by dense_plan_kernel
+    long long* pre;        // [blocks + 1] steps of the blocks before block b, per kv head
+    long long* cost;       // [blocks + 1] the same with the units' fixed costs (used by the plan kernel alone)
+    int* vis;              // [2 * blocks][F] visible keys per (tile, fragment)
+    int4* start;           // [ctas] block, kv head, step inside the unit, steps of this CTA
+    int4* merge;           // [blocks * Hkv] units left to the merge step: unit, first CTA, partials, one query tile
+    int* nmerge;
+    int4* rec;             // paged: [blocks] worker, first token, tokens
+    // Partials.  The one CTA c leaves of unit u is slot c + u (both only ever grow along the list).  Four columns of a row are one
+    // element and the rows are contiguous: a warp, one row per lane, stores and loads 512 consecutive bytes.
+    float4* ws_o;          // [slots][128 / 4][256]
+    float* ws_m;           // [slots][256]
+    float* ws_l;
+    int ctas;              // the grid; CTAs that get work: as many of them as there are steps
+    int* status;
+    void* out;             // [W, Hq, S, 128] or [total_q, Hq, 128]
+    int world, rank;       // > 0: every finished row goes to the full-size output of every rank
+    void* peer_out[HOGATT_MAX_PEERS];
 };
 
 struct DenseCfg {
     static constexpr int HD = 128;
     static constexpr int ATOM_BYTES = 128 * 128;            // [128 rows][64 16-bit columns], rows of 128 bytes, swizzled
     static constexpr int TILE_BYTES = 2 * ATOM_BYTES;       // a 128 x 128 operand tile: two column halves
-    static constexpr int NK = 3, NV = 3;                    // K ring, V ring
-    static constexpr int OFF_Q = 0;
-    static constexpr int OFF_K = OFF_Q + TILE_BYTES;
+    static constexpr int NK = 3, NV = 2;                    // K ring, V ring
+    static constexpr int OFF_Q = 0;                         // two query tiles
+    static constexpr int OFF_K = OFF_Q + 2 * TILE_BYTES;
     static constexpr int OFF_V = OFF_K + NK * TILE_BYTES;
     static constexpr int OFF_BAR = OFF_V + NV * TILE_BYTES;                 // 224 KiB of tiles
-    // barriers: q_full, k_full[NK], k_empty[NK], v_full[NV], v_empty[NV], s_full[2], s_free[2], p_full, o_done, l_ready[4]
-    static constexpr int NBAR = 1 + 2 * NK + 2 * NV + 2 + 2 + 1 + 1 + 4;
-    static constexpr int OFF_MISC = OFF_BAR + NBAR * 8;                     // tmem base, abort flag
-    static constexpr int OFF_PLAN = OFF_MISC + 16;                          // vis[F], pre[F + 1]
+    static constexpr int OFF_STAT = OFF_BAR;                                // [2 groups][2 halves][128 rows]: maxima or sums handed over
+    // barriers: q_full, k_full[NK], k_empty[NK], v_full[NV], v_empty[NV], s_full[2], s_free, p_full[2], o_done[2], segment full / empty
+    static constexpr int NBAR = 1 + 2 * NK + 2 * NV + 2 + 1 + 2 + 2 + 2 * 4;
+    static constexpr int OFF_MBAR = OFF_STAT + 2 * 2 * kDenseRows * 4;
+    static constexpr int OFF_SEG = (OFF_MBAR + NBAR * 8 + 15) / 16 * 16;
+    static constexpr int OFF_MISC = OFF_SEG + 4 * 32;                       // tmem base
+    static constexpr int OFF_END = OFF_MISC + 16;
     static constexpr int TMEM_COLS = 512;
-    static constexpr int COL_O = 0, COL_S0 = 128, COL_S1 = 256;
-    static constexpr int COL_P = 384;           // 64 columns: P, two 16-bit probabilities per 32-bit column
-    static constexpr int COL_L = 448;           // 2 x 4 columns: the column groups' shares of the row sums, handed over at a flush
+    static constexpr int COL_O = 0, COL_S = 256, COL_P = 384;               // O_g at 128 g, P_g at 384 + 64 g
 };
 
-__host__ __device__ inline size_t dense_smem_bytes(int F) {
-    return 1024 /* alignment slack: swizzled tiles start on 1 KiB boundaries */ + DenseCfg::OFF_PLAN + ((size_t)2 * F + 1) * 4;
-}
+constexpr size_t kDenseSmemBytes = DenseCfg::OFF_END;       // (227 KiB is all there is: dynamic shared memory starts on a 1 KiB boundary)
 
 // ---- tcgen05 / TMA wrappers -------------------------------------------------------------------------------------
 __device__ __forceinline__ void tmem_alloc(uint32_t smem_dst, uint32_t cols) {
@@ -133,6 +162,12 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map
         ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(bar)
         : "memory");
 }
+__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, int c3, uint32_t bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
+        ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bar)
+        : "memory");
+}
 __device__ __forceinline__ void tma_load_5d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, int c3, int c4,
                                             uint32_t bar) {
     asm volatile(
@@ -155,18 +190,6 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
         : "r"(taddr)
         : "memory");
 }
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const float (&v)[32]) {
-    const uint32_t* r = reinterpret_cast<const uint32_t*>(v);
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
-        "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
-        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
-          "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]),
-          "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]),
-          "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
-        : "memory");
-}
 // 2^x, the hardware approximation (about two units in the last place); -inf gives 0
 __device__ __forceinline__ float fast_exp2(float x) {
     float y;
@@ -178,79 +201,434 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
     asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
     return d;
 }
-__device__ __forceinline__ void tmem_st1(uint32_t taddr, float v) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(taddr), "r"(__float_as_uint(v)) : "memory");
-}
-__device__ __forceinline__ void tmem_ld4(uint32_t taddr, float (&v)[4]) {
-    uint32_t* r = reinterpret_cast<uint32_t*>(v);
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+// 16 consecutive 32-bit columns of this thread's tensor-memory lane
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+                   "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
                  : "r"(taddr)
                  : "memory");
+}
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+                 ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
+                 "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+                 : "memory");
+}
+// 32 bytes (a whole sector) in one store, 32-byte aligned
+__device__ __forceinline__ void store_sector(void* dst, const uint32_t (&v)[8]) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]),
+                 "r"(v[5]), "r"(v[6]), "r"(v[7])
+                 : "memory");
+}
+// two fp32 operations in one instruction (each half rounded as the scalar instruction rounds it)
+__device__ __forceinline__ uint64_t pair_f32(float lo, float hi) {
+    uint64_t d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+    return d;
+}
+__device__ __forceinline__ void unpair_f32(uint64_t v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
 }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
-// ---- the walk over this CTA's tiles, identical in every role ----------------------------------------------------
-struct DenseTile {
-    int u, f, tok0, ntok, hkv, rb;
-    bool first_of_unit;     // first tile of this CTA's share of the unit: O starts from zero
-    bool last_of_unit;      // last tile of the share: the partial result is due
-    bool new_segment;       // the query tile differs from the previous tile's (other fragment or other unit)
+// Bounded wait of a few instructions: kernels that move registers between warps (setmaxnreg) cannot have calls, and the
+// five roles' loops together have to stay in the instruction cache (with the timer of mbar_wait_bounded inlined at
+// every wait the kernel was 70 KB and twice as slow).  2^20 polls are between 10 ms and a few seconds.
+__device__ __forceinline__ bool mbar_wait_polls(uint32_t bar, uint32_t parity, int* status, int bit) {
+#pragma unroll 1
+    for (int i = 0; i < (1 << 20); ++i)
+        if (mbar_try_wait(bar, parity)) return true;
+    if (status) atomicOr(status, bit);
+    return false;
+}
+// bar.red over the two warps on hardware barrier `id`: is `x` true in any of their threads
+__device__ __forceinline__ bool pair_any(int id, bool x) {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %2, 0;\n\tbarrier.cta.red.or.pred q, %1, 64, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+                 : "=r"(r) : "r"(id), "r"((uint32_t)x) : "memory");
+    return r != 0;
+}
+// one lane of a converged warp
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
+
+// ---- geometry ----------------------------------------------------------------------------------------------------
+// Fragments: query rows of a kv head are (worker, row of G*S) and a tile holds whole workers (tile_span of them) or 128
+// rows of one worker.  Paged: a tile is tile_span tokens of one worker's packed run, G rows each.
+struct DenseRow {
+    bool valid;
+    int w, g, s;           // s: token of the worker (fragments), packed token index (paged)
 };
-struct DenseWalk {
-    const int *vis, *pre;
-    int F, Hkv, TH, j, fscan, prev_u, prev_f;
-    int64_t u, t, t1;
-    __device__ __forceinline__ DenseWalk(const int* vis_, const int* pre_, int F_, int Hkv_, int64_t t0, int64_t t1_)
-        : vis(vis_), pre(pre_), F(F_), Hkv(Hkv_), TH(pre_[F_]), fscan(0), prev_u(-1), prev_f(-1), t(t0), t1(t1_) {
-        u = TH > 0 ? t0 / TH : 0;
-        j = (int)(t0 - u * TH);
-    }
-    __device__ __forceinline__ bool done() const { return t >= t1; }
-    __device__ __forceinline__ DenseTile next() {
-        DenseTile d;
-        while (j >= pre[fscan + 1]) ++fscan;
-        d.u = (int)u;
-        d.f = fscan;
-        d.tok0 = (j - pre[fscan]) * kDenseTile;
-        d.ntok = min(kDenseTile, vis[fscan] - d.tok0);
-        d.hkv = d.u % Hkv;
-        d.rb = d.u / Hkv;
-        d.first_of_unit = d.u != prev_u;
-        d.new_segment = d.u != prev_u || d.f != prev_f;
-        d.last_of_unit = (j == TH - 1) || (t == t1 - 1);
-        prev_u = d.u;
-        prev_f = d.f;
-        ++t;
-        if (++j == TH) {
-            j = 0;
-            ++u;
-            fscan = 0;
+template <bool PAGED>
+__device__ __forceinline__ DenseRow dense_row(const DenseArgs& a, int tile, int i, const int4& rec) {
+    DenseRow r;
+    if constexpr (PAGED) {
+        const int tok = (tile & 1) * a.tile_span + i / a.G;
+        r.valid = i < a.tile_span * a.G && tok < rec.z;
+        r.w = rec.x;
+        r.g = i % a.G;
+        r.s = rec.y + tok;
+    } else {
+        const int gs = a.G * a.S;
+        int x = i;
+        if (gs > kDenseRows) {
+            r.w = tile / a.tile_span;
+            x += (tile - r.w * a.tile_span) * kDenseRows;
+        } else {
+            r.w = tile * a.tile_span + i / gs;
+            x = i % gs;
         }
-        return d;
+        r.valid = r.w < a.W && x < gs && (gs > kDenseRows || i < a.tile_span * gs);
+        r.g = x / a.S;
+        r.s = x - r.g * a.S;
+    }
+    return r;
+}
+// rows of fragment f that hold keys and values (worker w's, when paged)
+template <bool PAGED>
+__device__ __forceinline__ int dense_length(const DenseArgs& a, int f, int w) {
+    if constexpr (PAGED) return a.flen[f * a.W + w];
+    return a.flen ? min(a.cap[f], a.flen[f]) : a.cap[f];
+}
+template <bool PAGED>
+__device__ __forceinline__ int dense_location(const DenseArgs& a, int f, const DenseRow& r) {
+    if constexpr (PAGED) return a.loc[(size_t)f * a.total_q + r.s];
+    return a.loc[((size_t)f * a.W + r.w) * a.S + r.s];
+}
+// does block b hold one query tile only (its groups then take every other key tile each)
+template <bool PAGED>
+__device__ __forceinline__ bool dense_single(const DenseArgs& a, int b) {
+    if constexpr (PAGED) return a.rec[b].z <= a.tile_span;
+    return 2 * b + 1 >= a.tiles;
+}
+__device__ __forceinline__ int dense_steps(int vis0, int vis1, bool single) {
+    return single ? (vis0 + 2 * kDenseTile - 1) / (2 * kDenseTile) : (max(vis0, vis1) + kDenseTile - 1) / kDenseTile;
+}
+
+// ---- the plan: one CTA, beside the rotation kernel where there is one ----------------------------------------------
+// Writes what the other two kernels would otherwise each have to search for: visible keys per (tile, fragment), the prefix
+// of steps over blocks, where every CTA starts, and which units are left to the merge step.  The arrays stay in shared
+// memory while they are worked on, if they fit.
+constexpr int kDensePlanVis = 4096, kDensePlanBlocks = 1024;
+template <bool PAGED>
+__global__ void __launch_bounds__(kDensePlanThreads) dense_plan_kernel(const __grid_constant__ DenseArgs a) {
+    __shared__ int s_vis[kDensePlanVis];
+    __shared__ long long s_pre[kDensePlanBlocks + 1], s_cost[kDensePlanBlocks + 1], sums[kDensePlanThreads / 32], pos[kDenseMaxCtas + 1];
+    __shared__ int s_list;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = kDensePlanThreads / 32;
+    if (tid == 0) s_list = 0;
+    pdl_wait();
+    pdl_trigger();          // the rotation kernel writes nothing that is read here
+    // exclusive prefix of one value per thread over the CTA; *total gets the sum
+    auto scan = [&](long long v, long long* total) {
+        long long x = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const long long y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        __syncthreads();
+        if (lane == 31) sums[warp] = x;
+        __syncthreads();
+        long long w = sums[lane];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const long long y = __shfl_up_sync(0xffffffffu, w, o);
+            if (lane >= o) w += y;
+        }
+        *total = __shfl_sync(0xffffffffu, w, 31);
+        const long long before = __shfl_sync(0xffffffffu, w, warp > 0 ? warp - 1 : 0);
+        return (warp > 0 ? before : 0) + x - v;
+    };
+    int nb = a.blocks;
+    if constexpr (PAGED) {
+        const int per = (a.W + kDensePlanThreads - 1) / kDensePlanThreads, w0 = min(tid * per, a.W), w1 = min(w0 + per, a.W);
+        const int span = 2 * a.tile_span;
+        long long mine = 0, total;
+        for (int w = w0; w < w1; ++w) mine += (max(0, a.cu[w + 1] - a.cu[w]) + span - 1) / span;
+        long long at = scan(mine, &total);
+        nb = (int)min(total, (long long)a.blocks);
+        for (int w = w0; w < w1; ++w) {
+            const int first = a.cu[w], tokens = a.cu[w + 1] - first;
+            for (int s = 0; s < tokens; s += span, ++at)
+                if (at < a.blocks) a.rec[at] = make_int4(w, first + s, min(span, tokens - s), 0);
+        }
+        __syncthreads();
+    }
+    const bool small = nb <= kDensePlanBlocks && 2 * nb * (long long)a.F <= kDensePlanVis;
+    int* const vis = small ? s_vis : a.vis;
+    long long* const pre = small ? s_pre : a.pre;
+    long long* const cost = small ? s_cost : a.cost;
+    for (int i = warp; i < 2 * nb * a.F; i += nwarps) {
+        // Which tokens a tile's rows are: a run of locations (of one worker's tokens, round its end, if it has more
+        // than 128 rows).  Heads repeat the tokens, so no more than 128 locations are read.
+        const int tile = i / a.F, f = i - tile * a.F;
+        int from, tokens, wrap = INT_MAX, w = 0;      // locations [from, from + tokens); those at or past `wrap` are a.S further down
+        if constexpr (PAGED) {
+            const int4 rec = a.rec[tile >> 1];
+            const int skip = (tile & 1) * a.tile_span;
+            from = rec.y + skip;
+            tokens = min(a.tile_span, rec.z - skip);
+            w = rec.x;
+        } else {
+            const int gs = a.G * a.S;
+            if (gs > kDenseRows) {
+                w = tile / a.tile_span;
+                const int x = (tile - w * a.tile_span) * kDenseRows;
+                tokens = w < a.W ? min(min(kDenseRows, gs - x), a.S) : 0;
+                from = w * a.S + x % a.S;
+                wrap = (w + 1) * a.S;
+            } else {
+                w = tile * a.tile_span;
+                from = w * a.S;
+                tokens = (min(w + a.tile_span, a.W) - w) * a.S;
+            }
+        }
+        int top = -1;
+        const int* loc = a.loc + (size_t)f * (PAGED ? a.total_q : a.W * a.S);
+#pragma unroll
+        for (int k = 0; k < kDenseRows; k += 32) {
+            int at = from + k + lane;
+            if (at >= wrap) at -= a.S;
+            if (k + lane < tokens) top = max(top, loc[at]);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
+        top = tokens > 0 ? max(0, min(top, dense_length<PAGED>(a, f, w) - 1) + 1) : 0;
+        if (lane == 0) a.vis[i] = vis[i] = top;
+    }
+    __syncthreads();
+    const int per = (nb + kDensePlanThreads - 1) / kDensePlanThreads, b0 = min(tid * per, nb), b1 = min(b0 + per, nb);
+    auto block_steps = [&](int b) {
+        const bool single = dense_single<PAGED>(a, b);
+        long long n = 0;
+        for (int f = 0; f < a.F; ++f) n += dense_steps(vis[2 * b * a.F + f], vis[(2 * b + 1) * a.F + f], single);
+        return n;
+    };
+    long long mine = 0, mine_cost = 0, total, total_cost;
+    for (int b = b0; b < b1; ++b) {
+        const long long n = block_steps(b);
+        mine += n;
+        mine_cost += n > 0 ? n + kDenseUnitSteps : 0;
+    }
+    long long at = scan(mine, &total), at_cost = scan(mine_cost, &total_cost);
+    for (int b = b0; b < b1; ++b) {
+        const long long n = per == 1 ? mine : block_steps(b);
+        a.pre[b] = pre[b] = at;
+        cost[b] = at_cost;
+        at += n;
+        at_cost += n > 0 ? n + kDenseUnitSteps : 0;
+    }
+    if (tid == 0) {
+        a.pre[nb] = pre[nb] = total;
+        cost[nb] = total_cost;
+    }
+    __syncthreads();
+
+    // Where every CTA starts: equal shares of the steps and of the units' fixed costs.  pos[c]: its first step in the list of all.
+    const long long N = total * a.Hkv, C = total_cost * a.Hkv;
+    const int ctas = effective_ctas(N, a.ctas);
+    int4 st = make_int4(0, 0, 0, 0);
+    if (tid < ctas) {
+        const long long t = cta_first_tile(tid, C, ctas);
+        int lo = 0, hi = nb;                         // cost[lo] * Hkv <= t < cost[hi] * Hkv
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (cost[mid] * a.Hkv <= t) lo = mid;
+            else hi = mid;
+        }
+        const long long steps = pre[lo + 1] - pre[lo], off = t - cost[lo] * a.Hkv;
+        long long h = floor_div(off, steps + kDenseUnitSteps), j = min(off - h * (steps + kDenseUnitSteps), steps);
+        pos[tid] = pre[lo] * a.Hkv + h * steps + j;
+        if (j == steps) {                            // the unit's end is the next one's beginning
+            j = 0;
+            if (++h == a.Hkv) {
+                h = 0;
+                for (++lo; lo < nb && pre[lo + 1] == pre[lo]; ++lo) {}
+            }
+        }
+        st = make_int4(lo, (int)h, (int)j, 0);
+    }
+    if (tid == ctas) pos[ctas] = N;
+    __syncthreads();
+    // the partials of a unit that begins at step s: those of CTAs c0, c0 + 1, ...
+    auto parts = [&](int c0, long long s, long long steps) {
+        int c1 = c0;
+        while (c1 + 1 < ctas && pos[c1 + 1] < s + steps) ++c1;
+        return c1 - c0 + 1;
+    };
+    if (tid < a.ctas) {
+        if (tid < ctas) {
+            st.w = (int)(pos[tid + 1] - pos[tid]);
+            const long long s = pos[tid] - st.z;
+            // the unit this CTA starts inside of, if no earlier CTA does
+            if (st.z > 0 && !dense_single<PAGED>(a, st.x) && pos[tid - 1] <= s)
+                a.merge[atomicAdd(&s_list, 1)] = make_int4(st.x * a.Hkv + st.y, tid - 1, parts(tid - 1, s, pre[st.x + 1] - pre[st.x]), 0);
+        }
+        a.start[tid] = st;
+    }
+    // blocks of one tile (two halves per CTA that worked on them), blocks that see nothing
+    for (int b = b0; b < b1; ++b) {
+        const bool single = dense_single<PAGED>(a, b);
+        const long long steps = pre[b + 1] - pre[b];
+        if (!single && steps > 0) continue;
+        int at_list = atomicAdd(&s_list, a.Hkv);
+        for (int h = 0; h < a.Hkv; ++h, ++at_list) {
+            int c0 = 0, count = 0;
+            if (steps > 0) {
+                const long long s = pre[b] * a.Hkv + h * steps;
+                int hi = ctas;                       // pos[c0] <= s < pos[hi]
+                while (hi - c0 > 1) {
+                    const int mid = (c0 + hi) >> 1;
+                    if (pos[mid] <= s) c0 = mid;
+                    else hi = mid;
+                }
+                count = 2 * parts(c0, s, steps);
+            }
+            a.merge[at_list] = make_int4(b * a.Hkv + h, c0, count, single ? 1 : 0);
+        }
+    }
+    __syncthreads();
+    if (tid == 0) *a.nmerge = s_list;
+}
+
+// element offset of an output row
+template <bool PAGED>
+__device__ __forceinline__ size_t dense_out_offset(const DenseArgs& a, const DenseRow& r, int h) {
+    const int hq = h * a.G + r.g;
+    if constexpr (PAGED) return ((size_t)r.s * a.Hq + hq) * 128;
+    const int all = max(a.world, 1) * a.Hq, off = a.world > 0 ? a.rank * a.Hq : 0;
+    return (((size_t)r.w * all + off + hq) * a.S + r.s) * 128;
+}
+
+// ---- the walk over this CTA's share, segment by segment ----------------------------------------------------------------
+// A segment is a run of steps of one unit inside one fragment.  Its key tiles are [t0, t1); in a block with one query
+// tile, group g takes the tiles of parity g.  One warp walks (a step of it is two or three dependent loads) and hands
+// the segments to the others through a small ring in shared memory, one segment ahead.
+struct DenseSegment {
+    int b, h, f, flags;
+    int vis0, vis1;        // keys that the rows of query tile 0 / 1 see
+    int t0, t1;            // key tiles
+    static constexpr int SINGLE = 1, FIRST = 2, LAST = 4, WHOLE = 8, END = 16;
+    __device__ __forceinline__ bool single() const { return flags & SINGLE; }         // one query tile
+    __device__ __forceinline__ bool first() const { return flags & FIRST; }           // first segment of this CTA's share of the unit
+    __device__ __forceinline__ bool last() const { return flags & LAST; }             // last one
+    __device__ __forceinline__ bool whole() const { return flags & WHOLE; }           // the share is the whole unit
+    // does group g work on key tile t
+    __device__ __forceinline__ bool active(int g, int t) const { return single() ? (t & 1) == g : t * kDenseTile < (g ? vis1 : vis0); }
+};
+struct DenseSegments {     // a consumer's end of the ring (every lane of the warp takes part)
+    static constexpr int DEPTH = 4;
+    uint32_t slots, full, empty, n;
+    __device__ __forceinline__ bool next(DenseSegment& d, int lane, int* status) {
+        const uint32_t i = n % DEPTH;
+        bool ok = mbar_wait_polls(full + 8 * i, (n / DEPTH) & 1u, status, STATUS_WAIT_SYNC_TIMEOUT);
+        if (!__all_sync(0xffffffffu, ok)) return false;
+        const uint32_t at = slots + i * (uint32_t)sizeof(DenseSegment);
+        asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(d.b), "=r"(d.h), "=r"(d.f), "=r"(d.flags) : "r"(at) : "memory");
+        asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(d.vis0), "=r"(d.vis1), "=r"(d.t0), "=r"(d.t1) : "r"(at + 16) : "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(empty + 8 * i);
+        ++n;
+        return !(d.flags & DenseSegment::END);
+    }
+};
+template <bool PAGED>
+struct DenseWalk {
+    const DenseArgs& a;
+    int b, h, f, vis0, vis1, t0, t1;
+    bool single, first, last, whole;
+    int j, n, left, skip;
+    __device__ __forceinline__ DenseWalk(const DenseArgs& a_, const int4& start)
+        : a(a_), b(start.x), h(start.y - 1), last(true), j(start.z), n(start.w) {}
+    __device__ __forceinline__ bool next() {
+        if (last) {
+            if (n <= 0) return false;
+            if (++h == a.Hkv) {
+                h = 0;
+                ++b;
+                while (a.pre[b + 1] == a.pre[b]) ++b;                // (blocks that see nothing have no steps)
+            }
+            const int rest = (int)min(a.pre[b + 1] - a.pre[b] - j, (long long)INT_MAX);
+            single = dense_single<PAGED>(a, b);
+            whole = j == 0 && n >= rest;
+            left = min(n, rest);
+            n -= left;
+            skip = j;
+            j = 0;
+            f = -1;
+        }
+        first = last;
+        int steps, j0;
+        do {
+            ++f;
+            vis0 = a.vis[2 * b * a.F + f];
+            vis1 = a.vis[(2 * b + 1) * a.F + f];
+            steps = dense_steps(vis0, vis1, single);
+            j0 = min(skip, steps);
+            skip -= j0;
+        } while (j0 == steps);
+        steps = min(steps - j0, left);
+        left -= steps;
+        last = left == 0;
+        t0 = single ? 2 * j0 : j0;
+        t1 = single ? min(2 * (j0 + steps), (vis0 + kDenseTile - 1) / kDenseTile) : j0 + steps;
+        return true;
     }
 };
 
-template <class T>
-__global__ void __launch_bounds__(kDenseThreads, 1)
-dense_attention_kernel(const __grid_constant__ KernelArgs a, const __grid_constant__ DenseMaps maps) {
+// One K or V tile (keys tok0 .. tok0 + 127 of fragment f) of kv head h into shared memory.  Whole warp.
+template <bool PAGED>
+__device__ __forceinline__ void dense_fetch(const DenseArgs& a, const CUtensorMap* maps, int f, int w, int h, int tok0, uint32_t dst,
+                                            uint32_t bar, int lane) {
     using C = DenseCfg;
-    extern __shared__ unsigned char smem_dyn[];
-    unsigned char* base = reinterpret_cast<unsigned char*>(((uintptr_t)smem_dyn + 1023) & ~(uintptr_t)1023);
+    if constexpr (PAGED) {
+        // a lane per (cache block, column half); blocks past the sequence's end are not fetched
+        const int step = min(a.block_size, kDenseTile);
+        const int rows = min(kDenseTile, a.flen[f * a.W + w] - tok0), n = (rows + step - 1) / step;
+        const int i = lane >> 1, half = lane & 1;
+        const int tok = tok0 + i * step, blk = tok / a.block_size;
+        int place = 0;
+        if (i < n) place = a.block_table[(size_t)w * a.max_blocks + min(blk, a.max_blocks - 1)];
+        if (lane == 0) mbar_arrive_expect_tx(bar, (uint32_t)n * step * 256u);
+        __syncwarp();
+        if (i < n) tma_load_4d(dst + half * C::ATOM_BYTES + i * step * 128, maps, half * 64, tok - blk * a.block_size, h, place, bar);
+    } else {
+        if (lane == 0) {
+            mbar_arrive_expect_tx(bar, C::TILE_BYTES);
+            tma_load_3d(dst, maps + f, 0, tok0, h, bar);
+            tma_load_3d(dst + C::ATOM_BYTES, maps + f, 64, tok0, h, bar);
+        }
+    }
+}
+
+template <class T, bool PAGED>
+__global__ void __launch_bounds__(kDenseThreads, 1)
+dense_attention_kernel(const __grid_constant__ DenseArgs a, const __grid_constant__ DenseMaps maps) {
+    using C = DenseCfg;
+    extern __shared__ __align__(1024) unsigned char dense_smem[];       // swizzled tiles start on 1 KiB boundaries
+    unsigned char* const base = dense_smem;
     const uint32_t sbase = smem_u32(base);
-    const uint32_t bars = sbase + C::OFF_BAR;
-    const uint32_t q_full = bars, k_full = q_full + 8, k_empty = k_full + 8 * C::NK, v_full = k_empty + 8 * C::NK,
-                   v_empty = v_full + 8 * C::NV, s_full = v_empty + 8 * C::NV, s_free = s_full + 16, p_full = s_free + 16,
-                   o_done = p_full + 8, l_ready = o_done + 8;
+    const uint32_t q_full = sbase + C::OFF_MBAR, k_full = q_full + 8, k_empty = k_full + 8 * C::NK, v_full = k_empty + 8 * C::NK,
+                   v_empty = v_full + 8 * C::NV, s_full = v_empty + 8 * C::NV, s_free = s_full + 16, p_full = s_free + 8,
+                   o_done = p_full + 16, seg_full = o_done + 16, seg_empty = seg_full + 8 * DenseSegments::DEPTH;
+    constexpr int W_K = kDenseSoftmaxWarps, W_S = W_K + 1, W_V = W_K + 3;        // (W_K + 2: the PV products)
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(base + C::OFF_MISC);
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(base + C::OFF_MISC + 8);
-    int* vis = reinterpret_cast<int*>(base + C::OFF_PLAN);
-    int* pre = vis + a.F;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    HOGATT_TL_DECL;
-
     if (tid == 0) {
         mbar_init(q_full, 1);
         for (int s = 0; s < C::NK; ++s) {
@@ -261,356 +639,478 @@ dense_attention_kernel(const __grid_constant__ KernelArgs a, const __grid_consta
             mbar_init(v_full + 8 * s, 1);
             mbar_init(v_empty + 8 * s, 1);
         }
-        for (int s = 0; s < 2; ++s) {
-            mbar_init(s_full + 8 * s, 1);
-            mbar_init(s_free + 8 * s, kDenseSoftmaxWarps);      // one arrival per softmax warp
+        for (int g = 0; g < 2; ++g) {
+            mbar_init(s_full + 8 * g, 1);
+            mbar_init(p_full + 8 * g, kDenseSoftmaxWarps / 2);            // one arrival per softmax warp of the group
+            mbar_init(o_done + 8 * g, 1);
         }
-        mbar_init(p_full, kDenseSoftmaxWarps);
-        mbar_init(o_done, 1);
-        for (int s = 0; s < 4; ++s) mbar_init(l_ready + 8 * s, kDenseSplit - 1);
-        *abort_flag = 0;
+        mbar_init(s_free, kDenseSoftmaxWarps / 2);
+        for (int i = 0; i < DenseSegments::DEPTH; ++i) {
+            mbar_init(seg_full + 8 * i, 1);
+            mbar_init(seg_empty + 8 * i, kDenseSoftmaxWarps + 3);
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         fence_proxy_async_smem();
     }
-    if (warp == kDenseSoftmaxWarps + 1) tmem_alloc(smem_u32(tmem_slot), C::TMEM_COLS);
-    if (a.host_plan) {
-        if (warp == 0) host_tile_prefix(a, kDenseTile, vis, pre);
-        tc_fence_before();
-        __syncthreads();
-    } else {
-        tc_fence_before();
-        build_tile_prefix(a, kDenseTile, vis, pre);        // ends with __syncthreads()
-    }
+    if (warp == W_S) tmem_alloc(smem_u32(tmem_slot), C::TMEM_COLS);
+    tc_fence_before();
+    __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+//TL TLD;
+    //TX TLD; if (warp == 0) {TLG(0, 98); TL(0, 99);}
+    DenseSegments segs{sbase + C::OFF_SEG, seg_full, seg_empty, 0};
+    DenseSegment d;
+    bool ok = true;
 
-    const int TH = pre[a.F];
-    const int units = a.row_blocks * a.Hkv;
-    const int64_t N = (int64_t)units * TH;
-    const int ctas = a.host_plan ? a.plan_ctas : effective_ctas(N, gridDim.x);
-    if (!a.host_plan && blockIdx.x == 0 && tid == 0) {
-        a.header[0] = TH;
-        a.header[1] = ctas;
-    }
-    int64_t t0 = 0, t1 = 0;
-    if ((int)blockIdx.x < ctas) {
-        t0 = cta_first_tile(blockIdx.x, N, ctas);
-        t1 = cta_first_tile(blockIdx.x + 1, N, ctas);
-    }
-    const int GS = a.G * a.S;
-
-    if (warp == kDenseSoftmaxWarps) {
-        // ============================== K / V copies ==============================
-        if (lane == 0) {
-            DenseWalk walk(vis, pre, a.F, a.Hkv, t0, t1);
-            bool ok = true;
-            for (int it = 0; !walk.done() && ok; ++it) {
-                const DenseTile d = walk.next();
-                const int ks = it % C::NK, vs = it % C::NV;
-                ok = mbar_wait_bounded(k_empty + 8 * ks, (((uint32_t)(it / C::NK)) & 1u) ^ 1u, abort_flag, a.status,
-                                       STATUS_WAIT_EMPTY_TIMEOUT);
-                if (!ok) break;
-                mbar_arrive_expect_tx(k_full + 8 * ks, C::TILE_BYTES);
-                const uint32_t kdst = sbase + C::OFF_K + ks * C::TILE_BYTES;
-                tma_load_3d(kdst, &maps.k[d.f], 0, d.tok0, d.hkv, k_full + 8 * ks);
-                tma_load_3d(kdst + C::ATOM_BYTES, &maps.k[d.f], 64, d.tok0, d.hkv, k_full + 8 * ks);
-                ok = mbar_wait_bounded(v_empty + 8 * vs, (((uint32_t)(it / C::NV)) & 1u) ^ 1u, abort_flag, a.status,
-                                       STATUS_WAIT_EMPTY_TIMEOUT);
-                if (!ok) break;
-                mbar_arrive_expect_tx(v_full + 8 * vs, C::TILE_BYTES);
-                const uint32_t vdst = sbase + C::OFF_V + vs * C::TILE_BYTES;
-                tma_load_3d(vdst, &maps.v[d.f], 0, d.tok0, d.hkv, v_full + 8 * vs);
-                tma_load_3d(vdst + C::ATOM_BYTES, &maps.v[d.f], 64, d.tok0, d.hkv, v_full + 8 * vs);
+    if (warp >= W_K) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
+        if (warp == W_K) {
+            // ============================== K copies ==============================
+            int stage = 0;
+            uint32_t phase = 1;                      // of k_empty: the first round finds every stage free
+            while (ok && segs.next(d, lane, a.status)) {
+                const int w = PAGED ? a.rec[d.b].x : 0;
+#pragma unroll 1
+                for (int t = d.t0; t < d.t1; ++t) {
+                    ok = mbar_wait_polls(k_empty + 8 * stage, phase, a.status, STATUS_WAIT_EMPTY_TIMEOUT);
+                    ok = __all_sync(0xffffffffu, ok);
+                    if (!ok) break;
+                    dense_fetch<PAGED>(a, maps.k, d.f, w, d.h, t * kDenseTile, sbase + C::OFF_K + stage * C::TILE_BYTES, k_full + 8 * stage, lane);
+                    if (++stage == C::NK) {
+                        stage = 0;
+                        phase ^= 1u;
+                    }
+                }
             }
-        }
-    } else if (warp == kDenseSoftmaxWarps + 1) {
-        // ============================== Q copies and the S MMAs ==============================
-        // Issuing a tcgen05.mma costs the issuing thread some 60-70 cycles, sixteen of them per tile about as long as
-        // the tensor pipe needs to execute them -- so the two GEMMs of a tile are issued by two threads that only meet at
-        // barriers: this one runs ahead with S = Q K^T, the next warp follows the softmax warps with O += P V.
-        if (lane == 0) {
+        } else if (warp == W_V) {
+            // ============================== the walk, and the V copies ==============================
+            DenseWalk<PAGED> walk(a, a.start[blockIdx.x]);
+            uint32_t n = 0;
+            auto publish = [&]() {                   // the walk's next segment into the ring; false when there is none left
+                const uint32_t i = n % DenseSegments::DEPTH;
+                ok = mbar_wait_polls(seg_empty + 8 * i, ((n / DenseSegments::DEPTH) & 1u) ^ 1u, a.status, STATUS_WAIT_EMPTY_TIMEOUT) && ok;
+                ok = __all_sync(0xffffffffu, ok);
+                const bool more = walk.next();
+                if (lane == 0) {
+                    DenseSegment* slot = reinterpret_cast<DenseSegment*>(base + C::OFF_SEG) + i;
+                    slot->b = walk.b;
+                    slot->h = walk.h;
+                    slot->f = walk.f;
+                    slot->flags = more ? (walk.single ? DenseSegment::SINGLE : 0) | (walk.first ? DenseSegment::FIRST : 0) |
+                                             (walk.last ? DenseSegment::LAST : 0) | (walk.whole ? DenseSegment::WHOLE : 0)
+                                       : DenseSegment::END;
+                    slot->vis0 = walk.vis0;
+                    slot->vis1 = walk.vis1;
+                    slot->t0 = walk.t0;
+                    slot->t1 = walk.t1;
+                    mbar_arrive(seg_full + 8 * i);
+                }
+                __syncwarp();
+                ++n;
+                return more;
+            };
+            int stage = 0;
+            uint32_t phase = 1;
+            bool more = publish();
+#pragma unroll 1
+            while (ok && more) {
+                const int f = walk.f, h = walk.h, t0 = walk.t0, t1 = walk.t1, w = PAGED ? a.rec[walk.b].x : 0;
+                more = publish();
+#pragma unroll 1
+                for (int t = t0; t < t1 && ok; ++t) {
+                    ok = mbar_wait_polls(v_empty + 8 * stage, phase, a.status, STATUS_WAIT_EMPTY_TIMEOUT);
+                    ok = __all_sync(0xffffffffu, ok);
+                    if (!ok) break;
+                    dense_fetch<PAGED>(a, maps.v, f, w, h, t * kDenseTile, sbase + C::OFF_V + stage * C::TILE_BYTES, v_full + 8 * stage, lane);
+                    if (++stage == C::NV) {
+                        stage = 0;
+                        phase ^= 1u;
+                    }
+                }
+            }
+        } else if (warp == W_S) {
+            // ============================== Q copies and the S MMAs ==============================
             constexpr uint32_t IDESC_S = umma_idesc<T>(false, kDenseRows, kDenseTile);
-            const uint32_t q_smem = sbase + C::OFF_Q;
-            uint32_t q_phase = 0;
-            // the matrix descriptors are built once (a k-step only moves the start-address field: +32 bytes inside a
-            // 64-column swizzle atom, +16 KiB to the second atom)
-            const uint64_t q_desc = umma_desc(q_smem, 16, 1024);
-            uint64_t k_desc[C::NK];
-#pragma unroll
-            for (int i = 0; i < C::NK; ++i) k_desc[i] = umma_desc(sbase + C::OFF_K + i * C::TILE_BYTES, 16, 1024);
-            DenseWalk walk(vis, pre, a.F, a.Hkv, t0, t1);
-            bool ok = true;
-            for (int it = 0; !walk.done() && ok; ++it) {
-                const DenseTile d = walk.next();
-                const int ks = it % C::NK, sb = it & 1;
-                if (d.new_segment) {
-                    // the query tile changes: S_{it-1}, the last reader of the old one, must have finished
-                    if (it > 0)
-                        ok = mbar_wait_bounded(s_full + 8 * ((it - 1) & 1), ((uint32_t)((it - 1) >> 1)) & 1u, abort_flag, a.status,
-                                               STATUS_WAIT_SYNC_TIMEOUT);
-                    if (!ok) break;
-                    const int r0 = d.rb * kDenseRows;
-                    mbar_arrive_expect_tx(q_full, C::TILE_BYTES);
-                    tma_load_5d(q_smem, &maps.q, 0, r0 % GS, d.hkv, r0 / GS, d.f, q_full);
-                    tma_load_5d(q_smem + C::ATOM_BYTES, &maps.q, 64, r0 % GS, d.hkv, r0 / GS, d.f, q_full);
-                    ok = mbar_wait_bounded(q_full, q_phase, abort_flag, a.status, STATUS_WAIT_FULL_TIMEOUT);
-                    q_phase ^= 1u;
-                    if (!ok) break;
-                }
-                // S_it = Q K^T into S buffer it & 1 (K ring stage it % NK); the stage is handed back when the MMAs are done
-                ok = mbar_wait_bounded(k_full + 8 * ks, ((uint32_t)(it / C::NK)) & 1u, abort_flag, a.status, STATUS_WAIT_FULL_TIMEOUT) &&
-                     mbar_wait_bounded(s_free + 8 * sb, (((uint32_t)(it >> 1)) & 1u) ^ 1u, abort_flag, a.status, STATUS_WAIT_SYNC_TIMEOUT);
+            // (a k-step only moves the descriptor's start-address field: +32 bytes inside a 64-column swizzle atom,
+            // +16 KiB to the second atom)
+            const uint64_t q_desc = umma_desc(sbase + C::OFF_Q, 16, 1024), k_desc = umma_desc(sbase + C::OFF_K, 16, 1024);
+            int stage = 0, last_g = 0;
+            uint32_t k_phase = 0, q_phase = 0, s_phase = 1, g_phase = 0;      // g_phase: bit g, the parity of S_g's next completion
+            bool any = false;
+            while (ok && segs.next(d, lane, a.status)) {
+                // the query tiles change: the last reader of the old ones must have finished
+                if (any)
+                    ok = mbar_wait_polls(s_full + 8 * last_g, ((g_phase >> last_g) & 1u) ^ 1u, a.status, STATUS_WAIT_SYNC_TIMEOUT);
+                ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
-                tc_fence_after();
-                const uint64_t kd = ks == 0 ? k_desc[0] : (ks == 1 ? k_desc[1] : k_desc[2]);
-                const uint32_t d_tmem = tmem + (sb ? C::COL_S1 : C::COL_S0);
-#pragma unroll
-                for (int kk = 0; kk < C::HD / 16; ++kk) {
-                    const uint64_t off = (uint64_t)(((kk >> 2) * C::ATOM_BYTES + (kk & 3) * 32) >> 4);
-                    tc_mma(d_tmem, q_desc + off, kd + off, IDESC_S, kk > 0);
+                const int gs = a.G * a.S, tiles = d.single() ? 1 : 2;
+                if (elect_one()) {
+                    const uint32_t bytes = (uint32_t)(PAGED ? a.tile_span * a.G : (gs > kDenseRows ? kDenseRows : a.tile_span * gs)) * 256u;
+                    mbar_arrive_expect_tx(q_full, tiles * bytes);
+#pragma unroll 1
+                    for (int i = 0; i < 2 * tiles; ++i) {       // (query tile, column half)
+                        const int c = (i & 1) * 64, g = i >> 1;
+                        const uint32_t dst = sbase + C::OFF_Q + i * C::ATOM_BYTES;
+                        if constexpr (PAGED) {
+                            tma_load_5d(dst, &maps.q, c, 0, d.h, a.rec[d.b].y + g * a.tile_span, d.f, q_full);
+                        } else {
+                            const int tile = 2 * d.b + g;
+                            const int w = gs > kDenseRows ? tile / a.tile_span : tile * a.tile_span;
+                            tma_load_5d(dst, &maps.q, c, gs > kDenseRows ? (tile - w * a.tile_span) * kDenseRows : 0, d.h, w, d.f, q_full);
+                        }
+                    }
                 }
-                tc_commit(s_full + 8 * sb);
-                tc_commit(k_empty + 8 * ks);
-                HOGATT_TL(0, 3000 + it);
+                __syncwarp();
+                ok = mbar_wait_polls(q_full, q_phase, a.status, STATUS_WAIT_FULL_TIMEOUT);
+                q_phase ^= 1u;
+#pragma unroll 1
+                for (int t = d.t0; t < d.t1 && ok; ++t) {
+                    ok = mbar_wait_polls(k_full + 8 * stage, k_phase, a.status, STATUS_WAIT_FULL_TIMEOUT);
+                    const uint64_t kd = k_desc + (uint64_t)(uint32_t)(stage * (C::TILE_BYTES >> 4));
+#pragma unroll 1
+                    for (int g = 0; g < 2; ++g) {
+                        if (!d.active(g, t)) continue;
+                        // S = Q K^T into the S buffer once the scores before it have been read
+                        ok = mbar_wait_polls(s_free, s_phase, a.status, STATUS_WAIT_SYNC_TIMEOUT) && ok;
+                        ok = __all_sync(0xffffffffu, ok);
+                        if (!ok) break;
+                        s_phase ^= 1u;
+                        tc_fence_after();
+                        const uint64_t qd = q_desc + (uint64_t)(uint32_t)(d.single() ? 0 : g * (C::TILE_BYTES >> 4));
+                        if (elect_one()) {
+#pragma unroll
+                            for (int kk = 0; kk < C::HD / 16; ++kk) {
+                                const uint64_t off = (uint64_t)(((kk >> 2) * C::ATOM_BYTES + (kk & 3) * 32) >> 4);
+                                tc_mma(tmem + C::COL_S, qd + off, kd + off, IDESC_S, kk > 0);
+                            }
+                            tc_commit(s_full + 8 * g);
+                        }
+                        __syncwarp();
+                        //TL TL(2, g);
+                        g_phase ^= 1u << g;
+                        last_g = g;
+                        any = true;
+                    }
+                    if (!ok) break;
+                    if (elect_one()) tc_commit(k_empty + 8 * stage);
+                    __syncwarp();
+                    if (++stage == C::NK) {
+                        stage = 0;
+                        k_phase ^= 1u;
+                    }
+                }
             }
-        }
-    } else if (warp == kDenseSoftmaxWarps + 2) {
-        // ============================== the O += P V MMAs ==============================
-        if (lane == 0) {
+        } else {
+            // ============================== the O += P V MMAs ==============================
             constexpr uint32_t IDESC_O = umma_idesc<T>(true, kDenseRows, C::HD);
-            uint64_t v_desc[C::NV];
+            const uint64_t v_desc = umma_desc(sbase + C::OFF_V, C::ATOM_BYTES, 1024);
+            int stage = 0;
+            uint32_t v_phase = 0, g_phase = 0, started = 0;      // bit g: parity of P_g; O_g holds something
+            while (ok && segs.next(d, lane, a.status)) {
+                if (d.first()) started = 0;
+                const int vlen = dense_length<PAGED>(a, d.f, PAGED ? a.rec[d.b].x : 0);
+#pragma unroll 1
+                for (int t = d.t0; t < d.t1 && ok; ++t) {
+                    ok = mbar_wait_polls(v_full + 8 * stage, v_phase, a.status, STATUS_WAIT_FULL_TIMEOUT);
+                    if ((t + 1) * kDenseTile > vlen && ok) {
+                        // The tile runs past the rows in use: those rows may hold anything (spare rows of a slab or cache
+                        // block).  Their probabilities are exactly zero, but 0 * NaN would poison O.
+                        unsigned char* vt = base + C::OFF_V + stage * C::TILE_BYTES;
+#pragma unroll 1
+                        for (int i = (vlen - t * kDenseTile) * 8 + lane; i < kDenseTile * 8; i += 32) {
+                            *reinterpret_cast<int4*>(vt + i * 16) = make_int4(0, 0, 0, 0);
+                            *reinterpret_cast<int4*>(vt + C::ATOM_BYTES + i * 16) = make_int4(0, 0, 0, 0);
+                        }
+                        fence_proxy_async_smem();      // generic-proxy writes before the MMA's async-proxy reads
+                        __syncwarp();
+                    }
+                    const uint64_t vd = v_desc + (uint64_t)(uint32_t)(stage * (C::TILE_BYTES >> 4));
+#pragma unroll 1
+                    for (int g = 0; g < 2; ++g) {
+                        if (!d.active(g, t)) continue;
+                        ok = mbar_wait_polls(p_full + 8 * g, (g_phase >> g) & 1u, a.status, STATUS_WAIT_SYNC_TIMEOUT) && ok;
+                        ok = __all_sync(0xffffffffu, ok);
+                        if (!ok) break;
+                        g_phase ^= 1u << g;
+                        tc_fence_after();
+                        const uint32_t acc = (started >> g) & 1u;
+                        if (elect_one()) {
 #pragma unroll
-            for (int i = 0; i < C::NV; ++i) v_desc[i] = umma_desc(sbase + C::OFF_V + i * C::TILE_BYTES, C::ATOM_BYTES, 1024);
-            DenseWalk walk(vis, pre, a.F, a.Hkv, t0, t1);
-            bool ok = true;
-            for (int it = 0; !walk.done() && ok; ++it) {
-                const DenseTile cur = walk.next();
-                const int vs = it % C::NV;
-                ok = mbar_wait_bounded(p_full, ((uint32_t)it) & 1u, abort_flag, a.status, STATUS_WAIT_SYNC_TIMEOUT) &&
-                     mbar_wait_bounded(v_full + 8 * vs, ((uint32_t)(it / C::NV)) & 1u, abort_flag, a.status, STATUS_WAIT_FULL_TIMEOUT);
-                if (!ok) break;
-                tc_fence_after();
-                const uint64_t vd = vs == 0 ? v_desc[0] : (vs == 1 ? v_desc[1] : v_desc[2]);
-                const uint32_t acc0 = cur.first_of_unit ? 0u : 1u;
-#pragma unroll
-                for (int kk = 0; kk < kDenseTile / 16; ++kk) {
-                    // A = P from tensor memory: 16 keys are 8 columns.  V is [key][Ev]: Ev (the MMA's N) is contiguous ->
-                    // MN-major; 16 keys per step = two 8-key swizzle atoms (2 KiB)
-                    tc_mma_ts(tmem + C::COL_O, tmem + C::COL_P + kk * 8, vd + (uint64_t)(kk * 2048 >> 4), IDESC_O, kk > 0 ? 1u : acc0);
+                            for (int kk = 0; kk < kDenseTile / 16; ++kk) {
+                                // A = P from tensor memory: 16 keys are 8 columns.  V is [key][Ev]: Ev (the MMA's N) is
+                                // contiguous -> MN-major; 16 keys per step = two 8-key swizzle atoms (2 KiB)
+                                tc_mma_ts(tmem + C::COL_O + g * 128, tmem + C::COL_P + g * 64 + kk * 8, vd + (uint64_t)(kk * 2048 >> 4), IDESC_O,
+                                          kk > 0 ? 1u : acc);
+                            }
+                            tc_commit(o_done + 8 * g);
+                        }
+                        __syncwarp();
+                        //TL TL(3, g);
+                        started |= 1u << g;
+                    }
+                    if (!ok) break;
+                    if (elect_one()) tc_commit(v_empty + 8 * stage);
+                    __syncwarp();
+                    if (++stage == C::NV) {
+                        stage = 0;
+                        v_phase ^= 1u;
+                    }
                 }
-                tc_commit(o_done);
-                tc_commit(v_empty + 8 * vs);
-                HOGATT_TL(0, 2000 + it);
             }
         }
     } else {
-        // ============================== softmax: SPLIT threads per query row, 128 / SPLIT columns each ==============================
-        constexpr int SPLIT = kDenseSplit, COLS = kDenseTile / SPLIT;      // COLS is 32 or 64
-        static_assert(COLS == 32 || COLS == 64, "a thread owns one or two 32-column tensor-memory loads");
-        const int row = (warp & 3) * 32 + lane;                // row of the block == tensor-memory lane
-        const int part = warp >> 2;                            // which COLS columns of S, P and O this thread owns
-        const int col0 = part * COLS;
-        const uint32_t lane_base = ((uint32_t)((warp & 3) * 32)) << 16;
+        // ============================== softmax: warps 0-7 group 0, 8-15 group 1; warps w and w + 4 share 32 rows ==============================
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
+        constexpr int COLS = kDenseTile / 2;                              // this thread's columns of S, P and O
+        const int g = warp >> 3, half = (warp >> 2) & 1, row = (warp & 3) * 32 + lane;            // row of the tile == tensor-memory lane
+        const uint32_t lane_base = tmem + (((uint32_t)((warp & 3) * 32)) << 16);
+        const uint32_t s_addr = lane_base + C::COL_S + half * COLS, o_addr = lane_base + C::COL_O + g * 128 + half * COLS,
+                       p_addr = lane_base + C::COL_P + g * 64 + half * (COLS / 2);
+        float* const stat = reinterpret_cast<float*>(base + C::OFF_STAT) + (g * 2 + half) * kDenseRows + row;
+        const float* const other = reinterpret_cast<const float*>(base + C::OFF_STAT) + (g * 2 + (half ^ 1)) * kDenseRows + row;
+        const int pair_bar = 1 + g * 4 + (warp & 3);                      // hardware barrier of the two warps that share rows
         const float scale2 = a.l2scale;                        // scores are raw dot products; exp2((s - m) * scale2)
         const float grow_by = 8.f / scale2;                    // raw-score distance that equals a factor 2^8
-        float m_run = -INFINITY, l_run = 0.f;                  // running max (raw), this thread's share of the running sum
-        uint32_t nflush = 0;
-        int lim = 0, vlen = 0;
-        bool valid = false;
-        RowId id = {0, 0, 0};
-        DenseWalk walk(vis, pre, a.F, a.Hkv, t0, t1);
-        bool ok = true;
-        for (int it = 0; !walk.done() && ok; ++it) {
-            const DenseTile d = walk.next();
-            if (d.first_of_unit) {
-                const int gr = d.rb * kDenseRows + row;
-                valid = gr < a.rows_total;
-                id = decode_row(valid ? gr : 0, a.G, a.S);
+        float m_run = -INFINITY, l_run = 0.f;                  // running max (raw, the row's) and sum (of this half's columns)
+        uint32_t phase = 0;                                    // parity of this group's next S; its last PV has the other one
+        bool any = false, ever = false;                        // has worked on a tile of this unit; at all
+        DenseRow id = {false, 0, 0, 0};
+        // The two warps of a pair leave together, also when a wait has run out: a barrier the other one never reaches
+        // could not be given up.
+        while (true) {
+            const bool more = segs.next(d, lane, a.status);
+            if (pair_any(pair_bar, !more)) break;
+            //TX if (warp == 0) TL(0, 100);  if (warp == 8) TL(1, 100);
+            if (d.first()) {
+                int4 rec = make_int4(0, 0, 0, 0);
+                if constexpr (PAGED) rec = a.rec[d.b];
+                id = dense_row<PAGED>(a, 2 * d.b + (d.single() ? 0 : g), row, rec);
                 m_run = -INFINITY;
                 l_run = 0.f;
+                any = false;
             }
-            if (d.new_segment) {
-                vlen = vis[d.f];
-                if (a.host_plan && a.flen) vlen = min(vlen, a.flen[d.f]);
-                lim = valid ? min(a.loc[(d.f * a.W + id.w) * a.S + id.s], vlen - 1) + 1 : vlen;
-            }
-            const int sb = it & 1;
-            if (warp == 0) HOGATT_TL(1, 1000 + it);
-            ok = mbar_wait_bounded(s_full + 8 * sb, ((uint32_t)(it >> 1)) & 1u, abort_flag, a.status, STATUS_WAIT_FULL_TIMEOUT);
-            ok = __all_sync(0xffffffffu, ok);
-            if (!ok) break;
-            tc_fence_after();
-            if (warp == 0) HOGATT_TL(1, 2000 + it);
-            // ---- this thread's scores stay in registers; the other columns are only folded into the row maximum ----
-            const uint32_t src = tmem + lane_base + (sb ? C::COL_S1 : C::COL_S0);
-            const int nvis = lim - d.tok0;                      // keys of this tile the row sees: [0, nvis)
-            float s[COLS];
-            float mx0 = -INFINITY, mx1 = -INFINITY;
-            {
-                // every load is issued before the first is waited for (one tensor-memory round trip per tile)
-                constexpr int NOTHER = (kDenseTile - COLS) / 32;
-                float other[NOTHER][32];
-#pragma unroll
-                for (int c = 0; c < COLS / 32; ++c) tmem_ld32(src + col0 + c * 32, *reinterpret_cast<float(*)[32]>(&s[c * 32]));
-#pragma unroll
-                for (int c = 0; c < NOTHER; ++c) tmem_ld32(src + ((col0 + COLS + c * 32) & (kDenseTile - 1)), other[c]);
+            int lim = 0;                                       // keys of the fragment that the row sees: [0, lim)
+            if (id.valid) lim = min(dense_location<PAGED>(a, d.f, id), dense_length<PAGED>(a, d.f, id.w) - 1) + 1;
+            const int stride = d.single() ? 2 : 1, t1 = d.single() ? d.t1 : min(d.t1, ((g ? d.vis1 : d.vis0) + kDenseTile - 1) / kDenseTile);
+#pragma unroll 1
+            for (int t = d.t0 + (d.single() ? g : 0); t < t1; t += stride) {
+                ok = mbar_wait_polls(s_full + 8 * g, phase, a.status, STATUS_WAIT_FULL_TIMEOUT);
+                tc_fence_after();
+                __syncwarp();
+                //TL if (warp == 0) TL(0, 1);  if (warp == 8) TL(1, 1);
+                float s[COLS];
+                tmem_ld32(s_addr, *reinterpret_cast<float(*)[32]>(&s[0]));
+                tmem_ld32(s_addr + 32, *reinterpret_cast<float(*)[32]>(&s[32]));
                 tmem_wait_ld();
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(s_free + 8 * sb);    // the next S MMA may overwrite this buffer
-                if (nvis >= kDenseTile) {
+                if (lane == 0) mbar_arrive(s_free);            // the next S MMA may overwrite the buffer
+                //TL if (warp == 0) TL(0, 2);  if (warp == 8) TL(1, 2);
+                const int nvis = lim - t * kDenseTile - half * COLS;      // of this thread's keys the row sees [0, nvis)
+                float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+                if (__any_sync(0xffffffffu, nvis < COLS)) {
 #pragma unroll
-                    for (int c = 0; c < NOTHER; ++c)
-#pragma unroll
-                        for (int k = 0; k < 32; k += 4) {
-                            mx0 = max3(mx0, other[c][k], other[c][k + 1]);
-                            mx1 = max3(mx1, other[c][k + 2], other[c][k + 3]);
-                        }
-#pragma unroll
-                    for (int k = 0; k < COLS; k += 4) {
-                        mx0 = max3(mx0, s[k], s[k + 1]);
-                        mx1 = max3(mx1, s[k + 2], s[k + 3]);
-                    }
-                } else {
-#pragma unroll
-                    for (int c = 0; c < NOTHER; ++c) {
-                        const int ob = (col0 + COLS + c * 32) & (kDenseTile - 1);
-#pragma unroll
-                        for (int k = 0; k < 32; ++k) mx0 = fmaxf(mx0, ob + k < nvis ? other[c][k] : -INFINITY);
-                    }
-#pragma unroll
-                    for (int k = 0; k < COLS; ++k) {
-                        s[k] = col0 + k < nvis ? s[k] : -INFINITY;
-                        mx1 = fmaxf(mx1, s[k]);
-                    }
+                    for (int k = 0; k < COLS; ++k) s[k] = k < nvis ? s[k] : -INFINITY;
                 }
-            }
-            if (warp == 0) HOGATT_TL(1, 3000 + it);
-            const float mx = fmaxf(mx0, mx1);
-            // O is stored at scale 2^(-m_run * scale2).  It is only brought to a new scale when the row's max has
-            // grown by more than a factor 2^8 (so every exponent below stays <= 8) or nothing has been accumulated yet.
-            const bool grow = mx > m_run + grow_by;                     // (m_run = -inf: any finite max grows it)
-            const float m_new = grow ? mx : m_run;
-            const float mu = (m_new == -INFINITY) ? 0.f : m_new;
-            const float alpha = grow ? fast_exp2((m_run - mu) * scale2) : 1.f;      // (m_run = -inf -> 0)
-            m_run = m_new;
-            const float bias = -mu * scale2;
-            float sum0 = 0.f, sum1 = 0.f, sum2 = 0.f, sum3 = 0.f;
-            uint32_t packed[COLS / 2];
 #pragma unroll
-            for (int c = 0; c < COLS; c += 4) {
-                const float e0 = fast_exp2(fmaf(s[c], scale2, bias)), e1 = fast_exp2(fmaf(s[c + 1], scale2, bias));
-                const float e2 = fast_exp2(fmaf(s[c + 2], scale2, bias)), e3 = fast_exp2(fmaf(s[c + 3], scale2, bias));
-                sum0 += e0;
-                sum1 += e1;
-                sum2 += e2;
-                sum3 += e3;
-                packed[c / 2] = pack2<T>(e0, e1);
-                packed[c / 2 + 1] = pack2<T>(e2, e3);
-            }
-            l_run = l_run * alpha + ((sum0 + sum1) + (sum2 + sum3));
-
-            if (warp == 0) HOGATT_TL(1, 4000 + it);
-            // ---- P and O become writable once the previous tile's second MMA has finished ----
-            if (it > 0) {
-                ok = mbar_wait_bounded(o_done, ((uint32_t)(it - 1)) & 1u, abort_flag, a.status, STATUS_WAIT_SYNC_TIMEOUT);
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok) break;
-                tc_fence_after();
-            }
-            if (!d.first_of_unit && __any_sync(0xffffffffu, grow)) {
-                const uint32_t o_addr = tmem + lane_base + C::COL_O + col0;
-#pragma unroll 1
-                for (int c = 0; c < COLS / 32; ++c) {
-                    float o[32];
-                    tmem_ld32(o_addr + c * 32, o);
-                    tmem_wait_ld();
+                for (int k = 0; k < COLS; k += 8)
 #pragma unroll
-                    for (int k = 0; k < 32; ++k) o[k] *= alpha;
-                    tmem_st32(o_addr + c * 32, o);
-                }
-                tmem_wait_st();
-            }
-            if (warp == 0) HOGATT_TL(1, 5000 + it);
-            // ---- P (storage type, two per column) into tensor memory: this row's lane, this thread's columns ----
-            static_assert(COLS == 64, "one 32-column store of packed probabilities per thread");
-            tmem_st32(tmem + lane_base + C::COL_P + col0 / 2, *reinterpret_cast<const float(*)[32]>(&packed[0]));
-            tmem_wait_st();
-            // V rows at or past the fragment's true length may hold anything (spare rows of a slab, fetched as they
-            // are): their probabilities are exactly zero, but 0 * NaN would poison O.  Zero them in the staged tile
-            // (each thread its share of the row's bytes).
-            if (d.tok0 + kDenseTile > vlen) {
-                const int vs = it % C::NV;
-                ok = mbar_wait_bounded(v_full + 8 * vs, ((uint32_t)(it / C::NV)) & 1u, abort_flag, a.status, STATUS_WAIT_FULL_TIMEOUT);
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok) break;
-                if (d.tok0 + row >= vlen) {
-                    unsigned char* vrow = base + C::OFF_V + vs * C::TILE_BYTES + (col0 >> 6) * C::ATOM_BYTES + row * 128 + (col0 & 63) * 2;
-#pragma unroll
-                    for (int c = 0; c < COLS / 8; ++c) *reinterpret_cast<int4*>(vrow + c * 16) = make_int4(0, 0, 0, 0);
-                }
-                fence_proxy_async_smem();      // generic-proxy writes (V rows) before the MMA's async-proxy reads
-            }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(p_full);
-            if (warp == 0) HOGATT_TL(1, 6000 + it);
-
-            // ---- end of this CTA's share of the unit: leave the partial result ----
-            if (d.last_of_unit) {
-                ok = mbar_wait_bounded(o_done, ((uint32_t)it) & 1u, abort_flag, a.status, STATUS_WAIT_SYNC_TIMEOUT);
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok) break;
-                tc_fence_after();
-                int first, count;
-                unit_ctas(d.u, TH, N, ctas, &first, &count);
-                const size_t slot = (size_t)d.u * a.parts_per_unit + (blockIdx.x - first);
-                float* wo = a.ws_o + (slot * kDenseRows + row) * C::HD + col0;
-                const uint32_t o_addr = tmem + lane_base + C::COL_O + col0;
-#pragma unroll 1
-                for (int c = 0; c < COLS / 32; ++c) {
-                    float o[32];
-                    tmem_ld32(o_addr + c * 32, o);
-                    tmem_wait_ld();
-#pragma unroll
-                    for (int k = 0; k < 8; ++k)
-                        *reinterpret_cast<float4*>(wo + c * 32 + k * 4) = make_float4(o[4 * k], o[4 * k + 1], o[4 * k + 2], o[4 * k + 3]);
-                }
-                // The row's sum is the column groups' shares added up.  Groups 1.. hand theirs to group 0 through four
-                // spare tensor-memory columns (two sets, alternating: group 0 may still be reading the previous set).
-                const uint32_t l_addr = tmem + lane_base + C::COL_L + (nflush & 1u) * 4;
-                if (part != 0) {
-                    tmem_st1(l_addr + part, l_run);
-                    tmem_wait_st();
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(l_ready + 8 * (warp & 3));
-                } else {
-                    ok = mbar_wait_bounded(l_ready + 8 * (warp & 3), nflush & 1u, abort_flag, a.status, STATUS_WAIT_SYNC_TIMEOUT);
-                    ok = __all_sync(0xffffffffu, ok);
-                    if (!ok) break;
+                    for (int i = 0; i < 4; ++i) mx[i] = max3(mx[i], s[k + 2 * i], s[k + 2 * i + 1]);
+                float mt = max3(fmaxf(mx[0], mx[1]), mx[2], mx[3]);
+                //TL if (warp == 0) TL(0, 3);  if (warp == 8) TL(1, 3);
+                // ---- P and O become writable once this group's previous second MMA has finished ----
+                if (ever) {
+                    ok = mbar_wait_polls(o_done + 8 * g, phase ^ 1u, a.status, STATUS_WAIT_SYNC_TIMEOUT) && ok;
                     tc_fence_after();
-                    float shares[4];
-                    tmem_ld4(l_addr, shares);
-                    tmem_wait_ld();
-                    float total = l_run;
-#pragma unroll
-                    for (int k = 1; k < SPLIT; ++k) total += shares[k];
-                    a.ws_m[slot * kDenseRows + row] = m_run == -INFINITY ? -INFINITY : m_run * scale2;
-                    a.ws_l[slot * kDenseRows + row] = total;
                 }
-                ++nflush;
+                // O is stored at scale 2^(-m_run * scale2).  It is only brought to a new scale when a row's max has grown by
+                // more than a factor 2^8 (so every exponent below stays <= 8) or nothing has been accumulated yet.  Only
+                // then do the two halves of the rows need each other's maxima.
+                if (pair_any(pair_bar, mt > m_run + grow_by || !ok)) {
+                    ok = !pair_any(pair_bar, !ok);
+                    if (!ok) break;
+                    *stat = mt;
+                    named_barrier_sync(pair_bar, 64);
+                    mt = fmaxf(mt, *other);
+                    named_barrier_sync(pair_bar, 64);          // (read before it is written again)
+                    const bool grow = mt > m_run + grow_by;                     // (m_run = -inf: any finite max grows it)
+                    const float m_new = grow ? mt : m_run;
+                    const float alpha = grow ? fast_exp2((m_run - m_new) * scale2) : 1.f;      // (m_run = -inf -> 0)
+                    m_run = m_new;
+                    l_run *= alpha;
+                    if (any) {
+#pragma unroll 1
+                        for (int c = 0; c < COLS; c += 16) {
+                            uint32_t o[16];
+                            tmem_ld16(o_addr + c, o);
+                            tmem_wait_ld();
+#pragma unroll
+                            for (int k = 0; k < 16; ++k) o[k] = __float_as_uint(__uint_as_float(o[k]) * alpha);
+                            tmem_st16(o_addr + c, o);
+                        }
+                    }
+                }
+                //TL if (warp == 0) TL(0, 4);  if (warp == 8) TL(1, 4);
+                const float bias = (m_run == -INFINITY) ? 0.f : -m_run * scale2;
+                const uint64_t scale_pair = pair_f32(scale2, scale2), bias_pair = pair_f32(bias, bias);
+                uint64_t sum[2] = {0ull, 0ull};                             // (two fp32 zeros each)
+#pragma unroll
+                for (int c = 0; c < COLS / 32; ++c) {
+                    uint32_t packed[16];
+#pragma unroll
+                    for (int k = 0; k < 16; ++k) {
+                        float x0, x1;
+                        unpair_f32(fma2(pair_f32(s[c * 32 + 2 * k], s[c * 32 + 2 * k + 1]), scale_pair, bias_pair), x0, x1);
+                        x0 = fast_exp2(x0);
+                        x1 = fast_exp2(x1);
+                        sum[k & 1] = add2(sum[k & 1], pair_f32(x0, x1));
+                        packed[k] = pack2<T>(x0, x1);
+                    }
+                    tmem_st16(p_addr + c * 16, packed);        // P (storage type, two per column): this row's lane
+                }
+                float l0, l1;
+                unpair_f32(add2(sum[0], sum[1]), l0, l1);
+                l_run += l0 + l1;
+                tmem_wait_st();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(p_full + 8 * g);
+                //TL if (warp == 0) TL(0, 5);  if (warp == 8) TL(1, 5);
+                phase ^= 1u;
+                any = ever = true;
+            }
+            if (!ok) break;
+
+            // ---- end of this CTA's share of the unit: the rows themselves, or a partial result ----
+            //TX if (warp == 0) TL(0, 101);  if (warp == 8) TL(1, 101);
+            if (d.last()) {
+                if (any) {
+                    ok = mbar_wait_polls(o_done + 8 * g, phase ^ 1u, a.status, STATUS_WAIT_SYNC_TIMEOUT);
+                    tc_fence_after();
+                }
+                *stat = l_run;
+                ok = !pair_any(pair_bar, !ok);
+                if (!ok) break;
+                const float total = half ? *other + l_run : l_run + *other;
+                named_barrier_sync(pair_bar, 64);              // (read before it is written again)
+                const bool direct = d.whole() && !d.single();
+                const bool sectors = a.world == 0 && ((uintptr_t)a.out & 31u) == 0;
+                // (a group that saw nothing never touched its O: zeros)
+                const float factor = !any ? 0.f : direct ? (total > 0.f ? 1.f / total : 0.f) : 1.f;
+                const size_t slot = (size_t)blockIdx.x + (size_t)d.b * a.Hkv + d.h;
+                const int slot_row = g * kDenseRows + row;
+                float o[COLS];
+                tmem_ld32(o_addr, *reinterpret_cast<float(*)[32]>(&o[0]));
+                tmem_ld32(o_addr + 32, *reinterpret_cast<float(*)[32]>(&o[32]));
+                tmem_wait_ld();
+#pragma unroll
+                for (int k = 0; k < COLS; ++k) o[k] = any ? o[k] * factor : 0.f;
+                if (!direct) {
+                    float4* const wo = a.ws_o + (slot * (C::HD / 4) + half * (COLS / 4)) * kDenseBlock + slot_row;
+#pragma unroll
+                    for (int k = 0; k < COLS / 4; ++k) wo[k * kDenseBlock] = make_float4(o[4 * k], o[4 * k + 1], o[4 * k + 2], o[4 * k + 3]);
+                    if (half == 0) {
+                        a.ws_m[slot * kDenseBlock + slot_row] = m_run == -INFINITY ? -INFINITY : m_run * scale2;
+                        a.ws_l[slot * kDenseBlock + slot_row] = total;
+                    }
+                } else if (id.valid) {
+                    const size_t offset = dense_out_offset<PAGED>(a, id, d.h) + half * COLS;
+                    uint32_t v[COLS / 16][8];
+#pragma unroll
+                    for (int k = 0; k < COLS / 2; ++k) v[k >> 3][k & 7] = pack2<T>(o[2 * k], o[2 * k + 1]);
+#pragma unroll 1
+                    for (int p = 0; p < max(a.world, 1); ++p) {
+                        T* const dst = static_cast<T*>(a.world > 0 ? a.peer_out[p] : a.out) + offset;
+                        if (sectors) {
+#pragma unroll
+                            for (int k = 0; k < COLS / 16; ++k) store_sector(dst + k * 16, v[k]);
+                        } else {
+#pragma unroll
+                            for (int k = 0; k < COLS / 8; ++k)
+                                reinterpret_cast<uint4*>(dst)[k] = make_uint4(v[k >> 1][(k & 1) * 4], v[k >> 1][(k & 1) * 4 + 1],
+                                                                              v[k >> 1][(k & 1) * 4 + 2], v[k >> 1][(k & 1) * 4 + 3]);
+                        }
+                    }
+                }
                 tc_fence_before();
             }
         }
     }
 
-    // ---- common exit: nobody leaves before tensor memory can be handed back ----
+    //TX if (warp == 0) { TL(0, 103); TLG(0, 104); } if (warp == 8) TL(1, 103);
+    // ---- common exit: nobody leaves before the copies in flight have landed and tensor memory can be handed back ----
+    if (!ok && lane == 0 && warp >= W_K) {
+        const uint64_t since = global_timer_ns();              // (given up: a pending stage completes its transfer at the latest)
+        while (global_timer_ns() - since < 1000000ull) {}
+    }
     tc_fence_before();
     __syncthreads();
-    if (warp == kDenseSoftmaxWarps + 1) {
+    if (warp == W_S) {
         tc_fence_after();
         tmem_dealloc(tmem, C::TMEM_COLS);
+    }
+}
+
+// The units on the plan's list -- more than one CTA worked on them, or one left two halves, or nothing is visible --: fold
+// the partials, normalise, store.  Grid (units, 32-row groups, column groups of 64); a warp takes 32 rows, one per lane, and 16
+// columns: every load of a partial is 512 consecutive bytes, a lane stores one 32-byte sector.
+//   out = sum_p O_p * 2^(m_p - M) / sum_p l_p * 2^(m_p - M),   M = max_p m_p
+template <class T, bool PAGED>
+__global__ void __launch_bounds__(kDenseMergeWarps * 32) dense_merge_kernel(const __grid_constant__ DenseArgs a) {
+    const int lane = threadIdx.x & 31, r = blockIdx.y * 32 + lane, c4 = (blockIdx.z * kDenseMergeWarps + (threadIdx.x >> 5)) * 4;
+    pdl_wait();
+    const int n = *a.nmerge;
+    for (int i = blockIdx.x; i < n; i += gridDim.x) {
+        const int4 e = a.merge[i];
+        const int b = e.x / a.Hkv, h = e.x - b * a.Hkv, count = e.z;
+        const bool single = e.w != 0;
+        // a block of one tile: both 128-row halves of a slot are partials of the same rows
+        if (single && r >= kDenseRows) continue;
+        const int sub = single ? 1 : 0;
+        const size_t slot0 = (size_t)e.y + e.x;
+        auto where = [&](int p) { return (slot0 + (p >> sub)) * kDenseBlock + (single ? (p & 1) * kDenseRows : 0) + r; };
+        float M = -INFINITY;
+#pragma unroll 4
+        for (int p = 0; p < count; ++p) M = fmaxf(M, __ldcg(a.ws_m + where(p)));
+        float den = 0.f;
+        float4 acc[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) acc[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+        for (int p = 0; p < count; ++p) {
+            const size_t at = where(p);
+            const float m = __ldcg(a.ws_m + at), l = __ldcg(a.ws_l + at);
+            const float4* src = a.ws_o + (slot0 + (p >> sub)) * (32 * kDenseBlock) + (size_t)c4 * kDenseBlock + (at - (slot0 + (p >> sub)) * kDenseBlock);
+            const float wgt = m == -INFINITY ? 0.f : exp2f(m - M);       // (a partial that saw nothing holds zeros)
+            den = fmaf(l, wgt, den);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const float4 x = __ldcg(src + k * kDenseBlock);
+                acc[k].x = fmaf(x.x, wgt, acc[k].x);
+                acc[k].y = fmaf(x.y, wgt, acc[k].y);
+                acc[k].z = fmaf(x.z, wgt, acc[k].z);
+                acc[k].w = fmaf(x.w, wgt, acc[k].w);
+            }
+        }
+        int4 rec = make_int4(0, 0, 0, 0);
+        if constexpr (PAGED) rec = a.rec[b];
+        const DenseRow id = dense_row<PAGED>(a, 2 * b + r / kDenseRows, r % kDenseRows, rec);
+        if (!id.valid) continue;
+        const float inv = den > 0.f ? 1.f / den : 0.f;
+        const size_t offset = dense_out_offset<PAGED>(a, id, h) + c4 * 4;
+        uint4 v[2];
+        uint32_t* o = reinterpret_cast<uint32_t*>(v);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            o[2 * k] = pack2<T>(acc[k].x * inv, acc[k].y * inv);
+            o[2 * k + 1] = pack2<T>(acc[k].z * inv, acc[k].w * inv);
+        }
+        for (int p = 0; p < max(a.world, 1); ++p) {
+            uint4* dst = reinterpret_cast<uint4*>(static_cast<T*>(a.world > 0 ? a.peer_out[p] : a.out) + offset);
+            dst[0] = v[0];
+            dst[1] = v[1];
+        }
     }
 }
 

@@ -401,6 +401,7 @@ __global__ void __launch_bounds__(128) rope_kernel(T* __restrict__ rq, const T* 
                                                    int E, int R) {
     write_rotated_queries<T>(q, rq, cosines, sines, F, W, Hq, S, E, R, blockIdx.x * blockDim.x + threadIdx.x,
                              gridDim.x * blockDim.x);
+    pdl_wait();      // launched beside its predecessor: ends after it (otherwise returns at once)
 }
 
 // The same for 16-bit types with the whole head rotated (R == E, E a multiple of 16): a thread owns one pair of
@@ -414,7 +415,10 @@ __global__ void __launch_bounds__(128) rope_pairs_kernel(T* __restrict__ rq, con
                                                          int F, int W, int Hq, int S, int E) {
     const int pairs = E >> 4, half = E >> 1;
     const int item = blockIdx.x * blockDim.x + threadIdx.x;
-    if (item >= F * W * S * pairs) return;
+    if (item >= F * W * S * pairs) {
+        pdl_wait();
+        return;
+    }
     const int j = item % pairs;
     int t = item / pairs;
     const int s = t % S;
@@ -464,6 +468,7 @@ __global__ void __launch_bounds__(128) rope_pairs_kernel(T* __restrict__ rq, con
         *reinterpret_cast<uint4*>(dst) = lo;
         *reinterpret_cast<uint4*>(dst + half) = hi;
     }
+    pdl_wait();      // launched beside its predecessor: ends after it (otherwise returns at once)
 }
 
 }  // namespace hogatt
