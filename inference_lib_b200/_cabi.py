@@ -44,7 +44,7 @@ class PagedProblem(C.Structure):
         ("dtype", C.c_int32), ("scale", C.c_float),
         ("out", C.c_void_p), ("queries", C.c_void_p), ("locations", C.c_void_p), ("fragment_lengths", C.c_void_p),
         ("key_cache", C.c_void_p), ("value_cache", C.c_void_p), ("block_table", C.c_void_p), ("cu_seqlens_q", C.c_void_p),
-        ("workspace", C.c_void_p), ("workspace_bytes", C.c_size_t), ("kernel", C.c_int32), ("reserved_", C.c_int32),
+        ("workspace", C.c_void_p), ("workspace_bytes", C.c_size_t), ("kernel", C.c_int32), ("num_blocks", C.c_int32),
     ]
 
 
@@ -321,7 +321,7 @@ def bind_paged(*, out, queries, locations, fragment_lengths, key_cache, value_ca
     else:
         p.F, p.W, p.Hq, p.S, p.E = queries.shape
     p.Hkv, p.block_size, p.Ev = key_cache.shape[1], key_cache.shape[2], value_cache.shape[3]
-    p.max_blocks_per_seq = block_table.shape[1]
+    p.max_blocks_per_seq, p.num_blocks = block_table.shape[1], key_cache.shape[0]
     p.dtype, p.scale, p.kernel = dtype_code(out.dtype), float(scale), int(kernel)
     p.out, p.queries, p.locations = out.data_ptr(), queries.data_ptr(), locations.data_ptr()
     p.fragment_lengths, p.key_cache, p.value_cache = fragment_lengths.data_ptr(), key_cache.data_ptr(), value_cache.data_ptr()

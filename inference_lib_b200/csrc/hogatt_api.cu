@@ -211,13 +211,17 @@ struct WorkspaceLayout {
     int parts;
 };
 
-// Query tiles per kv head of a fragment call on the tcgen05 kernel: whole workers, or 128-row pieces of one worker.
-void dense_geometry(int W, int64_t gs, int* tiles, int* span) {
+// Query tiles per kv head of a fragment call on the tcgen05 kernel (dense_row in hogatt_dense.cuh): whole workers, or pieces
+// of one worker.
+void dense_geometry(int W, int G, int S, int* tiles, int* span, int* tokens) {
+    const int gs = G * S;
+    *tokens = 0;
     if (gs > kDenseRows) {
-        *span = (int)((gs + kDenseRows - 1) / kDenseRows);
+        if (kDenseRows % G == 0) *tokens = kDenseRows / G;
+        *span = *tokens ? ceil_div(S, *tokens) : ceil_div(gs, kDenseRows);
         *tiles = W * *span;
     } else {
-        *span = kDenseRows / (int)gs;
+        *span = kDenseRows / gs;
         *tiles = ceil_div(W, *span);
     }
 }
@@ -243,8 +247,8 @@ void carve_dense(WorkspaceLayout* w, int64_t blocks, int Hkv, int F, int grid, b
 WorkspaceLayout carve(const hogatt_problem* p, const Resolved& r, int grid) {
     WorkspaceLayout w = {};
     if (r.kernel == HOGATT_KERNEL_DENSE) {
-        int tiles, span;
-        dense_geometry(p->W, (int64_t)(p->Hq / p->Hkv) * p->S, &tiles, &span);
+        int tiles, span, tokens;
+        dense_geometry(p->W, p->Hq / p->Hkv, p->S, &tiles, &span, &tokens);
         carve_dense(&w, (tiles + 1) / 2, p->Hkv, p->F, grid, false);
         // the tcgen05 kernel reads rotated queries from memory: room for them in case the caller does not want them back
         w.total += align_up((size_t)p->F * p->W * p->Hq * p->S * p->E * dtype_size(p->dtype), 256);
@@ -664,8 +668,7 @@ int launch_dense_kernels(const DenseArgs& d, const DenseMaps& maps, int dev, int
     if (kDenseSmemBytes > (size_t)smem_optin) return HOGATT_ERR_CUDA;
     const int rc = ensure_smem_limit(dense_attention_kernel<T, PAGED>, dev, kDenseSmemBytes, granted);
     if (rc != HOGATT_OK) return rc;
-    dense_attention_kernel<T, PAGED><<<dim3(d.ctas), dim3(kDenseThreads), kDenseSmemBytes, stream>>>(d, maps);
-    HOGATT_CUDA_OK(cudaGetLastError());
+    HOGATT_CUDA_OK(launch_kernel(dense_attention_kernel<T, PAGED>, dim3(d.ctas), dim3(kDenseThreads), kDenseSmemBytes, stream, d, maps));
     // at most ctas - 1 units are split; more on the list are blocks of one tile or blind ones (the kernel walks the list)
     const dim3 grid((unsigned)std::min<int64_t>((int64_t)d.blocks * d.Hkv, 2 * (int64_t)d.ctas), kDenseBlock / 32, 128 / (16 * kDenseMergeWarps));
     HOGATT_CUDA_OK(launch_kernel(dense_merge_kernel<T, PAGED>, grid, dim3(kDenseMergeWarps * 32), 0, stream, d));
@@ -696,7 +699,7 @@ int launch_dense(const hogatt_problem* p, const KernelArgs& args, const Workspac
     memset(&d, 0, sizeof(d));
     d.F = args.F; d.W = args.W; d.Hq = args.Hq; d.Hkv = args.Hkv; d.G = args.G; d.S = args.S;
     const int gs = args.G * args.S;
-    dense_geometry(args.W, gs, &d.tiles, &d.tile_span);
+    dense_geometry(args.W, args.G, args.S, &d.tiles, &d.tile_span, &d.tile_tokens);
     d.blocks = (d.tiles + 1) / 2;
     d.l2scale = args.l2scale;
     for (int f = 0; f < args.F; ++f) d.cap[f] = args.host_plan ? args.ft.e[f].vis : args.ft.e[f].rows;
@@ -720,9 +723,11 @@ int launch_dense(const hogatt_problem* p, const KernelArgs& args, const Workspac
         if (rc == HOGATT_OK) rc = fragment_map(args.ft.e[f].v, args.ft.e[f].rows, args.Hkv, p->dtype, &maps.v[f]);
         if (rc != HOGATT_OK) return rc;
     }
-    {   // rotated queries [F, W, Hq, S, E] seen as [F, W, Hkv, G*S, E]; a tile is one box
-        const cuuint64_t dims[5] = {128, (cuuint64_t)gs, (cuuint64_t)args.Hkv, (cuuint64_t)args.W, (cuuint64_t)args.F};
-        const cuuint32_t box[5] = {64, (cuuint32_t)std::min(gs, kDenseRows), 1, (cuuint32_t)(gs > kDenseRows ? 1 : d.tile_span), 1};
+    {   // rotated queries [F, W, Hq, S, E]; a tile is one box of them, or of their view as [F, W, Hkv, G*S, E]
+        const bool tokens = d.tile_tokens > 0;
+        const cuuint64_t dims[5] = {128, (cuuint64_t)(tokens ? args.S : gs), (cuuint64_t)(tokens ? args.Hq : args.Hkv), (cuuint64_t)args.W, (cuuint64_t)args.F};
+        const cuuint32_t box[5] = {64, (cuuint32_t)(tokens ? d.tile_tokens : std::min(gs, kDenseRows)), (cuuint32_t)(tokens ? args.G : 1),
+                                   (cuuint32_t)(gs > kDenseRows ? 1 : d.tile_span), 1};
         const int rc = encode_map(&maps.q, q_rot, p->dtype, 5, dims, box);
         if (rc != HOGATT_OK) return rc;
     }
@@ -890,8 +895,24 @@ int attention_launch(const hogatt_problem* p, bool fused, cudaStream_t stream, c
 
 struct PagedPlan {
     int tokens_per_group, head_blocks, groups_bound, units, splits;
+    bool dense;                     // the tcgen05 kernel
+    int tokens, blocks;             // ... its query tokens per tile, blocks per kv head (upper bound)
+    WorkspaceLayout w;              // ... its workspace
     size_t o, m, l, total;
 };
+
+// Packed queries on the tcgen05 kernel: 16-bit types, head size 128, cache blocks that tile a 128-key tile in whole
+// 8-row swizzle groups (or hold whole tiles), the number of blocks known (a tensor map needs the extent).  AUTO takes it
+// when the prompt chunks of the batch -- the tokens beyond one per sequence -- fill at least one 128-row tile per kv
+// head: the mma.sync kernel reads every sequence once per 16 rows.
+bool paged_dense_wanted(const hogatt_paged_problem* p) {
+    if (p->kernel != HOGATT_KERNEL_AUTO || p->cu_seqlens_q == nullptr || dense_disabled() || p->num_blocks <= 0) return false;
+    if ((p->dtype != HOGATT_F16 && p->dtype != HOGATT_BF16) || p->E != 128 || p->Ev != 128) return false;
+    const int G = p->Hq / p->Hkv, bs = p->block_size;
+    if (G > kDenseRows || !(bs % kDenseTile == 0 || (kDenseTile % bs == 0 && bs % 8 == 0))) return false;
+    if ((int64_t)p->total_q_tokens * p->Hq * p->F >= ((int64_t)1 << 31)) return false;
+    return ((int64_t)p->total_q_tokens - p->W) * G >= kDenseRows;
+}
 
 int plan_paged(const hogatt_paged_problem* p, int sms, PagedPlan* pl) {
     if (p == nullptr) return HOGATT_ERR_NULL_POINTER;
@@ -922,7 +943,48 @@ int plan_paged(const hogatt_paged_problem* p, int sms, PagedPlan* pl) {
     pl->m = pl->o + align_up(slots * p->Ev * sizeof(float), 256);
     pl->l = pl->m + align_up(slots * sizeof(float), 256);
     pl->total = pl->l + align_up(slots * sizeof(float), 256);
+    pl->dense = paged_dense_wanted(p);
+    if (pl->dense) {
+        pl->tokens = kDenseRows / G;
+        pl->blocks = p->total_q_tokens / (2 * pl->tokens) + p->W;
+        carve_dense(&pl->w, pl->blocks, p->Hkv, p->F, std::min(sms, kDenseMaxCtas), true);
+        pl->total = pl->w.total;
+    }
     return HOGATT_OK;
+}
+
+// A packed call on the tcgen05 kernel.
+template <class T>
+int launch_paged_dense(const hogatt_paged_problem* p, const PagedPlan& pl, int dev, int sms, int smem_optin, cudaStream_t stream) {
+    DenseArgs d;
+    memset(&d, 0, sizeof(d));
+    d.F = p->F; d.W = p->W; d.Hq = p->Hq; d.Hkv = p->Hkv; d.G = p->Hq / p->Hkv;
+    d.tiles = 2 * pl.blocks;
+    d.blocks = pl.blocks;
+    d.tile_span = pl.tokens;
+    d.total_q = p->total_q_tokens;
+    d.block_size = p->block_size;
+    d.max_blocks = p->max_blocks_per_seq;
+    d.l2scale = p->scale * 1.4426950408889634f;
+    d.loc = p->locations;
+    d.flen = p->fragment_lengths;
+    d.cu = p->cu_seqlens_q;
+    d.block_table = p->block_table;
+    dense_workspace(&d, static_cast<unsigned char*>(p->workspace), pl.w);
+    d.ctas = std::min(sms, kDenseMaxCtas);
+    d.out = p->out;
+    DenseMaps maps;
+    memset(&maps, 0, sizeof(maps));
+    const cuuint64_t qdims[5] = {128, (cuuint64_t)d.G, (cuuint64_t)d.Hkv, (cuuint64_t)d.total_q, (cuuint64_t)d.F};
+    const cuuint32_t qbox[5] = {64, (cuuint32_t)d.G, 1, (cuuint32_t)d.tile_span, 1};
+    int rc = encode_map(&maps.q, p->queries, p->dtype, 5, qdims, qbox);
+    const cuuint64_t dims[4] = {128, (cuuint64_t)p->block_size, (cuuint64_t)d.Hkv, (cuuint64_t)p->num_blocks};
+    const cuuint32_t box[4] = {64, (cuuint32_t)std::min(p->block_size, kDenseTile), 1, 1};
+    if (rc == HOGATT_OK) rc = encode_map(&maps.k[0], p->key_cache, p->dtype, 4, dims, box);
+    if (rc == HOGATT_OK) rc = encode_map(&maps.v[0], p->value_cache, p->dtype, 4, dims, box);
+    if (rc != HOGATT_OK) return rc;
+    HOGATT_CUDA_OK(launch_kernel(dense_plan_kernel<true>, dim3(1), dim3(kDensePlanThreads), 0, stream, d));
+    return launch_dense_kernels<T, true>(d, maps, dev, smem_optin, stream);
 }
 
 template <class T, int EV>
@@ -1117,6 +1179,10 @@ int hogatt_paged_sdpa_launch(const hogatt_paged_problem* p, hogatt_stream_t stre
     if (p->workspace_bytes < pl.total) return HOGATT_ERR_WORKSPACE_TOO_SMALL;
     const bool packed = p->cu_seqlens_q != nullptr;
     if (packed && p->total_q_tokens == 0) return HOGATT_OK;
+
+    if (pl.dense)
+        return p->dtype == HOGATT_F16 ? launch_paged_dense<__half>(p, pl, dev, sms, smem_optin, stream)
+                                      : launch_paged_dense<__nv_bfloat16>(p, pl, dev, sms, smem_optin, stream);
 
     PagedArgs a;
     memset(&a, 0, sizeof(a));

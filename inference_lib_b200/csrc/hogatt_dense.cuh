@@ -45,11 +45,13 @@ constexpr int kDenseSoftmaxWarps = 16;      // two groups of eight: one group pe
 constexpr int kDenseThreads = (kDenseSoftmaxWarps + 4) * 32;
 constexpr int kDensePlanThreads = 1024;
 constexpr int kDenseMaxCtas = 256;
-constexpr int kDenseUnitSteps = 2;          // what starting and finishing a unit costs, in steps
+// What the balanced shares count (cycles on B200: a step 2,660, starting and finishing a unit 8,200, a step of a block of one
+// tile, whose two key tiles the short value ring cannot keep coming, 5,000).
+constexpr int kDenseUnitSteps = 3, kDenseSingleSteps = 2;
 constexpr int kDenseMergeWarps = 4;         // warps per CTA of the merge step
 
 struct alignas(64) DenseMaps {
-    CUtensorMap q;                          // fragments: [F, W, Hkv, G*S, E] view of the rotated queries; paged: [F, total_q, Hkv, G, E]
+    CUtensorMap q;                          // rotated queries as [F, W, Hq, S, E] or [F, W, Hkv, G*S, E]; paged: [F, total_q, Hkv, G, E]
     CUtensorMap k[kDenseMaxFragments];      // fragments: [Hkv, rows, E] each; paged: k[0] = [blocks, Hkv, block_size, E]
     CUtensorMap v[kDenseMaxFragments];
 };
@@ -59,6 +61,7 @@ struct DenseArgs {
     int tiles;             // query tiles per kv head (paged: upper bound)
     int blocks;            // blocks per kv head: pairs of tiles (paged: upper bound)
     int tile_span;         // fragments: workers per tile (G*S <= 128) or tiles per worker; paged: query tokens per tile
+    int tile_tokens;       // fragments, G*S > 128: tokens per tile, all G heads of each (0: 128 consecutive rows, token fastest)
     int total_q;           // paged: packed query tokens
     int block_size, max_blocks;
     float l2scale;         // scale * log2(e)
@@ -266,8 +269,9 @@ __device__ __forceinline__ bool elect_one() {
 }
 
 // ---- geometry ----------------------------------------------------------------------------------------------------
-// Fragments: query rows of a kv head are (worker, row of G*S) and a tile holds whole workers (tile_span of them) or 128
-// rows of one worker.  Paged: a tile is tile_span tokens of one worker's packed run, G rows each.
+// Fragments: a tile holds whole workers (tile_span of them), or tile_tokens tokens of one worker with all their heads, so
+// that its rows end at nearly the same key of a causal prompt; where G does not divide 128, 128 consecutive rows of a
+// worker, tokens fastest.  Paged: a tile is tile_span tokens of one worker's packed run, G rows each.
 struct DenseRow {
     bool valid;
     int w, g, s;           // s: token of the worker (fragments), packed token index (paged)
@@ -281,6 +285,11 @@ __device__ __forceinline__ DenseRow dense_row(const DenseArgs& a, int tile, int 
         r.w = rec.x;
         r.g = i % a.G;
         r.s = rec.y + tok;
+    } else if (a.tile_tokens > 0) {
+        r.w = tile / a.tile_span;
+        r.g = i / a.tile_tokens;
+        r.s = (tile - r.w * a.tile_span) * a.tile_tokens + i - r.g * a.tile_tokens;
+        r.valid = r.w < a.W && r.s < a.S;
     } else {
         const int gs = a.G * a.S;
         int x = i;
@@ -300,8 +309,8 @@ __device__ __forceinline__ DenseRow dense_row(const DenseArgs& a, int tile, int 
 // rows of fragment f that hold keys and values (worker w's, when paged)
 template <bool PAGED>
 __device__ __forceinline__ int dense_length(const DenseArgs& a, int f, int w) {
-    if constexpr (PAGED) return a.flen[f * a.W + w];
-    return a.flen ? min(a.cap[f], a.flen[f]) : a.cap[f];
+    if constexpr (PAGED) return __ldg(a.flen + f * a.W + w);
+    return a.flen ? min(a.cap[f], __ldg(a.flen + f)) : a.cap[f];
 }
 template <bool PAGED>
 __device__ __forceinline__ int dense_location(const DenseArgs& a, int f, const DenseRow& r) {
@@ -322,16 +331,16 @@ __device__ __forceinline__ int dense_steps(int vis0, int vis1, bool single) {
 // Writes what the other two kernels would otherwise each have to search for: visible keys per (tile, fragment), the prefix
 // of steps over blocks, where every CTA starts, and which units are left to the merge step.  The arrays stay in shared
 // memory while they are worked on, if they fit.
-constexpr int kDensePlanVis = 4096, kDensePlanBlocks = 1024;
+constexpr int kDensePlanVis = 4096, kDensePlanBlocks = 1024, kDensePlanRecs = 512;
 template <bool PAGED>
 __global__ void __launch_bounds__(kDensePlanThreads) dense_plan_kernel(const __grid_constant__ DenseArgs a) {
     __shared__ int s_vis[kDensePlanVis];
     __shared__ long long s_pre[kDensePlanBlocks + 1], s_cost[kDensePlanBlocks + 1], sums[kDensePlanThreads / 32], pos[kDenseMaxCtas + 1];
+    __shared__ int4 s_rec[PAGED ? kDensePlanRecs : 1];
     __shared__ int s_list;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = kDensePlanThreads / 32;
     if (tid == 0) s_list = 0;
     pdl_wait();
-    pdl_trigger();          // the rotation kernel writes nothing that is read here
     // exclusive prefix of one value per thread over the CTA; *total gets the sum
     auto scan = [&](long long v, long long* total) {
         long long x = v;
@@ -364,28 +373,43 @@ __global__ void __launch_bounds__(kDensePlanThreads) dense_plan_kernel(const __g
         for (int w = w0; w < w1; ++w) {
             const int first = a.cu[w], tokens = a.cu[w + 1] - first;
             for (int s = 0; s < tokens; s += span, ++at)
-                if (at < a.blocks) a.rec[at] = make_int4(w, first + s, min(span, tokens - s), 0);
+                if (at < a.blocks) {
+                    const int4 r = make_int4(w, first + s, min(span, tokens - s), 0);
+                    a.rec[at] = r;
+                    if (at < kDensePlanRecs) s_rec[at] = r;
+                }
         }
         __syncthreads();
     }
+    auto record = [&](int b) { return b < kDensePlanRecs ? s_rec[b] : a.rec[b]; };
+    auto single_block = [&](int b) {
+        if constexpr (PAGED) return record(b).z <= a.tile_span;
+        return dense_single<PAGED>(a, b);
+    };
     const bool small = nb <= kDensePlanBlocks && 2 * nb * (long long)a.F <= kDensePlanVis;
     int* const vis = small ? s_vis : a.vis;
     long long* const pre = small ? s_pre : a.pre;
     long long* const cost = small ? s_cost : a.cost;
+#pragma unroll 4
     for (int i = warp; i < 2 * nb * a.F; i += nwarps) {
         // Which tokens a tile's rows are: a run of locations (of one worker's tokens, round its end, if it has more
         // than 128 rows).  Heads repeat the tokens, so no more than 128 locations are read.
         const int tile = i / a.F, f = i - tile * a.F;
         int from, tokens, wrap = INT_MAX, w = 0;      // locations [from, from + tokens); those at or past `wrap` are a.S further down
         if constexpr (PAGED) {
-            const int4 rec = a.rec[tile >> 1];
+            const int4 rec = record(tile >> 1);
             const int skip = (tile & 1) * a.tile_span;
             from = rec.y + skip;
             tokens = min(a.tile_span, rec.z - skip);
             w = rec.x;
         } else {
             const int gs = a.G * a.S;
-            if (gs > kDenseRows) {
+            if (a.tile_tokens > 0) {
+                w = tile / a.tile_span;
+                const int s0 = (tile - w * a.tile_span) * a.tile_tokens;
+                tokens = w < a.W ? min(a.tile_tokens, a.S - s0) : 0;
+                from = w * a.S + s0;
+            } else if (gs > kDenseRows) {
                 w = tile / a.tile_span;
                 const int x = (tile - w * a.tile_span) * kDenseRows;
                 tokens = w < a.W ? min(min(kDenseRows, gs - x), a.S) : 0;
@@ -403,7 +427,7 @@ __global__ void __launch_bounds__(kDensePlanThreads) dense_plan_kernel(const __g
         for (int k = 0; k < kDenseRows; k += 32) {
             int at = from + k + lane;
             if (at >= wrap) at -= a.S;
-            if (k + lane < tokens) top = max(top, loc[at]);
+            if (k + lane < tokens) top = max(top, __ldg(loc + at));
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
@@ -411,9 +435,10 @@ __global__ void __launch_bounds__(kDensePlanThreads) dense_plan_kernel(const __g
         if (lane == 0) a.vis[i] = vis[i] = top;
     }
     __syncthreads();
+    pdl_trigger();          // the rotation kernel writes nothing that is read here (let go before, it crowds out these loads)
     const int per = (nb + kDensePlanThreads - 1) / kDensePlanThreads, b0 = min(tid * per, nb), b1 = min(b0 + per, nb);
     auto block_steps = [&](int b) {
-        const bool single = dense_single<PAGED>(a, b);
+        const bool single = single_block(b);
         long long n = 0;
         for (int f = 0; f < a.F; ++f) n += dense_steps(vis[2 * b * a.F + f], vis[(2 * b + 1) * a.F + f], single);
         return n;
@@ -422,7 +447,7 @@ __global__ void __launch_bounds__(kDensePlanThreads) dense_plan_kernel(const __g
     for (int b = b0; b < b1; ++b) {
         const long long n = block_steps(b);
         mine += n;
-        mine_cost += n > 0 ? n + kDenseUnitSteps : 0;
+        mine_cost += n > 0 ? n * (single_block(b) ? kDenseSingleSteps : 1) + kDenseUnitSteps : 0;
     }
     long long at = scan(mine, &total), at_cost = scan(mine_cost, &total_cost);
     for (int b = b0; b < b1; ++b) {
@@ -430,7 +455,7 @@ __global__ void __launch_bounds__(kDensePlanThreads) dense_plan_kernel(const __g
         a.pre[b] = pre[b] = at;
         cost[b] = at_cost;
         at += n;
-        at_cost += n > 0 ? n + kDenseUnitSteps : 0;
+        at_cost += n > 0 ? n * (single_block(b) ? kDenseSingleSteps : 1) + kDenseUnitSteps : 0;
     }
     if (tid == 0) {
         a.pre[nb] = pre[nb] = total;
@@ -450,8 +475,8 @@ __global__ void __launch_bounds__(kDensePlanThreads) dense_plan_kernel(const __g
             if (cost[mid] * a.Hkv <= t) lo = mid;
             else hi = mid;
         }
-        const long long steps = pre[lo + 1] - pre[lo], off = t - cost[lo] * a.Hkv;
-        long long h = floor_div(off, steps + kDenseUnitSteps), j = min(off - h * (steps + kDenseUnitSteps), steps);
+        const long long steps = pre[lo + 1] - pre[lo], unit = cost[lo + 1] - cost[lo], off = t - cost[lo] * a.Hkv;
+        long long h = floor_div(off, unit), j = min((off - h * unit) / (single_block(lo) ? kDenseSingleSteps : 1), steps);
         pos[tid] = pre[lo] * a.Hkv + h * steps + j;
         if (j == steps) {                            // the unit's end is the next one's beginning
             j = 0;
@@ -475,14 +500,14 @@ __global__ void __launch_bounds__(kDensePlanThreads) dense_plan_kernel(const __g
             st.w = (int)(pos[tid + 1] - pos[tid]);
             const long long s = pos[tid] - st.z;
             // the unit this CTA starts inside of, if no earlier CTA does
-            if (st.z > 0 && !dense_single<PAGED>(a, st.x) && pos[tid - 1] <= s)
+            if (st.z > 0 && !single_block(st.x) && pos[tid - 1] <= s)
                 a.merge[atomicAdd(&s_list, 1)] = make_int4(st.x * a.Hkv + st.y, tid - 1, parts(tid - 1, s, pre[st.x + 1] - pre[st.x]), 0);
         }
         a.start[tid] = st;
     }
     // blocks of one tile (two halves per CTA that worked on them), blocks that see nothing
     for (int b = b0; b < b1; ++b) {
-        const bool single = dense_single<PAGED>(a, b);
+        const bool single = single_block(b);
         const long long steps = pre[b + 1] - pre[b];
         if (!single && steps > 0) continue;
         int at_list = atomicAdd(&s_list, a.Hkv);
@@ -657,8 +682,11 @@ dense_attention_kernel(const __grid_constant__ DenseArgs a, const __grid_constan
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    pdl_wait();             // rotated queries, plan
+    pdl_trigger();
 //TL TLD;
     //TX TLD; if (warp == 0) {TLG(0, 98); TL(0, 99);}
+    //TC long long c_begin = clock64(), c_end = 0; int c_units = 0, c_segs = 0;
     DenseSegments segs{sbase + C::OFF_SEG, seg_full, seg_empty, 0};
     DenseSegment d;
     bool ok = true;
@@ -754,6 +782,9 @@ dense_attention_kernel(const __grid_constant__ DenseArgs a, const __grid_constan
                         const uint32_t dst = sbase + C::OFF_Q + i * C::ATOM_BYTES;
                         if constexpr (PAGED) {
                             tma_load_5d(dst, &maps.q, c, 0, d.h, a.rec[d.b].y + g * a.tile_span, d.f, q_full);
+                        } else if (a.tile_tokens > 0) {
+                            const int tile = 2 * d.b + g, w = tile / a.tile_span;
+                            tma_load_5d(dst, &maps.q, c, (tile - w * a.tile_span) * a.tile_tokens, d.h * a.G, w, d.f, q_full);
                         } else {
                             const int tile = 2 * d.b + g;
                             const int w = gs > kDenseRows ? tile / a.tile_span : tile * a.tile_span;
@@ -881,6 +912,7 @@ dense_attention_kernel(const __grid_constant__ DenseArgs a, const __grid_constan
         while (true) {
             const bool more = segs.next(d, lane, a.status);
             if (pair_any(pair_bar, !more)) break;
+            //TC ++c_segs; if (d.first()) ++c_units;
             //TX if (warp == 0) TL(0, 100);  if (warp == 8) TL(1, 100);
             if (d.first()) {
                 int4 rec = make_int4(0, 0, 0, 0);
@@ -1038,6 +1070,7 @@ dense_attention_kernel(const __grid_constant__ DenseArgs a, const __grid_constan
         }
     }
 
+    //TC if (tid == 0) { c_end = clock64(); g_cta[blockIdx.x][0] = c_end - c_begin; g_cta[blockIdx.x][1] = c_units; g_cta[blockIdx.x][2] = c_segs; g_cta[blockIdx.x][3] = a.start[blockIdx.x].w; }
     //TX if (warp == 0) { TL(0, 103); TLG(0, 104); } if (warp == 8) TL(1, 103);
     // ---- common exit: nobody leaves before the copies in flight have landed and tensor memory can be handed back ----
     if (!ok && lane == 0 && warp >= W_K) {
@@ -1060,6 +1093,7 @@ template <class T, bool PAGED>
 __global__ void __launch_bounds__(kDenseMergeWarps * 32) dense_merge_kernel(const __grid_constant__ DenseArgs a) {
     const int lane = threadIdx.x & 31, r = blockIdx.y * 32 + lane, c4 = (blockIdx.z * kDenseMergeWarps + (threadIdx.x >> 5)) * 4;
     pdl_wait();
+    pdl_trigger();
     const int n = *a.nmerge;
     for (int i = blockIdx.x; i < n; i += gridDim.x) {
         const int4 e = a.merge[i];

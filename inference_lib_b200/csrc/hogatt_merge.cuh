@@ -399,6 +399,7 @@ __global__ void __launch_bounds__(128) rope_kernel(T* __restrict__ rq, const T* 
                                                    const float* __restrict__ cosines,
                                                    const float* __restrict__ sines, int F, int W, int Hq, int S,
                                                    int E, int R) {
+    pdl_trigger();   // (whoever follows waits for this whole grid before it reads)
     write_rotated_queries<T>(q, rq, cosines, sines, F, W, Hq, S, E, R, blockIdx.x * blockDim.x + threadIdx.x,
                              gridDim.x * blockDim.x);
     pdl_wait();      // launched beside its predecessor: ends after it (otherwise returns at once)
@@ -413,6 +414,7 @@ template <class T>
 __global__ void __launch_bounds__(128) rope_pairs_kernel(T* __restrict__ rq, const T* __restrict__ q,
                                                          const float* __restrict__ cosines, const float* __restrict__ sines,
                                                          int F, int W, int Hq, int S, int E) {
+    pdl_trigger();   // (whoever follows waits for this whole grid before it reads)
     const int pairs = E >> 4, half = E >> 1;
     const int item = blockIdx.x * blockDim.x + threadIdx.x;
     if (item >= F * W * S * pairs) {

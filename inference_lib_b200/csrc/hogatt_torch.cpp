@@ -237,6 +237,7 @@ void run_paged(at::Tensor& out, double scale, const at::Tensor& locations, const
     p.Hkv = (int32_t)key_cache.size(1);
     p.block_size = (int32_t)key_cache.size(2);
     p.max_blocks_per_seq = (int32_t)block_table.size(1);
+    p.num_blocks = (int32_t)std::min<int64_t>(key_cache.size(0), value_cache.size(0));
     TORCH_CHECK_EQ(value_cache.size(1), key_cache.size(1));
     TORCH_CHECK_EQ(value_cache.size(2), key_cache.size(2));
     if (packed) {
