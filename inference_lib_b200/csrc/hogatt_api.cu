@@ -8,6 +8,7 @@
 #include <cstring>
 
 #include "hogatt_device.cuh"
+#include "hogatt_f32.cuh"
 #include "hogatt_fma.cuh"
 #include "hogatt_merge.cuh"
 #include "hogatt_mma.cuh"
@@ -487,6 +488,26 @@ int launch_fma_dims(const KernelArgs& args, int dev, int smem_optin, int grid, c
     return HOGATT_ERR_UNSUPPORTED_HEAD_DIM;
 }
 
+// fp32 with E == Ev == 64 or 128.  Up to 8 query rows per kv head take the instantiation of 8 rows, whose warps hold half as
+// many (it stays on the memory's side of the line where 16 rows reach it).
+template <int HD, int R>
+int launch_f32(const KernelArgs& args, int dev, int smem_optin, int grid, cudaStream_t stream) {
+    static std::atomic<size_t> granted[kMaxDevices];
+    const size_t smem = f32_smem_bytes<HD, R>(args.F);
+    if (smem > (size_t)smem_optin) return HOGATT_ERR_TOO_MANY_FRAGMENTS;
+    const int rc = ensure_smem_limit(f32_attention_kernel<HD, R>, dev, smem, granted);
+    if (rc != HOGATT_OK) return rc;
+    HOGATT_CUDA_OK(launch_kernel(f32_attention_kernel<HD, R>, dim3(grid), dim3(F32Cfg<HD, R>::THREADS), smem, stream, args));
+    return HOGATT_OK;
+}
+
+int launch_f32_dims(const KernelArgs& args, int dev, int smem_optin, int grid, cudaStream_t stream) {
+    if (args.E != args.Ev || (args.E != 64 && args.E != 128)) return launch_fma_dims<float>(args, dev, smem_optin, grid, stream);
+    if (args.E == 128)
+        return args.rows_total <= 8 ? launch_f32<128, 8>(args, dev, smem_optin, grid, stream) : launch_f32<128, 16>(args, dev, smem_optin, grid, stream);
+    return args.rows_total <= 8 ? launch_f32<64, 8>(args, dev, smem_optin, grid, stream) : launch_f32<64, 16>(args, dev, smem_optin, grid, stream);
+}
+
 // The merge step after a persistent-grid attention kernel.  Up to 32 partial slots per unit: one warp per output row
 // (lean instantiation; 8 kv heads on one GPU leave 19-20 partials per row).  More -- kv heads sharded over GPUs, one
 // unit cut into 37 ... 148 partials -- one CTA per row whose eight warps share the partials (one memory round trip
@@ -764,7 +785,7 @@ int launch_all(const KernelArgs& args, const Resolved& r, int dev, int smem_opti
 
 template <>
 int launch_all<float>(const KernelArgs& args, const Resolved& r, int dev, int smem_optin, int grid, cudaStream_t stream) {
-    int rc = launch_fma_dims<float>(args, dev, smem_optin, grid, stream);
+    int rc = launch_f32_dims(args, dev, smem_optin, grid, stream);
     if (rc != HOGATT_OK) return rc;
     return launch_merge<float>(args, r, stream);
 }

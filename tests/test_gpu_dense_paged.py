@@ -1,0 +1,72 @@
+"""Packed queries over a paged cache on the tcgen05 kernel: AUTO's choice once the prompt chunks of a batch fill a query tile."""
+import numpy as np
+import pytest
+import torch
+
+from inference_lib_b200 import _cabi
+from oracle import hogwild_oracle as oracle
+from tests.gpu_util import check_against
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.mark.parametrize("dtype,G,bs,seqs,lens", [
+    (torch.bfloat16, 4, 16, [65, 1, 0, 40, 64], [200, 129, 77, 40, 64]),     # 64 tokens are a block of two tiles
+    (torch.bfloat16, 5, 8, [51, 1, 26], [300, 513, 127]),                    # 25 tokens per tile, 3 rows of it unused
+    (torch.float16, 1, 32, [257, 3], [257, 400]),                            # a tile is 128 tokens
+    (torch.bfloat16, 7, 256, [40, 2], [700, 259]),                           # cache blocks of two key tiles
+    (torch.float16, 128, 64, [3, 1], [90, 256]),                             # a tile is one token
+])
+@pytest.mark.parametrize("F", [1, 2])
+def test_prompt_chunks_match_the_oracle(dtype, G, bs, seqs, lens, F):
+    rng = np.random.default_rng(G * 100 + bs)
+    W, Hkv, E = len(seqs), 2, 128
+    cu = torch.tensor([0] + list(np.cumsum(seqs)), dtype=torch.int32)
+    total = int(cu[-1])
+    gen = torch.Generator().manual_seed(G)
+    per = max(lens) // bs + 2
+    kc, vc = (torch.randn(W * per, Hkv, bs, E, generator=gen).to(dtype) for _ in range(2))
+    table = torch.from_numpy(rng.permutation(W * per).astype(np.int32)).reshape(W, per)
+    length = torch.tensor([[max(1, n - 13 * f) for n in lens] for f in range(F)], dtype=torch.int32)
+    loc = torch.tensor([[int(length[f, w]) - s + t for w, s in enumerate(seqs) for t in range(s)] for f in range(F)], dtype=torch.int32)
+    loc[0, 0] = -1 if F == 2 else loc[0, 0]                                  # a row that sees nothing of one fragment
+    rq = torch.randn(F, total, Hkv * G, E, generator=gen).to(dtype)
+    ref = oracle.varlen_paged_sdpa(rq, loc, length, kc, vc, table, cu, E ** -0.5)
+    # rows of the last cache block past a sequence's end may hold anything
+    for w in range(W):
+        n = int(length[:, w].max())
+        for x in range(n, per * bs):
+            vc[table[w, x // bs], :, x % bs] = float("nan")
+            kc[table[w, x // bs], :, x % bs] = float("inf")
+    dev = [t.to(DEV) for t in (rq, loc, length, kc, vc, table, cu)]
+    outs = []
+    for kernel in (_cabi.KERNEL_AUTO, _cabi.KERNEL_MMA):                     # the general path over the same inputs
+        out = torch.full((total, Hkv * G, E), float("nan"), dtype=dtype, device=DEV)
+        rc, keep = _cabi.paged_sdpa(out=out, queries=dev[0], locations=dev[1], fragment_lengths=dev[2], key_cache=dev[3], value_cache=dev[4],
+                                    block_table=dev[5], scale=E ** -0.5, cu_seqlens_q=dev[6], kernel=kernel,
+                                    stream=torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        assert rc == 0
+        check_against(out, ref.numpy(), dtype, what=f"kernel {kernel}")
+        outs.append(out.float())
+    assert float((outs[0] - outs[1]).abs().max()) <= 2e-2
+
+
+def test_which_calls_take_it():
+    """The workspace tells the routes apart: a chunk that fills a 128-row tile beyond one token per sequence, the cache's extent known."""
+    p = _cabi.PagedProblem()
+    p.F, p.W, p.Hq, p.Hkv, p.E, p.Ev, p.block_size, p.max_blocks_per_seq = 1, 4, 16, 4, 128, 128, 16, 64
+    p.dtype, p.num_blocks, p.cu_seqlens_q = _cabi.BF16, 256, 1
+    lib = _cabi.load()
+
+    def need(**kw):
+        for k, v in dict(dict(total_q_tokens=36, num_blocks=256, block_size=16, kernel=_cabi.KERNEL_AUTO), **kw).items():
+            setattr(p, k, v)
+        return lib.hogatt_paged_workspace_bytes(p)
+
+    general = need(kernel=_cabi.KERNEL_MMA)
+    assert need() != general
+    for kw in (dict(num_blocks=0), dict(block_size=12), dict(block_size=4)):
+        assert need(**kw) == general
+    assert need(total_q_tokens=35) == need(total_q_tokens=35, kernel=_cabi.KERNEL_MMA)
