@@ -11,7 +11,7 @@
 //     quarter warp take the same key of the eight groups: no bank conflicts although bulk copies land rows unpadded.
 //   * P V: a lane is four columns, probabilities are broadcasts.  Products go two at a time (fma.rn.f32x2, each rounded
 //     as the scalar instruction rounds it).
-// Warps keep their own running maximum, sum and O; the two warps that share rows are folded where the CTA's share of a unit
+// Warps keep their own running maximum, sum and O; the four warps that share rows are folded where the CTA's share of a unit
 // ends.  Row counts above 16 run as several blocks; the repeats of the keys are served by L2.
 #pragma once
 #include "hogatt_device.cuh"
@@ -20,11 +20,13 @@ namespace hogatt {
 
 template <int HD, int R>
 struct F32Cfg {
-    static constexpr int TILE = 64, WARPS = 4, THREADS = (WARPS + 1) * 32;
-    static constexpr int RW = R / 2;                        // rows per warp: warps w and w + 2 share keys, w and w ^ 1 rows
+    // Eight warps: w & 1 the half of a tile's keys, (w >> 1) & 1 the half of the rows, w >> 2 which tiles (every other one).
+    // One team of four had each scheduler wait out the latencies of its only warp.
+    static constexpr int TILE = 64, TEAMS = 2, WARPS = 4 * TEAMS, THREADS = (WARPS + 1) * 32;
+    static constexpr int RW = R / 2;                        // rows per warp
     static constexpr int GROUP_STRIDE = 8 * HD * 4 + 16;
     static constexpr int BUF_BYTES = 8 * GROUP_STRIDE;      // one K or V tile
-    static constexpr int NBUF = HD == 128 ? 6 : 8;          // K and V tiles in turn
+    static constexpr int NBUF = HD == 128 ? 4 : 8;          // K and V tiles in turn; a multiple of 4, so that a buffer always serves the same team (parities)
     static constexpr int QPITCH = HD + 4;                   // floats
     static constexpr int CPL = HD / 32;                     // columns of O per lane and key: lanes cover 128 columns, or 64 twice
     static constexpr int OFF_Q = NBUF * BUF_BYTES;
@@ -76,7 +78,7 @@ __global__ void __launch_bounds__(F32Cfg<HD, R>::THREADS, 1) f32_attention_kerne
     if (tid == 0) {
         for (int i = 0; i < C::NBUF; ++i) {
             mbar_init(full + 8 * i, 1);
-            mbar_init(empty + 8 * i, C::WARPS);
+            mbar_init(empty + 8 * i, 4);             // the warps of one team
         }
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -135,7 +137,7 @@ __global__ void __launch_bounds__(F32Cfg<HD, R>::THREADS, 1) f32_attention_kerne
     }
 
     // ============================== scores, softmax, values ==============================
-    const int kh = warp & 1, rw0 = (warp >> 1) * RW;        // this warp's half of the keys, first row
+    const int kh = warp & 1, rw0 = ((warp >> 1) & 1) * RW, team = warp >> 2;        // half of the keys, first row, which tiles
     const float* const q = static_cast<const float*>(a.q);
     float* const p_s = reinterpret_cast<float*>(base + C::OFF_P) + warp * 32 * RW;
     float* const fold = reinterpret_cast<float*>(base + C::OFF_FOLD);
@@ -207,94 +209,95 @@ __global__ void __launch_bounds__(F32Cfg<HD, R>::THREADS, 1) f32_attention_kerne
 
         // ---- S = Q K^T: this lane's key against the warp's rows.  (A wait that runs out raises the CTA's abort flag: the
         // waits after it return at once, the results are void, and every warp still reaches every barrier.) ----
-        uint32_t i = n % C::NBUF;
-        mbar_wait_bounded(full + 8 * i, (n / C::NBUF) & 1u, abort_flag, a.status, STATUS_WAIT_FULL_TIMEOUT);
-        __syncwarp();
-        uint64_t s2[RW];
+        if (((n >> 1) & 1u) == (uint32_t)team) {
+            uint32_t i = n % C::NBUF;
+            mbar_wait_bounded(full + 8 * i, (n / C::NBUF) & 1u, abort_flag, a.status, STATUS_WAIT_FULL_TIMEOUT);
+            __syncwarp();
+            uint64_t s2[RW];
 #pragma unroll
-        for (int r = 0; r < RW; ++r) s2[r] = 0ull;
-        {
-            const ulonglong2* k = reinterpret_cast<const ulonglong2*>(base + i * C::BUF_BYTES + (lane & 7) * C::GROUP_STRIDE + (my_key & 7) * HD * 4);
-            const float* qr = qs + rw0 * C::QPITCH;
+            for (int r = 0; r < RW; ++r) s2[r] = 0ull;
+            {
+                const ulonglong2* k = reinterpret_cast<const ulonglong2*>(base + i * C::BUF_BYTES + (lane & 7) * C::GROUP_STRIDE + (my_key & 7) * HD * 4);
+                const float* qr = qs + rw0 * C::QPITCH;
 #pragma unroll 4
-            for (int c = 0; c < HD / 4; ++c) {
-                const ulonglong2 kv = k[c];
+                for (int c = 0; c < HD / 4; ++c) {
+                    const ulonglong2 kv = k[c];
 #pragma unroll
-                for (int r = 0; r < RW; ++r) {
-                    const ulonglong2 qv = *reinterpret_cast<const ulonglong2*>(qr + r * C::QPITCH + c * 4);
-                    s2[r] = f32x2_fma(kv.x, qv.x, s2[r]);
-                    s2[r] = f32x2_fma(kv.y, qv.y, s2[r]);
-                }
-            }
-        }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(empty + 8 * i);
-        ++n;
-
-        // ---- online softmax, base 2 ----
-        const int key = tok0 + my_key;
-        float s[RW];
-        bool grew = false;
-        float top[RW];
-#pragma unroll
-        for (int r = 0; r < RW; ++r) {
-            s[r] = my_key < ntok && key < lim[r] ? f32x2_sum(s2[r]) * a.l2scale : -INFINITY;
-            top[r] = fmaxf(m[r], warp_max(s[r]));
-            grew |= top[r] != m[r];
-        }
-        if (grew) {                                           // (the same in every lane)
-#pragma unroll
-            for (int r = 0; r < RW; ++r) {
-                const float alpha = m[r] == -INFINITY ? 0.f : exp2f(m[r] - top[r]);
-                const uint64_t al2 = f32x2(alpha, alpha);
-                l[r] *= alpha;
-                o[r][0] = f32x2_fma(o[r][0], al2, 0ull);
-                o[r][1] = f32x2_fma(o[r][1], al2, 0ull);
-                m[r] = top[r];
-            }
-        }
-#pragma unroll
-        for (int r = 0; r < RW; ++r) {
-            s[r] = m[r] == -INFINITY ? 0.f : exp2f(s[r] - m[r]);
-            l[r] += s[r];
-        }
-#pragma unroll
-        for (int r = 0; r < RW; r += 4) *reinterpret_cast<float4*>(p_s + lane * RW + r) = make_float4(s[r], s[r + 1], s[r + 2], s[r + 3]);
-        __syncwarp();
-
-        // ---- O += P V: this lane's four columns ----
-        i = n % C::NBUF;
-        mbar_wait_bounded(full + 8 * i, (n / C::NBUF) & 1u, abort_flag, a.status, STATUS_WAIT_FULL_TIMEOUT);
-        __syncwarp();
-        {
-            const float* v = reinterpret_cast<const float*>(base + i * C::BUF_BYTES) + col;
-            constexpr int STEP = HD == 64 ? 2 : 1;
-            auto values = [&](auto whole) {
-#pragma unroll 8
-                for (int kk = 0; kk < 32; kk += STEP) {
-                    const int x = kk + vhalf;                 // key of the warp's 32: lane x's
-                    const int tk = (x & 7) * 8 + kh * 4 + (x >> 3);
-                    ulonglong2 vv = make_ulonglong2(0ull, 0ull);
-                    if (decltype(whole)::value || tk < ntok) vv = *reinterpret_cast<const ulonglong2*>(v + tk * HD);
-#pragma unroll
-                    for (int r = 0; r < RW; r += 4) {
-                        const float4 p = *reinterpret_cast<const float4*>(p_s + x * RW + r);
-                        const float pr[4] = {p.x, p.y, p.z, p.w};
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            const uint64_t pp = f32x2(pr[e], pr[e]);
-                            o[r + e][0] = f32x2_fma(vv.x, pp, o[r + e][0]);
-                            o[r + e][1] = f32x2_fma(vv.y, pp, o[r + e][1]);
-                        }
+                    for (int r = 0; r < RW; ++r) {
+                        const ulonglong2 qv = *reinterpret_cast<const ulonglong2*>(qr + r * C::QPITCH + c * 4);
+                        s2[r] = f32x2_fma(kv.x, qv.x, s2[r]);
+                        s2[r] = f32x2_fma(kv.y, qv.y, s2[r]);
                     }
                 }
-            };
-            if (ntok == C::TILE) values(std::true_type());
-            else values(std::false_type());
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(empty + 8 * i);
+            i = (n + 1) % C::NBUF;
+
+            // ---- online softmax, base 2 ----
+            const int key = tok0 + my_key;
+            float s[RW];
+            bool grew = false;
+            float top[RW];
+#pragma unroll
+            for (int r = 0; r < RW; ++r) {
+                s[r] = my_key < ntok && key < lim[r] ? f32x2_sum(s2[r]) * a.l2scale : -INFINITY;
+                top[r] = fmaxf(m[r], warp_max(s[r]));
+                grew |= top[r] != m[r];
+            }
+            if (grew) {                                           // (the same in every lane)
+#pragma unroll
+                for (int r = 0; r < RW; ++r) {
+                    const float alpha = m[r] == -INFINITY ? 0.f : exp2f(m[r] - top[r]);
+                    const uint64_t al2 = f32x2(alpha, alpha);
+                    l[r] *= alpha;
+                    o[r][0] = f32x2_fma(o[r][0], al2, 0ull);
+                    o[r][1] = f32x2_fma(o[r][1], al2, 0ull);
+                    m[r] = top[r];
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < RW; ++r) {
+                s[r] = m[r] == -INFINITY ? 0.f : exp2f(s[r] - m[r]);
+                l[r] += s[r];
+            }
+#pragma unroll
+            for (int r = 0; r < RW; r += 4) *reinterpret_cast<float4*>(p_s + lane * RW + r) = make_float4(s[r], s[r + 1], s[r + 2], s[r + 3]);
+            __syncwarp();
+
+            // ---- O += P V: this lane's four columns ----
+            mbar_wait_bounded(full + 8 * i, ((n + 1) / C::NBUF) & 1u, abort_flag, a.status, STATUS_WAIT_FULL_TIMEOUT);
+            __syncwarp();
+            {
+                const float* v = reinterpret_cast<const float*>(base + i * C::BUF_BYTES) + col;
+                constexpr int STEP = HD == 64 ? 2 : 1;
+                auto values = [&](auto whole) {
+#pragma unroll 8
+                    for (int kk = 0; kk < 32; kk += STEP) {
+                        const int x = kk + vhalf;                 // key of the warp's 32: lane x's
+                        const int tk = (x & 7) * 8 + kh * 4 + (x >> 3);
+                        ulonglong2 vv = make_ulonglong2(0ull, 0ull);
+                        if (decltype(whole)::value || tk < ntok) vv = *reinterpret_cast<const ulonglong2*>(v + tk * HD);
+#pragma unroll
+                        for (int r = 0; r < RW; r += 4) {
+                            const float4 p = *reinterpret_cast<const float4*>(p_s + x * RW + r);
+                            const float pr[4] = {p.x, p.y, p.z, p.w};
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) {
+                                const uint64_t pp = f32x2(pr[e], pr[e]);
+                                o[r + e][0] = f32x2_fma(vv.x, pp, o[r + e][0]);
+                                o[r + e][1] = f32x2_fma(vv.y, pp, o[r + e][1]);
+                            }
+                        }
+                    }
+                };
+                if (ntok == C::TILE) values(std::true_type());
+                else values(std::false_type());
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(empty + 8 * i);
         }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(empty + 8 * i);
-        ++n;
+        n += 2;
 
         // ---- leave a partial result where this CTA's share of the unit ends: fold the two key halves of every row ----
         if (j == TH - 1 || t == t1 - 1) {
@@ -322,15 +325,27 @@ __global__ void __launch_bounds__(F32Cfg<HD, R>::THREADS, 1) f32_attention_kerne
             named_barrier_sync(1, C::WARPS * 32);
             for (int idx = tid; idx < R * HD / 4; idx += C::WARPS * 32) {
                 const int r = idx / (HD / 4), c = (idx - r * (HD / 4)) * 4;
-                const int w0 = (r / RW) * 2, s0 = w0 * RW + r % RW, s1 = s0 + RW;        // the two warps' slots of row r
-                const float M = fmaxf(fold_m[s0], fold_m[s1]), mu = M == -INFINITY ? 0.f : M;
-                const float w_a = exp2f(fold_m[s0] - mu), w_b = exp2f(fold_m[s1] - mu);
-                const float4 x = *reinterpret_cast<const float4*>(fold + s0 * HD + c), y = *reinterpret_cast<const float4*>(fold + s1 * HD + c);
-                *reinterpret_cast<float4*>(a.ws_o + (row0 + r) * HD + c) =
-                    make_float4(fmaf(y.x, w_b, x.x * w_a), fmaf(y.y, w_b, x.y * w_a), fmaf(y.z, w_b, x.z * w_a), fmaf(y.w, w_b, x.w * w_a));
+                // the row's warps: both key halves of both teams
+                float M = -INFINITY, sum = 0.f;
+#pragma unroll
+                for (int x = 0; x < 2 * C::TEAMS; ++x) M = fmaxf(M, fold_m[((x >> 1) * 4 + (r / RW) * 2 + (x & 1)) * RW + r % RW]);
+                const float mu = M == -INFINITY ? 0.f : M;
+                float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                for (int x = 0; x < 2 * C::TEAMS; ++x) {
+                    const int slot = ((x >> 1) * 4 + (r / RW) * 2 + (x & 1)) * RW + r % RW;
+                    const float w = exp2f(fold_m[slot] - mu);
+                    const float4 y = *reinterpret_cast<const float4*>(fold + slot * HD + c);
+                    acc.x = fmaf(y.x, w, acc.x);
+                    acc.y = fmaf(y.y, w, acc.y);
+                    acc.z = fmaf(y.z, w, acc.z);
+                    acc.w = fmaf(y.w, w, acc.w);
+                    sum = fmaf(fold_l[slot], w, sum);
+                }
+                *reinterpret_cast<float4*>(a.ws_o + (row0 + r) * HD + c) = acc;
                 if (c == 0) {
                     a.ws_m[row0 + r] = M;
-                    a.ws_l[row0 + r] = fmaf(fold_l[s1], w_b, fold_l[s0] * w_a);
+                    a.ws_l[row0 + r] = sum;
                 }
             }
             named_barrier_sync(1, C::WARPS * 32);            // (read before the next share's fold)
