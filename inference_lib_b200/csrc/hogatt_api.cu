@@ -1031,18 +1031,26 @@ bool paged_mma_disabled() {
     return off;
 }
 
-// Two ring stages: measured best at 8 sequences x 16 K keys (deeper rings cost resident CTAs: three stages 53 us
-// against 40).
-template <class T, int HD>
+template <class T, int HD, bool BULK>
 int launch_paged_mma(const PagedArgs& a, const PagedPlan& pl, int dev, int smem_optin, cudaStream_t stream) {
     static std::atomic<size_t> granted[kMaxDevices];
-    const size_t smem = paged_mma_smem_bytes<HD>(a.F);
+    const size_t smem = paged_mma_smem_bytes<HD, BULK>(a.F);
     if (smem > (size_t)smem_optin) return HOGATT_ERR_TOO_MANY_FRAGMENTS;
-    int rc = ensure_smem_limit(paged_mma_kernel<T, HD>, dev, smem, granted);
+    int rc = ensure_smem_limit(paged_mma_kernel<T, HD, BULK>, dev, smem, granted);
     if (rc != HOGATT_OK) return rc;
-    HOGATT_CUDA_OK(launch_kernel(paged_mma_kernel<T, HD>, dim3(pl.units, pl.splits), dim3(PagedMmaCfg<HD>::THREADS), smem, stream, a));
+    HOGATT_CUDA_OK(launch_kernel(paged_mma_kernel<T, HD, BULK>, dim3(pl.units, a.splits), dim3(PagedMmaCfg<HD, BULK>::THREADS), smem, stream, a));
     HOGATT_CUDA_OK(launch_kernel(paged_merge_kernel<T>, dim3(pl.units, kFmaRows / kMergeWarps), dim3(kMergeWarps * 32), 0, stream, a));
     return HOGATT_OK;
+}
+
+// Bulk copies need runs of 8 rows.  Their ring of three leaves room for two CTAs per SM at head size 128 (at 64: three of four): splits
+// that fill them once.  (More fragments than fit beside that ring: row by row, as before.)
+template <class T, int HD>
+int launch_paged_mma_rows(PagedArgs a, const PagedPlan& pl, int dev, int sms, int smem_optin, cudaStream_t stream) {
+    if (a.block_size % 8 != 0 || paged_mma_smem_bytes<HD, true>(a.F) > (size_t)smem_optin)
+        return launch_paged_mma<T, HD, false>(a, pl, dev, smem_optin, stream);
+    a.splits = std::max(1, std::min(pl.splits, (HD == 128 ? 2 : 3) * sms / pl.units));
+    return launch_paged_mma<T, HD, true>(a, pl, dev, smem_optin, stream);
 }
 
 template <class T>
@@ -1051,13 +1059,13 @@ bool paged_mma_eligible(const PagedArgs& a) {
 }
 
 template <class T>
-int launch_paged_dims(const PagedArgs& a, const PagedPlan& pl, int kernel, int dev, int smem_optin, cudaStream_t stream) {
+int launch_paged_dims(const PagedArgs& a, const PagedPlan& pl, int kernel, int dev, int sms, int smem_optin, cudaStream_t stream) {
     if (kernel != HOGATT_KERNEL_AUTO && kernel != HOGATT_KERNEL_FMA && kernel != HOGATT_KERNEL_MMA) return HOGATT_ERR_BAD_KERNEL_CHOICE;
     if (kernel == HOGATT_KERNEL_MMA && !paged_mma_eligible<T>(a)) return HOGATT_ERR_BAD_KERNEL_CHOICE;
     if constexpr (!std::is_same<T, float>::value) {
         if (kernel == HOGATT_KERNEL_MMA || (kernel == HOGATT_KERNEL_AUTO && paged_mma_eligible<T>(a) && !paged_mma_disabled()))
-            return a.E == 128 ? launch_paged_mma<T, 128>(a, pl, dev, smem_optin, stream)
-                              : launch_paged_mma<T, 64>(a, pl, dev, smem_optin, stream);
+            return a.E == 128 ? launch_paged_mma_rows<T, 128>(a, pl, dev, sms, smem_optin, stream)
+                              : launch_paged_mma_rows<T, 64>(a, pl, dev, sms, smem_optin, stream);
     }
     switch (a.Ev) {
         case 32: return launch_paged<T, 32>(a, pl, dev, smem_optin, stream);
@@ -1230,9 +1238,9 @@ int hogatt_paged_sdpa_launch(const hogatt_paged_problem* p, hogatt_stream_t stre
     a.ws_m = reinterpret_cast<float*>(ws + pl.m);
     a.ws_l = reinterpret_cast<float*>(ws + pl.l);
     switch (p->dtype) {
-        case HOGATT_F32: return launch_paged_dims<float>(a, pl, p->kernel, dev, smem_optin, stream);
-        case HOGATT_F16: return launch_paged_dims<__half>(a, pl, p->kernel, dev, smem_optin, stream);
-        case HOGATT_BF16: return launch_paged_dims<__nv_bfloat16>(a, pl, p->kernel, dev, smem_optin, stream);
+        case HOGATT_F32: return launch_paged_dims<float>(a, pl, p->kernel, dev, sms, smem_optin, stream);
+        case HOGATT_F16: return launch_paged_dims<__half>(a, pl, p->kernel, dev, sms, smem_optin, stream);
+        case HOGATT_BF16: return launch_paged_dims<__nv_bfloat16>(a, pl, p->kernel, dev, sms, smem_optin, stream);
     }
     return HOGATT_ERR_UNSUPPORTED_DTYPE;
 }

@@ -244,15 +244,12 @@ __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
-// Bounded wait of a few instructions: kernels that move registers between warps (setmaxnreg) cannot have calls, and the
-// five roles' loops together have to stay in the instruction cache (with the timer of mbar_wait_bounded inlined at
-// every wait the kernel was 70 KB and twice as slow).  2^20 polls are between 10 ms and a few seconds.
+// Kernels that move registers between warps (setmaxnreg) cannot have calls, and the roles' loops together have to stay in
+// the instruction cache: with the timer of mbar_wait_bounded inlined at every wait the kernel was 70 KB and twice as slow.
 __device__ __forceinline__ bool mbar_wait_polls(uint32_t bar, uint32_t parity, int* status, int bit) {
-#pragma unroll 1
-    for (int i = 0; i < (1 << 20); ++i)
-        if (mbar_try_wait(bar, parity)) return true;
-    if (status) atomicOr(status, bit);
-    return false;
+    const bool ok = wait_polls(bar, parity);
+    if (!ok && status) atomicOr(status, bit);
+    return ok;
 }
 // bar.red over the two warps on hardware barrier `id`: is `x` true in any of their threads
 __device__ __forceinline__ bool pair_any(int id, bool x) {

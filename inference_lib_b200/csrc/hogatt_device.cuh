@@ -212,6 +212,15 @@ __device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, volat
     return true;
 }
 
+// A bounded wait of a few instructions and without a call, for kernels that cannot have calls or must stay small: 2^20 polls
+// are between 10 ms and a few seconds.
+__device__ __forceinline__ bool wait_polls(uint32_t bar, uint32_t parity) {
+#pragma unroll 1
+    for (int i = 0; i < (1 << 20); ++i)
+        if (mbar_try_wait(bar, parity)) return true;
+    return false;
+}
+
 // Programmatic dependent launch: a kernel launched with the "programmatic stream serialization"
 // attribute may start while its predecessor in the stream is still running; it must call
 // pdl_wait() before it touches anything the predecessor reads or writes.  pdl_trigger() lets the

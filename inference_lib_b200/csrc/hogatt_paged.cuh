@@ -192,28 +192,36 @@ __global__ void __launch_bounds__(kFmaThreads) paged_attention_kernel(const __gr
 
 // ---- tensor-core paged kernel (f16 / bf16, E = Ev = 64 or 128) --------------------------------------------------
 // Same units, splits, partial format and merge as paged_attention_kernel; what differs is the tile core: a tile is
-// 64 keys, fetched row by row through the block table with 16-byte cp.async copies into a two-stage ring (rows past
-// the tile's end are zero-filled by the copy itself), and the four warps each take 16 keys of it:
-// S = Q K^T and O += P V with mma.sync m16n8k16 (query rows are the M of both), online softmax in base 2 in
-// registers, P handed from the first MMA's accumulators to the second's A operand without leaving the registers.
-// At the end the four warps' (O, max, sum) are folded through shared memory into the one partial the split leaves.
+// 64 keys and the four warps each take 16 of them: S = Q K^T and O += P V with mma.sync m16n8k16 (query rows are the M of
+// both), online softmax in base 2 in registers, P handed from the first MMA's accumulators to the second's A operand
+// without leaving the registers.  At the end the four warps' (O, max, sum) are folded through shared memory into the one
+// partial the split leaves.
+// How a tile comes in (BULK): where the cache's blocks are whole runs of 8 rows (block_size a multiple of 8), 16 lanes of a
+// fifth warp issue one bulk copy each -- 8 consecutive rows of K or V -- into a ring of three; they look the next tile's
+// blocks up while this one's copies go out (with the lookup in front of the copies, on a warp that also computes, a tile
+// took 1.6 us).  Keys lie in 8 groups of 8 with 16 bytes between groups, a warp's 16 keys are positions 2w and 2w + 1 of
+// all groups, and the 8 rows of an ldmatrix phase fall into 8 bank groups.  Other block sizes go row by row with 16-byte cp.async
+// copies of all threads into a ring of two (rows past the tile's end zero-filled by the copy), padded rows, consecutive keys.
 // Replaces the CUDA-core loops of src/kernels/kernel_v21.cuh:318-602 (paged) and :658-949 (varlen paged).
-template <int HD, int NS = 2>
+template <int HD, bool BULK>
 struct PagedMmaCfg {
-    static constexpr int TILE = 64, WARPS = 4, THREADS = WARPS * 32, NSTAGE = NS;
-    static constexpr int PITCH = HD * 2 + 16;                    // bytes between staged rows: 8 consecutive rows hit 8 bank groups
+    static constexpr int TILE = 64, WARPS = 4, CONSUMERS = WARPS * 32, NSTAGE = BULK ? 3 : 2;
+    static constexpr int THREADS = CONSUMERS + (BULK ? 32 : 0);
+    static constexpr int PITCH = HD * 2 + 16;                    // bytes between staged rows (queries; K and V row by row)
+    static constexpr int GROUP_STRIDE = 8 * HD * 2 + 16;         // (BULK) bytes between groups of 8 keys
     static constexpr int QBYTES = kFmaRows * PITCH;
     static constexpr int OFF_LIM = QBYTES;                       // int[16]: visibility limit per query row
-    static constexpr int OFF_STAGE = (QBYTES + 64 + 127) / 128 * 128;
-    static constexpr int KV_BYTES = TILE * PITCH;                // K (or V) rows of one tile
+    static constexpr int OFF_BAR = OFF_LIM + 64;                 // full and empty barriers of the stages
+    static constexpr int OFF_STAGE = (OFF_BAR + 2 * NSTAGE * 8 + 127) / 128 * 128;
+    static constexpr int KV_BYTES = BULK ? 8 * GROUP_STRIDE : TILE * PITCH;                // K (or V) rows of one tile
     static constexpr int STAGE_BYTES = 2 * KV_BYTES;
     static constexpr int OFF_PLAN = OFF_STAGE + NSTAGE * STAGE_BYTES;       // int vis[F], pre[F + 1]
     static constexpr int FOLD_FLOATS = kFmaRows * HD + 2 * kFmaRows;        // per warp: O, max, sum
     static_assert(WARPS * FOLD_FLOATS * 4 <= NSTAGE * STAGE_BYTES, "the fold reuses the K/V ring");
 };
-template <int HD, int NS = 2>
+template <int HD, bool BULK>
 __host__ __device__ inline size_t paged_mma_smem_bytes(int F) {
-    return PagedMmaCfg<HD, NS>::OFF_PLAN + ((size_t)2 * F + 1) * sizeof(int);
+    return PagedMmaCfg<HD, BULK>::OFF_PLAN + ((size_t)2 * F + 1) * sizeof(int);
 }
 
 __device__ __forceinline__ void cp_async_16(uint32_t dst, const void* src, bool real) {
@@ -224,9 +232,9 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-template <class T, int HD, int NS = 2>
-__global__ void __launch_bounds__(PagedMmaCfg<HD, NS>::THREADS) paged_mma_kernel(const __grid_constant__ PagedArgs a) {
-    using C = PagedMmaCfg<HD, NS>;
+template <class T, int HD, bool BULK>
+__global__ void __launch_bounds__(PagedMmaCfg<HD, BULK>::THREADS) paged_mma_kernel(const __grid_constant__ PagedArgs a) {
+    using C = PagedMmaCfg<HD, BULK>;
     constexpr int KSTEPS = HD / 16, NT_O = HD / 8, CPR = HD / 8;     // k-steps of QK^T, n-tiles of O, 16-byte chunks per row
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -235,6 +243,15 @@ __global__ void __launch_bounds__(PagedMmaCfg<HD, NS>::THREADS) paged_mma_kernel
     unsigned char* stages = smem_raw + C::OFF_STAGE;
     int* vis = reinterpret_cast<int*>(smem_raw + C::OFF_PLAN);
     int* pre = vis + a.F;
+    const uint32_t bars = smem_u32(smem_raw + C::OFF_BAR);
+    if (BULK && tid == 0) {
+        for (int k = 0; k < C::NSTAGE; ++k) {
+            mbar_init(bars + 8 * k, 1);
+            mbar_init(bars + 8 * (C::NSTAGE + k), C::WARPS);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        fence_proxy_async_smem();
+    }
 
     // Launched with programmatic stream serialization: wait for the stream's earlier work before anything is read,
     // then let the merge kernel take its place on the SMs (it waits for this whole grid itself).
@@ -272,6 +289,40 @@ __global__ void __launch_bounds__(PagedMmaCfg<HD, NS>::THREADS) paged_mma_kernel
     __syncthreads();
     const int T_u = pre[a.F];
     const int t0 = (int)((int64_t)split * T_u / a.splits), t1 = (int)((int64_t)(split + 1) * T_u / a.splits);
+
+    if (BULK && warp == C::WARPS) {
+        // ---- copies: lane g + 8 v takes group g of K (v = 0) or V ----
+        int f = 0, stage = 0, ntok = 0, ntok_next = 0;
+        uint32_t phase = 1;                                         // the first round finds every stage free
+        long long row = 0, row_next = 0;
+        auto look_up = [&](int t) {                                 // first row of this lane's group of tile t
+            while (t >= pre[f + 1]) ++f;
+            const int tok0 = (t - pre[f]) * C::TILE;
+            ntok_next = min(C::TILE, vis[f] - tok0);
+            // (a length beyond the block table is the caller's error; the lookup stays inside the table regardless)
+            const int l = tok0 + min((lane & 7) * 8, ntok_next - 1), blk = l / a.block_size;
+            row_next = ((long long)table[min(blk, a.max_blocks - 1)] * a.Hkv + u.hkv) * a.block_size + (l - blk * a.block_size);
+        };
+        if (t0 < t1) look_up(t0);
+#pragma unroll 1
+        for (int t = t0; t < t1; ++t) {
+            row = row_next;
+            ntok = ntok_next;
+            if (t + 1 < t1) look_up(t + 1);
+            const int rows = min(8, ntok - (lane & 7) * 8);
+            if (!__all_sync(0xffffffffu, wait_polls(bars + 8 * (C::NSTAGE + stage), phase))) break;
+            if (lane == 0) mbar_arrive_expect_tx(bars + 8 * stage, (uint32_t)ntok * HD * 4);
+            __syncwarp();
+            if (lane < 16 && rows > 0)
+                bulk_load(smem_u32(stages + stage * C::STAGE_BYTES) + (lane >> 3) * C::KV_BYTES + (lane & 7) * C::GROUP_STRIDE,
+                          (lane < 8 ? kc : vc) + row * HD, (uint32_t)rows * HD * 2, bars + 8 * stage);
+            if (++stage == C::NSTAGE) {
+                stage = 0;
+                phase ^= 1u;
+            }
+        }
+        return;
+    }
 
     // One tile's rows into a stage.  The copies are dealt as pass k = 0 .. NP-1 of RP rows, a thread takes chunk
     // lane % CPR of row (tid / CPR) + k * RP; a warp therefore touches 16 distinct rows of the tile, and lane j < 16
@@ -311,24 +362,29 @@ __global__ void __launch_bounds__(PagedMmaCfg<HD, NS>::THREADS) paged_mma_kernel
     uint32_t qf[KSTEPS][4];
     int lim0 = 0, lim1 = 0, cur_f = -1, fscan = 0;
     // the ring: tiles t .. t + NSTAGE - 2 are in flight while tile t is used (one commit group per tile, empty past the end)
+    if constexpr (!BULK) {
 #pragma unroll
-    for (int k = 0; k < C::NSTAGE - 1; ++k) {
-        if (t0 + k < t1) fetch(t0 + k, k, 0);
-        else cp_async_commit();
+        for (int k = 0; k < C::NSTAGE - 1; ++k) {
+            if (t0 + k < t1) fetch(t0 + k, k, 0);
+            else cp_async_commit();
+        }
     }
 #pragma unroll 1
     for (int t = t0, it = 0; t < t1; ++t, ++it) {
         while (t >= pre[fscan + 1]) ++fscan;
         const int f = fscan;
-        cp_async_wait<C::NSTAGE - 2>();                             // this thread's copies of tile t have landed
-        __syncthreads();                                            // everyone's have, and everyone has left tile t - 1
-        if (t + C::NSTAGE - 1 < t1) fetch(t + C::NSTAGE - 1, (it + C::NSTAGE - 1) % C::NSTAGE, fscan);   // into tile t - 1's stage
-        else cp_async_commit();
+        if constexpr (!BULK) {
+            cp_async_wait<C::NSTAGE - 2>();                         // this thread's copies of tile t have landed
+            __syncthreads();                                        // everyone's have, and everyone has left tile t - 1
+            if (t + C::NSTAGE - 1 < t1) fetch(t + C::NSTAGE - 1, (it + C::NSTAGE - 1) % C::NSTAGE, fscan);   // into tile t - 1's stage
+            else cp_async_commit();
+        }
         if (f != cur_f) {
             // this fragment's query rows (already rotated) and their limits; the query tile is only read right after
             // it is written (the A fragments stay in registers), and a barrier has passed since
             cur_f = f;
-            for (int i = tid; i < kFmaRows * CPR; i += C::THREADS) {
+            if (BULK && it > 0) named_barrier_sync(1, C::CONSUMERS);        // (everyone has read the limits and queries before)
+            for (int i = tid; i < kFmaRows * CPR; i += C::CONSUMERS) {
                 const int r = i / CPR, c = i - r * CPR;
                 int s_abs, hq;
                 uint4 val = make_uint4(0u, 0u, 0u, 0u);
@@ -345,7 +401,7 @@ __global__ void __launch_bounds__(PagedMmaCfg<HD, NS>::THREADS) paged_mma_kernel
                 }
                 lim_s[tid] = lim;
             }
-            __syncthreads();
+            named_barrier_sync(1, C::CONSUMERS);
             const uint32_t qaddr = smem_u32(qtile) + ((lane & 7) + ((lane >> 3) & 1) * 8) * C::PITCH + (lane >> 4) * 16;
 #pragma unroll
             for (int kk = 0; kk < KSTEPS; ++kk) ldmatrix_x4(qaddr + kk * 32, qf[kk][0], qf[kk][1], qf[kk][2], qf[kk][3]);
@@ -355,10 +411,29 @@ __global__ void __launch_bounds__(PagedMmaCfg<HD, NS>::THREADS) paged_mma_kernel
 
         const int tok0 = (t - pre[f]) * C::TILE;
         const uint32_t sk = smem_u32(stages + (it % C::NSTAGE) * C::STAGE_BYTES), sv = sk + C::KV_BYTES;
-        const int kw0 = warp * 16;                                  // this warp's 16 keys of the tile
+        const int kw0 = warp * 16;                                  // this warp's 16 keys of the tile (row by row)
+        if constexpr (BULK) {
+            // (a wait that runs out leaves a void result, never a hung CTA; the status word is the fragment calls')
+            wait_polls(bars + 8 * (it % C::NSTAGE), (uint32_t)(it / C::NSTAGE) & 1u);
+            const int ntok = vis[f] - tok0;
+            if (ntok < C::TILE) {
+                // the copies wrote nothing past the tile's end: probabilities there are exactly zero, but 0 * NaN would
+                // poison the sums, so this warp's V rows there are made finite
+                for (int i = lane; i < 16 * CPR; i += 32) {
+                    const int x = i / CPR, key = (x & 7) * 8 + warp * 2 + (x >> 3);
+                    if (key >= ntok)
+                        *reinterpret_cast<uint4*>(stages + (it % C::NSTAGE) * C::STAGE_BYTES + C::KV_BYTES + (x & 7) * C::GROUP_STRIDE +
+                                                  (warp * 2 + (x >> 3)) * HD * 2 + (i % CPR) * 16) = make_uint4(0u, 0u, 0u, 0u);
+                }
+                fence_proxy_async_smem();                           // (a later copy may land where these were written)
+                __syncwarp();
+            }
+        }
         float s[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
         {
-            const uint32_t kaddr = sk + (kw0 + (lane & 7) + ((lane >> 4) & 1) * 8) * C::PITCH + ((lane >> 3) & 1) * 16;
+            const uint32_t kaddr = sk + ((lane >> 3) & 1) * 16 +
+                                   (BULK ? (lane & 7) * C::GROUP_STRIDE + (warp * 2 + ((lane >> 4) & 1)) * HD * 2
+                                         : (kw0 + (lane & 7) + ((lane >> 4) & 1) * 8) * C::PITCH);
 #pragma unroll
             for (int kk = 0; kk < KSTEPS; ++kk) {
                 uint32_t b0, b1, b2, b3;
@@ -368,13 +443,14 @@ __global__ void __launch_bounds__(PagedMmaCfg<HD, NS>::THREADS) paged_mma_kernel
             }
         }
         // mask, online softmax (base 2); a key is visible to a row iff its index is below the row's limit
-        const int key0 = tok0 + kw0 + (lane & 3) * 2;
+        // (n-tile j, column n: key n + 8 j of the warp's 16 -- in groups, position j of group n)
+        const int key0 = BULK ? tok0 + (lane & 3) * 16 + warp * 2 : tok0 + kw0 + (lane & 3) * 2;
         float mx0 = -INFINITY, mx1 = -INFINITY;
 #pragma unroll
         for (int j = 0; j < 2; ++j)
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
-                const int key = key0 + j * 8 + i;
+                const int key = key0 + (BULK ? j + i * 8 : j * 8 + i);
                 s[j][i] = key < lim0 ? s[j][i] * a.l2scale : -INFINITY;
                 s[j][2 + i] = key < lim1 ? s[j][2 + i] * a.l2scale : -INFINITY;
                 mx0 = fmaxf(mx0, s[j][i]);
@@ -409,7 +485,9 @@ __global__ void __launch_bounds__(PagedMmaCfg<HD, NS>::THREADS) paged_mma_kernel
         pa[2] = pack2<T>(s[1][0], s[1][1]);
         pa[3] = pack2<T>(s[1][2], s[1][3]);
         {
-            const uint32_t vaddr = sv + (kw0 + (lane & 7) + ((lane >> 3) & 1) * 8) * C::PITCH + ((lane >> 4) & 1) * 16;
+            const uint32_t vaddr = sv + ((lane >> 4) & 1) * 16 +
+                                   (BULK ? (lane & 7) * C::GROUP_STRIDE + (warp * 2 + ((lane >> 3) & 1)) * HD * 2
+                                         : (kw0 + (lane & 7) + ((lane >> 3) & 1) * 8) * C::PITCH);
 #pragma unroll
             for (int n = 0; n < NT_O; n += 2) {
                 uint32_t b0, b1, b2, b3;
@@ -422,8 +500,12 @@ __global__ void __launch_bounds__(PagedMmaCfg<HD, NS>::THREADS) paged_mma_kernel
                 mma_16816<T>(o[n + 1], pa, b2, b3);
             }
         }
+        if constexpr (BULK) {
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bars + 8 * (C::NSTAGE + it % C::NSTAGE));
+        }
     }
-    __syncthreads();                                                // every warp has left the last tile: the ring is free
+    named_barrier_sync(1, C::CONSUMERS);                            // every warp has left the last tile: the ring is free
 
     // ---- fold the four warps' results into the split's partial -------------------------------------------------
     l0 += __shfl_xor_sync(0xffffffffu, l0, 1);
@@ -445,10 +527,10 @@ __global__ void __launch_bounds__(PagedMmaCfg<HD, NS>::THREADS) paged_mma_kernel
             fold[kFmaRows * HD + kFmaRows + r0 + 8] = l1;
         }
     }
-    __syncthreads();
+    named_barrier_sync(1, C::CONSUMERS);
     const float* all = reinterpret_cast<const float*>(stages);
     const size_t slot = (size_t)blockIdx.x * a.splits + split;
-    for (int i = tid; i < kFmaRows * (HD / 4); i += C::THREADS) {
+    for (int i = tid; i < kFmaRows * (HD / 4); i += C::CONSUMERS) {
         const int r = i / (HD / 4), c = (i - r * (HD / 4)) * 4;
         float M = -INFINITY;
 #pragma unroll
