@@ -14,7 +14,7 @@
 #include "hogatt_mma.cuh"
 #include "hogatt_paged.cuh"
 #include "hogatt_cache.cuh"
-#include "hogatt_dense.cuh"
+#include "hogatt_dense_tile.cuh"
 
 #include <mutex>
 #include <unordered_map>
@@ -245,23 +245,31 @@ void carve_dense(WorkspaceLayout* w, int64_t blocks, int Hkv, int F, int grid, b
     w->total = w->rq;
 }
 
+size_t rotated_bytes(const hogatt_problem* p) {
+    return align_up((size_t)p->F * p->W * p->Hq * p->S * p->E * dtype_size(p->dtype), 256);
+}
+
+// The layout of a fragment call on the tcgen05 kernel of two query tiles per block.
+WorkspaceLayout carve_pairs(const hogatt_problem* p, int grid) {
+    WorkspaceLayout w = {};
+    int tiles, span, tokens;
+    dense_geometry(p->W, p->Hq / p->Hkv, p->S, &tiles, &span, &tokens);
+    carve_dense(&w, (tiles + 1) / 2, p->Hkv, p->F, std::min(grid, kDenseMaxCtas), false);
+    w.total += rotated_bytes(p);
+    return w;
+}
+
 WorkspaceLayout carve(const hogatt_problem* p, const Resolved& r, int grid) {
     WorkspaceLayout w = {};
-    if (r.kernel == HOGATT_KERNEL_DENSE) {
-        int tiles, span, tokens;
-        dense_geometry(p->W, p->Hq / p->Hkv, p->S, &tiles, &span, &tokens);
-        carve_dense(&w, (tiles + 1) / 2, p->Hkv, p->F, grid, false);
-        // the tcgen05 kernel reads rotated queries from memory: room for them in case the caller does not want them back
-        w.total += align_up((size_t)p->F * p->W * p->Hq * p->S * p->E * dtype_size(p->dtype), 256);
-        return w;
-    }
     w.parts = max_parts_per_unit(r.units, grid);
     const size_t slots = (size_t)r.units * w.parts * r.rows_per_block;
     w.header = 0;
     w.o = 256;
     w.m = w.o + align_up(slots * p->Ev * sizeof(float), 256);
     w.l = w.m + align_up(slots * sizeof(float), 256);
-    w.total = w.l + align_up(slots * sizeof(float), 256);
+    w.rq = w.l + align_up(slots * sizeof(float), 256);
+    // the tcgen05 kernels read rotated queries from memory: room for them in case the caller does not want them back
+    w.total = w.rq + (r.kernel == HOGATT_KERNEL_DENSE ? rotated_bytes(p) : 0);
     return w;
 }
 
@@ -281,6 +289,18 @@ int64_t tiles_upper_bound(const hogatt_problem* p, const Resolved& r) {
         th += ceil_div(rows, r.tile_tokens);
     }
     return th;
+}
+
+// Which tcgen05 kernel a call of at least 128 query rows per kv head runs on.  Blocks of two query tiles where they give every
+// CTA a step and do not fall apart into many partials each, unless the work is long enough to carry that (figures in
+// hogatt_dense_tile.cuh; two units cut into 74 parts each, 16,100 keys: 35 us against 27; one unit, 131,000 keys, 7 steps a
+// CTA: 52 against 44).  One tile per unit otherwise, and where the workspace is too small for the partials of the other (a
+// caller's fixed one).
+bool dense_pairs(const hogatt_problem* p, const Resolved& r, int grid) {
+    if (r.kernel != HOGATT_KERNEL_DENSE || r.row_blocks < 2) return false;
+    const int64_t units = (int64_t)((r.row_blocks + 1) / 2) * p->Hkv, steps = units * tiles_upper_bound(p, r);
+    if (steps < grid || (8 * units < grid && steps < 16 * (int64_t)grid)) return false;
+    return p->workspace_bytes >= carve_pairs(p, grid).total;
 }
 
 // How many query rows a CTA of the mma.sync kernel keeps (16, 32 or 64): resolve() takes the smallest block that
@@ -691,8 +711,14 @@ int launch_dense_kernels(const DenseArgs& d, const DenseMaps& maps, int dev, int
     if (rc != HOGATT_OK) return rc;
     HOGATT_CUDA_OK(launch_kernel(dense_attention_kernel<T, PAGED>, dim3(d.ctas), dim3(kDenseThreads), kDenseSmemBytes, stream, d, maps));
     // at most ctas - 1 units are split; more on the list are blocks of one tile or blind ones (the kernel walks the list)
-    const dim3 grid((unsigned)std::min<int64_t>((int64_t)d.blocks * d.Hkv, 2 * (int64_t)d.ctas), kDenseBlock / 32, 128 / (16 * kDenseMergeWarps));
-    HOGATT_CUDA_OK(launch_kernel(dense_merge_kernel<T, PAGED>, grid, dim3(kDenseMergeWarps * 32), 0, stream, d));
+    const int64_t units = (int64_t)d.blocks * d.Hkv;
+    const unsigned gx = (unsigned)std::min<int64_t>(units, 2 * (int64_t)d.ctas);
+    if (d.ctas > 8 * units)
+        HOGATT_CUDA_OK(launch_kernel(dense_merge_kernel<T, PAGED, kDenseMergeSplit>, dim3(gx, kDenseBlock / 32, 128 / 16),
+                                     dim3(kDenseMergeSplit * 32), 0, stream, d));
+    else
+        HOGATT_CUDA_OK(launch_kernel(dense_merge_kernel<T, PAGED, 1>, dim3(gx, kDenseBlock / 32, 128 / (16 * kDenseMergeWarps)),
+                                     dim3(kDenseMergeWarps * 32), 0, stream, d));
     return HOGATT_OK;
 }
 
@@ -762,9 +788,39 @@ int launch_dense(const hogatt_problem* p, const KernelArgs& args, const Workspac
 }
 
 template <class T>
-int launch_all(const KernelArgs& args, const Resolved& r, int dev, int smem_optin, int grid, cudaStream_t stream) {
+int launch_dense_tile(const KernelArgs& args, const void* q_rot, int dtype, int dev, int smem_optin, int grid, cudaStream_t stream) {
+    static std::atomic<size_t> granted[kMaxDevices];
+    const size_t smem = tile_smem_bytes(args.F);
+    if (smem > (size_t)smem_optin) return HOGATT_ERR_TOO_MANY_FRAGMENTS;
+    int rc = ensure_smem_limit(tile_attention_kernel<T>, dev, smem, granted);
+    if (rc != HOGATT_OK) return rc;
+    TileMaps maps;
+    memset(&maps, 0, sizeof(maps));
+    for (int f = 0; f < args.F; ++f) {
+        if (args.ft.e[f].rows == 0) continue;             // never addressed: no tile lies in an empty fragment
+        rc = fragment_map(args.ft.e[f].k, args.ft.e[f].rows, args.Hkv, dtype, &maps.k[f]);
+        if (rc == HOGATT_OK) rc = fragment_map(args.ft.e[f].v, args.ft.e[f].rows, args.Hkv, dtype, &maps.v[f]);
+        if (rc != HOGATT_OK) return rc;
+    }
+    {   // rotated queries [F, W, Hq, S, E] seen as [F, W, Hkv, G*S, E]; a 128-row block is one box
+        const int gs = args.G * args.S;
+        const cuuint64_t dims[5] = {128, (cuuint64_t)gs, (cuuint64_t)args.Hkv, (cuuint64_t)args.W, (cuuint64_t)args.F};
+        const cuuint32_t box[5] = {64, (cuuint32_t)std::min(gs, kDenseRows), 1, (cuuint32_t)(gs < kDenseRows ? kDenseRows / gs : 1), 1};
+        rc = encode_map(&maps.q, q_rot, dtype, 5, dims, box);
+        if (rc != HOGATT_OK) return rc;
+    }
+    tile_attention_kernel<T><<<dim3(grid), dim3(kTileThreads), smem, stream>>>(args, maps);
+    HOGATT_CUDA_OK(cudaGetLastError());
+    return HOGATT_OK;
+}
+
+template <class T>
+int launch_all(const KernelArgs& args, const Resolved& r, int dev, int smem_optin, int grid, cudaStream_t stream,
+               const void* q_rot = nullptr) {
     int rc;
-    if (r.kernel == HOGATT_KERNEL_MMA) {
+    if (r.kernel == HOGATT_KERNEL_DENSE) {
+        rc = launch_dense_tile<T>(args, q_rot, std::is_same<T, __half>::value ? HOGATT_F16 : HOGATT_BF16, dev, smem_optin, grid, stream);
+    } else if (r.kernel == HOGATT_KERNEL_MMA) {
         bool ef = r.row_blocks == 1;             // every K/V byte is read once: do not let it displace L2 contents
 #ifdef HOGATT_EXPERIMENT
         if (getenv("HOGATT_STREAM_ONLY")) return launch_mma_dims<T>(args, args.F, args.E, r.mt, dev, smem_optin,
@@ -784,7 +840,8 @@ int launch_all(const KernelArgs& args, const Resolved& r, int dev, int smem_opti
 }
 
 template <>
-int launch_all<float>(const KernelArgs& args, const Resolved& r, int dev, int smem_optin, int grid, cudaStream_t stream) {
+int launch_all<float>(const KernelArgs& args, const Resolved& r, int dev, int smem_optin, int grid, cudaStream_t stream,
+                      const void*) {
     int rc = launch_f32_dims(args, dev, smem_optin, grid, stream);
     if (rc != HOGATT_OK) return rc;
     return launch_merge<float>(args, r, stream);
@@ -890,16 +947,25 @@ int attention_launch(const hogatt_problem* p, bool fused, cudaStream_t stream, c
         args.stable_fragments = pdl_enabled() ? std::max(0, std::min(p->F, p->stable_fragments)) : 0;
     }
 
-    const bool dense = r.kernel == HOGATT_KERNEL_DENSE;
+    const bool pairs = dense_pairs(p, r, grid);
+    // The tcgen05 kernels take their queries already rotated, from memory: the rotated-query output of the call (or
+    // room in the workspace when the caller does not want it) is written by the stand-alone rotation kernel first.
+    const void* q_rot = p->queries;
+    if (r.kernel == HOGATT_KERNEL_DENSE && fused && !pairs) {
+        void* dst = p->rq ? p->rq : static_cast<void*>(ws + w.rq);
+        rc = rope_launch(dst, p->queries, p->cosines, p->sines, p->F, p->W, p->Hq, p->S, p->E, p->rotary_dim, p->dtype, stream);
+        if (rc != HOGATT_OK) return rc;
+        q_rot = dst;
+    }
     switch (p->dtype) {
-        case HOGATT_F32: rc = launch_all<float>(args, r, dev, smem_optin, grid, stream); break;
+        case HOGATT_F32: rc = launch_all<float>(args, r, dev, smem_optin, grid, stream, nullptr); break;
         case HOGATT_F16:
-            rc = dense ? launch_dense<__half>(p, args, w, fused, dev, smem_optin, grid, stream)
-                       : launch_all<__half>(args, r, dev, smem_optin, grid, stream);
+            rc = pairs ? launch_dense<__half>(p, args, carve_pairs(p, grid), fused, dev, smem_optin, grid, stream)
+                       : launch_all<__half>(args, r, dev, smem_optin, grid, stream, q_rot);
             break;
         case HOGATT_BF16:
-            rc = dense ? launch_dense<__nv_bfloat16>(p, args, w, fused, dev, smem_optin, grid, stream)
-                       : launch_all<__nv_bfloat16>(args, r, dev, smem_optin, grid, stream);
+            rc = pairs ? launch_dense<__nv_bfloat16>(p, args, carve_pairs(p, grid), fused, dev, smem_optin, grid, stream)
+                       : launch_all<__nv_bfloat16>(args, r, dev, smem_optin, grid, stream, q_rot);
             break;
         default: return HOGATT_ERR_UNSUPPORTED_DTYPE;
     }
@@ -924,15 +990,17 @@ struct PagedPlan {
 
 // Packed queries on the tcgen05 kernel: 16-bit types, head size 128, cache blocks that tile a 128-key tile in whole
 // 8-row swizzle groups (or hold whole tiles), the number of blocks known (a tensor map needs the extent).  AUTO takes it
-// when the prompt chunks of the batch -- the tokens beyond one per sequence -- fill at least one 128-row tile per kv
-// head: the mma.sync kernel reads every sequence once per 16 rows.
+// when the prompt chunks of the batch -- the tokens beyond one per sequence -- fill at least four 128-row tiles per kv
+// head: the mma.sync kernel reads every sequence once per 16 rows (two chunks of 512 tokens at 6,000 keys: 813 us against
+// 119), but has some 12 us less before and after (a chunk of 64 tokens beside one sequence, 600 keys: 19 against 30; two of
+// 64 beside six: 36 against 34).
 bool paged_dense_wanted(const hogatt_paged_problem* p) {
     if (p->kernel != HOGATT_KERNEL_AUTO || p->cu_seqlens_q == nullptr || dense_disabled() || p->num_blocks <= 0) return false;
     if ((p->dtype != HOGATT_F16 && p->dtype != HOGATT_BF16) || p->E != 128 || p->Ev != 128) return false;
     const int G = p->Hq / p->Hkv, bs = p->block_size;
     if (G > kDenseRows || !(bs % kDenseTile == 0 || (kDenseTile % bs == 0 && bs % 8 == 0))) return false;
     if ((int64_t)p->total_q_tokens * p->Hq * p->F >= ((int64_t)1 << 31)) return false;
-    return ((int64_t)p->total_q_tokens - p->W) * G >= kDenseRows;
+    return ((int64_t)p->total_q_tokens - p->W) * G >= 4 * kDenseRows;
 }
 
 int plan_paged(const hogatt_paged_problem* p, int sms, PagedPlan* pl) {
@@ -1031,26 +1099,32 @@ bool paged_mma_disabled() {
     return off;
 }
 
-template <class T, int HD, bool BULK>
+template <class T, int HD, bool BULK, int NS>
 int launch_paged_mma(const PagedArgs& a, const PagedPlan& pl, int dev, int smem_optin, cudaStream_t stream) {
     static std::atomic<size_t> granted[kMaxDevices];
-    const size_t smem = paged_mma_smem_bytes<HD, BULK>(a.F);
+    const size_t smem = paged_mma_smem_bytes<HD, BULK, NS>(a.F);
     if (smem > (size_t)smem_optin) return HOGATT_ERR_TOO_MANY_FRAGMENTS;
-    int rc = ensure_smem_limit(paged_mma_kernel<T, HD, BULK>, dev, smem, granted);
+    int rc = ensure_smem_limit(paged_mma_kernel<T, HD, BULK, NS>, dev, smem, granted);
     if (rc != HOGATT_OK) return rc;
-    HOGATT_CUDA_OK(launch_kernel(paged_mma_kernel<T, HD, BULK>, dim3(pl.units, a.splits), dim3(PagedMmaCfg<HD, BULK>::THREADS), smem, stream, a));
+    HOGATT_CUDA_OK(launch_kernel(paged_mma_kernel<T, HD, BULK, NS>, dim3(pl.units, a.splits), dim3(PagedMmaCfg<HD, BULK, NS>::THREADS), smem, stream, a));
     HOGATT_CUDA_OK(launch_kernel(paged_merge_kernel<T>, dim3(pl.units, kFmaRows / kMergeWarps), dim3(kMergeWarps * 32), 0, stream, a));
     return HOGATT_OK;
 }
 
-// Bulk copies need runs of 8 rows.  Their ring of three leaves room for two CTAs per SM at head size 128 (at 64: three of four): splits
-// that fill them once.  (More fragments than fit beside that ring: row by row, as before.)
+// Bulk copies need runs of 8 rows.  Where every unit has keys of its own (one group of query tokens per sequence) the stream from
+// HBM decides: a ring of three and two CTAs per SM, filled once (8 sequences x 16 K keys over 8 kv heads 96 us; with a ring
+// of two and three CTAs 125, row by row 138).  Where the groups of a prompt chunk share a sequence's keys through L2, three CTAs
+// with a ring of two (34 tokens over 4 sequences of 2,000 keys, GQA 8: 28 us; ring of three 42, row by row 33) -- at head size 64,
+// where a tile is half the bytes and the same work, row by row (467 us against 521 for two chunks of 512 tokens).
 template <class T, int HD>
 int launch_paged_mma_rows(PagedArgs a, const PagedPlan& pl, int dev, int sms, int smem_optin, cudaStream_t stream) {
-    if (a.block_size % 8 != 0 || paged_mma_smem_bytes<HD, true>(a.F) > (size_t)smem_optin)
-        return launch_paged_mma<T, HD, false>(a, pl, dev, smem_optin, stream);
-    a.splits = std::max(1, std::min(pl.splits, (HD == 128 ? 2 : 3) * sms / pl.units));
-    return launch_paged_mma<T, HD, true>(a, pl, dev, smem_optin, stream);
+    const bool own_keys = a.cu_seqlens == nullptr && a.S <= a.tokens_per_group && a.head_blocks == 1 && pl.units <= sms;
+    if (a.block_size % 8 == 0 && own_keys && paged_mma_smem_bytes<HD, true, 3>(a.F) <= (size_t)smem_optin) {
+        a.splits = std::min(pl.splits, (HD == 128 ? 2 : 3) * sms / pl.units);
+        return launch_paged_mma<T, HD, true, 3>(a, pl, dev, smem_optin, stream);
+    }
+    if (HD == 128 && a.block_size % 8 == 0) return launch_paged_mma<T, HD, true, 2>(a, pl, dev, smem_optin, stream);
+    return launch_paged_mma<T, HD, false, 2>(a, pl, dev, smem_optin, stream);
 }
 
 template <class T>
@@ -1132,6 +1206,7 @@ size_t hogatt_workspace_bytes(const hogatt_problem* p) {
     if (current_device_info(&dev, &sms, &smem_optin) != HOGATT_OK) return 0;
     const int grid = grid_size(p, sms);
     size_t need = carve(p, r, grid).total;
+    if (r.kernel == HOGATT_KERNEL_DENSE && r.row_blocks >= 2) need = std::max(need, carve_pairs(p, grid).total);
     if (r.kernel == HOGATT_KERNEL_MMA && !r.cluster_forced) {
         // a launch may cut the query rows into smaller blocks than resolve() did (refine_row_blocks): room for any of them
         const int64_t rows_total = (int64_t)p->W * (p->Hq / p->Hkv) * p->S;
@@ -1163,21 +1238,18 @@ int hogatt_fused_launch_static(const hogatt_problem* p, hogatt_stream_t stream) 
         const int rc = resolve(p, &r);
         return rc != HOGATT_OK ? rc : HOGATT_ERR_CUDA;
     }
-    hogatt_problem q = *p;
     if (need > (size_t)HOGATT_STATIC_SCRATCH_BYTES) {
-        // the tcgen05 kernel needs a slot per CTA: with up to half of the CTAs it may fit
+        // (the tcgen05 kernel that a launch takes when the other one's partials do not fit needs less)
         Resolved r;
         int dev, sms, smem_optin;
-        if (resolve(p, &r) != HOGATT_OK || r.kernel != HOGATT_KERNEL_DENSE) return HOGATT_ERR_EXCEEDS_STATIC_SCRATCH;
-        if (current_device_info(&dev, &sms, &smem_optin) != HOGATT_OK) return HOGATT_ERR_CUDA;
-        const int grid = grid_size(p, sms);
-        q.max_ctas = grid;
-        while (2 * q.max_ctas > grid && carve(&q, r, q.max_ctas).total > (size_t)HOGATT_STATIC_SCRATCH_BYTES) --q.max_ctas;
-        if (q.max_ctas < 1 || 2 * q.max_ctas <= grid) return HOGATT_ERR_EXCEEDS_STATIC_SCRATCH;
+        if (resolve(p, &r) != HOGATT_OK || current_device_info(&dev, &sms, &smem_optin) != HOGATT_OK) return HOGATT_ERR_CUDA;
+        if (r.kernel != HOGATT_KERNEL_DENSE || carve(p, r, grid_size(p, sms)).total > (size_t)HOGATT_STATIC_SCRATCH_BYTES)
+            return HOGATT_ERR_EXCEEDS_STATIC_SCRATCH;
     }
     void* scratch = nullptr;
     const int rc = static_scratch_for_current_device(&scratch);
     if (rc != HOGATT_OK) return rc;
+    hogatt_problem q = *p;
     q.workspace = scratch;
     q.workspace_bytes = HOGATT_STATIC_SCRATCH_BYTES;
     return attention_launch(&q, /*fused=*/true, reinterpret_cast<cudaStream_t>(stream));

@@ -48,7 +48,8 @@ constexpr int kDenseMaxCtas = 256;
 // What the balanced shares count (cycles on B200: a step 2,660, starting and finishing a unit 8,200, a step of a block of one
 // tile, whose two key tiles the short value ring cannot keep coming, 5,000).
 constexpr int kDenseUnitSteps = 3, kDenseSingleSteps = 2;
-constexpr int kDenseMergeWarps = 4;         // warps per CTA of the merge step
+constexpr int kDenseMergeWarps = 4;         // warps per CTA of the merge step, with few partials per row
+constexpr int kDenseMergeSplit = 8;         // ... with many: they share a row's partials
 
 struct alignas(64) DenseMaps {
     CUtensorMap q;                          // rotated queries as [F, W, Hq, S, E] or [F, W, Hkv, G*S, E]; paged: [F, total_q, Hkv, G, E]
@@ -681,9 +682,6 @@ dense_attention_kernel(const __grid_constant__ DenseArgs a, const __grid_constan
     const uint32_t tmem = *tmem_slot;
     pdl_wait();             // rotated queries, plan
     pdl_trigger();
-//TL TLD;
-    //TX TLD; if (warp == 0) {TLG(0, 98); TL(0, 99);}
-    //TC long long c_begin = clock64(), c_end = 0; int c_units = 0, c_segs = 0;
     DenseSegments segs{sbase + C::OFF_SEG, seg_full, seg_empty, 0};
     DenseSegment d;
     bool ok = true;
@@ -815,7 +813,6 @@ dense_attention_kernel(const __grid_constant__ DenseArgs a, const __grid_constan
                             tc_commit(s_full + 8 * g);
                         }
                         __syncwarp();
-                        //TL TL(2, g);
                         g_phase ^= 1u << g;
                         last_g = g;
                         any = true;
@@ -874,7 +871,6 @@ dense_attention_kernel(const __grid_constant__ DenseArgs a, const __grid_constan
                             tc_commit(o_done + 8 * g);
                         }
                         __syncwarp();
-                        //TL TL(3, g);
                         started |= 1u << g;
                     }
                     if (!ok) break;
@@ -909,8 +905,6 @@ dense_attention_kernel(const __grid_constant__ DenseArgs a, const __grid_constan
         while (true) {
             const bool more = segs.next(d, lane, a.status);
             if (pair_any(pair_bar, !more)) break;
-            //TC ++c_segs; if (d.first()) ++c_units;
-            //TX if (warp == 0) TL(0, 100);  if (warp == 8) TL(1, 100);
             if (d.first()) {
                 int4 rec = make_int4(0, 0, 0, 0);
                 if constexpr (PAGED) rec = a.rec[d.b];
@@ -927,7 +921,6 @@ dense_attention_kernel(const __grid_constant__ DenseArgs a, const __grid_constan
                 ok = mbar_wait_polls(s_full + 8 * g, phase, a.status, STATUS_WAIT_FULL_TIMEOUT);
                 tc_fence_after();
                 __syncwarp();
-                //TL if (warp == 0) TL(0, 1);  if (warp == 8) TL(1, 1);
                 float s[COLS];
                 tmem_ld32(s_addr, *reinterpret_cast<float(*)[32]>(&s[0]));
                 tmem_ld32(s_addr + 32, *reinterpret_cast<float(*)[32]>(&s[32]));
@@ -935,7 +928,6 @@ dense_attention_kernel(const __grid_constant__ DenseArgs a, const __grid_constan
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(s_free);            // the next S MMA may overwrite the buffer
-                //TL if (warp == 0) TL(0, 2);  if (warp == 8) TL(1, 2);
                 const int nvis = lim - t * kDenseTile - half * COLS;      // of this thread's keys the row sees [0, nvis)
                 float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
                 if (__any_sync(0xffffffffu, nvis < COLS)) {
@@ -947,7 +939,6 @@ dense_attention_kernel(const __grid_constant__ DenseArgs a, const __grid_constan
 #pragma unroll
                     for (int i = 0; i < 4; ++i) mx[i] = max3(mx[i], s[k + 2 * i], s[k + 2 * i + 1]);
                 float mt = max3(fmaxf(mx[0], mx[1]), mx[2], mx[3]);
-                //TL if (warp == 0) TL(0, 3);  if (warp == 8) TL(1, 3);
                 // ---- P and O become writable once this group's previous second MMA has finished ----
                 if (ever) {
                     ok = mbar_wait_polls(o_done + 8 * g, phase ^ 1u, a.status, STATUS_WAIT_SYNC_TIMEOUT) && ok;
@@ -980,7 +971,6 @@ dense_attention_kernel(const __grid_constant__ DenseArgs a, const __grid_constan
                         }
                     }
                 }
-                //TL if (warp == 0) TL(0, 4);  if (warp == 8) TL(1, 4);
                 const float bias = (m_run == -INFINITY) ? 0.f : -m_run * scale2;
                 const uint64_t scale_pair = pair_f32(scale2, scale2), bias_pair = pair_f32(bias, bias);
                 uint64_t sum[2] = {0ull, 0ull};                             // (two fp32 zeros each)
@@ -1005,14 +995,12 @@ dense_attention_kernel(const __grid_constant__ DenseArgs a, const __grid_constan
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(p_full + 8 * g);
-                //TL if (warp == 0) TL(0, 5);  if (warp == 8) TL(1, 5);
                 phase ^= 1u;
                 any = ever = true;
             }
             if (!ok) break;
 
             // ---- end of this CTA's share of the unit: the rows themselves, or a partial result ----
-            //TX if (warp == 0) TL(0, 101);  if (warp == 8) TL(1, 101);
             if (d.last()) {
                 if (any) {
                     ok = mbar_wait_polls(o_done + 8 * g, phase ^ 1u, a.status, STATUS_WAIT_SYNC_TIMEOUT);
@@ -1067,8 +1055,6 @@ dense_attention_kernel(const __grid_constant__ DenseArgs a, const __grid_constan
         }
     }
 
-    //TC if (tid == 0) { c_end = clock64(); g_cta[blockIdx.x][0] = c_end - c_begin; g_cta[blockIdx.x][1] = c_units; g_cta[blockIdx.x][2] = c_segs; g_cta[blockIdx.x][3] = a.start[blockIdx.x].w; }
-    //TX if (warp == 0) { TL(0, 103); TLG(0, 104); } if (warp == 8) TL(1, 103);
     // ---- common exit: nobody leaves before the copies in flight have landed and tensor memory can be handed back ----
     if (!ok && lane == 0 && warp >= W_K) {
         const uint64_t since = global_timer_ns();              // (given up: a pending stage completes its transfer at the latest)
@@ -1083,12 +1069,15 @@ dense_attention_kernel(const __grid_constant__ DenseArgs a, const __grid_constan
 }
 
 // The units on the plan's list -- more than one CTA worked on them, or one left two halves, or nothing is visible --: fold
-// the partials, normalise, store.  Grid (units, 32-row groups, column groups of 64); a warp takes 32 rows, one per lane, and 16
-// columns: every load of a partial is 512 consecutive bytes, a lane stores one 32-byte sector.
+// the partials, normalise, store.  Grid (units, 32-row groups, column groups); a warp takes 32 rows, one per lane, and 16
+// columns: every load of a partial is 512 consecutive bytes, a lane stores one 32-byte sector.  With SPLIT warps per CTA they
+// share the partials of the same rows and columns (a unit cut into a hundred parts would be a chain of as many loads).
 //   out = sum_p O_p * 2^(m_p - M) / sum_p l_p * 2^(m_p - M),   M = max_p m_p
-template <class T, bool PAGED>
-__global__ void __launch_bounds__(kDenseMergeWarps * 32) dense_merge_kernel(const __grid_constant__ DenseArgs a) {
-    const int lane = threadIdx.x & 31, r = blockIdx.y * 32 + lane, c4 = (blockIdx.z * kDenseMergeWarps + (threadIdx.x >> 5)) * 4;
+template <class T, bool PAGED, int SPLIT>
+__global__ void __launch_bounds__((SPLIT > 1 ? SPLIT : kDenseMergeWarps) * 32) dense_merge_kernel(const __grid_constant__ DenseArgs a) {
+    __shared__ float part[SPLIT > 1 ? SPLIT : 1][18][32];                // 16 columns, maximum, sum; by row
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, r = blockIdx.y * 32 + lane;
+    const int c4 = (SPLIT > 1 ? blockIdx.z : blockIdx.z * kDenseMergeWarps + warp) * 4;
     pdl_wait();
     pdl_trigger();
     const int n = *a.nmerge;
@@ -1097,22 +1086,24 @@ __global__ void __launch_bounds__(kDenseMergeWarps * 32) dense_merge_kernel(cons
         const int b = e.x / a.Hkv, h = e.x - b * a.Hkv, count = e.z;
         const bool single = e.w != 0;
         // a block of one tile: both 128-row halves of a slot are partials of the same rows
-        if (single && r >= kDenseRows) continue;
+        if (single && blockIdx.y * 32 >= kDenseRows) continue;
         const int sub = single ? 1 : 0;
         const size_t slot0 = (size_t)e.y + e.x;
-        auto where = [&](int p) { return (slot0 + (p >> sub)) * kDenseBlock + (single ? (p & 1) * kDenseRows : 0) + r; };
+        const int p0 = SPLIT > 1 ? warp : 0;
+        auto row_of = [&](int p) { return (single ? (p & 1) * kDenseRows : 0) + r; };
+        auto slot_of = [&](int p) { return slot0 + (p >> sub); };
         float M = -INFINITY;
 #pragma unroll 4
-        for (int p = 0; p < count; ++p) M = fmaxf(M, __ldcg(a.ws_m + where(p)));
+        for (int p = p0; p < count; p += SPLIT) M = fmaxf(M, __ldcg(a.ws_m + slot_of(p) * kDenseBlock + row_of(p)));
         float den = 0.f;
         float4 acc[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) acc[k] = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 4
-        for (int p = 0; p < count; ++p) {
-            const size_t at = where(p);
+        for (int p = p0; p < count; p += SPLIT) {
+            const size_t at = slot_of(p) * kDenseBlock + row_of(p);
             const float m = __ldcg(a.ws_m + at), l = __ldcg(a.ws_l + at);
-            const float4* src = a.ws_o + (slot0 + (p >> sub)) * (32 * kDenseBlock) + (size_t)c4 * kDenseBlock + (at - (slot0 + (p >> sub)) * kDenseBlock);
+            const float4* src = a.ws_o + (slot_of(p) * 32 + c4) * kDenseBlock + row_of(p);
             const float wgt = m == -INFINITY ? 0.f : exp2f(m - M);       // (a partial that saw nothing holds zeros)
             den = fmaf(l, wgt, den);
 #pragma unroll
@@ -1124,6 +1115,30 @@ __global__ void __launch_bounds__(kDenseMergeWarps * 32) dense_merge_kernel(cons
                 acc[k].w = fmaf(x.w, wgt, acc[k].w);
             }
         }
+        float* o = reinterpret_cast<float*>(acc);
+        if constexpr (SPLIT > 1) {
+            __syncthreads();                             // (the unit before has been read)
+#pragma unroll
+            for (int k = 0; k < 16; ++k) part[warp][k][lane] = o[k];
+            part[warp][16][lane] = M;
+            part[warp][17][lane] = den;
+            __syncthreads();
+            if (warp != 0) continue;
+            float top = M;
+#pragma unroll
+            for (int w = 1; w < SPLIT; ++w) top = fmaxf(top, part[w][16][lane]);
+            const float mine = M == -INFINITY ? 0.f : exp2f(M - top);
+            den *= mine;
+#pragma unroll
+            for (int k = 0; k < 16; ++k) o[k] *= mine;
+#pragma unroll
+            for (int w = 1; w < SPLIT; ++w) {
+                const float mw = part[w][16][lane], wgt = mw == -INFINITY ? 0.f : exp2f(mw - top);
+                den = fmaf(part[w][17][lane], wgt, den);
+#pragma unroll
+                for (int k = 0; k < 16; ++k) o[k] = fmaf(part[w][k][lane], wgt, o[k]);
+            }
+        }
         int4 rec = make_int4(0, 0, 0, 0);
         if constexpr (PAGED) rec = a.rec[b];
         const DenseRow id = dense_row<PAGED>(a, 2 * b + r / kDenseRows, r % kDenseRows, rec);
@@ -1131,12 +1146,9 @@ __global__ void __launch_bounds__(kDenseMergeWarps * 32) dense_merge_kernel(cons
         const float inv = den > 0.f ? 1.f / den : 0.f;
         const size_t offset = dense_out_offset<PAGED>(a, id, h) + c4 * 4;
         uint4 v[2];
-        uint32_t* o = reinterpret_cast<uint32_t*>(v);
+        uint32_t* out = reinterpret_cast<uint32_t*>(v);
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            o[2 * k] = pack2<T>(acc[k].x * inv, acc[k].y * inv);
-            o[2 * k + 1] = pack2<T>(acc[k].z * inv, acc[k].w * inv);
-        }
+        for (int k = 0; k < 8; ++k) out[k] = pack2<T>(o[2 * k] * inv, o[2 * k + 1] * inv);
         for (int p = 0; p < max(a.world, 1); ++p) {
             uint4* dst = reinterpret_cast<uint4*>(static_cast<T*>(a.world > 0 ? a.peer_out[p] : a.out) + offset);
             dst[0] = v[0];

@@ -197,15 +197,15 @@ __global__ void __launch_bounds__(kFmaThreads) paged_attention_kernel(const __gr
 // without leaving the registers.  At the end the four warps' (O, max, sum) are folded through shared memory into the one
 // partial the split leaves.
 // How a tile comes in (BULK): where the cache's blocks are whole runs of 8 rows (block_size a multiple of 8), 16 lanes of a
-// fifth warp issue one bulk copy each -- 8 consecutive rows of K or V -- into a ring of three; they look the next tile's
+// fifth warp issue one bulk copy each -- 8 consecutive rows of K or V -- into a ring of two or three; they look the next tile's
 // blocks up while this one's copies go out (with the lookup in front of the copies, on a warp that also computes, a tile
 // took 1.6 us).  Keys lie in 8 groups of 8 with 16 bytes between groups, a warp's 16 keys are positions 2w and 2w + 1 of
 // all groups, and the 8 rows of an ldmatrix phase fall into 8 bank groups.  Other block sizes go row by row with 16-byte cp.async
 // copies of all threads into a ring of two (rows past the tile's end zero-filled by the copy), padded rows, consecutive keys.
 // Replaces the CUDA-core loops of src/kernels/kernel_v21.cuh:318-602 (paged) and :658-949 (varlen paged).
-template <int HD, bool BULK>
+template <int HD, bool BULK, int NS>
 struct PagedMmaCfg {
-    static constexpr int TILE = 64, WARPS = 4, CONSUMERS = WARPS * 32, NSTAGE = BULK ? 3 : 2;
+    static constexpr int TILE = 64, WARPS = 4, CONSUMERS = WARPS * 32, NSTAGE = NS;
     static constexpr int THREADS = CONSUMERS + (BULK ? 32 : 0);
     static constexpr int PITCH = HD * 2 + 16;                    // bytes between staged rows (queries; K and V row by row)
     static constexpr int GROUP_STRIDE = 8 * HD * 2 + 16;         // (BULK) bytes between groups of 8 keys
@@ -219,9 +219,9 @@ struct PagedMmaCfg {
     static constexpr int FOLD_FLOATS = kFmaRows * HD + 2 * kFmaRows;        // per warp: O, max, sum
     static_assert(WARPS * FOLD_FLOATS * 4 <= NSTAGE * STAGE_BYTES, "the fold reuses the K/V ring");
 };
-template <int HD, bool BULK>
+template <int HD, bool BULK, int NS>
 __host__ __device__ inline size_t paged_mma_smem_bytes(int F) {
-    return PagedMmaCfg<HD, BULK>::OFF_PLAN + ((size_t)2 * F + 1) * sizeof(int);
+    return PagedMmaCfg<HD, BULK, NS>::OFF_PLAN + ((size_t)2 * F + 1) * sizeof(int);
 }
 
 __device__ __forceinline__ void cp_async_16(uint32_t dst, const void* src, bool real) {
@@ -232,9 +232,9 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-template <class T, int HD, bool BULK>
-__global__ void __launch_bounds__(PagedMmaCfg<HD, BULK>::THREADS) paged_mma_kernel(const __grid_constant__ PagedArgs a) {
-    using C = PagedMmaCfg<HD, BULK>;
+template <class T, int HD, bool BULK, int NS>
+__global__ void __launch_bounds__(PagedMmaCfg<HD, BULK, NS>::THREADS, BULK && NS == 2 ? 3 : 1) paged_mma_kernel(const __grid_constant__ PagedArgs a) {
+    using C = PagedMmaCfg<HD, BULK, NS>;
     constexpr int KSTEPS = HD / 16, NT_O = HD / 8, CPR = HD / 8;     // k-steps of QK^T, n-tiles of O, 16-byte chunks per row
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;

@@ -13,10 +13,10 @@ DEV = "cuda:0"
 
 @pytest.mark.parametrize("dtype,G,bs,seqs,lens", [
     (torch.bfloat16, 4, 16, [65, 1, 0, 40, 64], [200, 129, 77, 40, 64]),     # 64 tokens are a block of two tiles
-    (torch.bfloat16, 5, 8, [51, 1, 26], [300, 513, 127]),                    # 25 tokens per tile, 3 rows of it unused
-    (torch.float16, 1, 32, [257, 3], [257, 400]),                            # a tile is 128 tokens
-    (torch.bfloat16, 7, 256, [40, 2], [700, 259]),                           # cache blocks of two key tiles
-    (torch.float16, 128, 64, [3, 1], [90, 256]),                             # a tile is one token
+    (torch.bfloat16, 5, 8, [81, 1, 26], [300, 513, 127]),                    # 25 tokens per tile, 3 rows of it unused
+    (torch.float16, 1, 32, [513, 3], [513, 400]),                            # a tile is 128 tokens
+    (torch.bfloat16, 7, 256, [75, 2], [700, 259]),                           # cache blocks of two key tiles
+    (torch.float16, 128, 64, [5, 1], [90, 256]),                             # a tile is one token
 ])
 @pytest.mark.parametrize("F", [1, 2])
 def test_prompt_chunks_match_the_oracle(dtype, G, bs, seqs, lens, F):
@@ -54,14 +54,14 @@ def test_prompt_chunks_match_the_oracle(dtype, G, bs, seqs, lens, F):
 
 
 def test_which_calls_take_it():
-    """The workspace tells the routes apart: a chunk that fills a 128-row tile beyond one token per sequence, the cache's extent known."""
+    """The workspace tells the routes apart: chunks that fill four 128-row tiles beyond one token per sequence, the cache's extent known."""
     p = _cabi.PagedProblem()
     p.F, p.W, p.Hq, p.Hkv, p.E, p.Ev, p.block_size, p.max_blocks_per_seq = 1, 4, 16, 4, 128, 128, 16, 64
     p.dtype, p.num_blocks, p.cu_seqlens_q = _cabi.BF16, 256, 1
     lib = _cabi.load()
 
     def need(**kw):
-        for k, v in dict(dict(total_q_tokens=36, num_blocks=256, block_size=16, kernel=_cabi.KERNEL_AUTO), **kw).items():
+        for k, v in dict(dict(total_q_tokens=132, num_blocks=256, block_size=16, kernel=_cabi.KERNEL_AUTO), **kw).items():
             setattr(p, k, v)
         return lib.hogatt_paged_workspace_bytes(p)
 
@@ -69,4 +69,4 @@ def test_which_calls_take_it():
     assert need() != general
     for kw in (dict(num_blocks=0), dict(block_size=12), dict(block_size=4)):
         assert need(**kw) == general
-    assert need(total_q_tokens=35) == need(total_q_tokens=35, kernel=_cabi.KERNEL_MMA)
+    assert need(total_q_tokens=131) == need(total_q_tokens=131, kernel=_cabi.KERNEL_MMA)
