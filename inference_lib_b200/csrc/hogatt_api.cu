@@ -990,17 +990,19 @@ struct PagedPlan {
 
 // Packed queries on the tcgen05 kernel: 16-bit types, head size 128, cache blocks that tile a 128-key tile in whole
 // 8-row swizzle groups (or hold whole tiles), the number of blocks known (a tensor map needs the extent).  AUTO takes it
-// when the prompt chunks of the batch -- the tokens beyond one per sequence -- fill at least four 128-row tiles per kv
-// head: the mma.sync kernel reads every sequence once per 16 rows (two chunks of 512 tokens at 6,000 keys: 813 us against
-// 119), but has some 12 us less before and after (a chunk of 64 tokens beside one sequence, 600 keys: 19 against 30; two of
-// 64 beside six: 36 against 34).
+// where the prompt chunks of the batch -- the tokens beyond one per sequence, over as many keys as the block table has room
+// for -- would keep the mma.sync kernel (115 TFLOP/s: it reads every sequence once per 16 rows) busy for some 20 us: the
+// tcgen05 kernel takes 12 us more before and after.  Two chunks of 512 tokens at 6,000 keys: 119 us against 813, one of 300 at
+// 1,000 keys 29 against 71, one of 33 at 6,000 keys 68 against 81; one of 175 over 2 kv heads and 718 keys 27 against 21.
 bool paged_dense_wanted(const hogatt_paged_problem* p) {
     if (p->kernel != HOGATT_KERNEL_AUTO || p->cu_seqlens_q == nullptr || dense_disabled() || p->num_blocks <= 0) return false;
     if ((p->dtype != HOGATT_F16 && p->dtype != HOGATT_BF16) || p->E != 128 || p->Ev != 128) return false;
     const int G = p->Hq / p->Hkv, bs = p->block_size;
     if (G > kDenseRows || !(bs % kDenseTile == 0 || (kDenseTile % bs == 0 && bs % 8 == 0))) return false;
     if ((int64_t)p->total_q_tokens * p->Hq * p->F >= ((int64_t)1 << 31)) return false;
-    return ((int64_t)p->total_q_tokens - p->W) * G >= 4 * kDenseRows;
+    const int64_t tokens = (int64_t)p->total_q_tokens - p->W;
+    if (tokens * G < kDenseRows || tokens * p->Hq < 8 * kDenseRows) return false;
+    return (double)tokens * p->Hq * p->max_blocks_per_seq * bs >= 4.5e6;
 }
 
 int plan_paged(const hogatt_paged_problem* p, int sms, PagedPlan* pl) {

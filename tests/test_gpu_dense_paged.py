@@ -28,6 +28,9 @@ def test_prompt_chunks_match_the_oracle(dtype, G, bs, seqs, lens, F):
     per = max(lens) // bs + 2
     kc, vc = (torch.randn(W * per, Hkv, bs, E, generator=gen).to(dtype) for _ in range(2))
     table = torch.from_numpy(rng.permutation(W * per).astype(np.int32)).reshape(W, per)
+    # (room in the table for the keys that make AUTO take the kernel)
+    columns = max(per, int(4.5e6 / ((total - W) * Hkv * G * bs)) + 1)
+    table = torch.cat([table, torch.zeros(W, columns - per, dtype=torch.int32)], 1).contiguous()
     length = torch.tensor([[max(1, n - 13 * f) for n in lens] for f in range(F)], dtype=torch.int32)
     loc = torch.tensor([[int(length[f, w]) - s + t for w, s in enumerate(seqs) for t in range(s)] for f in range(F)], dtype=torch.int32)
     loc[0, 0] = -1 if F == 2 else loc[0, 0]                                  # a row that sees nothing of one fragment
@@ -54,19 +57,23 @@ def test_prompt_chunks_match_the_oracle(dtype, G, bs, seqs, lens, F):
 
 
 def test_which_calls_take_it():
-    """The workspace tells the routes apart: chunks that fill four 128-row tiles beyond one token per sequence, the cache's extent known."""
+    """The workspace tells the routes apart: enough chunk tokens beyond one per sequence for the room in the block table, the
+    cache's extent known, blocks of whole swizzle groups."""
     p = _cabi.PagedProblem()
-    p.F, p.W, p.Hq, p.Hkv, p.E, p.Ev, p.block_size, p.max_blocks_per_seq = 1, 4, 16, 4, 128, 128, 16, 64
-    p.dtype, p.num_blocks, p.cu_seqlens_q = _cabi.BF16, 256, 1
+    p.F, p.W, p.Hq, p.Hkv, p.E, p.Ev = 1, 4, 16, 4, 128, 128
+    p.dtype, p.cu_seqlens_q = _cabi.BF16, 1
     lib = _cabi.load()
 
     def need(**kw):
-        for k, v in dict(dict(total_q_tokens=132, num_blocks=256, block_size=16, kernel=_cabi.KERNEL_AUTO), **kw).items():
+        for k, v in dict(dict(total_q_tokens=300, num_blocks=256, block_size=16, max_blocks_per_seq=64, kernel=_cabi.KERNEL_AUTO), **kw).items():
             setattr(p, k, v)
         return lib.hogatt_paged_workspace_bytes(p)
 
-    general = need(kernel=_cabi.KERNEL_MMA)
-    assert need() != general
-    for kw in (dict(num_blocks=0), dict(block_size=12), dict(block_size=4)):
-        assert need(**kw) == general
-    assert need(total_q_tokens=131) == need(total_q_tokens=131, kernel=_cabi.KERNEL_MMA)
+    def general(**kw):
+        return need(**dict(kw, kernel=_cabi.KERNEL_MMA))
+
+    assert need() != general()
+    for kw in (dict(num_blocks=0), dict(block_size=12, max_blocks_per_seq=90), dict(block_size=4, max_blocks_per_seq=300),
+               dict(total_q_tokens=270), dict(max_blocks_per_seq=58), dict(total_q_tokens=60, max_blocks_per_seq=4096)):
+        assert need(**kw) == general(**kw)
+    assert need(total_q_tokens=70, max_blocks_per_seq=4096) != general(total_q_tokens=70, max_blocks_per_seq=4096)
