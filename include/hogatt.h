@@ -80,12 +80,12 @@ typedef enum hogatt_status {
  * heads, where they are faster (hogatt_plan_describe reports the outcome).
  *
  * DENSE is the kernel for calls with many query rows per kv head (W x Hq/Hkv x S >= 128, e.g. workers that
- * each issue a 16-token chunk), where the op is bound by the tensor pipe, not by HBM: 128-row query blocks,
- * tcgen05.mma with accumulators in tensor memory, K / V / Q tiles fetched by tensor-map TMA.  f16 / bf16,
+ * each issue a 16-token chunk), where the op is bound by the tensor pipe, not by HBM: 128-row query tiles, two to
+ * a block where the call is long enough, tcgen05.mma with accumulators in tensor memory, K / V / Q tiles fetched by tensor-map TMA.  f16 / bf16,
  * E == Ev == 128, at most 16 fragments, and Hq/Hkv x S must divide 128 or be a multiple of it; AUTO takes it
  * whenever a problem qualifies, DENSE forces it (HOGATT_ERR_BAD_KERNEL_CHOICE otherwise).  It reads rotated
  * queries from memory, so the fused entry point first runs the stand-alone rotation kernel into `rq` (or into
- * the workspace when rq is NULL): three kernels per call. */
+ * the workspace when rq is NULL): three kernels per call, four with the plan kernel of the two-tile blocks. */
 typedef enum hogatt_kernel_choice {
     HOGATT_KERNEL_AUTO = 0,
     HOGATT_KERNEL_FMA = 1,

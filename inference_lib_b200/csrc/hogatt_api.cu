@@ -665,8 +665,8 @@ int rope_launch(void* rq, const void* queries, const float* cosines, const float
     if (rows > (1 << 30) || rows * std::max(E, 8) >= ((int64_t)1 << 31)) return HOGATT_ERR_TOO_LARGE;   // 32-bit element counts
     cudaError_t rc = cudaSuccess;
     auto go = [&](auto kernel, dim3 grid, auto... args) {
-        if (beside_predecessor) return launch_kernel(kernel, grid, dim3(128), 0, stream, args...);
-        kernel<<<grid, 128, 0, stream>>>(args...);
+        if (beside_predecessor) return launch_kernel(kernel, grid, dim3(128), 0, stream, args..., 1);
+        kernel<<<grid, 128, 0, stream>>>(args..., 0);
         return cudaGetLastError();
     };
     const int64_t work = rows * ((dtype != HOGATT_F32 && E % 8 == 0) ? E / 8 : E);      // chunks or channels
@@ -1530,7 +1530,9 @@ int hogatt_launch_shape(const hogatt_problem* p, int32_t shape[4]) {
     shape[0] = cluster ? HOGATT_KERNEL_MMA_CLUSTER : r.kernel;
     shape[1] = cluster ? r.units * cluster : grid;
     shape[2] = cluster;
-    shape[3] = cluster ? 1 : (r.kernel == HOGATT_KERNEL_DENSE && p->cosines ? 3 : 2);
+    hogatt_problem q = *p;
+    if (!q.workspace) q.workspace_bytes = SIZE_MAX;          // (asked before there is one: as with hogatt_workspace_bytes of it)
+    shape[3] = cluster ? 1 : 2 + (r.kernel == HOGATT_KERNEL_DENSE && p->cosines ? 1 : 0) + (dense_pairs(&q, r, grid) ? 1 : 0);
     return HOGATT_OK;
 }
 

@@ -1,7 +1,6 @@
 // CUDA-core (FMA) fragment attention: any storage type (fp32 / fp16 / bf16), any qk head size
-// up to 256, v head size in {32, 64, 128, 256}.  This is the path for shapes whose query tile is
-// too thin or too oddly sized for the tensor-core kernel (and for fp32, where tensor cores would
-// mean tf32 rounding); it uses the same persistent split-K decomposition, workspace format and
+// up to 256, v head size in {32, 64, 128, 256}.  This is the path for head sizes that neither the
+// tensor-core kernels nor the fp32 kernel take; it uses the same persistent split-K decomposition, workspace format and
 // merge step as the tensor-core kernel.
 //
 // Same math as the reference kernel (src/kernels/kernel_v21.cuh:95-203: per fragment, dot

@@ -398,11 +398,11 @@ template <class T>
 __global__ void __launch_bounds__(128) rope_kernel(T* __restrict__ rq, const T* __restrict__ q,
                                                    const float* __restrict__ cosines,
                                                    const float* __restrict__ sines, int F, int W, int Hq, int S,
-                                                   int E, int R) {
-    pdl_trigger();   // (whoever follows waits for this whole grid before it reads)
+                                                   int E, int R, int chained) {
+    if (chained) pdl_trigger();      // (whoever follows waits for this whole grid before it reads)
     write_rotated_queries<T>(q, rq, cosines, sines, F, W, Hq, S, E, R, blockIdx.x * blockDim.x + threadIdx.x,
                              gridDim.x * blockDim.x);
-    pdl_wait();      // launched beside its predecessor: ends after it (otherwise returns at once)
+    if (chained) pdl_wait();         // launched beside its predecessor: ends after it
 }
 
 // The same for 16-bit types with the whole head rotated (R == E, E a multiple of 16): a thread owns one pair of
@@ -413,12 +413,12 @@ constexpr int kRopeHeads = 4;
 template <class T>
 __global__ void __launch_bounds__(128) rope_pairs_kernel(T* __restrict__ rq, const T* __restrict__ q,
                                                          const float* __restrict__ cosines, const float* __restrict__ sines,
-                                                         int F, int W, int Hq, int S, int E) {
-    pdl_trigger();   // (whoever follows waits for this whole grid before it reads)
+                                                         int F, int W, int Hq, int S, int E, int chained) {
+    if (chained) pdl_trigger();      // (whoever follows waits for this whole grid before it reads)
     const int pairs = E >> 4, half = E >> 1;
     const int item = blockIdx.x * blockDim.x + threadIdx.x;
     if (item >= F * W * S * pairs) {
-        pdl_wait();
+        if (chained) pdl_wait();
         return;
     }
     const int j = item % pairs;
@@ -470,7 +470,7 @@ __global__ void __launch_bounds__(128) rope_pairs_kernel(T* __restrict__ rq, con
         *reinterpret_cast<uint4*>(dst) = lo;
         *reinterpret_cast<uint4*>(dst + half) = hi;
     }
-    pdl_wait();      // launched beside its predecessor: ends after it (otherwise returns at once)
+    if (chained) pdl_wait();         // launched beside its predecessor: ends after it
 }
 
 }  // namespace hogatt
