@@ -6,21 +6,21 @@
 // Decomposition.  Query rows are cut into tiles of 128 (the MMA's M).  A block is two tiles that read the same keys, a
 // unit is (block, kv head).  dense_plan_kernel finds, per tile and fragment, how many keys any of its rows sees; a
 // block walks only those, 128 keys per step -- of a causal prompt just over half (4,000 tokens: 543 us per call when
-// every block walked every key, see below) -- and the steps of all units are one list that a persistent grid of one
+// every block walked every key, 168 now) -- and the steps of all units are one list that a persistent grid of one
 // CTA per SM cuts into balanced contiguous ranges.  A unit that lies inside one range is normalised and stored by
 // its CTA; the others leave unnormalised partials for dense_merge_kernel.
 //
 // A step.  Both tiles of the block use the K and V tile (64 KiB of copies per 16.8 MFLOP; each tile alone would be at
 // the SM's L2 bandwidth).  Where a block has only one tile, the second softmax group takes every other key tile
 // of the same queries instead, and the two halves are two partials.
-//   warp 8   K copies (TMA, ring of 3 tiles)         warp 11  V copies (ring of 2)
-//   warp 9   query copies and S = Q K^T: one S buffer in tensor memory, used by the two groups in turn
-//   warp 10  O_g += P_g V, P as the tensor-memory A operand
-//   warps 0-3 / 4-7  softmax of group 0 / 1: one thread per query row.  The 128 scores go to registers at once, which
-//            frees the S buffer for the other group's product; row maximum, exponentials and sums need no
-//            exchange between threads.  The groups run half a step apart: one's tensor-memory round trips and waits lie
-//            under the other's exponentials (128 x 128 per tile = 1,024 cycles of the special-function unit, as
-//            long as the two products of the tile take the tensor pipe).
+//   warp 16  K copies (TMA, ring of 3 tiles)         warp 19  the walk over the steps, V copies (ring of 2)
+//   warp 17  query copies and S = Q K^T: one S buffer in tensor memory, used by the two groups in turn
+//   warp 18  O_g += P_g V, P as the tensor-memory A operand
+//   warps 0-7 / 8-15  softmax of group 0 / 1: two threads per query row, 64 columns each (with one, which has 128
+//            exponentials in a row, a 1,024-row chunk call took 128 us instead of 122).  The scores go to registers at once, which frees the S buffer for the other
+//            group's product; the halves of a row need each other's maximum only when the row's scale has to change, and
+//            each other's sum at the end.  The groups run half a step apart: one's tensor-memory round trips and waits lie
+//            under the other's exponentials.
 // Tensor memory, all 512 columns: O_0, O_1 (128 each), S (128), P_0, P_1 (64 each: two 16-bit probabilities a column).
 // Issuing one tcgen05.mma costs the issuing thread 60-70 cycles, hence two issuing threads.  O is rescaled in tensor
 // memory only when a row's maximum has grown by more than 2^8 since the scale it is stored at (then exp2 arguments
