@@ -409,7 +409,8 @@ int hogatt_plan_describe(const hogatt_problem* p, const int32_t* visible_rows, i
  * (hogatt_kernel_choice, never AUTO), shape[1] = CTAs of the attention grid, shape[2] = CTAs per
  * cluster (0: no clusters; an upper bound, a forced cluster launch shrinks it until all clusters are
  * resident), shape[3] = kernels per call (1 when the attention kernel merges by itself, 2 with the
- * merge kernel).  No reference counterpart.
+ * merge kernel, one more each for the rotation kernel in front of a tcgen05 kernel and for the plan kernel of
+ * the one with two query tiles per block).  No reference counterpart.
  */
 int hogatt_launch_shape(const hogatt_problem* p, int32_t shape[4]);
 
