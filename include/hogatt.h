@@ -422,6 +422,16 @@ int hogatt_launch_shape(const hogatt_problem* p, int32_t shape[4]);
 int hogatt_plan_ranges(int32_t tiles_per_unit, int32_t units, int32_t ctas, int32_t cta, int32_t unit,
                        int64_t range[4]);
 
+/*
+ * The same for the blocks of two query tiles of the tcgen05 kernel, by the arithmetic that its plan kernel runs on the
+ * device: block b has steps[b] steps per kv head (single[b] != 0: it holds one query tile), units are (block, kv head).
+ * Fills pos[0 .. grid]: the first step of every CTA's share in the list of all steps (a CTA without work: where the next
+ * share begins), and per unit parts[2u] = first CTA that works on it, parts[2u + 1] = how many of the following ones
+ * leave a partial (u = b * Hkv + kv head).  Host-only.
+ */
+int hogatt_dense_plan(const int32_t* steps, const uint8_t* single, int32_t blocks, int32_t Hkv, int32_t grid, int64_t* pos,
+                      int32_t* parts);
+
 #ifdef __cplusplus
 }
 #endif

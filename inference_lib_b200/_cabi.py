@@ -20,7 +20,7 @@ MAX_FRAGMENTS = 128
 EXPORTS = ["hogatt_abi_version", "hogatt_status_string", "hogatt_last_cuda_error", "hogatt_workspace_bytes",
            "hogatt_sdpa_launch", "hogatt_fused_launch", "hogatt_fused_launch_static", "hogatt_fused_launch_gather", "hogatt_rope_launch",
            "hogatt_paged_workspace_bytes", "hogatt_paged_sdpa_launch", "hogatt_copy_to_blocks_launch", "hogatt_plan_describe",
-           "hogatt_plan_ranges", "hogatt_launch_shape", "hogatt_step_plan_launch", "hogatt_append_launch"]
+           "hogatt_plan_ranges", "hogatt_dense_plan", "hogatt_launch_shape", "hogatt_step_plan_launch", "hogatt_append_launch"]
 
 
 class Problem(C.Structure):
@@ -96,6 +96,9 @@ def load() -> C.CDLL:
         lib.hogatt_plan_describe.argtypes = [C.POINTER(Problem), C.POINTER(C.c_int32), C.c_int32, C.POINTER(C.c_int32)]
         lib.hogatt_plan_ranges.restype = C.c_int
         lib.hogatt_plan_ranges.argtypes = [C.c_int32] * 5 + [C.POINTER(C.c_int64)]
+        lib.hogatt_dense_plan.restype = C.c_int
+        lib.hogatt_dense_plan.argtypes = [C.POINTER(C.c_int32), C.POINTER(C.c_uint8)] + [C.c_int32] * 3 + [C.POINTER(C.c_int64),
+                                                                                                      C.POINTER(C.c_int32)]
         _lib = lib
     return _lib
 

@@ -18,6 +18,7 @@
 
 #include <mutex>
 #include <unordered_map>
+#include <vector>
 
 namespace hogatt {
 namespace {
@@ -1548,6 +1549,36 @@ int hogatt_plan_ranges(int32_t tiles_per_unit, int32_t units, int32_t ctas, int3
     unit_ctas(unit, tiles_per_unit, n, ctas, &first, &count);
     range[2] = first;
     range[3] = count;
+    return HOGATT_OK;
+}
+
+int hogatt_dense_plan(const int32_t* steps, const uint8_t* single, int32_t blocks, int32_t Hkv, int32_t grid, int64_t* pos,
+                      int32_t* parts) {
+    if (!steps || !single || !pos || !parts) return HOGATT_ERR_NULL_POINTER;
+    if (blocks <= 0 || Hkv <= 0 || grid <= 0) return HOGATT_ERR_BAD_SHAPE;
+    std::vector<long long> pre(blocks + 1, 0), cost(blocks + 1, 0);
+    bool singles = false;
+    for (int b = 0; b < blocks; ++b) {
+        if (steps[b] < 0) return HOGATT_ERR_BAD_SHAPE;
+        pre[b + 1] = pre[b] + steps[b];
+        cost[b + 1] = cost[b] + dense_cost(steps[b], single[b] != 0);
+        singles |= single[b] != 0;
+    }
+    const long long N = pre[blocks] * Hkv, C = cost[blocks] * Hkv;
+    const int ctas = dense_ctas(N, C, singles, std::min(grid, kDenseMaxCtas));
+    std::vector<long long> at(ctas + 1, N);
+    for (int c = 0; c < ctas; ++c) {
+        DenseStart d;
+        at[c] = dense_share_start(pre.data(), cost.data(), blocks, Hkv, [&](int b) { return single[b] != 0; }, cta_first_tile(c, C, ctas), &d);
+    }
+    for (int c = 0; c <= grid; ++c) pos[c] = c < ctas ? at[c] : N;
+    for (int b = 0; b < blocks; ++b)
+        for (int h = 0; h < Hkv; ++h) {
+            int32_t* e = parts + 2 * ((int64_t)b * Hkv + h);
+            const long long s = pre[b] * Hkv + (long long)h * steps[b];
+            e[0] = steps[b] > 0 ? dense_first_cta(at.data(), ctas, s) : 0;
+            e[1] = steps[b] > 0 ? dense_parts(at.data(), ctas, e[0], s + steps[b]) : 0;
+        }
     return HOGATT_OK;
 }
 

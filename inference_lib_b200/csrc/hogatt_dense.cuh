@@ -45,9 +45,6 @@ constexpr int kDenseSoftmaxWarps = 16;      // two groups of eight: one group pe
 constexpr int kDenseThreads = (kDenseSoftmaxWarps + 4) * 32;
 constexpr int kDensePlanThreads = 1024;
 constexpr int kDenseMaxCtas = 256;
-// What the balanced shares count (cycles on B200: a step 2,660, starting and finishing a unit 8,200, a step of a block of one
-// tile, whose two key tiles the short value ring cannot keep coming, 5,000).
-constexpr int kDenseUnitSteps = 3, kDenseSingleSteps = 2;
 constexpr int kDenseMergeWarps = 4;         // warps per CTA of the merge step, with few partials per row
 constexpr int kDenseMergeSplit = 8;         // ... with many: they share a row's partials
 
@@ -442,10 +439,12 @@ __global__ void __launch_bounds__(kDensePlanThreads) dense_plan_kernel(const __g
         return n;
     };
     long long mine = 0, mine_cost = 0, total, total_cost;
+    bool singles = false;
     for (int b = b0; b < b1; ++b) {
         const long long n = block_steps(b);
         mine += n;
-        mine_cost += n > 0 ? n * (single_block(b) ? kDenseSingleSteps : 1) + kDenseUnitSteps : 0;
+        mine_cost += dense_cost(n, single_block(b));
+        singles |= single_block(b);
     }
     long long at = scan(mine, &total), at_cost = scan(mine_cost, &total_cost);
     for (int b = b0; b < b1; ++b) {
@@ -453,53 +452,32 @@ __global__ void __launch_bounds__(kDensePlanThreads) dense_plan_kernel(const __g
         a.pre[b] = pre[b] = at;
         cost[b] = at_cost;
         at += n;
-        at_cost += n > 0 ? n * (single_block(b) ? kDenseSingleSteps : 1) + kDenseUnitSteps : 0;
+        at_cost += dense_cost(n, single_block(b));
     }
     if (tid == 0) {
         a.pre[nb] = pre[nb] = total;
         cost[nb] = total_cost;
     }
-    __syncthreads();
+    singles = __syncthreads_or(singles);
 
     // Where every CTA starts: equal shares of the steps and of the units' fixed costs.  pos[c]: its first step in the list of all.
     const long long N = total * a.Hkv, C = total_cost * a.Hkv;
-    const int ctas = effective_ctas(N, a.ctas);
+    const int ctas = dense_ctas(N, C, singles, a.ctas);
     int4 st = make_int4(0, 0, 0, 0);
     if (tid < ctas) {
-        const long long t = cta_first_tile(tid, C, ctas);
-        int lo = 0, hi = nb;                         // cost[lo] * Hkv <= t < cost[hi] * Hkv
-        while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (cost[mid] * a.Hkv <= t) lo = mid;
-            else hi = mid;
-        }
-        const long long steps = pre[lo + 1] - pre[lo], unit = cost[lo + 1] - cost[lo], off = t - cost[lo] * a.Hkv;
-        long long h = floor_div(off, unit), j = min((off - h * unit) / (single_block(lo) ? kDenseSingleSteps : 1), steps);
-        pos[tid] = pre[lo] * a.Hkv + h * steps + j;
-        if (j == steps) {                            // the unit's end is the next one's beginning
-            j = 0;
-            if (++h == a.Hkv) {
-                h = 0;
-                for (++lo; lo < nb && pre[lo + 1] == pre[lo]; ++lo) {}
-            }
-        }
-        st = make_int4(lo, (int)h, (int)j, 0);
+        DenseStart d;
+        pos[tid] = dense_share_start(pre, cost, nb, a.Hkv, single_block, cta_first_tile(tid, C, ctas), &d);
+        st = make_int4(d.block, d.head, d.step, 0);
     }
     if (tid == ctas) pos[ctas] = N;
     __syncthreads();
-    // the partials of a unit that begins at step s: those of CTAs c0, c0 + 1, ...
-    auto parts = [&](int c0, long long s, long long steps) {
-        int c1 = c0;
-        while (c1 + 1 < ctas && pos[c1 + 1] < s + steps) ++c1;
-        return c1 - c0 + 1;
-    };
     if (tid < a.ctas) {
         if (tid < ctas) {
             st.w = (int)(pos[tid + 1] - pos[tid]);
             const long long s = pos[tid] - st.z;
             // the unit this CTA starts inside of, if no earlier CTA does
             if (st.z > 0 && !single_block(st.x) && pos[tid - 1] <= s)
-                a.merge[atomicAdd(&s_list, 1)] = make_int4(st.x * a.Hkv + st.y, tid - 1, parts(tid - 1, s, pre[st.x + 1] - pre[st.x]), 0);
+                a.merge[atomicAdd(&s_list, 1)] = make_int4(st.x * a.Hkv + st.y, tid - 1, dense_parts(pos, ctas, tid - 1, s + pre[st.x + 1] - pre[st.x]), 0);
         }
         a.start[tid] = st;
     }
@@ -513,13 +491,8 @@ __global__ void __launch_bounds__(kDensePlanThreads) dense_plan_kernel(const __g
             int c0 = 0, count = 0;
             if (steps > 0) {
                 const long long s = pre[b] * a.Hkv + h * steps;
-                int hi = ctas;                       // pos[c0] <= s < pos[hi]
-                while (hi - c0 > 1) {
-                    const int mid = (c0 + hi) >> 1;
-                    if (pos[mid] <= s) c0 = mid;
-                    else hi = mid;
-                }
-                count = 2 * parts(c0, s, steps);
+                c0 = dense_first_cta(pos, ctas, s);
+                count = 2 * dense_parts(pos, ctas, c0, s + steps);
             }
             a.merge[at_list] = make_int4(b * a.Hkv + h, c0, count, single ? 1 : 0);
         }

@@ -95,4 +95,69 @@ HOGATT_HD int max_parts_per_unit(int units, int grid) {
 
 HOGATT_HD int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
+// ---- shares of the tcgen05 kernel of two query tiles per block (hogatt_dense.cuh) ----------------------------------------
+// There the units of a kv head differ: block b has pre[b + 1] - pre[b] steps, every kv head repeats the list, and what is cut
+// into equal shares is cost[] -- a step counts 1 (kDenseSingleSteps in a block of one query tile), a unit that has steps
+// kDenseUnitSteps more (cycles on B200: a step 2,660, starting and finishing a unit 8,200, a step of a block of one tile,
+// whose two key tiles the short value ring cannot keep coming, 5,000).
+constexpr int kDenseUnitSteps = 3, kDenseSingleSteps = 2;
+
+HOGATT_HD long long dense_cost(long long steps, bool single) {
+    return steps > 0 ? steps * (single ? kDenseSingleSteps : 1) + kDenseUnitSteps : 0;
+}
+
+// CTAs that get work.  The merge step takes every CTA whose share starts inside a unit for a partial of it, so two shares must
+// never start at the same step there: a share counts at least what one step does.
+HOGATT_HD int dense_ctas(long long steps, long long cost, bool singles, int grid) {
+    const int ctas = effective_ctas(steps, grid);
+    return singles && cost < (long long)kDenseSingleSteps * ctas ? (int)(cost / kDenseSingleSteps) : ctas;
+}
+
+// Where the share at cost t begins: block, kv head and step (st), and its place in the list of all steps (returned).
+struct DenseStart {
+    int block, head, step;
+};
+template <class Single>
+HOGATT_HD long long dense_share_start(const long long* pre, const long long* cost, int nb, int Hkv, Single single, long long t,
+                                      DenseStart* st) {
+    int lo = 0, hi = nb;                         // cost[lo] * Hkv <= t < cost[hi] * Hkv
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (cost[mid] * Hkv <= t) lo = mid;
+        else hi = mid;
+    }
+    const long long steps = pre[lo + 1] - pre[lo], unit = cost[lo + 1] - cost[lo], off = t - cost[lo] * Hkv;
+    long long h = floor_div(off, unit), j = (off - h * unit) / (single(lo) ? kDenseSingleSteps : 1);
+    if (j > steps) j = steps;
+    const long long pos = pre[lo] * Hkv + h * steps + j;
+    if (j == steps) {                            // the unit's end is the next one's beginning
+        j = 0;
+        if (++h == Hkv) {
+            h = 0;
+            for (++lo; lo < nb && pre[lo + 1] == pre[lo]; ++lo) {}
+        }
+    }
+    st->block = lo;
+    st->head = (int)h;
+    st->step = (int)j;
+    return pos;
+}
+
+// pos[c]: the first step of CTA c, pos[ctas] the number of steps.  The first CTA that works on a unit beginning at step s ...
+HOGATT_HD int dense_first_cta(const long long* pos, int ctas, long long s) {
+    int lo = 0, hi = ctas;                       // pos[lo] <= s < pos[hi]
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (pos[mid] <= s) lo = mid;
+        else hi = mid;
+    }
+    return lo;
+}
+// ... and how many from there on do, if it ends before step `end`.
+HOGATT_HD int dense_parts(const long long* pos, int ctas, int first, long long end) {
+    int last = first;
+    while (last + 1 < ctas && pos[last + 1] < end) ++last;
+    return last - first + 1;
+}
+
 }  // namespace hogatt

@@ -77,3 +77,45 @@ def test_which_calls_take_it():
                dict(total_q_tokens=270), dict(max_blocks_per_seq=58), dict(total_q_tokens=60, max_blocks_per_seq=4096)):
         assert need(**kw) == general(**kw)
     assert need(total_q_tokens=70, max_blocks_per_seq=4096) != general(total_q_tokens=70, max_blocks_per_seq=4096)
+
+
+def _packed(dtype, Hkv, G, bs, seqs, lens, room, seed=3):
+    """A packed batch on the device, its table as wide as `room` keys, and what the oracle says of it."""
+    W, E = len(seqs), 128
+    gen = torch.Generator().manual_seed(seed)
+    cu = torch.tensor([0] + list(np.cumsum(seqs)), dtype=torch.int32)
+    per = -(-max(lens) // bs)
+    kc, vc = (torch.randn(W * per, Hkv, bs, E, generator=gen).to(dtype) for _ in range(2))
+    table = torch.randperm(W * per, generator=gen).to(torch.int32).reshape(W, per)
+    table = torch.cat([table, torch.zeros(W, max(0, -(-room // bs) - per), dtype=torch.int32)], 1).contiguous()
+    length = torch.tensor([lens], dtype=torch.int32)
+    loc = torch.tensor([[n - s + t for n, s in zip(lens, seqs) for t in range(s)]], dtype=torch.int32)
+    rq = torch.randn(1, int(cu[-1]), Hkv * G, E, generator=gen).to(dtype)
+    names = ("queries", "locations", "fragment_lengths", "key_cache", "value_cache", "block_table", "cu_seqlens_q")
+    return dict(zip(names, (rq, loc, length, kc, vc, table, cu)))
+
+
+def _run(p, scale, kernel=_cabi.KERNEL_AUTO):
+    """One call with the workspace and the output filled with NaN."""
+    d = {k: v.to(DEV) for k, v in p.items()}
+    out = torch.full(p["queries"].shape[1:], float("nan"), dtype=p["queries"].dtype, device=DEV)
+    problem, keep = _cabi.bind_paged(out=out, scale=scale, kernel=kernel, **d)
+    keep[0].fill_(0xFF)
+    assert _cabi.launch_paged(problem, torch.cuda.current_stream().cuda_stream) == 0
+    torch.cuda.synchronize()
+    return out
+
+
+def _oracle(p, scale):
+    return oracle.varlen_paged_sdpa(*(p[k] for k in ("queries", "locations", "fragment_lengths", "key_cache", "value_cache", "block_table",
+                                                     "cu_seqlens_q")), scale)
+
+
+@pytest.mark.parametrize("Hkv,G,seqs,lens", [
+    (2, 4, [367, 1, 1], [1675, 1666, 1657]),
+    (1, 4, [300, 1], [4000, 4000]),
+    (1, 8, [300], [2000]),
+])
+def test_every_partial_that_is_folded_has_been_written(Hkv, G, seqs, lens):
+    p = _packed(torch.bfloat16, Hkv, G, 16, seqs, lens, room=int(4.6e6 / ((sum(seqs) - len(seqs)) * Hkv * G)))
+    check_against(_run(p, 128 ** -0.5), _oracle(p, 128 ** -0.5).numpy(), torch.bfloat16)

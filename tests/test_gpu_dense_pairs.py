@@ -76,3 +76,17 @@ def test_too_small_a_workspace_runs_on_the_other_kernel():
     torch.cuda.synchronize()
     ref, _ = oracle.fused(p.queries, p.cos, p.sin, p.locations, p.keys, p.values, p.scale)
     check_against(out, ref.numpy(), p.dtype)
+
+
+@pytest.mark.parametrize("W,G,S,lengths,Hkv", [
+    (1, 4, 160, [640, 360], 8),                             # five tiles: the last block holds one; shares of 1.9 steps
+    (3, 4, 96, [400, 160, 160, 160], 4),
+    (1, 8, 304, [700, 404], 2),
+])
+def test_every_partial_that_is_folded_has_been_written(W, G, S, lengths, Hkv):
+    """On all SMs a share of a block of one tile can be shorter than its steps count for; the workspace is NaN beforehand."""
+    p = _problem(W, G, S, lengths, Hkv=Hkv)
+    ref, _ = oracle.fused(p.queries, p.cos, p.sin, p.locations, p.keys, p.values, p.scale)
+    r = run_cabi(p)
+    assert r.rc == 0 and r.status == 0
+    check_against(r.out, ref.numpy(), p.dtype)
