@@ -807,13 +807,13 @@ dense_attention_kernel(const __grid_constant__ DenseArgs a, const __grid_constan
             uint32_t v_phase = 0, g_phase = 0, started = 0;      // bit g: parity of P_g; O_g holds something
             while (ok && segs.next(d, lane, a.status)) {
                 if (d.first()) started = 0;
-                const int vlen = dense_length<PAGED>(a, d.f, PAGED ? a.rec[d.b].x : 0);
+                const int vlen = max(d.vis0, d.vis1);
 #pragma unroll 1
                 for (int t = d.t0; t < d.t1 && ok; ++t) {
                     ok = mbar_wait_polls(v_full + 8 * stage, v_phase, a.status, STATUS_WAIT_FULL_TIMEOUT);
                     if ((t + 1) * kDenseTile > vlen && ok) {
-                        // The tile runs past the rows in use: those rows may hold anything (spare rows of a slab or cache
-                        // block).  Their probabilities are exactly zero, but 0 * NaN would poison O.
+                        // The tile runs past the keys that any row of the block sees: what follows may hold anything (spare
+                        // rows of a slab or cache block).  Those probabilities are exactly zero, but 0 * NaN would poison O.
                         unsigned char* vt = base + C::OFF_V + stage * C::TILE_BYTES;
 #pragma unroll 1
                         for (int i = (vlen - t * kDenseTile) * 8 + lane; i < kDenseTile * 8; i += 32) {

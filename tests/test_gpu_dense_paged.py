@@ -119,3 +119,14 @@ def _oracle(p, scale):
 def test_every_partial_that_is_folded_has_been_written(Hkv, G, seqs, lens):
     p = _packed(torch.bfloat16, Hkv, G, 16, seqs, lens, room=int(4.6e6 / ((sum(seqs) - len(seqs)) * Hkv * G)))
     check_against(_run(p, 128 ** -0.5), _oracle(p, 128 ** -0.5).numpy(), torch.bfloat16)
+
+
+def test_rows_that_nobody_sees_never_reach_a_result():
+    """A sequence that already holds keys behind the ones this call's tokens may see."""
+    p = _packed(torch.bfloat16, 2, 4, 16, [130, 1], [700, 300], room=5000)
+    p["locations"] = (p["locations"] - 100).contiguous()
+    ref = _oracle(p, 128 ** -0.5)
+    for w, n in enumerate((600, 200)):
+        for x in range(n, 16 * (n // 16 + 6)):
+            p["value_cache"][p["block_table"][w, x // 16], :, x % 16] = float("nan")
+    check_against(_run(p, 128 ** -0.5), ref.numpy(), torch.bfloat16)

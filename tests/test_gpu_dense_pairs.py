@@ -90,3 +90,25 @@ def test_every_partial_that_is_folded_has_been_written(W, G, S, lengths, Hkv):
     r = run_cabi(p)
     assert r.rc == 0 and r.status == 0
     check_against(r.out, ref.numpy(), p.dtype)
+
+
+@pytest.mark.parametrize("W,G,S,lengths", [(2, 4, 64, [300, 130, 257]), (1, 4, 160, [290])])
+@pytest.mark.parametrize("with_lengths", [False, True])
+def test_rows_that_nobody_sees_never_reach_a_result(W, G, S, lengths, with_lengths):
+    """Fragments that hold more rows than any query sees (no lengths given, or lengths that count those rows)."""
+    p = _problem(W, G, S, lengths)
+    loc = torch.minimum(p.locations, torch.tensor(lengths, dtype=torch.int32)[:, None, None] - 1)      # (else a row sees all there is)
+    p = wl.Problem(**{**p.__dict__, "locations": loc})
+    ref, _ = oracle.fused(p.queries, p.cos, p.sin, p.locations, p.keys, p.values, p.scale)
+    more = [torch.cat([t, torch.full_like(t[:, :, :100], float("nan"))], 2) for t in p.keys + p.values]
+    d = p.to("cuda:0")
+    keys, values = [t.cuda() for t in more[:p.F]], [t.cuda() for t in more[p.F:]]
+    rows = torch.tensor([k.shape[2] for k in keys], dtype=torch.int32, device="cuda:0") if with_lengths else None
+    for max_ctas in (1, 3, 0):
+        out = torch.full((p.W, p.Hq, p.S, p.Ev), float("nan"), dtype=p.dtype, device="cuda:0")
+        bp = _cabi.bind(out=out, queries=d.queries, locations=d.locations, keys=keys, values=values, scale=p.scale, fragment_lengths=rows,
+                        cos=d.cos, sin=d.sin, max_ctas=max_ctas)
+        _cabi.attach_workspace(bp, torch.device("cuda:0"))
+        assert _cabi.launch(bp, torch.cuda.current_stream().cuda_stream) == 0
+        torch.cuda.synchronize()
+        check_against(out, ref.numpy(), p.dtype, what=f"{max_ctas} CTAs")
