@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(F32Cfg<HD, R>::THREADS, 1) f32_attention_kerne
             }
 #pragma unroll
             for (int r = 0; r < RW; ++r) {
-                s[r] = m[r] == -INFINITY ? 0.f : exp2f(s[r] - m[r]);
+                s[r] = exp2f(s[r] - (m[r] == -INFINITY ? 0.f : m[r]));      // (hidden: 0; not a number stays one)
                 l[r] += s[r];
             }
 #pragma unroll

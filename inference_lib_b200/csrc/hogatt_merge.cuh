@@ -90,7 +90,7 @@ __device__ __forceinline__ void merge_partials_rows(const float* __restrict__ ws
                     den += __ldcg(ws_l + (slot0 + p) * rpb + row) * exp2f(__ldcg(ws_m + (slot0 + p) * rpb + row) - M);
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) den += __shfl_xor_sync(0xffffffffu, den, o);
-            blind = !(den > 0.f);
+            blind = den == 0.f;                     // (not a number: not blind, and it shows)
             inv = blind ? 0.f : 1.f / den;
 #ifdef HOGATT_TIMELINE
             if (stamp && lane == 0) *stamp = global_timer_ns_();      // the statistics have arrived
@@ -321,8 +321,8 @@ __global__ void __launch_bounds__(WW * 32, (WW == 4 && KP == 16) ? 5 : 1) merge_
             sum.z = fmaf(y.z, f, sum.z);
             sum.w = fmaf(y.w, f, sum.w);
         }
-        const float inv = den > 0.f ? 1.f / den : 0.f;
-        if (!(den > 0.f)) sum = make_float4(0.f, 0.f, 0.f, 0.f);
+        const float inv = den == 0.f ? 0.f : 1.f / den;
+        if (den == 0.f) sum = make_float4(0.f, 0.f, 0.f, 0.f);
         const RowId id = decode_row(gr, a.G, a.S);
         T* const local_out = static_cast<T*>(a.out);
         const int nbases = a.world > 0 ? a.world : 1;

@@ -823,8 +823,8 @@ mma_attention_kernel(const __grid_constant__ KernelArgs a, const int use_evict_f
                     sum.w += y.w;
                 }
                 const float den = scr[C::CL_DEN + ri * SPLIT];
-                const float inv = den > 0.f ? 1.f / den : 0.f;
-                if (!(den > 0.f)) sum = make_float4(0.f, 0.f, 0.f, 0.f);
+                const float inv = den == 0.f ? 0.f : 1.f / den;
+                if (den == 0.f) sum = make_float4(0.f, 0.f, 0.f, 0.f);
                 const RowId id = decode_row(gr, a.G, a.S);
                 const size_t offset = dst.row_offset(id.w, hkv_u * a.G + id.g, id.s, a.S, HD) + c4 * 4;
                 uint2 packed;
