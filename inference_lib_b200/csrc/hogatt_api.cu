@@ -155,6 +155,10 @@ bool dense_eligible(const hogatt_problem* p) {
     return gs <= kDenseRows ? kDenseRows % gs == 0 : gs % kDenseRows == 0;
 }
 
+// The tcgen05 kernels take a row's maximum over unscaled scores and bring O to a new scale when it has grown by 8 / scale: the
+// scale has to be positive, and both it and that quotient finite.  AUTO sends other calls to the mma.sync kernels, which scale first.
+bool dense_scale(float scale) { return scale >= 1e-30f && scale <= 1e30f; }
+
 bool fma_eligible(const hogatt_problem* p) {
     const int vec = 16 / (int)dtype_size(p->dtype);
     if (p->Ev != 32 && p->Ev != 64 && p->Ev != 128 && p->Ev != 256) return false;
@@ -179,8 +183,8 @@ int resolve(const hogatt_problem* p, Resolved* r) {
     r->cluster_forced = kernel == HOGATT_KERNEL_MMA_CLUSTER;
     if (kernel == HOGATT_KERNEL_MMA_CLUSTER) kernel = HOGATT_KERNEL_MMA;
     if (kernel == HOGATT_KERNEL_AUTO)
-        kernel = (dense_eligible(p) && !dense_disabled()) ? HOGATT_KERNEL_DENSE
-                                                           : (mma_eligible(p) ? HOGATT_KERNEL_MMA : HOGATT_KERNEL_FMA);
+        kernel = (dense_eligible(p) && dense_scale(p->scale) && !dense_disabled()) ? HOGATT_KERNEL_DENSE
+                 : mma_eligible(p) ? HOGATT_KERNEL_MMA : HOGATT_KERNEL_FMA;
     if (kernel == HOGATT_KERNEL_DENSE) {
         if (!dense_eligible(p)) return HOGATT_ERR_BAD_KERNEL_CHOICE;
         r->cluster_mode = -1;
@@ -979,6 +983,29 @@ int attention_launch(const hogatt_problem* p, bool fused, cudaStream_t stream, c
     return HOGATT_OK;
 }
 
+size_t workspace_need(const hogatt_problem* p) {
+    Resolved r;
+    if (resolve(p, &r) != HOGATT_OK) return 0;
+    int dev, sms, smem_optin;
+    if (current_device_info(&dev, &sms, &smem_optin) != HOGATT_OK) return 0;
+    const int grid = grid_size(p, sms);
+    size_t need = carve(p, r, grid).total;
+    if (r.kernel == HOGATT_KERNEL_DENSE && r.row_blocks >= 2) need = std::max(need, carve_pairs(p, grid).total);
+    if (r.kernel == HOGATT_KERNEL_MMA && !r.cluster_forced) {
+        // a launch may cut the query rows into smaller blocks than resolve() did (refine_row_blocks): room for any of them
+        const int64_t rows_total = (int64_t)p->W * (p->Hq / p->Hkv) * p->S;
+        for (int mt = 1; mt < r.mt; mt *= 2) {
+            Resolved q = r;
+            q.mt = mt;
+            q.rows_per_block = 16 * mt;
+            q.row_blocks = (int)((rows_total + q.rows_per_block - 1) / q.rows_per_block);
+            q.units = q.row_blocks * p->Hkv;
+            need = std::max(need, carve(p, q, grid).total);
+        }
+    }
+    return need;
+}
+
 // ---- paged variants ----------------------------------------------------------------------------------
 
 struct PagedPlan {
@@ -986,7 +1013,7 @@ struct PagedPlan {
     bool dense;                     // the tcgen05 kernel
     int tokens, blocks;             // ... its query tokens per tile, blocks per kv head (upper bound)
     WorkspaceLayout w;              // ... its workspace
-    size_t o, m, l, total;
+    size_t o, m, l, total;          // the other kernels' workspace
 };
 
 // Packed queries on the tcgen05 kernel: 16-bit types, head size 128, cache blocks that tile a 128-key tile in whole
@@ -1040,7 +1067,6 @@ int plan_paged(const hogatt_paged_problem* p, int sms, PagedPlan* pl) {
         pl->tokens = kDenseRows / G;
         pl->blocks = p->total_q_tokens / (2 * pl->tokens) + p->W;
         carve_dense(&pl->w, pl->blocks, p->Hkv, p->F, std::min(sms, kDenseMaxCtas), true);
-        pl->total = pl->w.total;
     }
     return HOGATT_OK;
 }
@@ -1203,24 +1229,11 @@ const char* hogatt_status_string(int status) {
 int hogatt_last_cuda_error(void) { return tl_last_cuda_error; }
 
 size_t hogatt_workspace_bytes(const hogatt_problem* p) {
-    Resolved r;
-    if (resolve(p, &r) != HOGATT_OK) return 0;
-    int dev, sms, smem_optin;
-    if (current_device_info(&dev, &sms, &smem_optin) != HOGATT_OK) return 0;
-    const int grid = grid_size(p, sms);
-    size_t need = carve(p, r, grid).total;
-    if (r.kernel == HOGATT_KERNEL_DENSE && r.row_blocks >= 2) need = std::max(need, carve_pairs(p, grid).total);
-    if (r.kernel == HOGATT_KERNEL_MMA && !r.cluster_forced) {
-        // a launch may cut the query rows into smaller blocks than resolve() did (refine_row_blocks): room for any of them
-        const int64_t rows_total = (int64_t)p->W * (p->Hq / p->Hkv) * p->S;
-        for (int mt = 1; mt < r.mt; mt *= 2) {
-            Resolved q = r;
-            q.mt = mt;
-            q.rows_per_block = 16 * mt;
-            q.row_blocks = (int)((rows_total + q.rows_per_block - 1) / q.rows_per_block);
-            q.units = q.row_blocks * p->Hkv;
-            need = std::max(need, carve(p, q, grid).total);
-        }
+    size_t need = workspace_need(p);
+    if (p != nullptr && !dense_scale(p->scale)) {        // one not filled in yet, say: room for the kernel of an ordinary one too
+        hogatt_problem q = *p;
+        q.scale = 1.f;
+        need = std::max(need, workspace_need(&q));
     }
     return need;
 }
@@ -1235,7 +1248,7 @@ int hogatt_fused_launch(const hogatt_problem* p, hogatt_stream_t stream) {
 
 int hogatt_fused_launch_static(const hogatt_problem* p, hogatt_stream_t stream) {
     if (p == nullptr) return HOGATT_ERR_NULL_POINTER;
-    const size_t need = hogatt_workspace_bytes(p);
+    const size_t need = workspace_need(p);
     if (need == 0) {                         // let the regular path name what is wrong with the problem
         Resolved r;
         const int rc = resolve(p, &r);
@@ -1263,7 +1276,7 @@ size_t hogatt_paged_workspace_bytes(const hogatt_paged_problem* p) {
     if (current_device_info(&dev, &sms, &smem_optin) != HOGATT_OK) return 0;
     PagedPlan pl;
     if (plan_paged(p, sms, &pl) != HOGATT_OK) return 0;
-    return pl.total;
+    return pl.dense ? std::max(pl.total, pl.w.total) : pl.total;       // (whatever the scale, which may not be filled in yet)
 }
 
 int hogatt_paged_sdpa_launch(const hogatt_paged_problem* p, hogatt_stream_t stream_) {
@@ -1280,11 +1293,12 @@ int hogatt_paged_sdpa_launch(const hogatt_paged_problem* p, hogatt_stream_t stre
     if (!aligned16(p->out) || !aligned16(p->queries) || !aligned16(p->key_cache) || !aligned16(p->value_cache) ||
         ((uintptr_t)p->workspace & 255u))
         return HOGATT_ERR_MISALIGNED;
-    if (p->workspace_bytes < pl.total) return HOGATT_ERR_WORKSPACE_TOO_SMALL;
+    const bool dense = pl.dense && dense_scale(p->scale);
+    if (p->workspace_bytes < (dense ? pl.w.total : pl.total)) return HOGATT_ERR_WORKSPACE_TOO_SMALL;
     const bool packed = p->cu_seqlens_q != nullptr;
     if (packed && p->total_q_tokens == 0) return HOGATT_OK;
 
-    if (pl.dense)
+    if (dense)
         return p->dtype == HOGATT_F16 ? launch_paged_dense<__half>(p, pl, dev, sms, smem_optin, stream)
                                       : launch_paged_dense<__nv_bfloat16>(p, pl, dev, sms, smem_optin, stream);
 

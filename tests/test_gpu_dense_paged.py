@@ -130,3 +130,12 @@ def test_rows_that_nobody_sees_never_reach_a_result():
         for x in range(n, 16 * (n // 16 + 6)):
             p["value_cache"][p["block_table"][w, x // 16], :, x % 16] = float("nan")
     check_against(_run(p, 128 ** -0.5), ref.numpy(), torch.bfloat16)
+
+
+@pytest.mark.parametrize("scale", [0.0, -0.05, 1e-40])
+def test_scales_that_are_not_positive(scale):
+    """The result for -scale is that of the negated queries for scale; a scale of nothing is an average over what a token sees.
+    (The oracle masks before it scales and cannot say either by itself.)"""
+    p = _packed(torch.bfloat16, 2, 4, 16, [200, 1], [700, 650], room=5000)
+    flipped = dict(p, queries=-p["queries"] if scale < -0.01 else torch.zeros_like(p["queries"]))
+    check_against(_run(p, scale), _oracle(flipped, max(0.01, -scale)).numpy(), torch.bfloat16)

@@ -112,3 +112,23 @@ def test_rows_that_nobody_sees_never_reach_a_result(W, G, S, lengths, with_lengt
         assert _cabi.launch(bp, torch.cuda.current_stream().cuda_stream) == 0
         torch.cuda.synchronize()
         check_against(out, ref.numpy(), p.dtype, what=f"{max_ctas} CTAs")
+
+
+@pytest.mark.parametrize("W,G,S,lengths", [(1, 4, 160, [290]), (4, 4, 8, [260, 33, 20, 70, 129])])
+@pytest.mark.parametrize("scale", [0.0, -0.05, 1e-40])
+def test_scales_that_are_not_positive(W, G, S, lengths, scale):
+    """AUTO keeps such calls off both tcgen05 kernels.  (The oracle masks before it scales: negated queries, or none.)"""
+    p = _problem(W, G, S, lengths)
+    q = -p.queries if scale < -0.01 else torch.zeros_like(p.queries)
+    ref, _ = oracle.fused(q, p.cos, p.sin, p.locations, p.keys, p.values, max(0.01, -scale))
+    for max_ctas in (0, 2):
+        r = run_cabi(wl.Problem(**{**p.__dict__, "scale": scale}), max_ctas=max_ctas)
+        assert r.rc == 0 and r.status == 0
+        check_against(r.out, ref.numpy(), p.dtype)
+
+
+def test_a_workspace_asked_for_before_the_scale_is_known_is_enough():
+    p = _cabi.shape_problem(F=1, W=1, Hq=32, Hkv=8, E=128, Ev=128, S=512, dtype=_cabi.BF16)
+    q = _cabi.shape_problem(F=1, W=1, Hq=32, Hkv=8, E=128, Ev=128, S=512, dtype=_cabi.BF16, scale=0.0)
+    lib = _cabi.load()
+    assert lib.hogatt_workspace_bytes(q) >= lib.hogatt_workspace_bytes(p) > 0
