@@ -34,7 +34,7 @@
 extern "C" {
 #endif
 
-#define HOGATT_ABI_VERSION 2
+#define HOGATT_ABI_VERSION 3   /* 3: hogatt_paged_problem: num_blocks (reserved before), device_status */
 #ifndef HOGATT_MAX_FRAGMENTS
 #define HOGATT_MAX_FRAGMENTS 128   /* the fragment table travels by value in the kernel arguments (24 bytes per
                                       fragment); the reference's device pointer table admits 512
@@ -293,6 +293,7 @@ typedef struct hogatt_paged_problem {
     int32_t num_blocks;            /* extent of the caches' first dimension, or 0 if unknown: packed calls with prompt chunks
                                       (f16 / bf16, E == Ev == 128, block_size 8 ... 128 a power of two or a multiple of
                                       128) run on the tcgen05 kernel where AUTO knows it */
+    int32_t* device_status;        /* device int or NULL: as in hogatt_problem; the rows of a wait that ran out are NaN */
 } hogatt_paged_problem;
 
 size_t hogatt_paged_workspace_bytes(const hogatt_paged_problem* p);

@@ -45,6 +45,7 @@ class PagedProblem(C.Structure):
         ("out", C.c_void_p), ("queries", C.c_void_p), ("locations", C.c_void_p), ("fragment_lengths", C.c_void_p),
         ("key_cache", C.c_void_p), ("value_cache", C.c_void_p), ("block_table", C.c_void_p), ("cu_seqlens_q", C.c_void_p),
         ("workspace", C.c_void_p), ("workspace_bytes", C.c_size_t), ("kernel", C.c_int32), ("num_blocks", C.c_int32),
+        ("device_status", C.c_void_p),
     ]
 
 
@@ -310,7 +311,7 @@ def append(*, keys, values, cosines, sines, write_to, key_fragments, value_fragm
 
 
 def bind_paged(*, out, queries, locations, fragment_lengths, key_cache, value_cache, block_table, scale,
-               cu_seqlens_q=None, kernel=KERNEL_AUTO):
+               cu_seqlens_q=None, kernel=KERNEL_AUTO, status=None):
     """Fill a ``PagedProblem`` from torch CUDA tensors (fixed layout: ``queries [F,W,Hq,S,E]``, ``out [W,Hq,S,Ev]``;
     packed layout with ``cu_seqlens_q``: ``queries [F,total_q,Hq,E]``, ``out [total_q,Hq,Ev]``) and give it a
     workspace allocated with torch.  Returns ``(problem, keepalive)``; ``problem`` is ``None`` when the library
@@ -330,12 +331,13 @@ def bind_paged(*, out, queries, locations, fragment_lengths, key_cache, value_ca
     p.fragment_lengths, p.key_cache, p.value_cache = fragment_lengths.data_ptr(), key_cache.data_ptr(), value_cache.data_ptr()
     p.block_table = block_table.data_ptr()
     p.cu_seqlens_q = cu_seqlens_q.data_ptr() if packed else None
+    p.device_status = status.data_ptr() if status is not None else None
     need = int(load().hogatt_paged_workspace_bytes(C.byref(p)))
     if need == 0:
         return None, None
     ws = torch.empty(need + 256, dtype=torch.uint8, device=out.device)
     p.workspace, p.workspace_bytes = ws.data_ptr() + (-ws.data_ptr()) % 256, need
-    return p, [ws, out, queries, locations, fragment_lengths, key_cache, value_cache, block_table, cu_seqlens_q]
+    return p, [ws, out, queries, locations, fragment_lengths, key_cache, value_cache, block_table, cu_seqlens_q, status]
 
 
 def launch_paged(problem: PagedProblem, stream: int = 0) -> int:

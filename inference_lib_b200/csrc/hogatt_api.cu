@@ -1090,6 +1090,7 @@ int launch_paged_dense(const hogatt_paged_problem* p, const PagedPlan& pl, int d
     d.block_table = p->block_table;
     dense_workspace(&d, static_cast<unsigned char*>(p->workspace), pl.w);
     d.ctas = std::min(sms, kDenseMaxCtas);
+    d.status = p->device_status;
     d.out = p->out;
     DenseMaps maps;
     memset(&maps, 0, sizeof(maps));
@@ -1326,6 +1327,7 @@ int hogatt_paged_sdpa_launch(const hogatt_paged_problem* p, hogatt_stream_t stre
     a.ws_o = reinterpret_cast<float*>(ws + pl.o);
     a.ws_m = reinterpret_cast<float*>(ws + pl.m);
     a.ws_l = reinterpret_cast<float*>(ws + pl.l);
+    a.status = p->device_status;
     switch (p->dtype) {
         case HOGATT_F32: return launch_paged_dims<float>(a, pl, p->kernel, dev, sms, smem_optin, stream);
         case HOGATT_F16: return launch_paged_dims<__half>(a, pl, p->kernel, dev, sms, smem_optin, stream);

@@ -221,6 +221,19 @@ __device__ __forceinline__ bool wait_polls(uint32_t bar, uint32_t parity) {
     return false;
 }
 
+// A CTA must not leave while copies may still be landing in its shared memory.  Unlike the waits above this one neither
+// goes by the abort flag -- after a wait that ran out the copies in flight still need their microseconds -- nor by the
+// configured limit.
+__device__ __noinline__ void drain_stage(uint32_t bar, uint32_t parity, int* status) {
+    if (mbar_try_wait(bar, parity)) return;              // (before the timer: a read of it takes a microsecond)
+    const uint64_t t0 = global_timer_ns();
+    while (!mbar_try_wait(bar, parity))
+        if (global_timer_ns() - t0 > kWaitLimitNs) {
+            if (status) atomicOr(status, STATUS_DRAIN_TIMEOUT);
+            return;
+        }
+}
+
 // Programmatic dependent launch: a kernel launched with the "programmatic stream serialization"
 // attribute may start while its predecessor in the stream is still running; it must call
 // pdl_wait() before it touches anything the predecessor reads or writes.  pdl_trigger() lets the

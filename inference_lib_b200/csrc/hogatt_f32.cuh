@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(F32Cfg<HD, R>::THREADS, 1) f32_attention_kerne
         // (do not leave while copies may still be landing in this CTA's shared memory)
         if (lane == 0)
             for (uint32_t k = n > C::NBUF ? n - C::NBUF : 0; k < n; ++k)
-                mbar_wait_bounded(full + 8 * (k % C::NBUF), (k / C::NBUF) & 1u, abort_flag, a.status, STATUS_DRAIN_TIMEOUT);
+                drain_stage(full + 8 * (k % C::NBUF), (k / C::NBUF) & 1u, a.status);
         return;
     }
 

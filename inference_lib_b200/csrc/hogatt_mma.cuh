@@ -319,9 +319,7 @@ mma_attention_kernel(const __grid_constant__ KernelArgs a, const int use_evict_f
         // Do not leave while copies may still be landing in this CTA's shared memory.
         if (lane == 0) {
             const int pending = min(it, C::NSTAGE);
-            for (int k = it - pending; k < it; ++k)
-                mbar_wait_bounded(full0 + 8 * (k % C::NSTAGE), (uint32_t)(k / C::NSTAGE) & 1u, abort_flag, a.status,
-                                  STATUS_DRAIN_TIMEOUT);
+            for (int k = it - pending; k < it; ++k) drain_stage(full0 + 8 * (k % C::NSTAGE), (uint32_t)(k / C::NSTAGE) & 1u, a.status);
         }
         HOGATT_SPAN_MAX(1);
         if constexpr (CL) {

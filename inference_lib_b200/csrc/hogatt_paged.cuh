@@ -41,6 +41,7 @@ struct PagedArgs {
     float* ws_o;
     float* ws_m;
     float* ws_l;
+    int* status;              // optional
 };
 
 // Which worker and which of its token groups a global group index is.  Linear scan over workers
@@ -212,7 +213,8 @@ struct PagedMmaCfg {
     static constexpr int QBYTES = kFmaRows * PITCH;
     static constexpr int OFF_LIM = QBYTES;                       // int[16]: visibility limit per query row
     static constexpr int OFF_BAR = OFF_LIM + 64;                 // full and empty barriers of the stages
-    static constexpr int OFF_STAGE = (OFF_BAR + 2 * NSTAGE * 8 + 127) / 128 * 128;
+    static constexpr int OFF_VOID = OFF_BAR + 2 * NSTAGE * 8;    // int: a wait has run out, the partial is void
+    static constexpr int OFF_STAGE = (OFF_VOID + 4 + 127) / 128 * 128;
     static constexpr int KV_BYTES = BULK ? 8 * GROUP_STRIDE : TILE * PITCH;                // K (or V) rows of one tile
     static constexpr int STAGE_BYTES = 2 * KV_BYTES;
     static constexpr int OFF_PLAN = OFF_STAGE + NSTAGE * STAGE_BYTES;       // int vis[F], pre[F + 1]
@@ -244,7 +246,9 @@ __global__ void __launch_bounds__(PagedMmaCfg<HD, BULK, NS>::THREADS, BULK && NS
     int* vis = reinterpret_cast<int*>(smem_raw + C::OFF_PLAN);
     int* pre = vis + a.F;
     const uint32_t bars = smem_u32(smem_raw + C::OFF_BAR);
+    volatile int* const is_void = reinterpret_cast<volatile int*>(smem_raw + C::OFF_VOID);
     if (BULK && tid == 0) {
+        *is_void = 0;
         for (int k = 0; k < C::NSTAGE; ++k) {
             mbar_init(bars + 8 * k, 1);
             mbar_init(bars + 8 * (C::NSTAGE + k), C::WARPS);
@@ -304,13 +308,14 @@ __global__ void __launch_bounds__(PagedMmaCfg<HD, BULK, NS>::THREADS, BULK && NS
             row_next = ((long long)table[min(blk, a.max_blocks - 1)] * a.Hkv + u.hkv) * a.block_size + (l - blk * a.block_size);
         };
         if (t0 < t1) look_up(t0);
+        int issued = 0;
 #pragma unroll 1
-        for (int t = t0; t < t1; ++t) {
+        for (int t = t0; t < t1; ++t, ++issued) {
             row = row_next;
             ntok = ntok_next;
             if (t + 1 < t1) look_up(t + 1);
             const int rows = min(8, ntok - (lane & 7) * 8);
-            if (!__all_sync(0xffffffffu, wait_polls(bars + 8 * (C::NSTAGE + stage), phase))) break;
+            if (!__all_sync(0xffffffffu, mbar_wait_bounded(bars + 8 * (C::NSTAGE + stage), phase, is_void, a.status, STATUS_WAIT_EMPTY_TIMEOUT))) break;
             if (lane == 0) mbar_arrive_expect_tx(bars + 8 * stage, (uint32_t)ntok * HD * 4);
             __syncwarp();
             if (lane < 16 && rows > 0)
@@ -321,6 +326,8 @@ __global__ void __launch_bounds__(PagedMmaCfg<HD, BULK, NS>::THREADS, BULK && NS
                 phase ^= 1u;
             }
         }
+        if (lane == 0)
+            for (int k = max(0, issued - C::NSTAGE); k < issued; ++k) drain_stage(bars + 8 * (k % C::NSTAGE), (uint32_t)(k / C::NSTAGE) & 1u, a.status);
         return;
     }
 
@@ -361,6 +368,7 @@ __global__ void __launch_bounds__(PagedMmaCfg<HD, BULK, NS>::THREADS, BULK && NS
     float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;    // rows lane / 4 and lane / 4 + 8
     uint32_t qf[KSTEPS][4];
     int lim0 = 0, lim1 = 0, cur_f = -1, fscan = 0;
+    bool ok = true;                                                 // (BULK) every tile has come; otherwise the warp goes on to the barriers only
     // the ring: tiles t .. t + NSTAGE - 2 are in flight while tile t is used (one commit group per tile, empty past the end)
     if constexpr (!BULK) {
 #pragma unroll
@@ -413,8 +421,9 @@ __global__ void __launch_bounds__(PagedMmaCfg<HD, BULK, NS>::THREADS, BULK && NS
         const uint32_t sk = smem_u32(stages + (it % C::NSTAGE) * C::STAGE_BYTES), sv = sk + C::KV_BYTES;
         const int kw0 = warp * 16;                                  // this warp's 16 keys of the tile (row by row)
         if constexpr (BULK) {
-            // (a wait that runs out leaves a void result, never a hung CTA; the status word is the fragment calls')
-            wait_polls(bars + 8 * (it % C::NSTAGE), (uint32_t)(it / C::NSTAGE) & 1u);
+            ok = ok && __all_sync(0xffffffffu, mbar_wait_bounded(bars + 8 * (it % C::NSTAGE), (uint32_t)(it / C::NSTAGE) & 1u, is_void, a.status,
+                                                                 STATUS_WAIT_FULL_TIMEOUT));
+            if (!ok) continue;
             const int ntok = vis[f] - tok0;
             if (ntok < C::TILE) {
                 // the copies wrote nothing past the tile's end: probabilities there are exactly zero, but 0 * NaN would
@@ -552,7 +561,7 @@ __global__ void __launch_bounds__(PagedMmaCfg<HD, BULK, NS>::THREADS, BULK && NS
         *reinterpret_cast<float4*>(a.ws_o + (slot * kFmaRows + r) * HD + c) = acc;
         if (c == 0) {
             a.ws_m[slot * kFmaRows + r] = M;
-            a.ws_l[slot * kFmaRows + r] = L;
+            a.ws_l[slot * kFmaRows + r] = BULK && *is_void ? NAN : L;       // (the rows come out as NaN, not as something plausible)
         }
     }
 }

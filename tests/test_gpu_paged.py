@@ -196,3 +196,24 @@ def test_tensor_core_paged_kernel_is_refused_where_it_cannot_run():
         assert torch.isnan(out).all()                    # nothing ran
         rc, out = _run_paged(_cabi.KERNEL_AUTO, rq, loc, lens, kc, vc, table, 0.1)
         assert rc == 0 and torch.isfinite(out).all()
+
+
+@pytest.mark.parametrize("seqs,block", [([1, 1], 16), ([1, 1], 12), ([130, 1], 16)])      # bulk copies, row by row, tcgen05
+def test_status_word(seqs, block):
+    """The paged calls report to a status word as the fragment calls do: nothing in an ordinary call."""
+    from inference_lib_b200 import _cabi
+    gen = torch.Generator(device=DEV).manual_seed(1)
+    kc, vc = (torch.randn(40, 2, block, 128, device=DEV, generator=gen).bfloat16() for _ in range(2))
+    table = torch.arange(1400, dtype=torch.int32, device=DEV).reshape(2, 700) % 40
+    total = sum(seqs)
+    lens = torch.full((1, 2), 20 * block, dtype=torch.int32, device=DEV)
+    loc = torch.arange(20 * block - total, 20 * block, dtype=torch.int32, device=DEV)[None]
+    out = torch.empty(total, 8, 128, dtype=torch.bfloat16, device=DEV)
+    status = torch.zeros(3, dtype=torch.int32, device=DEV)
+    problem, keep = _cabi.bind_paged(out=out, queries=torch.randn(1, total, 8, 128, device=DEV, generator=gen).bfloat16(), locations=loc,
+                                     fragment_lengths=lens, key_cache=kc, value_cache=vc, block_table=table, scale=0.1,
+                                     cu_seqlens_q=torch.tensor([0, seqs[0], total], dtype=torch.int32, device=DEV), status=status[1:2])
+    assert problem.device_status == status.data_ptr() + 4
+    assert _cabi.launch_paged(problem, torch.cuda.current_stream().cuda_stream) == 0
+    torch.cuda.synchronize()
+    assert status.tolist() == [0, 0, 0] and bool(torch.isfinite(out).all())
