@@ -293,7 +293,7 @@ typedef struct hogatt_paged_problem {
     int32_t num_blocks;            /* extent of the caches' first dimension, or 0 if unknown: packed calls with prompt chunks
                                       (f16 / bf16, E == Ev == 128, block_size 8 ... 128 a power of two or a multiple of
                                       128) run on the tcgen05 kernel where AUTO knows it */
-    int32_t* device_status;        /* device int or NULL: as in hogatt_problem; the rows of a wait that ran out are NaN */
+    int32_t* device_status;        /* device int or NULL: as in hogatt_problem; where a wait ran out the rows are NaN */
 } hogatt_paged_problem;
 
 size_t hogatt_paged_workspace_bytes(const hogatt_paged_problem* p);

@@ -53,8 +53,10 @@ int current_device_info(int* dev, int* sms, int* smem_optin) {
         HOGATT_CUDA_OK(cudaDeviceGetAttribute(&s, cudaDevAttrMultiProcessorCount, *dev));
         HOGATT_CUDA_OK(cudaDeviceGetAttribute(&m, cudaDevAttrMaxSharedMemoryPerBlockOptin, *dev));
         if (const char* ms = getenv("HOGATT_WAIT_LIMIT_MS")) {      // tests of the give-up path shorten every bounded wait
-            const unsigned long long ns = (unsigned long long)std::max(1, atoi(ms)) * 1000000ull;
+            const unsigned long long limit_ms = (unsigned long long)std::max(1, atoi(ms)), ns = limit_ms * 1000000ull;
+            const unsigned int polls = (unsigned int)std::min(limit_ms, 1000000ull) * kPollsPerMs;
             HOGATT_CUDA_OK(cudaMemcpyToSymbol(g_wait_limit_ns, &ns, sizeof(ns)));
+            HOGATT_CUDA_OK(cudaMemcpyToSymbol(g_wait_polls, &polls, sizeof(polls)));
         }
         d.smem_optin.store(m, std::memory_order_release);
         d.sms.store(s, std::memory_order_release);

@@ -74,7 +74,7 @@ struct DenseArgs {
     int* vis;              // [2 * blocks][F] visible keys per (tile, fragment)
     int4* start;           // [ctas] block, kv head, step inside the unit, steps of this CTA
     int4* merge;           // [blocks * Hkv] units left to the merge step: unit, first CTA, partials, one query tile
-    int* nmerge;
+    int* nmerge;           // [0] units on that list; [1] a CTA of the attention kernel gave up a wait: the call's result is void
     int4* rec;             // paged: [blocks] worker, first token, tokens
     // Partials.  The one CTA c leaves of unit u is slot c + u (both only ever grow along the list).  Four columns of a row are one
     // element and the rows are contiguous: a warp, one row per lane, stores and loads 512 consecutive bytes.
@@ -498,7 +498,10 @@ __global__ void __launch_bounds__(kDensePlanThreads) dense_plan_kernel(const __g
         }
     }
     __syncthreads();
-    if (tid == 0) *a.nmerge = s_list;
+    if (tid == 0) {
+        a.nmerge[0] = s_list;
+        a.nmerge[1] = 0;
+    }
 }
 
 // element offset of an output row
@@ -529,10 +532,13 @@ struct DenseSegment {
 struct DenseSegments {     // a consumer's end of the ring (every lane of the warp takes part)
     static constexpr int DEPTH = 4;
     uint32_t slots, full, empty, n;
-    __device__ __forceinline__ bool next(DenseSegment& d, int lane, int* status) {
+    __device__ __forceinline__ bool next(DenseSegment& d, int lane, int* status, bool& ok) {
         const uint32_t i = n % DEPTH;
-        bool ok = mbar_wait_polls(full + 8 * i, (n / DEPTH) & 1u, status, STATUS_WAIT_SYNC_TIMEOUT);
-        if (!__all_sync(0xffffffffu, ok)) return false;
+        const bool come = mbar_wait_polls(full + 8 * i, (n / DEPTH) & 1u, status, STATUS_WAIT_SYNC_TIMEOUT);
+        if (!__all_sync(0xffffffffu, come)) {
+            ok = false;
+            return false;
+        }
         const uint32_t at = slots + i * (uint32_t)sizeof(DenseSegment);
         asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(d.b), "=r"(d.h), "=r"(d.f), "=r"(d.flags) : "r"(at) : "memory");
         asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(d.vis0), "=r"(d.vis1), "=r"(d.t0), "=r"(d.t1) : "r"(at + 16) : "memory");
@@ -665,7 +671,7 @@ dense_attention_kernel(const __grid_constant__ DenseArgs a, const __grid_constan
             // ============================== K copies ==============================
             int stage = 0;
             uint32_t phase = 1;                      // of k_empty: the first round finds every stage free
-            while (ok && segs.next(d, lane, a.status)) {
+            while (ok && segs.next(d, lane, a.status, ok)) {
                 const int w = PAGED ? a.rec[d.b].x : 0;
 #pragma unroll 1
                 for (int t = d.t0; t < d.t1; ++t) {
@@ -734,7 +740,7 @@ dense_attention_kernel(const __grid_constant__ DenseArgs a, const __grid_constan
             int stage = 0, last_g = 0;
             uint32_t k_phase = 0, q_phase = 0, s_phase = 1, g_phase = 0;      // g_phase: bit g, the parity of S_g's next completion
             bool any = false;
-            while (ok && segs.next(d, lane, a.status)) {
+            while (ok && segs.next(d, lane, a.status, ok)) {
                 // the query tiles change: the last reader of the old ones must have finished
                 if (any)
                     ok = mbar_wait_polls(s_full + 8 * last_g, ((g_phase >> last_g) & 1u) ^ 1u, a.status, STATUS_WAIT_SYNC_TIMEOUT);
@@ -761,7 +767,7 @@ dense_attention_kernel(const __grid_constant__ DenseArgs a, const __grid_constan
                     }
                 }
                 __syncwarp();
-                ok = mbar_wait_polls(q_full, q_phase, a.status, STATUS_WAIT_FULL_TIMEOUT);
+                ok = __all_sync(0xffffffffu, mbar_wait_polls(q_full, q_phase, a.status, STATUS_WAIT_FULL_TIMEOUT));
                 q_phase ^= 1u;
 #pragma unroll 1
                 for (int t = d.t0; t < d.t1 && ok; ++t) {
@@ -805,12 +811,12 @@ dense_attention_kernel(const __grid_constant__ DenseArgs a, const __grid_constan
             const uint64_t v_desc = umma_desc(sbase + C::OFF_V, C::ATOM_BYTES, 1024);
             int stage = 0;
             uint32_t v_phase = 0, g_phase = 0, started = 0;      // bit g: parity of P_g; O_g holds something
-            while (ok && segs.next(d, lane, a.status)) {
+            while (ok && segs.next(d, lane, a.status, ok)) {
                 if (d.first()) started = 0;
                 const int vlen = max(d.vis0, d.vis1);
 #pragma unroll 1
                 for (int t = d.t0; t < d.t1 && ok; ++t) {
-                    ok = mbar_wait_polls(v_full + 8 * stage, v_phase, a.status, STATUS_WAIT_FULL_TIMEOUT);
+                    ok = __all_sync(0xffffffffu, mbar_wait_polls(v_full + 8 * stage, v_phase, a.status, STATUS_WAIT_FULL_TIMEOUT));
                     if ((t + 1) * kDenseTile > vlen && ok) {
                         // The tile runs past the keys that any row of the block sees: what follows may hold anything (spare
                         // rows of a slab or cache block).  Those probabilities are exactly zero, but 0 * NaN would poison O.
@@ -876,7 +882,7 @@ dense_attention_kernel(const __grid_constant__ DenseArgs a, const __grid_constan
         // The two warps of a pair leave together, also when a wait has run out: a barrier the other one never reaches
         // could not be given up.
         while (true) {
-            const bool more = segs.next(d, lane, a.status);
+            const bool more = segs.next(d, lane, a.status, ok);
             if (pair_any(pair_bar, !more)) break;
             if (d.first()) {
                 int4 rec = make_int4(0, 0, 0, 0);
@@ -1028,13 +1034,14 @@ dense_attention_kernel(const __grid_constant__ DenseArgs a, const __grid_constan
         }
     }
 
-    // ---- common exit: nobody leaves before the copies in flight have landed and tensor memory can be handed back ----
-    if (!ok && lane == 0 && warp >= W_K) {
-        const uint64_t since = global_timer_ns();              // (given up: a pending stage completes its transfer at the latest)
-        while (global_timer_ns() - since < 1000000ull) {}
-    }
+    // ---- common exit: nobody leaves before the copies and products in flight have ended and tensor memory can be handed
+    // back.  In an ordinary call the last segment's readers have waited for all of them. ----
     tc_fence_before();
-    __syncthreads();
+    if (__syncthreads_or(!ok)) {
+        if (tid == 0) a.nmerge[1] = 1;                         // the merge step leaves NaN
+        settle();
+        __syncthreads();
+    }
     if (warp == W_S) {
         tc_fence_after();
         tmem_dealloc(tmem, C::TMEM_COLS);
@@ -1053,7 +1060,19 @@ __global__ void __launch_bounds__((SPLIT > 1 ? SPLIT : kDenseMergeWarps) * 32) d
     const int c4 = (SPLIT > 1 ? blockIdx.z : blockIdx.z * kDenseMergeWarps + warp) * 4;
     pdl_wait();
     pdl_trigger();
-    const int n = *a.nmerge;
+    const int2 head = *reinterpret_cast<const int2*>(a.nmerge);
+    if (head.y != 0) {
+        // given up: nothing that looks like a result (0x7FFF is a NaN of both types)
+        const size_t per = (size_t)(PAGED ? a.total_q : a.S) * a.Hq * (128 / 8), all = (PAGED ? 1 : a.W) * per;
+        const size_t cta = blockIdx.x + (size_t)gridDim.x * (blockIdx.y + (size_t)gridDim.y * blockIdx.z), ctas = (size_t)gridDim.x * gridDim.y * gridDim.z;
+        for (size_t i = cta * blockDim.x + threadIdx.x; i < all; i += ctas * blockDim.x) {
+            const size_t w = i / per, at = a.world > 0 ? (w * a.world + a.rank) * per + i % per : i;
+            for (int p = 0; p < max(a.world, 1); ++p)
+                static_cast<uint4*>(a.world > 0 ? a.peer_out[p] : a.out)[at] = make_uint4(0x7FFF7FFFu, 0x7FFF7FFFu, 0x7FFF7FFFu, 0x7FFF7FFFu);
+        }
+        return;
+    }
+    const int n = head.x;
     for (int i = blockIdx.x; i < n; i += gridDim.x) {
         const int4 e = a.merge[i];
         const int b = e.x / a.Hkv, h = e.x - b * a.Hkv, count = e.z;

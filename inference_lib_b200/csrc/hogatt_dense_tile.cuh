@@ -476,9 +476,13 @@ tile_attention_kernel(const __grid_constant__ KernelArgs a, const __grid_constan
         }
     }
 
-    // ---- common exit: nobody leaves before tensor memory can be handed back ----
+    // ---- common exit: nobody leaves before tensor memory can be handed back (given up: before what is in flight has ended) ----
     tc_fence_before();
     __syncthreads();
+    if (*abort_flag) {
+        settle();
+        __syncthreads();
+    }
     if (warp == kTileSoftmaxWarps + 1) {
         tc_fence_after();
         tmem_dealloc(tmem, C::TMEM_COLS);

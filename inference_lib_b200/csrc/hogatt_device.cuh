@@ -212,13 +212,22 @@ __device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, volat
     return true;
 }
 
-// A bounded wait of a few instructions and without a call, for kernels that cannot have calls or must stay small: 2^20 polls
-// are between 10 ms and a few seconds.
+// The same limit without a call and in a few instructions, for kernels that cannot have calls or must stay small: it counts
+// failing polls, each of which the hardware holds for 3.96 us (B200).
+constexpr unsigned int kPollsPerMs = 250;
+__device__ unsigned int g_wait_polls = 1000u * kPollsPerMs;
 __device__ __forceinline__ bool wait_polls(uint32_t bar, uint32_t parity) {
+    unsigned int polls = 0;
 #pragma unroll 1
-    for (int i = 0; i < (1 << 20); ++i)
-        if (mbar_try_wait(bar, parity)) return true;
-    return false;
+    while (!mbar_try_wait(bar, parity))
+        if (++polls > g_wait_polls) return false;
+    return true;
+}
+
+// After a wait that ran out: copies and products in flight take microseconds; a millisecond later there are none.
+__device__ __forceinline__ void settle() {
+    const uint64_t since = global_timer_ns();
+    while (global_timer_ns() - since < 1000000ull) {}
 }
 
 // A CTA must not leave while copies may still be landing in its shared memory.  Unlike the waits above this one neither

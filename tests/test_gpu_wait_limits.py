@@ -67,3 +67,60 @@ def test_a_peer_that_never_reports_makes_the_wait_give_up():
     env = dict(os.environ, HOGATT_WAIT_LIMIT_MS="60")
     res = subprocess.run([sys.executable, "-c", SCRIPT.format(root=ROOT)], env=env, capture_output=True, text=True, timeout=300)
     assert res.returncode == 0 and "WAIT_LIMIT_OK" in res.stdout, res.stdout[-2000:] + res.stderr[-4000:]
+
+
+IDLE = r"""
+import os, sys, torch
+sys.path.insert(0, {root!r})
+from inference_lib_b200 import _cabi
+# One CTA, one block of two query tiles (a worker each).  The second worker sees nothing of the long first fragment: its
+# softmax warps wait for the first tile of the second fragment meanwhile, some ten milliseconds.
+dev, long, W, G, S, E = torch.device("cuda:0"), {keys}, 2, 8, 16, 128
+gen = torch.Generator(device=dev).manual_seed(1)
+lengths = [long, 300, 200]
+keys, values = ([torch.randn(1, n, E, device=dev, generator=gen).bfloat16() for n in lengths] for _ in range(2))
+q = torch.randn(3, W, G, S, E, device=dev, generator=gen).bfloat16()
+loc = torch.tensor(lengths, dtype=torch.int32)[:, None, None].expand(3, W, S).contiguous() - 1
+loc[0, 1] = -1
+status = torch.zeros(1, dtype=torch.int32, device=dev)
+
+def call(loc):
+    out = torch.zeros(W, G, S, E, dtype=torch.bfloat16, device=dev)
+    loc = loc.to(dev)
+    bp = _cabi.bind(out=out, queries=q, locations=loc, keys=keys, values=values, scale=E ** -0.5, status=status, max_ctas=1)
+    _cabi.attach_workspace(bp, dev)
+    assert _cabi.launch_shape(bp)["kernels_per_call"] == 3                   # plan, attention, merge
+    status.zero_()
+    rc = _cabi.launch(bp, torch.cuda.current_stream(dev).cuda_stream)
+    torch.cuda.synchronize()
+    assert rc == 0
+    return out, int(status.item())
+
+def check(out, w, fragments):
+    k, v = (torch.cat([x[f][0] for f in fragments]).float() for x in (keys, values))
+    s = torch.cat([q[f, w].float() @ keys[f][0].float().T for f in fragments], -1) * E ** -0.5
+    assert float((out[w].float() - torch.softmax(s, -1) @ v).abs().max()) < 3e-3
+
+out, code = call(loc)
+if "HOGATT_WAIT_LIMIT_MS" in os.environ:
+    assert code & 7 and bool(torch.isnan(out).all()), (code, out)            # said so, and nothing that looks like a result
+    loc[0] = -1                                                              # an ordinary call right after it
+    out, code = call(loc)
+    check(out, 0, [1, 2])
+else:
+    check(out, 0, [0, 1, 2])
+check(out, 1, [1, 2])
+assert code == 0, code
+print("IDLE_OK")
+"""
+
+
+@pytest.mark.parametrize("limit", [None, "1"])
+def test_a_long_idle_wait_is_not_given_up_before_the_limit(limit):
+    """Within the ordinary limit such a call is fine; with one of a millisecond the idle warps give up, the others follow, the
+    status word and the output say so, and the next call is fine."""
+    env = {k: v for k, v in os.environ.items() if k != "HOGATT_WAIT_LIMIT_MS"}
+    if limit:
+        env["HOGATT_WAIT_LIMIT_MS"] = limit
+    res = subprocess.run([sys.executable, "-c", IDLE.format(root=ROOT, keys=1 << 21)], env=env, capture_output=True, text=True, timeout=300)
+    assert res.returncode == 0 and "IDLE_OK" in res.stdout, res.stdout[-2000:] + res.stderr[-4000:]
