@@ -289,7 +289,8 @@ typedef struct hogatt_paged_problem {
     size_t  workspace_bytes;
     int32_t kernel;                /* HOGATT_KERNEL_AUTO, _FMA (CUDA cores: any dtype and head size above) or _MMA
                                       (mma.sync tensor cores: f16 / bf16 with E == Ev == 64 or 128; what AUTO takes
-                                      there unless HOGATT_PAGED_MMA=0 is set in the environment) */
+                                      there, or the tcgen05 kernel (num_blocks), unless HOGATT_PAGED_MMA=0 is set in
+                                      the environment) */
     int32_t num_blocks;            /* extent of the caches' first dimension, or 0 if unknown: packed calls with prompt chunks
                                       (f16 / bf16, E == Ev == 128, block_size 8 ... 128 a power of two or a multiple of
                                       128) run on the tcgen05 kernel where AUTO knows it */

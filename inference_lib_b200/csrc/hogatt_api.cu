@@ -1018,6 +1018,15 @@ struct PagedPlan {
     size_t o, m, l, total;          // the other kernels' workspace
 };
 
+// HOGATT_PAGED_MMA=0 in the environment keeps AUTO on the CUDA-core paged kernel (A/B measurements).
+bool paged_mma_disabled() {
+    static const bool off = [] {
+        const char* v = getenv("HOGATT_PAGED_MMA");
+        return v && v[0] == '0';
+    }();
+    return off;
+}
+
 // Packed queries on the tcgen05 kernel: 16-bit types, head size 128, cache blocks that tile a 128-key tile in whole
 // 8-row swizzle groups (or hold whole tiles), the number of blocks known (a tensor map needs the extent).  AUTO takes it
 // where the prompt chunks of the batch -- the tokens beyond one per sequence, over as many keys as the block table has room
@@ -1025,7 +1034,8 @@ struct PagedPlan {
 // tcgen05 kernel takes 12 us more before and after.  Two chunks of 512 tokens at 6,000 keys: 119 us against 813, one of 300 at
 // 1,000 keys 29 against 71, one of 33 at 6,000 keys 68 against 81; one of 175 over 2 kv heads and 718 keys 27 against 21.
 bool paged_dense_wanted(const hogatt_paged_problem* p) {
-    if (p->kernel != HOGATT_KERNEL_AUTO || p->cu_seqlens_q == nullptr || dense_disabled() || p->num_blocks <= 0) return false;
+    if (p->kernel != HOGATT_KERNEL_AUTO || p->cu_seqlens_q == nullptr || p->num_blocks <= 0) return false;
+    if (dense_disabled() || paged_mma_disabled()) return false;
     if ((p->dtype != HOGATT_F16 && p->dtype != HOGATT_BF16) || p->E != 128 || p->Ev != 128) return false;
     const int G = p->Hq / p->Hkv, bs = p->block_size;
     if (G > kDenseRows || !(bs % kDenseTile == 0 || (kDenseTile % bs == 0 && bs % 8 == 0))) return false;
@@ -1120,15 +1130,6 @@ int launch_paged(const PagedArgs& a, const PagedPlan& pl, int dev, int smem_opti
     paged_merge_kernel<T><<<dim3(pl.units, kFmaRows / kMergeWarps), kMergeWarps * 32, 0, stream>>>(a);
     HOGATT_CUDA_OK(cudaGetLastError());
     return HOGATT_OK;
-}
-
-// HOGATT_PAGED_MMA=0 in the environment keeps AUTO on the CUDA-core paged kernel (A/B measurements).
-bool paged_mma_disabled() {
-    static const bool off = [] {
-        const char* v = getenv("HOGATT_PAGED_MMA");
-        return v && v[0] == '0';
-    }();
-    return off;
 }
 
 template <class T, int HD, bool BULK, int NS>

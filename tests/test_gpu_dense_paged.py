@@ -1,4 +1,8 @@
 """Packed queries over a paged cache on the tcgen05 kernel: AUTO's choice once the prompt chunks of a batch fill a query tile."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 import torch
@@ -139,3 +143,22 @@ def test_scales_that_are_not_positive(scale):
     p = _packed(torch.bfloat16, 2, 4, 16, [200, 1], [700, 650], room=5000)
     flipped = dict(p, queries=-p["queries"] if scale < -0.01 else torch.zeros_like(p["queries"]))
     check_against(_run(p, scale), _oracle(flipped, max(0.01, -scale)).numpy(), torch.bfloat16)
+
+
+SWITCH = """
+from inference_lib_b200 import _cabi
+p = _cabi.PagedProblem()
+p.F, p.W, p.Hq, p.Hkv, p.E, p.Ev, p.dtype, p.cu_seqlens_q = 1, 4, 16, 4, 128, 128, _cabi.BF16, 1
+p.total_q_tokens, p.num_blocks, p.block_size, p.max_blocks_per_seq = 300, 256, 16, 64
+needs = []
+for p.kernel in (_cabi.KERNEL_AUTO, _cabi.KERNEL_FMA):
+    needs.append(_cabi.load().hogatt_paged_workspace_bytes(p))
+print("SAME" if needs[0] == needs[1] else "OTHER")
+"""
+
+
+@pytest.mark.parametrize("env,route", [({}, "OTHER"), ({"HOGATT_PAGED_MMA": "0"}, "SAME"), ({"HOGATT_DENSE": "0"}, "SAME")])
+def test_switches_keep_auto_off_it(env, route):
+    root = os.path.abspath(os.path.join(os.path.dirname(__file__), ".."))
+    res = subprocess.run([sys.executable, "-c", SWITCH], env=dict(os.environ, **env), capture_output=True, text=True, timeout=300, cwd=root)
+    assert res.returncode == 0 and res.stdout.split() == [route], res.stdout + res.stderr[-2000:]
