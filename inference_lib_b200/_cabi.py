@@ -325,7 +325,7 @@ def bind_paged(*, out, queries, locations, fragment_lengths, key_cache, value_ca
     else:
         p.F, p.W, p.Hq, p.S, p.E = queries.shape
     p.Hkv, p.block_size, p.Ev = key_cache.shape[1], key_cache.shape[2], value_cache.shape[3]
-    p.max_blocks_per_seq, p.num_blocks = block_table.shape[1], key_cache.shape[0]
+    p.max_blocks_per_seq, p.num_blocks = block_table.shape[1], min(key_cache.shape[0], value_cache.shape[0])
     p.dtype, p.scale, p.kernel = dtype_code(out.dtype), float(scale), int(kernel)
     p.out, p.queries, p.locations = out.data_ptr(), queries.data_ptr(), locations.data_ptr()
     p.fragment_lengths, p.key_cache, p.value_cache = fragment_lengths.data_ptr(), key_cache.data_ptr(), value_cache.data_ptr()

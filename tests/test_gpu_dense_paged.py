@@ -162,3 +162,12 @@ def test_switches_keep_auto_off_it(env, route):
     root = os.path.abspath(os.path.join(os.path.dirname(__file__), ".."))
     res = subprocess.run([sys.executable, "-c", SWITCH], env=dict(os.environ, **env), capture_output=True, text=True, timeout=300, cwd=root)
     assert res.returncode == 0 and res.stdout.split() == [route], res.stdout + res.stderr[-2000:]
+
+
+def test_the_extent_of_caches_of_different_sizes():
+    """A tensor map must not reach past the smaller cache."""
+    p = {k: v.to(DEV) for k, v in _packed(torch.bfloat16, 2, 4, 16, [130, 1], [300, 300], room=5000).items()}
+    for name in ("key_cache", "value_cache"):
+        q = dict(p, **{name: torch.cat([p[name], p[name][:3]])})
+        problem, _ = _cabi.bind_paged(out=torch.empty(131, 8, 128, dtype=torch.bfloat16, device=DEV), scale=0.1, **q)
+        assert problem.num_blocks == min(q["key_cache"].shape[0], q["value_cache"].shape[0])
