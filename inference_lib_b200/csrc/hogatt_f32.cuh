@@ -46,20 +46,10 @@ __device__ __forceinline__ float warp_max(float x) {
     asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(y) : "f"(x));
     return y;
 }
-__device__ __forceinline__ uint64_t f32x2(float lo, float hi) {
-    uint64_t d;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
-    return d;
-}
-__device__ __forceinline__ float f32x2_sum(uint64_t v) {
+__device__ __forceinline__ float pair_sum(uint64_t v) {
     float lo, hi;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+    unpair_f32(v, lo, hi);
     return lo + hi;
-}
-__device__ __forceinline__ uint64_t f32x2_fma(uint64_t a, uint64_t b, uint64_t c) {
-    uint64_t d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
 }
 
 template <int HD, int R>
@@ -225,8 +215,8 @@ __global__ void __launch_bounds__(F32Cfg<HD, R>::THREADS, 1) f32_attention_kerne
 #pragma unroll
                     for (int r = 0; r < RW; ++r) {
                         const ulonglong2 qv = *reinterpret_cast<const ulonglong2*>(qr + r * C::QPITCH + c * 4);
-                        s2[r] = f32x2_fma(kv.x, qv.x, s2[r]);
-                        s2[r] = f32x2_fma(kv.y, qv.y, s2[r]);
+                        s2[r] = fma2(kv.x, qv.x, s2[r]);
+                        s2[r] = fma2(kv.y, qv.y, s2[r]);
                     }
                 }
             }
@@ -241,7 +231,7 @@ __global__ void __launch_bounds__(F32Cfg<HD, R>::THREADS, 1) f32_attention_kerne
             float top[RW];
 #pragma unroll
             for (int r = 0; r < RW; ++r) {
-                s[r] = my_key < ntok && key < lim[r] ? f32x2_sum(s2[r]) * a.l2scale : -INFINITY;
+                s[r] = my_key < ntok && key < lim[r] ? pair_sum(s2[r]) * a.l2scale : -INFINITY;
                 top[r] = fmaxf(m[r], warp_max(s[r]));
                 grew |= top[r] != m[r];
             }
@@ -249,10 +239,10 @@ __global__ void __launch_bounds__(F32Cfg<HD, R>::THREADS, 1) f32_attention_kerne
 #pragma unroll
                 for (int r = 0; r < RW; ++r) {
                     const float alpha = m[r] == -INFINITY ? 0.f : exp2f(m[r] - top[r]);
-                    const uint64_t al2 = f32x2(alpha, alpha);
+                    const uint64_t al2 = pair_f32(alpha, alpha);
                     l[r] *= alpha;
-                    o[r][0] = f32x2_fma(o[r][0], al2, 0ull);
-                    o[r][1] = f32x2_fma(o[r][1], al2, 0ull);
+                    o[r][0] = fma2(o[r][0], al2, 0ull);
+                    o[r][1] = fma2(o[r][1], al2, 0ull);
                     m[r] = top[r];
                 }
             }
@@ -284,9 +274,9 @@ __global__ void __launch_bounds__(F32Cfg<HD, R>::THREADS, 1) f32_attention_kerne
                             const float pr[4] = {p.x, p.y, p.z, p.w};
 #pragma unroll
                             for (int e = 0; e < 4; ++e) {
-                                const uint64_t pp = f32x2(pr[e], pr[e]);
-                                o[r + e][0] = f32x2_fma(vv.x, pp, o[r + e][0]);
-                                o[r + e][1] = f32x2_fma(vv.y, pp, o[r + e][1]);
+                                const uint64_t pp = pair_f32(pr[e], pr[e]);
+                                o[r + e][0] = fma2(vv.x, pp, o[r + e][0]);
+                                o[r + e][1] = fma2(vv.y, pp, o[r + e][1]);
                             }
                         }
                     }
@@ -310,8 +300,8 @@ __global__ void __launch_bounds__(F32Cfg<HD, R>::THREADS, 1) f32_attention_kerne
 #pragma unroll
                 for (int x = 16; x > 0; x >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, x);
                 float x[4];
-                asm("mov.b64 {%0, %1}, %2;" : "=f"(x[0]), "=f"(x[1]) : "l"(o[r][0]));
-                asm("mov.b64 {%0, %1}, %2;" : "=f"(x[2]), "=f"(x[3]) : "l"(o[r][1]));
+                unpair_f32(o[r][0], x[0], x[1]);
+                unpair_f32(o[r][1], x[2], x[3]);
                 if constexpr (HD == 64) {
 #pragma unroll
                     for (int e = 0; e < 4; ++e) x[e] += __shfl_xor_sync(0xffffffffu, x[e], 16);
