@@ -22,7 +22,7 @@
  *     an error is returned.  Unsupported shapes are an error (the reference prints a message and
  *     reports success with the output untouched, src/kernels/kernel_v21.cuh:992-995).
  *   - A row that can see no key at all produces zeros (as the reference kernel does,
- *     src/kernels/kernel_v21.cuh:238-245).
+ *     src/kernels/kernel_v21.cuh:238-245).  A row with a query, or a key that it sees, that is not a number is NaN.
  */
 #ifndef HOGATT_H_
 #define HOGATT_H_
@@ -83,7 +83,8 @@ typedef enum hogatt_status {
  * each issue a 16-token chunk), where the op is bound by the tensor pipe, not by HBM: 128-row query tiles, two to
  * a block where the call is long enough, tcgen05.mma with accumulators in tensor memory, K / V / Q tiles fetched by tensor-map TMA.  f16 / bf16,
  * E == Ev == 128, at most 16 fragments, and Hq/Hkv x S must divide 128 or be a multiple of it; AUTO takes it
- * whenever a problem qualifies, DENSE forces it (HOGATT_ERR_BAD_KERNEL_CHOICE otherwise).  It reads rotated
+ * whenever a problem qualifies and the scale lies between 1e-30 and 1e30 (the maximum of a row is taken before the
+ * scale, which therefore has to be positive), DENSE forces it (HOGATT_ERR_BAD_KERNEL_CHOICE otherwise).  It reads rotated
  * queries from memory, so the fused entry point first runs the stand-alone rotation kernel into `rq` (or into
  * the workspace when rq is NULL): three kernels per call, four with the plan kernel of the two-tile blocks. */
 typedef enum hogatt_kernel_choice {
@@ -119,7 +120,9 @@ typedef struct hogatt_problem {
     const int32_t* locations;         /* device [F,W,S]: key l of fragment f is visible to (w,s)
                                          iff l <= locations[f,w,s]                            */
     const int32_t* fragment_lengths;  /* device [F] or NULL: visible length of each fragment;
-                                         NULL means fragment_rows[f]                          */
+                                         NULL means fragment_rows[f].  Rows past it may hold
+                                         anything.  With host_lengths, rows below both that no
+                                         query sees must hold numbers (0 * NaN is NaN)        */
 
     const void* const* key_fragments;    /* host array of F device pointers, each [Hkv, rows_f, E]  */
     const void* const* value_fragments;  /* host array of F device pointers, each [Hkv, rows_f, Ev] */
@@ -399,6 +402,10 @@ int hogatt_append_launch(const hogatt_append* p, hogatt_stream_t stream);
  * (cluster shape: units x CTAs per cluster), plan[6] = partial-result slots per unit (cluster shape:
  * CTAs per cluster), plan[7] = kernel chosen (hogatt_kernel_choice; HOGATT_KERNEL_MMA_CLUSTER when
  * the cluster shape would run, taking visible_rows as the fragments' row counts).
+ * It describes equal units cut into balanced ranges.  Two kinds of call run on a kernel with a cut of its own where this
+ * reports the general one: the tcgen05 kernel's blocks of two query tiles (256 rows, steps of 128 keys of which a block has
+ * only those that its rows see; see hogatt_dense_plan, and hogatt_launch_shape for whether a call takes them), and fp32 with
+ * E == Ev == 64 or 128 (tiles of 64 keys).
  * Used by the tests of the split-K decomposition; has no reference counterpart (the reference
  * derives `splits` inline, src/kernels/kernel_v21.cuh:957-964).
  */

@@ -1031,8 +1031,11 @@ bool paged_mma_disabled() {
 // 8-row swizzle groups (or hold whole tiles), the number of blocks known (a tensor map needs the extent).  AUTO takes it
 // where the prompt chunks of the batch -- the tokens beyond one per sequence, over as many keys as the block table has room
 // for -- would keep the mma.sync kernel (115 TFLOP/s: it reads every sequence once per 16 rows) busy for some 20 us: the
-// tcgen05 kernel takes 12 us more before and after.  Two chunks of 512 tokens at 6,000 keys: 119 us against 813, one of 300 at
-// 1,000 keys 29 against 71, one of 33 at 6,000 keys 68 against 81; one of 175 over 2 kv heads and 718 keys 27 against 21.
+// tcgen05 kernel takes up to 12 us more before and after.  The lengths are on the device; where the table has far more room than
+// the sequences have keys the rule guesses too high, and costs little.  Tables of 32,768 keys, 8 kv heads of 4 heads, us per call
+// on the tcgen05 / mma.sync kernel: a chunk of 512 tokens at 4,000 keys 46 / 245, at 512 keys 26 / 58; 128 tokens at 1,000 keys
+// 26 / 35, at 128 keys 17 / 19; 64 tokens at 64 keys 17 / 17; 40 at 40 16 / 16; 128 at 128 beside 64 single tokens at 300 keys 80 /
+// 67, at 4,000 keys 226 / 237; beside 200 at 1,000 keys 262 / 396.
 bool paged_dense_wanted(const hogatt_paged_problem* p) {
     if (p->kernel != HOGATT_KERNEL_AUTO || p->cu_seqlens_q == nullptr || p->num_blocks <= 0) return false;
     if (dense_disabled() || paged_mma_disabled()) return false;
