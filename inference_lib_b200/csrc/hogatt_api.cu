@@ -1358,18 +1358,19 @@ int hogatt_copy_to_blocks_launch(const void* key_states, const void* value_state
     int dev = 0, sms = 0, smem_optin = 0;
     if (const int rc = current_device_info(&dev, &sms, &smem_optin)) return rc;
     const unsigned blocks = (unsigned)std::min<int64_t>((total + 255) / 256, (int64_t)sms * 8);   // 8 CTAs of 256 threads per SM
+    cudaError_t err = cudaSuccess;
     switch (dtype) {
         case HOGATT_F32:
-            copy_to_blocks_kernel<float><<<blocks, 256, 0, stream>>>((const float*)key_states, (const float*)value_states, (float*)key_cache, (float*)value_cache, block_table, seq_lengths, B, Hkv, S_new, E, Ev, block_size, max_blocks);
+            err = launch_kernel(copy_to_blocks_kernel<float>, dim3(blocks), dim3(256), 0, stream, (const float*)key_states, (const float*)value_states, (float*)key_cache, (float*)value_cache, block_table, seq_lengths, B, Hkv, S_new, E, Ev, block_size, max_blocks);
             break;
         case HOGATT_F16:
-            copy_to_blocks_kernel<__half><<<blocks, 256, 0, stream>>>((const __half*)key_states, (const __half*)value_states, (__half*)key_cache, (__half*)value_cache, block_table, seq_lengths, B, Hkv, S_new, E, Ev, block_size, max_blocks);
+            err = launch_kernel(copy_to_blocks_kernel<__half>, dim3(blocks), dim3(256), 0, stream, (const __half*)key_states, (const __half*)value_states, (__half*)key_cache, (__half*)value_cache, block_table, seq_lengths, B, Hkv, S_new, E, Ev, block_size, max_blocks);
             break;
         default:
-            copy_to_blocks_kernel<__nv_bfloat16><<<blocks, 256, 0, stream>>>((const __nv_bfloat16*)key_states, (const __nv_bfloat16*)value_states, (__nv_bfloat16*)key_cache, (__nv_bfloat16*)value_cache, block_table, seq_lengths, B, Hkv, S_new, E, Ev, block_size, max_blocks);
+            err = launch_kernel(copy_to_blocks_kernel<__nv_bfloat16>, dim3(blocks), dim3(256), 0, stream, (const __nv_bfloat16*)key_states, (const __nv_bfloat16*)value_states, (__nv_bfloat16*)key_cache, (__nv_bfloat16*)value_cache, block_table, seq_lengths, B, Hkv, S_new, E, Ev, block_size, max_blocks);
             break;
     }
-    HOGATT_CUDA_OK(cudaGetLastError());
+    HOGATT_CUDA_OK(err);
     return HOGATT_OK;
 }
 
@@ -1478,8 +1479,7 @@ int hogatt_step_plan_launch(const hogatt_step_plan* p, hogatt_stream_t stream) {
     a.attention_scaling = p->attention_scaling;
     a.round_to = p->round_tables_to;
     a.loc = p->locations; a.cos = p->cosines; a.sin = p->sines;
-    step_plan_kernel<<<(unsigned)(p->F * p->W), 128, 0, reinterpret_cast<cudaStream_t>(stream)>>>(a);
-    HOGATT_CUDA_OK(cudaGetLastError());
+    HOGATT_CUDA_OK(launch_kernel(step_plan_kernel, dim3((unsigned)(p->F * p->W)), dim3(kStepPlanThreads), 0, reinterpret_cast<cudaStream_t>(stream), a));
     return HOGATT_OK;
 }
 
@@ -1530,11 +1530,10 @@ int hogatt_append_launch(const hogatt_append* p, hogatt_stream_t stream) {
     dim3 grid((unsigned)std::min<int64_t>((pieces + 255) / 256, 1 << 14), (unsigned)p->Hkv, (unsigned)p->W);
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     switch (p->dtype) {
-        case HOGATT_F32: append_kernel<float><<<grid, 256, 0, st>>>(a, 0); break;
-        case HOGATT_F16: append_kernel<__half><<<grid, 256, 0, st>>>(a, vectorised ? 1 : 0); break;
-        default: append_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(a, vectorised ? 1 : 0); break;
+        case HOGATT_F32: HOGATT_CUDA_OK(launch_kernel(append_kernel<float>, grid, dim3(256), 0, st, a, 0)); break;
+        case HOGATT_F16: HOGATT_CUDA_OK(launch_kernel(append_kernel<__half>, grid, dim3(256), 0, st, a, vectorised ? 1 : 0)); break;
+        default: HOGATT_CUDA_OK(launch_kernel(append_kernel<__nv_bfloat16>, grid, dim3(256), 0, st, a, vectorised ? 1 : 0)); break;
     }
-    HOGATT_CUDA_OK(cudaGetLastError());
     return HOGATT_OK;
 }
 

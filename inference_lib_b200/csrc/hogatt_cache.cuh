@@ -29,26 +29,41 @@ struct StepPlanArgs {
     float* sin;
 };
 
-// One CTA per (fragment, worker).  Thread 0 walks the worker's order backwards (at most F steps) to find
-// the fragment's end position; all threads then fill the S x R table rows.
-__global__ void __launch_bounds__(128) step_plan_kernel(const StepPlanArgs a) {
+// One CTA per (fragment, worker), four warps.  Bound by its chain of dependent loads, not by its few KB: lane k of warp 0
+// reads entry k, k + 32, ... of the worker's order and those fragments' lengths at once (walking the order from its end in one
+// thread was up to 2 F loads in a row).  All threads then fill the S x R table rows.
+constexpr int kStepPlanThreads = 128;
+__global__ void __launch_bounds__(kStepPlanThreads) step_plan_kernel(const StepPlanArgs a) {
     const int f = blockIdx.x / a.W, w = blockIdx.x % a.W;
     __shared__ int s_end;
-    if (threadIdx.x == 0) {
+    pdl_wait();
+    pdl_trigger();                    // (whoever follows waits for this grid before it reads what it writes)
+    if (threadIdx.x < 32) {
         // positions count from the end of the worker's sequence: the fragment that comes last in the order
         // ends at its own length, the one before it at the sum of both, ...  (attention.py:173-181)
-        int n = 0;
-        while (n < a.F && a.order[w * a.F + n] >= 0) ++n;
-        int pos = 0, end = -1;
-        for (int k = n - 1; k >= 0; --k) {
-            const int g = a.order[w * a.F + k];
-            pos += a.lengths[g];
-            if (g == f) {
-                end = pos;
-                break;
-            }
+        constexpr int PER = HOGATT_MAX_FRAGMENTS / 32;
+        const int lane = threadIdx.x;
+        int order[PER], n = a.F, at = -1, sum = 0;
+#pragma unroll
+        for (int i = 0; i < PER; ++i) order[i] = i * 32 + lane < a.F ? a.order[w * a.F + i * 32 + lane] : -1;
+#pragma unroll
+        for (int i = PER - 1; i >= 0; --i) {                       // the list ends at its first negative entry
+            const unsigned stop = __ballot_sync(0xffffffffu, order[i] < 0);
+            if (stop) n = min(a.F, i * 32 + __ffs(stop) - 1);
         }
-        s_end = end;
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {                            // where this fragment stands (the last time)
+            const unsigned here = __ballot_sync(0xffffffffu, order[i] == f && i * 32 + lane < n);
+            if (here) at = i * 32 + 31 - __clz(here);
+        }
+        if (at >= 0) {
+#pragma unroll
+            for (int i = 0; i < PER; ++i)
+                if (i * 32 + lane >= at && i * 32 + lane < n) sum += a.lengths[order[i]];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        }
+        if (lane == 0) s_end = at >= 0 ? sum : -1;
     }
     __syncthreads();
     const int end = s_end;            // -1: this worker does not have the fragment at all
@@ -115,77 +130,92 @@ __device__ __forceinline__ T rope_channel_lowp(const T* __restrict__ x, const T*
 }
 
 // grid: (row chunks, kv heads, sources); a thread handles one 16-byte piece of a key row and of a value row
-// when everything is 16-byte aligned, single elements otherwise.
+// when everything is 16-byte aligned, single elements otherwise.  A few KB: bound by launch and load latency.  The grid is
+// launched beside its predecessor, and lets its successor in once its own wait is over; a thread's source rows and tables are in
+// flight while the fragment's length is (four layers of 4 workers at 16 K keys, append and attention: 91.4 -> 80.0 us).
 template <class T>
 __global__ void __launch_bounds__(256) append_kernel(const __grid_constant__ AppendArgs a, const int vectorised) {
+    pdl_wait();
+    // (an attention call may read fragments that its caller declares stable before it waits for its predecessor: rows taken
+    // from another fragment may go to any fragment, so that form ends first)
+    if (!a.take_leading) pdl_trigger();
     const int w = blockIdx.z, h = blockIdx.y;
     const int f = a.write_to[w];
+    int start = a.len_in[f];
     const int n = a.new_rows ? min(max(a.new_rows[w], 0), a.S) : a.S;
     const int skip = a.take_leading ? 0 : a.S - n;      // left-masked: the first rows of the source are padding
-    int start = a.len_in[f];
+    const int cap = a.ft.e[f].rows;
+
+    const T* ksrc = static_cast<const T*>(a.k) + w * a.ks[0] + h * a.ks[1];
+    const T* vsrc = static_cast<const T*>(a.v) + w * a.vs[0] + h * a.vs[1];
+    constexpr int VEC = 16 / (int)sizeof(T);
+    const int kc = vectorised ? a.E / VEC : a.E, vc = vectorised ? a.Ev / VEC : a.Ev;     // pieces per row
+    const int per_row = kc + vc;
+    // piece c of source row sr: what goes into the fragment
+    auto piece = [&](int sr, int c) {
+        const T* krow = ksrc + sr * a.ks[2];
+        const size_t tab = (size_t)(w * a.ts[0] + sr * a.ts[1]);
+        uint4 out = make_uint4(0u, 0u, 0u, 0u);
+        T one;
+        if (c >= kc) {                                  // value piece: plain copy
+            const T* src = vsrc + sr * a.vs[2];
+            if (vectorised) return *reinterpret_cast<const uint4*>(src + (c - kc) * VEC);
+            one = src[c - kc];
+        } else if (!vectorised) {
+            if (a.tables_lowp || sizeof(T) == 4) {
+                // same type everywhere; in fp32 this is also exactly the fp32-table arithmetic
+                one = rope_channel_lowp<T>(krow, static_cast<const T*>(a.cos) + tab, static_cast<const T*>(a.sin) + tab, c, a.R);
+            } else {
+                one = Scalar<T>::from_float(rope_channel<T>(krow, static_cast<const float*>(a.cos) + tab,
+                                                            static_cast<const float*>(a.sin) + tab, c, a.R));
+            }
+        } else {
+            if constexpr (sizeof(T) == 2) {
+                if (a.tables_lowp) {
+                    T* tmp = reinterpret_cast<T*>(&out);
+#pragma unroll
+                    for (int e = 0; e < VEC; ++e)
+                        tmp[e] = rope_channel_lowp<T>(krow, static_cast<const T*>(a.cos) + tab, static_cast<const T*>(a.sin) + tab,
+                                                      c * VEC + e, a.R);
+                } else {
+                    out = rotate_chunk<T>(krow, static_cast<const float*>(a.cos) + tab, static_cast<const float*>(a.sin) + tab, c, a.R);
+                }
+            }
+            return out;
+        }
+        *reinterpret_cast<T*>(&out) = one;
+        return out;
+    };
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    int r = (int)floor_div(i, per_row), c = (int)(i - (int64_t)r * per_row);
+    uint4 got = make_uint4(0u, 0u, 0u, 0u);
+    if (r < n) got = piece(skip + r, c);
+
     for (int w2 = 0; w2 < w; ++w2)                      // sources that share a fragment append in source order
         if (a.write_to[w2] == f) start += a.new_rows ? min(max(a.new_rows[w2], 0), a.S) : a.S;
-    const int cap = a.ft.e[f].rows;
     const int fit = max(0, min(n, cap - start));
-    if (fit < n && threadIdx.x == 0 && blockIdx.x == 0 && h == 0 && a.status) atomicOr(a.status, STATUS_FRAGMENT_FULL);
+    T* kdst = static_cast<T*>(const_cast<void*>(a.ft.e[f].k)) + ((size_t)h * cap + start) * a.E;
+    T* vdst = static_cast<T*>(const_cast<void*>(a.ft.e[f].v)) + ((size_t)h * cap + start) * a.Ev;
+    while (r < fit) {
+        T* dst = c < kc ? kdst + (size_t)r * a.E : vdst + (size_t)r * a.Ev;
+        const int at = c < kc ? c : c - kc;
+        if (vectorised) *reinterpret_cast<uint4*>(dst + at * VEC) = got;
+        else dst[at] = *reinterpret_cast<const T*>(&got);
+        i += stride;
+        r = (int)floor_div(i, per_row);
+        c = (int)(i - (int64_t)r * per_row);
+        if (r < fit) got = piece(skip + r, c);
+    }
 
-    // lengths: one thread of the whole grid, from len_in (nobody writes it)
+    if (fit < n && threadIdx.x == 0 && blockIdx.x == 0 && h == 0 && a.status) atomicOr(a.status, STATUS_FRAGMENT_FULL);
+    // lengths: one warp of the whole grid, from len_in (nobody writes it)
     if (blockIdx.x == 0 && h == 0 && w == 0 && threadIdx.x < 32) {
         for (int g = threadIdx.x; g < a.F; g += 32) {
             int len = a.len_in[g];
             for (int w2 = 0; w2 < a.W; ++w2)
                 if (a.write_to[w2] == g) len += a.new_rows ? min(max(a.new_rows[w2], 0), a.S) : a.S;
             a.len_out[g] = min(len, a.ft.e[g].rows);
-        }
-    }
-
-    const T* ksrc = static_cast<const T*>(a.k) + w * a.ks[0] + h * a.ks[1];
-    const T* vsrc = static_cast<const T*>(a.v) + w * a.vs[0] + h * a.vs[1];
-    T* kdst = static_cast<T*>(const_cast<void*>(a.ft.e[f].k)) + ((size_t)h * cap + start) * a.E;
-    T* vdst = static_cast<T*>(const_cast<void*>(a.ft.e[f].v)) + ((size_t)h * cap + start) * a.Ev;
-    constexpr int VEC = 16 / (int)sizeof(T);
-    const int kc = vectorised ? a.E / VEC : a.E, vc = vectorised ? a.Ev / VEC : a.Ev;     // pieces per row
-    const int per_row = kc + vc;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < (int64_t)fit * per_row;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const int r = (int)(i / per_row), c = (int)(i % per_row);
-        const int sr = skip + r;
-        if (c >= kc) {                                  // value piece: plain copy
-            const int cv = c - kc;
-            if (vectorised)
-                *reinterpret_cast<uint4*>(vdst + (size_t)r * a.Ev + cv * VEC) =
-                    *reinterpret_cast<const uint4*>(vsrc + sr * a.vs[2] + cv * VEC);
-            else
-                vdst[(size_t)r * a.Ev + cv] = vsrc[sr * a.vs[2] + cv];
-            continue;
-        }
-        const T* krow = ksrc + sr * a.ks[2];
-        const size_t tab = (size_t)(w * a.ts[0] + sr * a.ts[1]);
-        if (!vectorised) {
-            T out;
-            if (a.tables_lowp || sizeof(T) == 4) {
-                // same type everywhere; in fp32 this is also exactly the fp32-table arithmetic
-                out = rope_channel_lowp<T>(krow, static_cast<const T*>(a.cos) + tab, static_cast<const T*>(a.sin) + tab, c, a.R);
-            } else {
-                out = Scalar<T>::from_float(rope_channel<T>(krow, static_cast<const float*>(a.cos) + tab,
-                                                            static_cast<const float*>(a.sin) + tab, c, a.R));
-            }
-            kdst[(size_t)r * a.E + c] = out;
-            continue;
-        }
-        if constexpr (sizeof(T) == 2) {
-            uint4 out;
-            if (a.tables_lowp) {
-                T tmp[VEC];
-#pragma unroll
-                for (int e = 0; e < VEC; ++e)
-                    tmp[e] = rope_channel_lowp<T>(krow, static_cast<const T*>(a.cos) + tab, static_cast<const T*>(a.sin) + tab,
-                                                  c * VEC + e, a.R);
-                out = *reinterpret_cast<const uint4*>(tmp);
-            } else {
-                out = rotate_chunk<T>(krow, static_cast<const float*>(a.cos) + tab, static_cast<const float*>(a.sin) + tab, c, a.R);
-            }
-            *reinterpret_cast<uint4*>(kdst + (size_t)r * a.E + c * VEC) = out;
         }
     }
 }
