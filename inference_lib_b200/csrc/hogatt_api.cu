@@ -215,7 +215,7 @@ int resolve(const hogatt_problem* p, Resolved* r) {
 }
 
 struct WorkspaceLayout {
-    size_t header, pre, cost, vis, start, merge, rec, o, m, l, rq, total;     // pre ... rec: the plan of the tcgen05 kernel
+    size_t header, pre, cost, vis, start, merge, fold, rec, o, m, l, rq, total;     // pre ... rec: the plan of the tcgen05 kernel
     int parts;
 };
 
@@ -244,7 +244,8 @@ void carve_dense(WorkspaceLayout* w, int64_t blocks, int Hkv, int F, int grid, b
     w->vis = w->cost + align_up((size_t)(blocks + 1) * sizeof(long long), 256);
     w->start = w->vis + align_up((size_t)blocks * 2 * F * sizeof(int), 256);
     w->merge = w->start + align_up((size_t)grid * sizeof(int4), 256);
-    w->rec = w->merge + align_up((size_t)blocks * Hkv * sizeof(int4), 256);
+    w->fold = w->merge + align_up((size_t)blocks * Hkv * sizeof(int4), 256);
+    w->rec = w->fold + align_up((size_t)blocks * Hkv * kDenseFoldInts * sizeof(int), 256);
     w->o = w->rec + (paged ? align_up((size_t)blocks * sizeof(int4), 256) : 0);
     w->m = w->o + slots * kDenseBlock * 128 * sizeof(float);
     w->l = w->m + align_up(slots * kDenseBlock * sizeof(float), 256);
@@ -717,15 +718,14 @@ int launch_dense_kernels(const DenseArgs& d, const DenseMaps& maps, int dev, int
     const int rc = ensure_smem_limit(dense_attention_kernel<T, PAGED>, dev, kDenseSmemBytes, granted);
     if (rc != HOGATT_OK) return rc;
     HOGATT_CUDA_OK(launch_kernel(dense_attention_kernel<T, PAGED>, dim3(d.ctas), dim3(kDenseThreads), kDenseSmemBytes, stream, d, maps));
-    // at most ctas - 1 units are split; more on the list are blocks of one tile or blind ones (the kernel walks the list)
+    // the merge step walks the plan's list, which holds few units or none where there are as many units as CTAs: no more CTAs
+    // than are resident at once
     const int64_t units = (int64_t)d.blocks * d.Hkv;
-    const unsigned gx = (unsigned)std::min<int64_t>(units, 2 * (int64_t)d.ctas);
+    const dim3 block(kDenseMergeWarps * 32);
     if (d.ctas > 8 * units)
-        HOGATT_CUDA_OK(launch_kernel(dense_merge_kernel<T, PAGED, kDenseMergeSplit>, dim3(gx, kDenseBlock / 32, 128 / 16),
-                                     dim3(kDenseMergeSplit * 32), 0, stream, d));
+        HOGATT_CUDA_OK(launch_kernel(dense_merge_kernel<T, PAGED, true>, dim3((unsigned)(64 * units)), block, 0, stream, d));
     else
-        HOGATT_CUDA_OK(launch_kernel(dense_merge_kernel<T, PAGED, 1>, dim3(gx, kDenseBlock / 32, 128 / (16 * kDenseMergeWarps)),
-                                     dim3(kDenseMergeWarps * 32), 0, stream, d));
+        HOGATT_CUDA_OK(launch_kernel(dense_merge_kernel<T, PAGED, false>, dim3((unsigned)std::min<int64_t>(8 * units, 2 * (int64_t)d.ctas)), block, 0, stream, d));
     return HOGATT_OK;
 }
 
@@ -733,6 +733,7 @@ void dense_workspace(DenseArgs* d, unsigned char* ws, const WorkspaceLayout& w) 
     d->nmerge = reinterpret_cast<int*>(ws + w.header);
     d->start = reinterpret_cast<int4*>(ws + w.start);
     d->merge = reinterpret_cast<int4*>(ws + w.merge);
+    d->fold = reinterpret_cast<int*>(ws + w.fold);
     d->pre = reinterpret_cast<long long*>(ws + w.pre);
     d->cost = reinterpret_cast<long long*>(ws + w.cost);
     d->vis = reinterpret_cast<int*>(ws + w.vis);

@@ -8,7 +8,8 @@
 // block walks only those, 128 keys per step -- of a causal prompt just over half (4,000 tokens: 543 us per call when
 // every block walked every key, 168 now) -- and the steps of all units are one list that a persistent grid of one
 // CTA per SM cuts into balanced contiguous ranges.  A unit that lies inside one range is normalised and stored by
-// its CTA; the others leave unnormalised partials for dense_merge_kernel.
+// its CTA; of a unit cut into a few parts, the CTA that finishes last folds the partials of the others; units of many
+// parts are left to dense_merge_kernel.
 //
 // A step.  Both tiles of the block use the K and V tile (64 KiB of copies per 16.8 MFLOP; each tile alone would be at
 // the SM's L2 bandwidth).  Where a block has only one tile, the second softmax group takes every other key tile
@@ -45,8 +46,15 @@ constexpr int kDenseSoftmaxWarps = 16;      // two groups of eight: one group pe
 constexpr int kDenseThreads = (kDenseSoftmaxWarps + 4) * 32;
 constexpr int kDensePlanThreads = 1024;
 constexpr int kDenseMaxCtas = 256;
-constexpr int kDenseMergeWarps = 4;         // warps per CTA of the merge step, with few partials per row
-constexpr int kDenseMergeSplit = 8;         // ... with many: they share a row's partials
+constexpr int kDenseMergeWarps = 8;         // warps per CTA of the merge step; with many partials per row they share a row's
+constexpr int kDenseMergeBatch = 4;         // partials of a row that a thread of it has in flight
+// CTAs of a unit up to which the last of them to finish folds the others' partials into its own rows, and nothing of it is left to
+// the merge step (which then ends 1.5 us after the attention kernel instead of 12).  It reads 128 KiB of each other one; more are
+// left to the merge step, which has the whole chip for them.  us per call with a line at 2 / 3 / 8: 5.6 CTAs per unit (1,024 rows
+// of 8 heads, 24,576 keys) 114.4 / 114.4 / 119.7; two or three (3 x 256 tokens, 5,700 keys) 125.4 / 124.9 / 124.9; before, with
+// every one of them in the merge step, 128 for the latter and 159 instead of 154 for a 4,000-token prompt.
+constexpr int kDenseFoldParts = 3;
+constexpr int kDenseFoldInts = 20;          // per unit: first CTA, CTAs (0: not folded there), two unused, arrivals left of 16 warps
 
 struct alignas(64) DenseMaps {
     CUtensorMap q;                          // rotated queries as [F, W, Hq, S, E] or [F, W, Hkv, G*S, E]; paged: [F, total_q, Hkv, G, E]
@@ -74,6 +82,7 @@ struct DenseArgs {
     int* vis;              // [2 * blocks][F] visible keys per (tile, fragment)
     int4* start;           // [ctas] block, kv head, step inside the unit, steps of this CTA
     int4* merge;           // [blocks * Hkv] units left to the merge step: unit, first CTA, partials, one query tile
+    int* fold;             // [blocks * Hkv][kDenseFoldInts], written for units that more than one CTA, or two halves of one, work on
     int* nmerge;           // [0] units on that list; [1] a CTA of the attention kernel gave up a wait: the call's result is void
     int4* rec;             // paged: [blocks] worker, first token, tokens
     // Partials.  The one CTA c leaves of unit u is slot c + u (both only ever grow along the list).  Four columns of a row are one
@@ -449,6 +458,18 @@ __global__ void __launch_bounds__(kDensePlanThreads) dense_plan_kernel(const __g
     // Where every CTA starts: equal shares of the steps and of the units' fixed costs.  pos[c]: its first step in the list of all.
     const long long N = total * a.Hkv, C = total_cost * a.Hkv;
     const int ctas = dense_ctas(N, C, singles, a.ctas);
+    // who folds unit u, which `count` CTAs from `first` on work on (in a block of one tile, two halves each)
+    auto leave = [&](int u, int first, int count, bool single) {
+        int4* const fold = reinterpret_cast<int4*>(a.fold + (size_t)u * kDenseFoldInts);
+        const int here = count <= kDenseFoldParts ? count : 0, left = single ? 2 * here : here;
+        fold[0] = make_int4(first, here, 0, 0);
+        if (here > 0) {
+#pragma unroll
+            for (int i = 1; i < kDenseFoldInts / 4; ++i) fold[i] = make_int4(left, left, left, left);
+        } else {
+            a.merge[atomicAdd(&s_list, 1)] = make_int4(u, first, single ? 2 * count : count, single ? 1 : 0);
+        }
+    };
     int4 st = make_int4(0, 0, 0, 0);
     if (tid < ctas) {
         DenseStart d;
@@ -463,7 +484,7 @@ __global__ void __launch_bounds__(kDensePlanThreads) dense_plan_kernel(const __g
             const long long s = pos[tid] - st.z;
             // the unit this CTA starts inside of, if no earlier CTA does
             if (st.z > 0 && !single_block(st.x) && pos[tid - 1] <= s)
-                a.merge[atomicAdd(&s_list, 1)] = make_int4(st.x * a.Hkv + st.y, tid - 1, dense_parts(pos, ctas, tid - 1, s + pre[st.x + 1] - pre[st.x]), 0);
+                leave(st.x * a.Hkv + st.y, tid - 1, dense_parts(pos, ctas, tid - 1, s + pre[st.x + 1] - pre[st.x]), false);
         }
         a.start[tid] = st;
     }
@@ -475,13 +496,13 @@ __global__ void __launch_bounds__(kDensePlanThreads) dense_plan_kernel(const __g
         const bool single = single_block(b);
         const long long steps = pre[b + 1] - pre[b];
         if (!single && steps > 0) continue;
-        int c0 = 0, count = 0;
         if (steps > 0) {
             const long long s = pre[b] * a.Hkv + h * steps;
-            c0 = dense_first_cta(pos, ctas, s);
-            count = 2 * dense_parts(pos, ctas, c0, s + steps);
+            const int c0 = dense_first_cta(pos, ctas, s);
+            leave((int)u, c0, dense_parts(pos, ctas, c0, s + steps), true);
+        } else {
+            a.merge[atomicAdd(&s_list, 1)] = make_int4((int)u, 0, 0, single ? 1 : 0);
         }
-        a.merge[atomicAdd(&s_list, 1)] = make_int4((int)u, c0, count, single ? 1 : 0);
     }
     __syncthreads();
     if (tid == 0) {
@@ -976,43 +997,112 @@ dense_attention_kernel(const __grid_constant__ DenseArgs a, const __grid_constan
                 if (!ok) break;
                 const float total = half ? *other + l_run : l_run + *other;
                 named_barrier_sync(pair_bar, 64);              // (read before it is written again)
-                const bool direct = d.whole() && !d.single();
-                const bool sectors = a.world == 0 && ((uintptr_t)a.out & 31u) == 0;
-                // (a group that saw nothing never touched its O: zeros)
-                const float factor = !any ? 0.f : direct ? (total > 0.f ? 1.f / total : 0.f) : 1.f;
-                const size_t slot = (size_t)blockIdx.x + (size_t)d.b * a.Hkv + d.h;
-                const int slot_row = g * kDenseRows + row;
-                float o[COLS];
-                tmem_ld32(o_addr, *reinterpret_cast<float(*)[32]>(&o[0]));
-                tmem_ld32(o_addr + 32, *reinterpret_cast<float(*)[32]>(&o[32]));
-                tmem_wait_ld();
-#pragma unroll
-                for (int k = 0; k < COLS; ++k) o[k] = any ? o[k] * factor : 0.f;
+                const bool direct = d.whole() && !d.single(), one_tile = d.single();
+                const int unit = d.b * a.Hkv + d.h, slot_row = g * kDenseRows + row;
+                const size_t slot = (size_t)blockIdx.x + unit;
+                const float m_own = m_run == -INFINITY ? -INFINITY : m_run * scale2;
+                int first = blockIdx.x, parts = 1;             // partials that make up the rows: CTAs from `first` on, or their halves
+                bool finish = direct;
                 if (!direct) {
-                    float4* const wo = a.ws_o + (slot * (C::HD / 4) + half * (COLS / 4)) * kDenseBlock + slot_row;
-#pragma unroll
-                    for (int k = 0; k < COLS / 4; ++k) wo[k * kDenseBlock] = make_float4(o[4 * k], o[4 * k + 1], o[4 * k + 2], o[4 * k + 3]);
-                    if (half == 0) {
-                        a.ws_m[slot * kDenseBlock + slot_row] = m_run == -INFINITY ? -INFINITY : m_run * scale2;
-                        a.ws_l[slot * kDenseBlock + slot_row] = total;
+                    // Warps of different CTAs that hold the same rows and columns count themselves off; the last one has all
+                    // that the others left.  Not known yet to be the last: leave a partial first.
+                    int* const fold = a.fold + (size_t)unit * kDenseFoldInts;
+                    int* const left = fold + 4 + (one_tile ? warp & 7 : warp);
+                    const int2 who = *reinterpret_cast<const int2*>(fold);
+                    if (who.y > 0) {
+                        first = who.x;
+                        parts = one_tile ? 2 * who.y : who.y;
+                        int n = 0;
+                        if (lane == 0) asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(n) : "l"(left) : "memory");
+                        finish = __shfl_sync(0xffffffffu, n, 0) == 1;
+                        __syncwarp();
                     }
-                } else if (id.valid) {
-                    const size_t offset = dense_out_offset<PAGED>(a, id, d.h) + half * COLS;
-                    uint32_t v[COLS / 16][8];
-#pragma unroll
-                    for (int k = 0; k < COLS / 2; ++k) v[k >> 3][k & 7] = pack2<T>(o[2 * k], o[2 * k + 1]);
+                    if (!finish) {
+                        float4* const wo = a.ws_o + (slot * (C::HD / 4) + half * (COLS / 4)) * kDenseBlock + slot_row;
 #pragma unroll 1
-                    for (int p = 0; p < max(a.world, 1); ++p) {
-                        T* const dst = static_cast<T*>(a.world > 0 ? a.peer_out[p] : a.out) + offset;
-                        if (sectors) {
+                        for (int c = 0; c < COLS; c += 32) {
+                            float o[32];
+                            tmem_ld32(o_addr + c, o);
+                            tmem_wait_ld();
 #pragma unroll
-                            for (int k = 0; k < COLS / 16; ++k) store_sector(dst + k * 16, v[k]);
-                        } else {
+                            for (int k = 0; k < 32; ++k) o[k] = any ? o[k] : 0.f;          // (a group that saw nothing never touched its O)
 #pragma unroll
-                            for (int k = 0; k < COLS / 8; ++k)
-                                reinterpret_cast<uint4*>(dst)[k] = make_uint4(v[k >> 1][(k & 1) * 4], v[k >> 1][(k & 1) * 4 + 1],
-                                                                              v[k >> 1][(k & 1) * 4 + 2], v[k >> 1][(k & 1) * 4 + 3]);
+                            for (int k = 0; k < 8; ++k) wo[(c / 4 + k) * kDenseBlock] = make_float4(o[4 * k], o[4 * k + 1], o[4 * k + 2], o[4 * k + 3]);
                         }
+                        a.ws_m[slot * kDenseBlock + slot_row] = m_own;                     // (both halves store the same)
+                        a.ws_l[slot * kDenseBlock + slot_row] = total;
+                        if (who.y > 0) {
+                            __syncwarp();
+                            int n = 0;
+                            if (lane == 0) {
+                                __threadfence();
+                                n = atomicSub(left, 1);
+                                __threadfence();
+                            }
+                            finish = __shfl_sync(0xffffffffu, n, 0) == 1;
+                            __syncwarp();
+                        }
+                    }
+                }
+                if (finish) {
+                    // out = sum_p O_p * 2^(m_p - M) / sum_p l_p * 2^(m_p - M), in the order of the parts whoever is last
+                    const bool sectors = a.world == 0 && ((uintptr_t)a.out & 31u) == 0;
+                    const int own = one_tile ? 2 * ((int)blockIdx.x - first) + g : (int)blockIdx.x - first;
+                    auto at = [&](int p) {
+                        const size_t sl = (size_t)first + unit + (one_tile ? p >> 1 : p);
+                        return sl * kDenseBlock + (one_tile ? (p & 1) * kDenseRows + row : slot_row);
+                    };
+                    float M = m_own, den = 0.f;
+#pragma unroll 1
+                    for (int p = 0; p < parts; ++p)
+                        if (p != own) M = fmaxf(M, __ldcg(a.ws_m + at(p)));
+                    const size_t offset = dense_out_offset<PAGED>(a, id, d.h) + half * COLS;
+#pragma unroll 1
+                    for (int c = 0; c < COLS; c += 32) {
+                        float acc[32];
+#pragma unroll
+                        for (int k = 0; k < 32; ++k) acc[k] = 0.f;
+                        den = 0.f;
+#pragma unroll 1
+                        for (int p = 0; p < parts; ++p) {
+                            float x[32], m = m_own, l = total;
+                            if (p == own) {
+                                tmem_ld32(o_addr + c, x);
+                                tmem_wait_ld();
+                            } else {
+                                const size_t i = at(p);
+                                m = __ldcg(a.ws_m + i);
+                                l = __ldcg(a.ws_l + i);
+                                const size_t sl = i / kDenseBlock, r = i % kDenseBlock;
+                                const float4* const src = a.ws_o + (sl * (C::HD / 4) + (half * COLS + c) / 4) * kDenseBlock + r;
+#pragma unroll
+                                for (int k = 0; k < 8; ++k) *reinterpret_cast<float4*>(x + 4 * k) = __ldcg(src + k * kDenseBlock);
+                            }
+                            const float w = m == -INFINITY ? 0.f : parts == 1 ? 1.f : exp2f(m - M);
+                            den = fmaf(l, w, den);
+                            if (p != own || any) {             // (what was never touched may hold anything)
+#pragma unroll
+                                for (int k = 0; k < 32; ++k) acc[k] = fmaf(x[k], w, acc[k]);
+                            }
+                        }
+                        const float inv = den > 0.f ? 1.f / den : 0.f;
+                        uint32_t v[2][8];
+#pragma unroll
+                        for (int k = 0; k < 16; ++k) v[k >> 3][k & 7] = pack2<T>(acc[2 * k] * inv, acc[2 * k + 1] * inv);
+#pragma unroll 1
+                        for (int q = 0; q < (id.valid ? max(a.world, 1) : 0); ++q) {
+                            T* const dst = static_cast<T*>(a.world > 0 ? a.peer_out[q] : a.out) + offset + c;
+                            if (sectors) {
+                                store_sector(dst, v[0]);
+                                store_sector(dst + 16, v[1]);
+                            } else {
+#pragma unroll
+                                for (int k = 0; k < 4; ++k)
+                                    reinterpret_cast<uint4*>(dst)[k] = make_uint4(v[k >> 1][(k & 1) * 4], v[k >> 1][(k & 1) * 4 + 1],
+                                                                                  v[k >> 1][(k & 1) * 4 + 2], v[k >> 1][(k & 1) * 4 + 3]);
+                            }
+                        }
+                        __syncwarp();
                     }
                 }
                 tc_fence_before();
@@ -1034,68 +1124,100 @@ dense_attention_kernel(const __grid_constant__ DenseArgs a, const __grid_constan
     }
 }
 
-// The units on the plan's list -- more than one CTA worked on them, or one left two halves, or nothing is visible --: fold
-// the partials, normalise, store.  Grid (units, 32-row groups, column groups); a warp takes 32 rows, one per lane, and 16
-// columns: every load of a partial is 512 consecutive bytes, a lane stores one 32-byte sector.  With SPLIT warps per CTA they
-// share the partials of the same rows and columns (a unit cut into a hundred parts would be a chain of as many loads).
+// The units on the plan's list -- more than kDenseFoldParts CTAs worked on them, or nothing is visible --: fold the partials,
+// normalise, store.  A warp takes 32 rows, one per lane, and 16 columns: every load of a partial is 512 consecutive bytes, a lane
+// stores one 32-byte sector.  A CTA is the eight column groups of 32 rows, or with SPLIT eight warps that share the partials of the
+// same rows and columns (a unit cut into a hundred parts would be a chain of as many loads); the grid walks the list.
+// Bound by its chain of dependent loads -- list, partials, store, about a microsecond each -- and by the wait in front of
+// them, so a row's statistics and values are fetched together, kDenseMergeBatch partials at a time, and rescaled when a
+// later batch has the larger maximum (1,024 rows of 8 heads, 24,576 keys, 5.6 partials each: 7 us from the attention kernel's
+// end to this one's, 10 when the list's length, its entry, the maxima and the values were fetched one after the other).
 //   out = sum_p O_p * 2^(m_p - M) / sum_p l_p * 2^(m_p - M),   M = max_p m_p
-template <class T, bool PAGED, int SPLIT>
-__global__ void __launch_bounds__((SPLIT > 1 ? SPLIT : kDenseMergeWarps) * 32) dense_merge_kernel(const __grid_constant__ DenseArgs a) {
-    __shared__ float part[SPLIT > 1 ? SPLIT : 1][18][32];                // 16 columns, maximum, sum; by row
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, r = blockIdx.y * 32 + lane;
-    const int c4 = (SPLIT > 1 ? blockIdx.z : blockIdx.z * kDenseMergeWarps + warp) * 4;
+template <class T, bool PAGED, bool SPLIT>
+__global__ void __launch_bounds__(kDenseMergeWarps * 32) dense_merge_kernel(const __grid_constant__ DenseArgs a) {
+    __shared__ float part[SPLIT ? kDenseMergeWarps : 1][18][32];         // 16 columns, maximum, sum; by row
+    constexpr int PER = SPLIT ? 64 : 8;                                  // CTAs' worth of work per unit
+    constexpr int STRIDE = SPLIT ? kDenseMergeWarps : 1, BATCH = kDenseMergeBatch;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     pdl_wait();
     pdl_trigger();
+    int4 e = a.merge[min((int)(blockIdx.x / PER), a.blocks * a.Hkv - 1)];       // (in flight with the list's length; not used past it)
     const int2 head = *reinterpret_cast<const int2*>(a.nmerge);
     if (head.y != 0) {
         // given up: nothing that looks like a result (0x7FFF is a NaN of both types)
         const size_t per = (size_t)(PAGED ? a.total_q : a.S) * a.Hq * (128 / 8), all = (PAGED ? 1 : a.W) * per;
-        const size_t cta = blockIdx.x + (size_t)gridDim.x * (blockIdx.y + (size_t)gridDim.y * blockIdx.z), ctas = (size_t)gridDim.x * gridDim.y * gridDim.z;
-        for (size_t i = cta * blockDim.x + threadIdx.x; i < all; i += ctas * blockDim.x) {
+        for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < all; i += (size_t)gridDim.x * blockDim.x) {
             const size_t w = i / per, at = a.world > 0 ? (w * a.world + a.rank) * per + i % per : i;
             for (int p = 0; p < max(a.world, 1); ++p)
                 static_cast<uint4*>(a.world > 0 ? a.peer_out[p] : a.out)[at] = make_uint4(0x7FFF7FFFu, 0x7FFF7FFFu, 0x7FFF7FFFu, 0x7FFF7FFFu);
         }
         return;
     }
-    const int n = head.x;
-    for (int i = blockIdx.x; i < n; i += gridDim.x) {
-        const int4 e = a.merge[i];
+    for (int64_t i = blockIdx.x; i < (int64_t)head.x * PER; i += gridDim.x) {
+        const int task = (int)(i % PER);
+        if (i != blockIdx.x) e = a.merge[i / PER];
+        const int r = (SPLIT ? task >> 3 : task) * 32 + lane, c4 = (SPLIT ? task & 7 : warp) * 4;
         const int b = e.x / a.Hkv, h = e.x - b * a.Hkv, count = e.z;
         const bool single = e.w != 0;
         // a block of one tile: both 128-row halves of a slot are partials of the same rows
-        if (single && blockIdx.y * 32 >= kDenseRows) continue;
+        if (single && (r & ~31) >= kDenseRows) continue;
+        int4 rec = make_int4(0, 0, 0, 0);
+        if constexpr (PAGED) rec = a.rec[b];
         const int sub = single ? 1 : 0;
         const size_t slot0 = (size_t)e.y + e.x;
-        const int p0 = SPLIT > 1 ? warp : 0;
-        auto row_of = [&](int p) { return (single ? (p & 1) * kDenseRows : 0) + r; };
-        auto slot_of = [&](int p) { return slot0 + (p >> sub); };
-        float M = -INFINITY;
-#pragma unroll 4
-        for (int p = p0; p < count; p += SPLIT) M = fmaxf(M, __ldcg(a.ws_m + slot_of(p) * kDenseBlock + row_of(p)));
-        float den = 0.f;
+        float M = -INFINITY, den = 0.f;
         float4 acc[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) acc[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 4
-        for (int p = p0; p < count; p += SPLIT) {
-            const size_t at = slot_of(p) * kDenseBlock + row_of(p);
-            const float m = __ldcg(a.ws_m + at), l = __ldcg(a.ws_l + at);
-            const float4* src = a.ws_o + (slot_of(p) * 32 + c4) * kDenseBlock + row_of(p);
-            const float wgt = m == -INFINITY ? 0.f : exp2f(m - M);       // (a partial that saw nothing holds zeros)
-            den = fmaf(l, wgt, den);
+#pragma unroll 1
+        for (int p0 = SPLIT ? warp : 0; p0 < count; p0 += BATCH * STRIDE) {
+            float m[BATCH], l[BATCH];
+            float4 x[BATCH][4];
+#pragma unroll
+            for (int j = 0; j < BATCH; ++j) {
+                const int p = p0 + j * STRIDE;
+                m[j] = -INFINITY;
+                l[j] = 0.f;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) x[j][k] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (p < count) {
+                    const size_t slot = slot0 + (p >> sub), row = (single ? (p & 1) * kDenseRows : 0) + r;
+                    m[j] = __ldcg(a.ws_m + slot * kDenseBlock + row);
+                    l[j] = __ldcg(a.ws_l + slot * kDenseBlock + row);
+                    const float4* src = a.ws_o + (slot * 32 + c4) * kDenseBlock + row;
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) x[j][k] = __ldcg(src + k * kDenseBlock);
+                }
+            }
+            float top = M;
+#pragma unroll
+            for (int j = 0; j < BATCH; ++j) top = fmaxf(top, m[j]);
+            const float old = M == -INFINITY ? 0.f : exp2f(M - top);
+            M = top;
+            den *= old;
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                const float4 x = __ldcg(src + k * kDenseBlock);
-                acc[k].x = fmaf(x.x, wgt, acc[k].x);
-                acc[k].y = fmaf(x.y, wgt, acc[k].y);
-                acc[k].z = fmaf(x.z, wgt, acc[k].z);
-                acc[k].w = fmaf(x.w, wgt, acc[k].w);
+                acc[k].x *= old;
+                acc[k].y *= old;
+                acc[k].z *= old;
+                acc[k].w *= old;
+            }
+#pragma unroll
+            for (int j = 0; j < BATCH; ++j) {
+                const float wgt = m[j] == -INFINITY ? 0.f : exp2f(m[j] - M);       // (a partial that saw nothing holds zeros)
+                den = fmaf(l[j], wgt, den);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    acc[k].x = fmaf(x[j][k].x, wgt, acc[k].x);
+                    acc[k].y = fmaf(x[j][k].y, wgt, acc[k].y);
+                    acc[k].z = fmaf(x[j][k].z, wgt, acc[k].z);
+                    acc[k].w = fmaf(x[j][k].w, wgt, acc[k].w);
+                }
             }
         }
         float* o = reinterpret_cast<float*>(acc);
-        if constexpr (SPLIT > 1) {
-            __syncthreads();                             // (the unit before has been read)
+        if constexpr (SPLIT) {
+            __syncthreads();                             // (the task before has been read)
 #pragma unroll
             for (int k = 0; k < 16; ++k) part[warp][k][lane] = o[k];
             part[warp][16][lane] = M;
@@ -1104,21 +1226,19 @@ __global__ void __launch_bounds__((SPLIT > 1 ? SPLIT : kDenseMergeWarps) * 32) d
             if (warp != 0) continue;
             float top = M;
 #pragma unroll
-            for (int w = 1; w < SPLIT; ++w) top = fmaxf(top, part[w][16][lane]);
+            for (int w = 1; w < kDenseMergeWarps; ++w) top = fmaxf(top, part[w][16][lane]);
             const float mine = M == -INFINITY ? 0.f : exp2f(M - top);
             den *= mine;
 #pragma unroll
             for (int k = 0; k < 16; ++k) o[k] *= mine;
 #pragma unroll
-            for (int w = 1; w < SPLIT; ++w) {
+            for (int w = 1; w < kDenseMergeWarps; ++w) {
                 const float mw = part[w][16][lane], wgt = mw == -INFINITY ? 0.f : exp2f(mw - top);
                 den = fmaf(part[w][17][lane], wgt, den);
 #pragma unroll
                 for (int k = 0; k < 16; ++k) o[k] = fmaf(part[w][k][lane], wgt, o[k]);
             }
         }
-        int4 rec = make_int4(0, 0, 0, 0);
-        if constexpr (PAGED) rec = a.rec[b];
         const DenseRow id = dense_row<PAGED>(a, 2 * b + r / kDenseRows, r % kDenseRows, rec);
         if (!id.valid) continue;
         const float inv = den > 0.f ? 1.f / den : 0.f;
