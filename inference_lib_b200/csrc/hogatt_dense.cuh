@@ -14,8 +14,8 @@
 // A step.  Both tiles of the block use the K and V tile (64 KiB of copies per 16.8 MFLOP; each tile alone would be at
 // the SM's L2 bandwidth).  Where a block has only one tile, the second softmax group takes every other key tile
 // of the same queries instead, and the two halves are two partials.
-//   warp 16  K copies (TMA, ring of 3 tiles)         warp 19  the walk over the steps, V copies (ring of 2)
-//   warp 17  query copies and S = Q K^T: one S buffer in tensor memory, used by the two groups in turn
+//   warp 16  query and K copies (TMA, rings of 2 and 3 tiles)      warp 19  the walk over the steps, V copies (ring of 2)
+//   warp 17  S = Q K^T: one S buffer in tensor memory, used by the two groups in turn
 //   warp 18  O_g += P_g V, P as the tensor-memory A operand
 //   warps 0-7 / 8-15  softmax of group 0 / 1: two threads per query row, 64 columns each (with one, which has 128
 //            exponentials in a row, a 1,024-row chunk call took 128 us instead of 122).  The scores go to registers at once, which frees the S buffer for the other
@@ -101,14 +101,15 @@ struct DenseCfg {
     static constexpr int HD = 128;
     static constexpr int ATOM_BYTES = 128 * 128;            // [128 rows][64 16-bit columns], rows of 128 bytes, swizzled
     static constexpr int TILE_BYTES = 2 * ATOM_BYTES;       // a 128 x 128 operand tile: two column halves
-    static constexpr int NK = 3, NV = 2;                    // K ring, V ring
-    static constexpr int OFF_Q = 0;                         // two query tiles
-    static constexpr int OFF_K = OFF_Q + 2 * TILE_BYTES;
+    static constexpr int NQ = 2, NK = 3, NV = 2;            // rings of query, K and V tiles
+    static constexpr int OFF_Q = 0;
+    static constexpr int OFF_K = OFF_Q + NQ * TILE_BYTES;
     static constexpr int OFF_V = OFF_K + NK * TILE_BYTES;
     static constexpr int OFF_BAR = OFF_V + NV * TILE_BYTES;                 // 224 KiB of tiles
     static constexpr int OFF_STAT = OFF_BAR;                                // [2 groups][2 halves][128 rows]: maxima or sums handed over
-    // barriers: q_full, k_full[NK], k_empty[NK], v_full[NV], v_empty[NV], s_full[2], s_free, p_full[2], o_done[2], segment full / empty
-    static constexpr int NBAR = 1 + 2 * NK + 2 * NV + 2 + 1 + 2 + 2 + 2 * 4;
+    // barriers: q_full[NQ], q_empty[NQ], k_full[NK], k_empty[NK], v_full[NV], v_empty[NV], s_full[2], s_free, p_full[2], o_done[2],
+    // segment full / empty
+    static constexpr int NBAR = 2 * NQ + 2 * NK + 2 * NV + 2 + 1 + 2 + 2 + 2 * 4;
     static constexpr int OFF_MBAR = OFF_STAT + 2 * 2 * kDenseRows * 4;
     static constexpr int OFF_SEG = (OFF_MBAR + NBAR * 8 + 15) / 16 * 16;
     static constexpr int OFF_MISC = OFF_SEG + 4 * 32;                       // tmem base
@@ -631,7 +632,7 @@ dense_attention_kernel(const __grid_constant__ DenseArgs a, const __grid_constan
     extern __shared__ __align__(1024) unsigned char dense_smem[];       // swizzled tiles start on 1 KiB boundaries
     unsigned char* const base = dense_smem;
     const uint32_t sbase = smem_u32(base);
-    const uint32_t q_full = sbase + C::OFF_MBAR, k_full = q_full + 8, k_empty = k_full + 8 * C::NK, v_full = k_empty + 8 * C::NK,
+    const uint32_t q_full = sbase + C::OFF_MBAR, q_empty = q_full + 8 * C::NQ, k_full = q_empty + 8 * C::NQ, k_empty = k_full + 8 * C::NK, v_full = k_empty + 8 * C::NK,
                    v_empty = v_full + 8 * C::NV, s_full = v_empty + 8 * C::NV, s_free = s_full + 16, p_full = s_free + 8,
                    o_done = p_full + 16, seg_full = o_done + 16, seg_empty = seg_full + 8 * DenseSegments::DEPTH;
     constexpr int W_K = kDenseSoftmaxWarps, W_S = W_K + 1, W_V = W_K + 3;        // (W_K + 2: the PV products)
@@ -639,7 +640,10 @@ dense_attention_kernel(const __grid_constant__ DenseArgs a, const __grid_constan
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid == 0) {
-        mbar_init(q_full, 1);
+        for (int s = 0; s < C::NQ; ++s) {
+            mbar_init(q_full + 8 * s, 1);
+            mbar_init(q_empty + 8 * s, 1);
+        }
         for (int s = 0; s < C::NK; ++s) {
             mbar_init(k_full + 8 * s, 1);
             mbar_init(k_empty + 8 * s, 1);
@@ -675,9 +679,11 @@ dense_attention_kernel(const __grid_constant__ DenseArgs a, const __grid_constan
     if (warp >= W_K) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
         if (warp == W_K) {
-            // ============================== K copies ==============================
-            int stage = 0;
-            uint32_t phase = 1;                      // of k_empty: the first round finds every stage free
+            // ============================== query and K copies ==============================
+            int stage = 0, q_slot = 0;
+            uint32_t phase = 1, q_phase = 1;         // of k_empty and q_empty: the first round finds every stage free
+            const int gs = a.G * a.S;
+            const uint32_t q_bytes = (uint32_t)(PAGED ? a.tile_span * a.G : (gs > kDenseRows ? kDenseRows : a.tile_span * gs)) * 256u;
             while (ok && segs.next(d, lane, a.status, ok)) {
                 const int w = PAGED ? a.rec[d.b].x : 0;
 #pragma unroll 1
@@ -690,6 +696,38 @@ dense_attention_kernel(const __grid_constant__ DenseArgs a, const __grid_constan
                         stage = 0;
                         phase ^= 1u;
                     }
+                    // The segment's query tiles, behind its first K tile: each as soon as the last product with the one before it
+                    // in its place has finished.
+#pragma unroll 1
+                    for (int part = 0; t == d.t0 && part < (d.single() ? 1 : 2); ++part) {
+                        ok = mbar_wait_polls(q_empty + 8 * q_slot, q_phase, a.status, STATUS_WAIT_EMPTY_TIMEOUT);
+                        ok = __all_sync(0xffffffffu, ok);
+                        if (!ok) break;
+                        if (elect_one()) {
+                            const uint32_t bar = q_full + 8 * q_slot;
+                            mbar_arrive_expect_tx(bar, q_bytes);
+#pragma unroll 1
+                            for (int i = 0; i < 2; ++i) {               // column halves
+                                const uint32_t dst = sbase + C::OFF_Q + q_slot * C::TILE_BYTES + i * C::ATOM_BYTES;
+                                const int tile = 2 * d.b + part;
+                                if constexpr (PAGED) {
+                                    tma_load_5d(dst, &maps.q, i * 64, 0, d.h, a.rec[d.b].y + part * a.tile_span, d.f, bar);
+                                } else if (a.tile_tokens > 0) {
+                                    const int qw = tile / a.tile_span;
+                                    tma_load_5d(dst, &maps.q, i * 64, (tile - qw * a.tile_span) * a.tile_tokens, d.h * a.G, qw, d.f, bar);
+                                } else {
+                                    const int qw = gs > kDenseRows ? tile / a.tile_span : tile * a.tile_span;
+                                    tma_load_5d(dst, &maps.q, i * 64, gs > kDenseRows ? (tile - qw * a.tile_span) * kDenseRows : 0, d.h, qw, d.f, bar);
+                                }
+                            }
+                        }
+                        __syncwarp();
+                        if (++q_slot == C::NQ) {
+                            q_slot = 0;
+                            q_phase ^= 1u;
+                        }
+                    }
+                    if (!ok) break;
                 }
             }
         } else if (warp == W_V) {
@@ -739,70 +777,50 @@ dense_attention_kernel(const __grid_constant__ DenseArgs a, const __grid_constan
                 }
             }
         } else if (warp == W_S) {
-            // ============================== Q copies and the S MMAs ==============================
+            // ============================== the S MMAs ==============================
             constexpr uint32_t IDESC_S = umma_idesc<T>(false, kDenseRows, kDenseTile);
             // (a k-step only moves the descriptor's start-address field: +32 bytes inside a 64-column swizzle atom,
             // +16 KiB to the second atom)
             const uint64_t q_desc = umma_desc(sbase + C::OFF_Q, 16, 1024), k_desc = umma_desc(sbase + C::OFF_K, 16, 1024);
-            int stage = 0, last_g = 0;
-            uint32_t k_phase = 0, q_phase = 0, s_phase = 1, g_phase = 0;      // g_phase: bit g, the parity of S_g's next completion
-            bool any = false;
+            int stage = 0, q_slot = 0;
+            uint32_t k_phase = 0, q_phase = 0, s_phase = 1;
             while (ok && segs.next(d, lane, a.status, ok)) {
-                // the query tiles change: the last reader of the old ones must have finished
-                if (any)
-                    ok = mbar_wait_polls(s_full + 8 * last_g, ((g_phase >> last_g) & 1u) ^ 1u, a.status, STATUS_WAIT_SYNC_TIMEOUT);
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok) break;
-                const int gs = a.G * a.S, tiles = d.single() ? 1 : 2;
-                if (elect_one()) {
-                    const uint32_t bytes = (uint32_t)(PAGED ? a.tile_span * a.G : (gs > kDenseRows ? kDenseRows : a.tile_span * gs)) * 256u;
-                    mbar_arrive_expect_tx(q_full, tiles * bytes);
-#pragma unroll 1
-                    for (int i = 0; i < 2 * tiles; ++i) {       // (query tile, column half)
-                        const int c = (i & 1) * 64, g = i >> 1;
-                        const uint32_t dst = sbase + C::OFF_Q + i * C::ATOM_BYTES;
-                        if constexpr (PAGED) {
-                            tma_load_5d(dst, &maps.q, c, 0, d.h, a.rec[d.b].y + g * a.tile_span, d.f, q_full);
-                        } else if (a.tile_tokens > 0) {
-                            const int tile = 2 * d.b + g, w = tile / a.tile_span;
-                            tma_load_5d(dst, &maps.q, c, (tile - w * a.tile_span) * a.tile_tokens, d.h * a.G, w, d.f, q_full);
-                        } else {
-                            const int tile = 2 * d.b + g;
-                            const int w = gs > kDenseRows ? tile / a.tile_span : tile * a.tile_span;
-                            tma_load_5d(dst, &maps.q, c, gs > kDenseRows ? (tile - w * a.tile_span) * kDenseRows : 0, d.h, w, d.f, q_full);
-                        }
-                    }
-                }
-                __syncwarp();
-                ok = __all_sync(0xffffffffu, mbar_wait_polls(q_full, q_phase, a.status, STATUS_WAIT_FULL_TIMEOUT));
-                q_phase ^= 1u;
+                // this segment's places in the ring of query tiles
+                const int slot0 = q_slot, slot1 = slot0 + 1 == C::NQ ? 0 : slot0 + 1;
+                const uint32_t phase0 = q_phase, phase1 = slot1 == 0 ? q_phase ^ 1u : q_phase;
 #pragma unroll 1
                 for (int t = d.t0; t < d.t1 && ok; ++t) {
                     ok = mbar_wait_polls(k_full + 8 * stage, k_phase, a.status, STATUS_WAIT_FULL_TIMEOUT);
                     const uint64_t kd = k_desc + (uint64_t)(uint32_t)(stage * (C::TILE_BYTES >> 4));
 #pragma unroll 1
                     for (int g = 0; g < 2; ++g) {
-                        if (!d.active(g, t)) continue;
-                        // S = Q K^T into the S buffer once the scores before it have been read
-                        ok = mbar_wait_polls(s_free, s_phase, a.status, STATUS_WAIT_SYNC_TIMEOUT) && ok;
-                        ok = __all_sync(0xffffffffu, ok);
-                        if (!ok) break;
-                        s_phase ^= 1u;
-                        tc_fence_after();
-                        const uint64_t qd = q_desc + (uint64_t)(uint32_t)(d.single() ? 0 : g * (C::TILE_BYTES >> 4));
-                        if (elect_one()) {
+                        const int slot = g && !d.single() ? slot1 : slot0;
+                        if (t == d.t0) ok = mbar_wait_polls(q_full + 8 * slot, g && !d.single() ? phase1 : phase0, a.status, STATUS_WAIT_FULL_TIMEOUT) && ok;
+                        if (d.active(g, t)) {
+                            // S = Q K^T into the S buffer once the scores before it have been read
+                            ok = mbar_wait_polls(s_free, s_phase, a.status, STATUS_WAIT_SYNC_TIMEOUT) && ok;
+                            ok = __all_sync(0xffffffffu, ok);
+                            if (!ok) break;
+                            s_phase ^= 1u;
+                            tc_fence_after();
+                            const uint64_t qd = q_desc + (uint64_t)(uint32_t)(slot * (C::TILE_BYTES >> 4));
+                            if (elect_one()) {
 #pragma unroll
-                            for (int kk = 0; kk < C::HD / 16; ++kk) {
-                                const uint64_t off = (uint64_t)(((kk >> 2) * C::ATOM_BYTES + (kk & 3) * 32) >> 4);
-                                tc_mma(tmem + C::COL_S, qd + off, kd + off, IDESC_S, kk > 0);
+                                for (int kk = 0; kk < C::HD / 16; ++kk) {
+                                    const uint64_t off = (uint64_t)(((kk >> 2) * C::ATOM_BYTES + (kk & 3) * 32) >> 4);
+                                    tc_mma(tmem + C::COL_S, qd + off, kd + off, IDESC_S, kk > 0);
+                                }
+                                tc_commit(s_full + 8 * g);
                             }
-                            tc_commit(s_full + 8 * g);
+                            __syncwarp();
                         }
-                        __syncwarp();
-                        g_phase ^= 1u << g;
-                        last_g = g;
-                        any = true;
+                        // a query tile is done with when the products so far are (in a block of one tile, the second group's)
+                        if (t == d.t1 - 1 && g >= (int)d.single()) {
+                            if (elect_one()) tc_commit(q_empty + 8 * slot);
+                            __syncwarp();
+                        }
                     }
+                    ok = __all_sync(0xffffffffu, ok);
                     if (!ok) break;
                     if (elect_one()) tc_commit(k_empty + 8 * stage);
                     __syncwarp();
@@ -810,6 +828,11 @@ dense_attention_kernel(const __grid_constant__ DenseArgs a, const __grid_constan
                         stage = 0;
                         k_phase ^= 1u;
                     }
+                }
+                q_slot += d.single() ? 1 : 2;
+                if (q_slot >= C::NQ) {
+                    q_slot -= C::NQ;
+                    q_phase ^= 1u;
                 }
             }
         } else {
