@@ -27,6 +27,17 @@ def _load_ops() -> None:
 
 _load_ops()
 
+# the operators' overloads, looked up once: a call through torch.ops.libhogatt.<name> finds them anew, 1 us of a 13 us decode call
+_SDPA = torch.ops.libhogatt.hogwild_sdpa.default
+_ROPE = torch.ops.libhogatt.hogwild_rope.default
+_FUSED = torch.ops.libhogatt.hogwild_fused.default
+_FUSED_PLANNED = torch.ops.libhogatt.hogwild_fused_planned.default
+_PAGED_SDPA = torch.ops.libhogatt.hogwild_paged_sdpa.default
+_VARLEN_PAGED_SDPA = torch.ops.libhogatt.hogwild_varlen_paged_sdpa.default
+_COPY_TO_BLOCKS = torch.ops.libhogatt.copy_to_blocks.default
+fragment_append = torch.ops.libhogatt.fragment_append.default              # FragmentCache.update's two steps
+fragment_step_plan = torch.ops.libhogatt.fragment_step_plan.default
+
 
 def hogwild_fused(queries: torch.Tensor, locations: torch.Tensor, keys: List[torch.Tensor], values: List[torch.Tensor],
                   scale: float, fragment_lengths: torch.Tensor, cosines: torch.Tensor, sines: torch.Tensor, *,
@@ -36,8 +47,8 @@ def hogwild_fused(queries: torch.Tensor, locations: torch.Tensor, keys: List[tor
     ``queries [W,Hq,S,E]`` un-rotated; ``rotated_queries [F,W,Hq,S,E]`` and ``out [W,Hq,S,Ev]`` are
     caller-owned buffers that are overwritten.
     """
-    torch.ops.libhogatt.hogwild_fused(out, rotated_queries, scale, locations, queries.contiguous(), fragment_lengths,
-                                      keys, values, cosines, sines)
+    _FUSED(out, rotated_queries, scale, locations, queries.contiguous(), fragment_lengths,
+           keys, values, cosines, sines)
     return out
 
 
@@ -51,9 +62,9 @@ def hogwild_fused_planned(queries: torch.Tensor, locations: torch.Tensor, keys: 
     fragments are not written by work enqueued before this call, e.g. the shared prompt.  With both, the kernel
     starts streaming keys and values without reading anything from device memory first.  No counterpart in the
     reference, whose fragment tensors always end at the fragment's length."""
-    torch.ops.libhogatt.hogwild_fused_planned(out, rotated_queries, scale, locations, queries.contiguous(),
-                                              fragment_lengths, keys, values, cosines, sines,
-                                              [int(x) for x in host_lengths], int(stable_fragments))
+    _FUSED_PLANNED(out, rotated_queries, scale, locations, queries.contiguous(),
+                   fragment_lengths, keys, values, cosines, sines,
+                   [int(x) for x in host_lengths], int(stable_fragments))
     return out
 
 
@@ -68,7 +79,7 @@ def hogwild_sdpa(queries: torch.Tensor, locations: torch.Tensor, keys: List[torc
         fragment_lengths = torch.tensor([k.size(-2) for k in keys], dtype=torch.int32, device=queries.device)
     keys = [k.contiguous() for k in keys]
     values = [v.contiguous() for v in values]
-    torch.ops.libhogatt.hogwild_sdpa(out, scale, locations, queries.contiguous(), fragment_lengths, keys, values)
+    _SDPA(out, scale, locations, queries.contiguous(), fragment_lengths, keys, values)
     return out
 
 
@@ -78,7 +89,7 @@ def hogwild_rope(queries: torch.Tensor, cosines: torch.Tensor, sines: torch.Tens
     if out is None:
         out = torch.empty((cosines.size(0), queries.size(0), queries.size(1), queries.size(2), queries.size(3)),
                           dtype=queries.dtype, device=queries.device)
-    torch.ops.libhogatt.hogwild_rope(out, queries, cosines, sines)
+    _ROPE(out, queries, cosines, sines)
     return out
 
 
@@ -91,8 +102,8 @@ def hogwild_paged_sdpa(queries: torch.Tensor, locations: torch.Tensor, key_cache
     if out is None:
         out = torch.empty((queries.size(1), queries.size(2), queries.size(3), value_cache.size(3)),
                           dtype=queries.dtype, device=queries.device)
-    torch.ops.libhogatt.hogwild_paged_sdpa(out, scale, locations, queries.contiguous(), fragment_lengths, key_cache,
-                                           value_cache, block_table)
+    _PAGED_SDPA(out, scale, locations, queries.contiguous(), fragment_lengths, key_cache,
+                value_cache, block_table)
     return out
 
 
@@ -106,8 +117,8 @@ def hogwild_varlen_paged_sdpa(queries: torch.Tensor, locations: torch.Tensor, ke
         out = torch.empty((queries.size(1), queries.size(2), value_cache.size(3)), dtype=queries.dtype, device=queries.device)
     if cu_seqlens_k is None:
         cu_seqlens_k = cu_seqlens_q
-    torch.ops.libhogatt.hogwild_varlen_paged_sdpa(out, scale, locations, queries.contiguous(), fragment_lengths, key_cache,
-                                                  value_cache, block_table, cu_seqlens_q, cu_seqlens_k)
+    _VARLEN_PAGED_SDPA(out, scale, locations, queries.contiguous(), fragment_lengths, key_cache,
+                       value_cache, block_table, cu_seqlens_q, cu_seqlens_k)
     return out
 
 
@@ -115,8 +126,8 @@ def copy_to_blocks(key_states: torch.Tensor, value_states: torch.Tensor, key_cac
                    block_table: torch.Tensor, seq_lengths: torch.Tensor) -> None:
     """Append ``key_states / value_states [B,Hkv,S_new,E]`` to the paged caches at ``seq_lengths[b] + t``
     (``src/binding.cu:370-371``)."""
-    torch.ops.libhogatt.copy_to_blocks(key_states.contiguous(), value_states.contiguous(), key_cache, value_cache,
-                                       block_table, seq_lengths)
+    _COPY_TO_BLOCKS(key_states.contiguous(), value_states.contiguous(), key_cache, value_cache,
+                    block_table, seq_lengths)
 
 
 def rotate_half(x: torch.Tensor) -> torch.Tensor:

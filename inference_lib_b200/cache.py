@@ -24,6 +24,7 @@ from typing import List, Optional, Sequence
 import torch
 
 from . import _cabi
+from . import attention as ops
 
 
 @dataclass
@@ -87,14 +88,10 @@ class FragmentCache:
         output), un-rotated; ``cos`` / ``sin`` ``[W,S,R]`` for the tokens' own positions, fp32 or the model's type
         (the latter reproduces the reference's arithmetic, ``attention.py:315``).  ``new_rows [W]`` int32 device:
         only the last ``new_rows[w]`` tokens of worker ``w`` are real (left-masked input, ``attention.py:139-145``)."""
-        stream = torch.cuda.current_stream(self.device).cuda_stream
         S = key_states.shape[2]
         src, dst = self.lengths[layer][self.cur[layer]], self.lengths[layer][1 - self.cur[layer]]
-        rc = _cabi.append(keys=key_states, values=value_states, cosines=cos, sines=sin, write_to=self.write_to,
-                          key_fragments=self.keys[layer], value_fragments=self.values[layer], lengths_in=src,
-                          lengths_out=dst, new_rows=new_rows, status=self.status, stream=stream)
-        if rc != 0:
-            raise RuntimeError(f"hogatt_append_launch: {_cabi.status_string(rc)}")
+        ops.fragment_append(key_states, value_states, cos, sin, self.write_to, self.keys[layer], self.values[layer], src, dst,
+                            new_rows, False, self.status)
         self.cur[layer] = 1 - self.cur[layer]
         for f in self.write_to:
             self.host_lengths[layer][f] = min(self.capacities[f], self.host_lengths[layer][f] + S)
@@ -104,11 +101,7 @@ class FragmentCache:
                 self.loc = torch.empty((self.F, self.W, S), dtype=torch.int32, device=self.device)
                 self.cos = torch.empty((self.F, self.W, S, R), dtype=torch.float32, device=self.device)
                 self.sin = torch.empty_like(self.cos)
-            rc = _cabi.step_plan(order=self.order, fragment_lengths=dst, inv_freq=self.inv_freq, S=S, locations=self.loc,
-                                 cosines=self.cos, sines=self.sin, attention_scaling=self.attention_scaling,
-                                 round_tables_to=self.round_to, stream=stream)
-            if rc != 0:
-                raise RuntimeError(f"hogatt_step_plan_launch: {_cabi.status_string(rc)}")
+            ops.fragment_step_plan(self.order, dst, self.inv_freq, self.loc, self.cos, self.sin, self.attention_scaling, self.round_to)
         return CacheStructure(keys=self.keys[layer], values=self.values[layer], frags=dst, cos=self.cos, sin=self.sin,
                               loc=self.loc, host_lengths=list(self.host_lengths[layer]), stable=min(self.write_to))
 

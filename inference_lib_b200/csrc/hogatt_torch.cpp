@@ -13,6 +13,7 @@
 #include <torch/library.h>
 
 #include <algorithm>
+#include <optional>
 #include <vector>
 
 #include "../../include/hogatt.h"
@@ -342,6 +343,84 @@ void copy_to_blocks(const at::Tensor& key_states, const at::Tensor& value_states
                  "copy_to_blocks");
 }
 
+// --- the steps either side of the op (FragmentCache.update) -------------------------------------------------
+// The C ABI's calls with their arguments gathered here: filling the same structures through ctypes took 16 us per layer, and
+// asking torch for the stream another 4, of the 28 that FragmentCache.update was.
+
+void fragment_append(const at::Tensor& keys, const at::Tensor& values, const at::Tensor& cosines, const at::Tensor& sines,
+                     at::IntArrayRef write_to, at::TensorList key_fragments, at::TensorList value_fragments, const at::Tensor& lengths_in,
+                     at::Tensor& lengths_out, const std::optional<at::Tensor>& new_rows, bool take_leading, at::Tensor& status) {
+    TORCH_CHECK(keys.is_cuda(), "libhogatt: tensors must live on a CUDA device");
+    const c10::cuda::CUDAGuard guard(keys.device());
+    TORCH_CHECK(keys.dim() == 4 && values.dim() == 4, "fragment_append: keys and values must be [W,Hkv,S,E]");
+    for (const at::Tensor* t : {&keys, &values, &cosines, &sines})
+        TORCH_CHECK(t->dim() > 0 && t->stride(-1) == 1, "fragment_append: the last axis of keys, values and tables must be contiguous");
+    const int64_t W = keys.size(0), S = keys.size(2);
+    TORCH_CHECK_EQ((int64_t)write_to.size(), W);
+    const size_t F = key_fragments.size();
+    TORCH_CHECK_EQ(value_fragments.size(), F);
+    hogatt_append p = {};
+    p.W = (int32_t)W; p.Hkv = (int32_t)keys.size(1); p.E = (int32_t)keys.size(3); p.Ev = (int32_t)values.size(3); p.S = (int32_t)S;
+    p.F = (int32_t)F;
+    p.rotary_dim = (int32_t)cosines.size(-1);
+    p.dtype = dtype_code(keys);
+    p.table_dtype = dtype_code(cosines);
+    p.keys = keys.const_data_ptr();
+    p.values = values.const_data_ptr();
+    for (int i = 0; i < 3; ++i) {
+        p.key_strides[i] = keys.stride(i);
+        p.value_strides[i] = values.stride(i);
+    }
+    p.cosines = cosines.const_data_ptr();
+    p.sines = sines.const_data_ptr();
+    if (cosines.dim() == 3 && cosines.size(0) == W && cosines.size(1) == S) {
+        p.table_strides[0] = cosines.stride(0);
+        p.table_strides[1] = cosines.stride(1);
+        TORCH_CHECK(sines.dim() == 3 && sines.stride(0) == cosines.stride(0) && sines.stride(1) == cosines.stride(1),
+                    "fragment_append: both tables must have the same strides");
+    } else {
+        TORCH_CHECK(cosines.numel() == cosines.size(-1), "fragment_append: tables are [W,S,R] or a single row");
+    }
+    p.new_rows = new_rows.has_value() ? static_cast<const int32_t*>(new_rows->const_data_ptr()) : nullptr;
+    p.take_leading = take_leading ? 1 : 0;
+    std::vector<int32_t> to(write_to.begin(), write_to.end()), rows(F);
+    std::vector<void*> kptr(F), vptr(F);
+    for (size_t f = 0; f < F; ++f) {
+        kptr[f] = key_fragments[f].data_ptr();
+        vptr[f] = value_fragments[f].data_ptr();
+        rows[f] = (int32_t)key_fragments[f].size(-2);
+    }
+    p.write_to = to.data();
+    p.key_fragments = kptr.data();
+    p.value_fragments = vptr.data();
+    p.fragment_rows = rows.data();
+    p.lengths_in = lengths_in.const_data_ptr<int>();
+    p.lengths_out = lengths_out.data_ptr<int>();
+    p.device_status = status.data_ptr<int>();
+    const cudaStream_t stream = c10::cuda::getCurrentCUDAStream();
+    check_status(hogatt_append_launch(&p, reinterpret_cast<hogatt_stream_t>(stream)), "fragment_append");
+}
+
+void fragment_step_plan(const at::Tensor& order, const at::Tensor& fragment_lengths, const at::Tensor& inv_freq, at::Tensor& locations,
+                        at::Tensor& cosines, at::Tensor& sines, double attention_scaling, int64_t round_tables_to) {
+    TORCH_CHECK(order.is_cuda(), "libhogatt: tensors must live on a CUDA device");
+    const c10::cuda::CUDAGuard guard(order.device());
+    TORCH_CHECK(order.dim() == 2 && locations.dim() == 3, "fragment_step_plan: order [W,F], locations [F,W,S]");
+    hogatt_step_plan p = {};
+    p.W = (int32_t)order.size(0); p.F = (int32_t)order.size(1); p.S = (int32_t)locations.size(2);
+    p.rotary_dim = 2 * (int32_t)inv_freq.numel();
+    p.order = order.const_data_ptr<int>();
+    p.fragment_lengths = fragment_lengths.const_data_ptr<int>();
+    p.inv_freq = inv_freq.const_data_ptr<float>();
+    p.attention_scaling = (float)attention_scaling;
+    p.round_tables_to = (int32_t)round_tables_to;
+    p.locations = locations.data_ptr<int>();
+    p.cosines = cosines.data_ptr<float>();
+    p.sines = sines.data_ptr<float>();
+    const cudaStream_t stream = c10::cuda::getCurrentCUDAStream();
+    check_status(hogatt_step_plan_launch(&p, reinterpret_cast<hogatt_stream_t>(stream)), "fragment_step_plan");
+}
+
 }  // namespace
 
 extern "C" {
@@ -371,6 +450,12 @@ TORCH_LIBRARY(libhogatt, m) {
     m.def("hogwild_fused_planned(Tensor(a!) output, Tensor(b!) rq, float scale, Tensor locations, Tensor queries, "
           "Tensor fragment_lengths, Tensor[] key_fragments, Tensor[] value_fragments, Tensor cosines, Tensor sines, "
           "int[] host_lengths, int stable_fragments) -> ()", tags, torch::_RegisterOrVerify::REGISTER);
+    // ... and the steps either side of it
+    m.def("fragment_append(Tensor keys, Tensor values, Tensor cosines, Tensor sines, int[] write_to, Tensor(a!)[] key_fragments, "
+          "Tensor(b!)[] value_fragments, Tensor lengths_in, Tensor(c!) lengths_out, Tensor? new_rows, bool take_leading, "
+          "Tensor(d!) status) -> ()", tags, torch::_RegisterOrVerify::REGISTER);
+    m.def("fragment_step_plan(Tensor order, Tensor fragment_lengths, Tensor inv_freq, Tensor(a!) locations, Tensor(b!) cosines, "
+          "Tensor(c!) sines, float attention_scaling, int round_tables_to) -> ()", tags, torch::_RegisterOrVerify::REGISTER);
 }
 
 TORCH_LIBRARY_IMPL(libhogatt, CUDA, m) {
@@ -381,4 +466,6 @@ TORCH_LIBRARY_IMPL(libhogatt, CUDA, m) {
     m.impl("copy_to_blocks", copy_to_blocks);
     m.impl("hogwild_varlen_paged_sdpa", hogwild_varlen_paged_attention);
     m.impl("hogwild_fused_planned", hogwild_fused_planned);
+    m.impl("fragment_append", fragment_append);
+    m.impl("fragment_step_plan", fragment_step_plan);
 }
