@@ -297,8 +297,8 @@ __device__ __forceinline__ DenseRow dense_row(const DenseArgs& a, int tile, int 
 // rows of fragment f that hold keys and values (worker w's, when paged)
 template <bool PAGED>
 __device__ __forceinline__ int dense_length(const DenseArgs& a, int f, int w) {
-    if constexpr (PAGED) return __ldg(a.flen + f * a.W + w);
-    return a.flen ? min(a.cap[f], __ldg(a.flen + f)) : a.cap[f];
+    if constexpr (PAGED) return a.flen[f * a.W + w];
+    return a.flen ? min(a.cap[f], a.flen[f]) : a.cap[f];
 }
 template <bool PAGED>
 __device__ __forceinline__ int dense_location(const DenseArgs& a, int f, const DenseRow& r) {
@@ -419,7 +419,7 @@ __global__ void __launch_bounds__(kDensePlanThreads) dense_plan_kernel(const __g
         for (int k = 0; k < kDenseRows; k += 32) {
             int at = from + k + lane;
             if (at >= wrap) at -= a.S;
-            if (k + lane < tokens) top = max(top, __ldg(loc + at));
+            if (k + lane < tokens) top = max(top, loc[at]);
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, o));

@@ -249,6 +249,15 @@ __device__ __noinline__ void drain_stage(uint32_t bar, uint32_t parity, int* sta
 // NEXT kernel in the stream start being scheduled.  Both are no-ops for a normal launch.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// 16 bytes of what a kernel of this library may still be writing when this one starts (appended rows, step metadata).  Not
+// __ldg, and no const __restrict__ kernel parameters either: ld.global.nc is for memory that nobody writes during the whole life
+// of the kernel, and nothing keeps such a load behind pdl_wait().  This one stays behind it (both are volatile) and may
+// move past stores to shared memory, as the staging loops want.
+__device__ __forceinline__ int4 load_16(const void* p) {
+    int4 v;
+    asm volatile("ld.global.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
 
 // ---- thread-block cluster helpers (distributed shared memory) -----------------------------------------
 // barrier.cluster is a hardware barrier over every thread of every CTA of the cluster (like bar.sync over

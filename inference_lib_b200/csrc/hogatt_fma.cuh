@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(kFmaThreads) fma_attention_kernel(const __grid
             const T* vsrc = static_cast<const T*>(a.ft.e[f].v) + row0 * EV;
             const int kvecs = ntok * E / VEC;
             for (int i = tid; i < kvecs; i += kFmaThreads) {
-                const int4 raw = __ldg(reinterpret_cast<const int4*>(ksrc) + i);
+                const int4 raw = load_16(ksrc + i * VEC);
                 const T* x = reinterpret_cast<const T*>(&raw);
                 const int idx = i * VEC, tok = idx / E, e = idx - tok * E;
 #pragma unroll
@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(kFmaThreads) fma_attention_kernel(const __grid
             const int vvecs = kFmaTile * EV / VEC, vvalid = ntok * EV / VEC;
             for (int i = tid; i < vvecs; i += kFmaThreads) {
                 int4 raw = make_int4(0, 0, 0, 0);          // rows past the tile end must be finite
-                if (i < vvalid) raw = __ldg(reinterpret_cast<const int4*>(vsrc) + i);
+                if (i < vvalid) raw = load_16(vsrc + i * VEC);
                 const T* x = reinterpret_cast<const T*>(&raw);
 #pragma unroll
                 for (int k = 0; k < VEC; ++k) Vs[i * VEC + k] = Scalar<T>::to_float(x[k]);

@@ -399,7 +399,9 @@ __device__ __forceinline__ void end_after_predecessor(int chained) {
 
 // rq[f,w,h,s,:] = rope(q[w,h,s,:], cos[f,w,s,:], sin[f,w,s,:]).
 // Replaces rope_kernel (src/rope.cuh:2-52), which uses one thread per channel and one CTA per row;
-// here a thread produces a 16-byte chunk of a row from 16-byte loads.
+// here a thread produces a 16-byte chunk of a row from 16-byte loads.  (Its inputs may be declared read-only, unlike those of the
+// other kernels that start beside their predecessor: that one is the plan kernel, which lets it in after its own wait, and nobody
+// writes them from then on.)
 template <class T>
 __global__ void __launch_bounds__(128) rope_kernel(T* __restrict__ rq, const T* __restrict__ q,
                                                    const float* __restrict__ cosines,

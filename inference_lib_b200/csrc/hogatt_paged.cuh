@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(kFmaThreads) paged_attention_kernel(const __gr
                 if (tok < ntok) {
                     const int l = tok0 + tok;
                     const size_t row = ((size_t)table[min(l / a.block_size, a.max_blocks - 1)] * a.Hkv + u.hkv) * a.block_size + l % a.block_size;
-                    const int4 raw = __ldg(reinterpret_cast<const int4*>(static_cast<const T*>(a.kcache) + row * E) + c);
+                    const int4 raw = load_16(static_cast<const T*>(a.kcache) + row * E + c * VEC);
                     const T* x = reinterpret_cast<const T*>(&raw);
 #pragma unroll
                     for (int k = 0; k < VEC; ++k) core.Ks[tok * (E + 1) + c * VEC + k] = Scalar<T>::to_float(x[k]);
@@ -177,7 +177,7 @@ __global__ void __launch_bounds__(kFmaThreads) paged_attention_kernel(const __gr
                 if (tok < ntok) {
                     const int l = tok0 + tok;
                     const size_t row = ((size_t)table[min(l / a.block_size, a.max_blocks - 1)] * a.Hkv + u.hkv) * a.block_size + l % a.block_size;
-                    raw = __ldg(reinterpret_cast<const int4*>(static_cast<const T*>(a.vcache) + row * EV) + c);
+                    raw = load_16(static_cast<const T*>(a.vcache) + row * EV + c * VEC);
                 }
                 const T* x = reinterpret_cast<const T*>(&raw);
 #pragma unroll
@@ -591,11 +591,9 @@ __global__ void __launch_bounds__(kMergeWarps * 32) paged_merge_kernel(const __g
 // thread of a (S_new x head-size) block copies a whole row element by element.  A few KB in a decode step: launched beside
 // its predecessor, and its successor beside it (8 sequences of 16 K keys, with the attention call: 37.1 -> 35.0 us).
 template <class T>
-__global__ void __launch_bounds__(256) copy_to_blocks_kernel(const T* __restrict__ k_states, const T* __restrict__ v_states,
-                                                             T* __restrict__ k_cache, T* __restrict__ v_cache,
-                                                             const int* __restrict__ block_table,
-                                                             const int* __restrict__ seq_lengths, int B, int Hkv,
-                                                             int S_new, int E, int Ev, int block_size, int max_blocks) {
+__global__ void __launch_bounds__(256) copy_to_blocks_kernel(const T* k_states, const T* v_states, T* k_cache, T* v_cache,
+                                                             const int* block_table, const int* seq_lengths, int B, int Hkv, int S_new,
+                                                             int E, int Ev, int block_size, int max_blocks) {
     constexpr int VEC = 16 / sizeof(T);
     const int kvr = E / VEC, vvr = Ev / VEC, per_row = kvr + vvr;
     const int64_t total = (int64_t)B * Hkv * S_new * per_row;
@@ -610,10 +608,9 @@ __global__ void __launch_bounds__(256) copy_to_blocks_kernel(const T* __restrict
         const size_t dst_row = (blk * Hkv + h) * block_size + pos % block_size;
         const size_t src_row = ((size_t)b * Hkv + h) * S_new + t;
         if (c < kvr)
-            reinterpret_cast<int4*>(k_cache + dst_row * E)[c] = __ldg(reinterpret_cast<const int4*>(k_states + src_row * E) + c);
+            reinterpret_cast<int4*>(k_cache + dst_row * E)[c] = load_16(k_states + src_row * E + c * VEC);
         else
-            reinterpret_cast<int4*>(v_cache + dst_row * Ev)[c - kvr] =
-                __ldg(reinterpret_cast<const int4*>(v_states + src_row * Ev) + (c - kvr));
+            reinterpret_cast<int4*>(v_cache + dst_row * Ev)[c - kvr] = load_16(v_states + src_row * Ev + (c - kvr) * VEC);
     }
 }
 
