@@ -353,14 +353,39 @@ void fragment_append(const at::Tensor& keys, const at::Tensor& values, const at:
     TORCH_CHECK(keys.is_cuda(), "libhogatt: tensors must live on a CUDA device");
     const c10::cuda::CUDAGuard guard(keys.device());
     TORCH_CHECK(keys.dim() == 4 && values.dim() == 4, "fragment_append: keys and values must be [W,Hkv,S,E]");
+    for (const at::Tensor* t : {&values, &cosines, &sines, &lengths_in, (const at::Tensor*)&lengths_out, (const at::Tensor*)&status})
+        TORCH_CHECK(t->device() == keys.device(), "fragment_append: every tensor must be on the keys' device");
     for (const at::Tensor* t : {&keys, &values, &cosines, &sines})
         TORCH_CHECK(t->dim() > 0 && t->stride(-1) == 1, "fragment_append: the last axis of keys, values and tables must be contiguous");
-    const int64_t W = keys.size(0), S = keys.size(2);
+    const int64_t W = keys.size(0), Hkv = keys.size(1), S = keys.size(2), E = keys.size(3), Ev = values.size(3);
+    for (int i = 0; i < 3; ++i) TORCH_CHECK_EQ(values.size(i), keys.size(i));
+    TORCH_CHECK(values.scalar_type() == keys.scalar_type(), "fragment_append: values must have the keys' dtype");
+    TORCH_CHECK(sines.scalar_type() == cosines.scalar_type() && sines.size(-1) == cosines.size(-1),
+                "fragment_append: both tables must have the same dtype and row length");
     TORCH_CHECK_EQ((int64_t)write_to.size(), W);
-    const size_t F = key_fragments.size();
-    TORCH_CHECK_EQ(value_fragments.size(), F);
+    const int64_t F = (int64_t)key_fragments.size();
+    TORCH_CHECK_EQ((int64_t)value_fragments.size(), F);
+    for (const int64_t f : write_to) TORCH_CHECK(f >= 0 && f < F, "fragment_append: write_to names fragment ", f, " of ", F);
+    for (int64_t f = 0; f < F; ++f) {
+        const at::Tensor &k = key_fragments[f], &v = value_fragments[f];
+        TORCH_CHECK(k.device() == keys.device() && v.device() == keys.device(), "fragment_append: fragments on another device");
+        TORCH_CHECK(k.scalar_type() == keys.scalar_type() && v.scalar_type() == keys.scalar_type(), "fragment_append: fragment dtype != keys' dtype");
+        TORCH_CHECK(k.is_contiguous() && v.is_contiguous() && k.dim() >= 3 && v.dim() >= 3, "fragment_append: fragments must be contiguous [Hkv,capacity,E]");
+        TORCH_CHECK_EQ(k.size(-1), E);
+        TORCH_CHECK_EQ(v.size(-1), Ev);
+        TORCH_CHECK_EQ(v.size(-2), k.size(-2));
+        TORCH_CHECK(k.size(-3) == Hkv && v.size(-3) == Hkv && k.numel() == Hkv * k.size(-2) * E && v.numel() == Hkv * k.size(-2) * Ev,
+                    "fragment_append: fragments must be [Hkv,capacity,E]");
+    }
+    for (const at::Tensor* t : {&lengths_in, (const at::Tensor*)&lengths_out})
+        TORCH_CHECK(t->dim() == 1 && t->size(0) == F && t->is_contiguous() && t->scalar_type() == at::kInt,
+                    "fragment_append: lengths must be contiguous int32 [F]");
+    TORCH_CHECK(status.numel() > 0 && status.scalar_type() == at::kInt, "fragment_append: status must be int32");
+    if (new_rows.has_value())
+        TORCH_CHECK(new_rows->device() == keys.device() && new_rows->dim() == 1 && new_rows->size(0) == W && new_rows->is_contiguous() &&
+                        new_rows->scalar_type() == at::kInt, "fragment_append: new_rows must be contiguous int32 [W]");
     hogatt_append p = {};
-    p.W = (int32_t)W; p.Hkv = (int32_t)keys.size(1); p.E = (int32_t)keys.size(3); p.Ev = (int32_t)values.size(3); p.S = (int32_t)S;
+    p.W = (int32_t)W; p.Hkv = (int32_t)Hkv; p.E = (int32_t)E; p.Ev = (int32_t)Ev; p.S = (int32_t)S;
     p.F = (int32_t)F;
     p.rotary_dim = (int32_t)cosines.size(-1);
     p.dtype = dtype_code(keys);
@@ -376,16 +401,16 @@ void fragment_append(const at::Tensor& keys, const at::Tensor& values, const at:
     if (cosines.dim() == 3 && cosines.size(0) == W && cosines.size(1) == S) {
         p.table_strides[0] = cosines.stride(0);
         p.table_strides[1] = cosines.stride(1);
-        TORCH_CHECK(sines.dim() == 3 && sines.stride(0) == cosines.stride(0) && sines.stride(1) == cosines.stride(1),
-                    "fragment_append: both tables must have the same strides");
+        TORCH_CHECK(sines.sizes() == cosines.sizes() && sines.stride(0) == cosines.stride(0) && sines.stride(1) == cosines.stride(1),
+                    "fragment_append: both tables must have the same shape and strides");
     } else {
-        TORCH_CHECK(cosines.numel() == cosines.size(-1), "fragment_append: tables are [W,S,R] or a single row");
+        TORCH_CHECK(cosines.numel() == cosines.size(-1) && sines.numel() == sines.size(-1), "fragment_append: tables are [W,S,R] or a single row");
     }
-    p.new_rows = new_rows.has_value() ? static_cast<const int32_t*>(new_rows->const_data_ptr()) : nullptr;
+    p.new_rows = new_rows.has_value() ? new_rows->const_data_ptr<int>() : nullptr;
     p.take_leading = take_leading ? 1 : 0;
     std::vector<int32_t> to(write_to.begin(), write_to.end()), rows(F);
     std::vector<void*> kptr(F), vptr(F);
-    for (size_t f = 0; f < F; ++f) {
+    for (int64_t f = 0; f < F; ++f) {
         kptr[f] = key_fragments[f].data_ptr();
         vptr[f] = value_fragments[f].data_ptr();
         rows[f] = (int32_t)key_fragments[f].size(-2);
@@ -405,10 +430,19 @@ void fragment_step_plan(const at::Tensor& order, const at::Tensor& fragment_leng
                         at::Tensor& cosines, at::Tensor& sines, double attention_scaling, int64_t round_tables_to) {
     TORCH_CHECK(order.is_cuda(), "libhogatt: tensors must live on a CUDA device");
     const c10::cuda::CUDAGuard guard(order.device());
+    for (const at::Tensor* t : {&order, &fragment_lengths, &inv_freq, (const at::Tensor*)&locations, (const at::Tensor*)&cosines, (const at::Tensor*)&sines})
+        TORCH_CHECK(t->is_contiguous() && t->device() == order.device(), "fragment_step_plan: tensors must be contiguous and on one device");
     TORCH_CHECK(order.dim() == 2 && locations.dim() == 3, "fragment_step_plan: order [W,F], locations [F,W,S]");
+    const int64_t W = order.size(0), F = order.size(1), S = locations.size(2), R = 2 * inv_freq.numel();
+    TORCH_CHECK_EQ(locations.size(0), F);
+    TORCH_CHECK_EQ(locations.size(1), W);
+    TORCH_CHECK(fragment_lengths.dim() == 1 && fragment_lengths.size(0) == F, "fragment_step_plan: fragment_lengths must be [F]");
+    for (const at::Tensor* t : {&cosines, &sines})
+        TORCH_CHECK(t->dim() == 4 && t->size(0) == F && t->size(1) == W && t->size(2) == S && t->size(3) == R,
+                    "fragment_step_plan: cosines / sines must be [F,W,S,2 * inv_freq]");
     hogatt_step_plan p = {};
-    p.W = (int32_t)order.size(0); p.F = (int32_t)order.size(1); p.S = (int32_t)locations.size(2);
-    p.rotary_dim = 2 * (int32_t)inv_freq.numel();
+    p.W = (int32_t)W; p.F = (int32_t)F; p.S = (int32_t)S;
+    p.rotary_dim = (int32_t)R;
     p.order = order.const_data_ptr<int>();
     p.fragment_lengths = fragment_lengths.const_data_ptr<int>();
     p.inv_freq = inv_freq.const_data_ptr<float>();
