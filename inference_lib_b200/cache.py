@@ -24,7 +24,17 @@ from typing import List, Optional, Sequence
 import torch
 
 from . import _cabi
-from . import attention as ops
+
+_ops = None
+
+
+def _operators():
+    """The operator library, loaded when the first cache needs it: importing this module takes the C ABI only."""
+    global _ops
+    if _ops is None:
+        from . import attention
+        _ops = attention
+    return _ops
 
 
 @dataclass
@@ -90,6 +100,7 @@ class FragmentCache:
         only the last ``new_rows[w]`` tokens of worker ``w`` are real (left-masked input, ``attention.py:139-145``)."""
         S = key_states.shape[2]
         src, dst = self.lengths[layer][self.cur[layer]], self.lengths[layer][1 - self.cur[layer]]
+        ops = _operators()
         ops.fragment_append(key_states, value_states, cos, sin, self.write_to, self.keys[layer], self.values[layer], src, dst,
                             new_rows, False, self.status)
         self.cur[layer] = 1 - self.cur[layer]
