@@ -121,7 +121,6 @@ class FragmentCache:
         """Append fragment ``source`` to fragment ``target`` in every layer, its keys re-rotated by the target's
         current length as one constant position, tables in the model's type (``merge_caches``,
         ``python/hogwild/attention.py:251-257``).  The source keeps its contents."""
-        stream = torch.cuda.current_stream(self.device).cuda_stream
         t_len = self.frags(0)[target:target + 1].to(torch.float32)          # stays on the device
         angle = t_len * self.inv_freq
         emb = torch.cat([angle, angle])
@@ -133,11 +132,8 @@ class FragmentCache:
             k = self.keys[layer][source].view(1, self.Hkv, cap, self.E)
             v = self.values[layer][source].view(1, self.Hkv, cap, self.Ev)
             # the source is a slab itself: its first lengths[source] rows are taken, the count stays on the device
-            rc = _cabi.append(keys=k, values=v, cosines=cos, sines=sin, write_to=[target], key_fragments=self.keys[layer],
-                              value_fragments=self.values[layer], lengths_in=src, lengths_out=dst,
-                              new_rows=src[source:source + 1], take_leading=True, status=self.status, stream=stream)
-            if rc != 0:
-                raise RuntimeError(f"hogatt_append_launch: {_cabi.status_string(rc)}")
+            _operators().fragment_append(k, v, cos, sin, [target], self.keys[layer], self.values[layer], src, dst,
+                                         src[source:source + 1], True, self.status)
             self.cur[layer] = 1 - self.cur[layer]
             self.host_lengths[layer][target] = min(self.capacities[target],
                                                    self.host_lengths[layer][target] + self.host_lengths[layer][source])
