@@ -8,8 +8,8 @@
 // block walks only those, 128 keys per step -- of a causal prompt just over half (4,000 tokens: 543 us per call when
 // every block walked every key, 168 now) -- and the steps of all units are one list that a persistent grid of one
 // CTA per SM cuts into balanced contiguous ranges.  A unit that lies inside one range is normalised and stored by
-// its CTA; of a unit cut into a few parts, the CTA that finishes last folds the partials of the others; units of many
-// parts are left to dense_merge_kernel.
+// its CTA; where units are cut into a few parts, the CTA that finishes last folds the partials of the others, else they are
+// left to dense_merge_kernel.
 //
 // A step.  Both tiles of the block use the K and V tile (64 KiB of copies per 16.8 MFLOP; each tile alone would be at
 // the SM's L2 bandwidth).  Where a block has only one tile, the second softmax group takes every other key tile
@@ -48,11 +48,16 @@ constexpr int kDensePlanThreads = 1024;
 constexpr int kDenseMaxCtas = 256;
 constexpr int kDenseMergeWarps = 8;         // warps per CTA of the merge step; with many partials per row they share a row's
 constexpr int kDenseMergeBatch = 4;         // partials of a row that a thread of it has in flight
-// CTAs of a unit up to which the last of them to finish folds the others' partials into its own rows, and nothing of it is left to
-// the merge step (which then ends 1.5 us after the attention kernel instead of 12).  It reads 128 KiB of each other one; more are
-// left to the merge step, which has the whole chip for them.  us per call with a line at 2 / 3 / 8: 5.6 CTAs per unit (1,024 rows
-// of 8 heads, 24,576 keys) 114.4 / 114.4 / 119.7; two or three (3 x 256 tokens, 5,700 keys) 125.4 / 124.9 / 124.9; before, with
-// every one of them in the merge step, 128 for the latter and 159 instead of 154 for a 4,000-token prompt.
+// Where no unit has more CTAs than this, the last CTA of a unit to finish folds the others' partials into its own rows, 128 KiB of
+// each, and nothing of it is left to the merge step (which then ends 1.5 us after the attention kernel instead of 12).  us per
+// call, folded up to 3 / merged: three parts at most (3 x 256 tokens, 5,700 keys, G = 5) 111.5 / 117.5, a 4,000-token prompt 134 /
+// 145 (a line at 2: 134).  Two more conditions, both for all units of a call:
+//   * one unit of more CTAs makes the call wait for the merge step anyway, which then gets every shared unit (512 tokens, 4,000
+//     packed keys, 64 units of which two have four CTAs: 49.4; folding the others as well 53.2; with a line at 4 50.2);
+//   * where the steps do not fill the SMs, the merge step's CTAs are resident on the idle ones before the attention kernel ends
+//     (128 tokens, 512 packed keys 22.7, folded 26.4).
+// The two halves that one CTA leaves of a block of one tile are always folded there (six single tokens beside two chunks of 512
+// tokens: 112, in the merge step 120).
 constexpr int kDenseFoldParts = 3;
 constexpr int kDenseFoldInts = 20;          // per unit: first CTA, CTAs (0: not folded there), two unused, arrivals left of 16 warps
 
@@ -325,9 +330,9 @@ __global__ void __launch_bounds__(kDensePlanThreads) dense_plan_kernel(const __g
     __shared__ int s_vis[kDensePlanVis];
     __shared__ long long s_pre[kDensePlanBlocks + 1], s_cost[kDensePlanBlocks + 1], sums[kDensePlanThreads / 32], pos[kDenseMaxCtas + 1];
     __shared__ int4 s_rec[PAGED ? kDensePlanRecs : 1];
-    __shared__ int s_list;
+    __shared__ int s_list, s_most;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = kDensePlanThreads / 32;
-    if (tid == 0) s_list = 0;
+    if (tid == 0) s_list = s_most = 0;
     pdl_wait();
     // The rotation kernel writes nothing that is read here.  It starts at once and makes the loads below slower, but its own
     // time is what the attention kernel waits for (let go behind them it began 4 us later: 4,000 tokens 25 -> 15 us to the end
@@ -459,18 +464,6 @@ __global__ void __launch_bounds__(kDensePlanThreads) dense_plan_kernel(const __g
     // Where every CTA starts: equal shares of the steps and of the units' fixed costs.  pos[c]: its first step in the list of all.
     const long long N = total * a.Hkv, C = total_cost * a.Hkv;
     const int ctas = dense_ctas(N, C, singles, a.ctas);
-    // who folds unit u, which `count` CTAs from `first` on work on (in a block of one tile, two halves each)
-    auto leave = [&](int u, int first, int count, bool single) {
-        int4* const fold = reinterpret_cast<int4*>(a.fold + (size_t)u * kDenseFoldInts);
-        const int here = count <= kDenseFoldParts ? count : 0, left = single ? 2 * here : here;
-        fold[0] = make_int4(first, here, 0, 0);
-        if (here > 0) {
-#pragma unroll
-            for (int i = 1; i < kDenseFoldInts / 4; ++i) fold[i] = make_int4(left, left, left, left);
-        } else {
-            a.merge[atomicAdd(&s_list, 1)] = make_int4(u, first, single ? 2 * count : count, single ? 1 : 0);
-        }
-    };
     int4 st = make_int4(0, 0, 0, 0);
     if (tid < ctas) {
         DenseStart d;
@@ -479,14 +472,31 @@ __global__ void __launch_bounds__(kDensePlanThreads) dense_plan_kernel(const __g
     }
     if (tid == ctas) pos[ctas] = N;
     __syncthreads();
-    if (tid < a.ctas) {
-        if (tid < ctas) {
-            st.w = (int)(pos[tid + 1] - pos[tid]);
-            const long long s = pos[tid] - st.z;
-            // the unit this CTA starts inside of, if no earlier CTA does
-            if (st.z > 0 && !single_block(st.x) && pos[tid - 1] <= s)
-                leave(st.x * a.Hkv + st.y, tid - 1, dense_parts(pos, ctas, tid - 1, s + pre[st.x + 1] - pre[st.x]), false);
+    int parts = 0;                               // CTAs of the unit this one starts inside of, if no earlier CTA does
+    if (tid < ctas) {
+        st.w = (int)(pos[tid + 1] - pos[tid]);
+        const long long s = pos[tid] - st.z;
+        if (st.z > 0 && pos[tid - 1] <= s) {
+            parts = dense_parts(pos, ctas, tid - 1, s + pre[st.x + 1] - pre[st.x]);
+            atomicMax(&s_most, parts);
         }
+    }
+    __syncthreads();
+    // Who folds unit u, which `count` CTAs from `first` on work on (in a block of one tile, two halves each).
+    const bool few = s_most <= kDenseFoldParts && ctas == a.ctas;
+    auto leave = [&](int u, int first, int count, bool single) {
+        int4* const fold = reinterpret_cast<int4*>(a.fold + (size_t)u * kDenseFoldInts);
+        const int here = count == 1 || few ? count : 0, left = single ? 2 * here : here;
+        fold[0] = make_int4(first, here, 0, 0);
+        if (here > 0) {
+#pragma unroll
+            for (int i = 1; i < kDenseFoldInts / 4; ++i) fold[i] = make_int4(left, left, left, left);
+        } else {
+            a.merge[atomicAdd(&s_list, 1)] = make_int4(u, first, single ? 2 * count : count, single ? 1 : 0);
+        }
+    };
+    if (tid < a.ctas) {
+        if (parts > 0 && !single_block(st.x)) leave(st.x * a.Hkv + st.y, tid - 1, parts, false);
         a.start[tid] = st;
     }
     // blocks of one tile (two halves per CTA that worked on them), blocks that see nothing.  (A thread per unit: with one per

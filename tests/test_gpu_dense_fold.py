@@ -1,5 +1,5 @@
-"""Who folds the partials of the tcgen05 kernel of two query tiles per block: the last CTA of a unit up to three of them, the merge
-step above that.  ``max_ctas`` CTAs cut the units of a small call into so many parts; the plan's list of what is left to the
+"""Who folds the partials of the tcgen05 kernel of two query tiles per block: the last CTA of a unit where no unit has more than three
+and every CTA has a step, the merge step otherwise.  ``max_ctas`` CTAs cut the units of a small call into so many parts; the plan's list of what is left to the
 merge step (its length is the workspace's first word) says which of the two it was."""
 import ctypes as C
 
@@ -13,7 +13,7 @@ from tests.gpu_util import check_against
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
-TILE, FOLDED = 128, 3            # rows of a query tile and keys of a step; CTAs of a unit that the last of them folds
+TILE, FOLDED = 128, 3            # rows of a query tile and keys of a step; CTAs of a unit up to which the last of them folds
 
 
 def _plan(blocks, Hkv, grid):
@@ -48,8 +48,9 @@ def _tiles(p):
 
 def _left_to_the_merge_step(blocks, Hkv, grid):
     """How many units are, and how many CTAs work on each unit."""
-    _, parts = _plan(blocks, Hkv, grid)
-    return sum(n == 0 or n > FOLDED for n in parts), parts
+    pos, parts = _plan(blocks, Hkv, grid)
+    few = max(parts) <= FOLDED and all(p < pos[grid] for p in pos[:grid])
+    return sum(n == 0 or (n > 1 and not few) for n in parts), parts
 
 
 def _problem(W, G, S, Hkv, dtype, prompt):
