@@ -718,14 +718,23 @@ int launch_dense_kernels(const DenseArgs& d, const DenseMaps& maps, int dev, int
     const int rc = ensure_smem_limit(dense_attention_kernel<T, PAGED>, dev, kDenseSmemBytes, granted);
     if (rc != HOGATT_OK) return rc;
     HOGATT_CUDA_OK(launch_kernel(dense_attention_kernel<T, PAGED>, dim3(d.ctas), dim3(kDenseThreads), kDenseSmemBytes, stream, d, maps));
-    // the merge step walks the plan's list, which holds few units or none where there are as many units as CTAs: no more CTAs
-    // than are resident at once
-    const int64_t units = (int64_t)d.blocks * d.Hkv;
+    // The merge step walks the plan's list, which holds few units or none where there are as many units as CTAs: no more CTAs than
+    // are resident at once, two per SM.  Few units have many partials each, and a unit's warps share them; where even so there
+    // are more CTAs than that, four per SM that fetch one partial at a time (64 tokens, 1,000 packed keys, 8 units of 16 parts: 23.1
+    // us per call, 24.9 with the other; one unit of 148 parts, 320,000 keys: 70.0, and 64.6 with the other).  A limit to the grid costs
+    // there (300 tokens of 8 heads, 16,000 keys: 40.7 without, 42.7 with one of four per SM).
+    const int64_t units = (int64_t)d.blocks * d.Hkv, resident = 2 * (int64_t)d.ctas;
     const dim3 block(kDenseMergeWarps * 32);
-    if (d.ctas > 8 * units)
-        HOGATT_CUDA_OK(launch_kernel(dense_merge_kernel<T, PAGED, true>, dim3((unsigned)(64 * units)), block, 0, stream, d));
-    else
-        HOGATT_CUDA_OK(launch_kernel(dense_merge_kernel<T, PAGED, false>, dim3((unsigned)std::min<int64_t>(8 * units, 2 * (int64_t)d.ctas)), block, 0, stream, d));
+    if (d.ctas <= 8 * units) {
+        HOGATT_CUDA_OK(launch_kernel(dense_merge_kernel<T, PAGED, false, kDenseMergeBatch>, dim3((unsigned)std::min(8 * units, resident)), block, 0, stream, d));
+        return HOGATT_OK;
+    }
+    if constexpr (!PAGED)                                      // (a packed call here has more units: 1,024 rows at least)
+        if (64 * units <= resident) {
+            HOGATT_CUDA_OK(launch_kernel(dense_merge_kernel<T, PAGED, true, kDenseMergeBatch>, dim3((unsigned)(64 * units)), block, 0, stream, d));
+            return HOGATT_OK;
+        }
+    HOGATT_CUDA_OK(launch_kernel(dense_merge_kernel<T, PAGED, true, 1>, dim3((unsigned)(64 * units)), block, 0, stream, d));
     return HOGATT_OK;
 }
 

@@ -47,7 +47,7 @@ constexpr int kDenseThreads = (kDenseSoftmaxWarps + 4) * 32;
 constexpr int kDensePlanThreads = 1024;
 constexpr int kDenseMaxCtas = 256;
 constexpr int kDenseMergeWarps = 8;         // warps per CTA of the merge step; with many partials per row they share a row's
-constexpr int kDenseMergeBatch = 4;         // partials of a row that a thread of it has in flight
+constexpr int kDenseMergeBatch = 4;         // partials of a row that a thread of it has in flight (one in the lean instantiation)
 // Where no unit has more CTAs than this, the last CTA of a unit to finish folds the others' partials into its own rows, 128 KiB of
 // each, and nothing of it is left to the merge step (which then ends 1.5 us after the attention kernel instead of 12).  us per
 // call, folded up to 3 / merged: three parts at most (3 x 256 tokens, 5,700 keys, G = 5) 111.5 / 117.5, a 4,000-token prompt 134 /
@@ -1157,20 +1157,20 @@ dense_attention_kernel(const __grid_constant__ DenseArgs a, const __grid_constan
     }
 }
 
-// The units on the plan's list -- more than kDenseFoldParts CTAs worked on them, or nothing is visible --: fold the partials,
-// normalise, store.  A warp takes 32 rows, one per lane, and 16 columns: every load of a partial is 512 consecutive bytes, a lane
-// stores one 32-byte sector.  A CTA is the eight column groups of 32 rows, or with SPLIT eight warps that share the partials of the
-// same rows and columns (a unit cut into a hundred parts would be a chain of as many loads); the grid walks the list.
+// The units on the plan's list -- those that several CTAs worked on and none of them folds, or where nothing is visible --: fold
+// the partials, normalise, store.  A warp takes 32 rows, one per lane, and 16 columns: every load of a partial is 512 consecutive
+// bytes, a lane stores one 32-byte sector.  A CTA is the eight column groups of 32 rows, or with SPLIT eight warps that share the
+// partials of the same rows and columns (a unit cut into a hundred parts would be a chain of as many loads); the grid walks the list.
 // Bound by its chain of dependent loads -- list, partials, store, about a microsecond each -- and by the wait in front of
-// them, so a row's statistics and values are fetched together, kDenseMergeBatch partials at a time, and rescaled when a
-// later batch has the larger maximum (1,024 rows of 8 heads, 24,576 keys, 5.6 partials each: 7 us from the attention kernel's
-// end to this one's, 10 when the list's length, its entry, the maxima and the values were fetched one after the other).
+// them, so a row's statistics and values are fetched together, BATCH partials at a time, and rescaled when a later batch has
+// the larger maximum (1,024 rows of 8 heads, 24,576 keys, 5.6 partials each: 7 us from the attention kernel's end to this
+// one's, 10 when the list's length, its entry, the maxima and the values were fetched one after the other).
 //   out = sum_p O_p * 2^(m_p - M) / sum_p l_p * 2^(m_p - M),   M = max_p m_p
-template <class T, bool PAGED, bool SPLIT>
-__global__ void __launch_bounds__(kDenseMergeWarps * 32) dense_merge_kernel(const __grid_constant__ DenseArgs a) {
+template <class T, bool PAGED, bool SPLIT, int BATCH>
+__global__ void __launch_bounds__(kDenseMergeWarps * 32, BATCH == 1 ? 4 : 2) dense_merge_kernel(const __grid_constant__ DenseArgs a) {
     __shared__ float part[SPLIT ? kDenseMergeWarps : 1][18][32];         // 16 columns, maximum, sum; by row
     constexpr int PER = SPLIT ? 64 : 8;                                  // CTAs' worth of work per unit
-    constexpr int STRIDE = SPLIT ? kDenseMergeWarps : 1, BATCH = kDenseMergeBatch;
+    constexpr int STRIDE = SPLIT ? kDenseMergeWarps : 1;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     pdl_wait();
     pdl_trigger();

@@ -82,7 +82,20 @@ def _bind(p, d, out, status, **kw):
 ])
 @pytest.mark.parametrize("max_ctas", [1, 2, 3, 4, 5, 7, 9])
 def test_units_of_any_number_of_parts(W, G, S, Hkv, dtype, max_ctas):
-    p = _problem(W, G, S, Hkv, dtype, 3000)
+    _check(_problem(W, G, S, Hkv, dtype, 3000), max_ctas)
+
+
+@pytest.mark.parametrize("W,max_ctas,prompt", [
+    (2, 9, 18500),                                          # one unit; the merge step's warps share its partials,
+    (2, 31, 64000), (2, 32, 66000),                         # ... the last form without and the first with several of them in flight
+    (2, 33, 68000), (3, 65, 67000),                         # two units, one of one query tile
+])
+def test_units_of_many_parts(W, max_ctas, prompt):
+    _check(_problem(W, 8, 16, 1, torch.bfloat16, prompt), max_ctas)
+
+
+def _check(p, max_ctas):
+    dtype, Hkv = p.dtype, p.Hkv
     ref, _ = oracle.fused(p.queries, p.cos, p.sin, p.locations, p.keys, p.values, p.scale)
     d = p.to(DEV)
     status = torch.zeros(1, dtype=torch.int32, device=DEV)
@@ -101,7 +114,7 @@ def test_units_of_any_number_of_parts(W, G, S, Hkv, dtype, max_ctas):
         torch.cuda.synchronize()
         assert int(status.item()) == 0 and left() == expected
         results.append(out.clone())
-    check_against(results[0], ref.numpy(), dtype, what=f"{W} workers, {max_ctas} CTAs")
+    check_against(results[0], ref.numpy(), dtype, what=f"{max_ctas} CTAs")
     assert all(torch.equal(r, results[0]) for r in results[1:])
 
 
