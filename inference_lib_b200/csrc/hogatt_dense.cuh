@@ -1023,6 +1023,16 @@ dense_attention_kernel(const __grid_constant__ DenseArgs a, const __grid_constan
 
             // ---- end of this CTA's share of the unit: the rows themselves, or a partial result ----
             if (d.last()) {
+                const bool direct = d.whole() && !d.single(), one_tile = d.single();
+                const int unit = d.b * a.Hkv + d.h;
+                int* const fold = a.fold + (size_t)unit * kDenseFoldInts;
+                int* const left = fold + 4 + (one_tile ? warp & 7 : warp);
+                int2 who = make_int2(0, 0);
+                int n_left = 0;                                // (asked for in front of the last wait; an old answer costs a partial)
+                if (!direct) {
+                    who = *reinterpret_cast<const int2*>(fold);
+                    if (lane == 0) asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(n_left) : "l"(left) : "memory");
+                }
                 if (any) {
                     ok = mbar_wait_polls(o_done + 8 * g, phase ^ 1u, a.status, STATUS_WAIT_SYNC_TIMEOUT);
                     tc_fence_after();
@@ -1032,24 +1042,21 @@ dense_attention_kernel(const __grid_constant__ DenseArgs a, const __grid_constan
                 if (!ok) break;
                 const float total = half ? *other + l_run : l_run + *other;
                 named_barrier_sync(pair_bar, 64);              // (read before it is written again)
-                const bool direct = d.whole() && !d.single(), one_tile = d.single();
-                const int unit = d.b * a.Hkv + d.h, slot_row = g * kDenseRows + row;
+                const int slot_row = g * kDenseRows + row;
                 const size_t slot = (size_t)blockIdx.x + unit;
                 const float m_own = m_run == -INFINITY ? -INFINITY : m_run * scale2;
                 int first = blockIdx.x, parts = 1;             // partials that make up the rows: CTAs from `first` on, or their halves
                 bool finish = direct;
                 if (!direct) {
                     // Warps of different CTAs that hold the same rows and columns count themselves off; the last one has all
-                    // that the others left.  Not known yet to be the last: leave a partial first.
-                    int* const fold = a.fold + (size_t)unit * kDenseFoldInts;
-                    int* const left = fold + 4 + (one_tile ? warp & 7 : warp);
-                    const int2 who = *reinterpret_cast<const int2*>(fold);
+                    // that the others left.  Not known yet to be the last: leave a partial first.  (The count releases the
+                    // warp's partial and acquires the others', once: with a full fence on either side of it, the question asked
+                    // only here, and the other parts' maxima fetched one after the other, the fold was 1-2 us more: 640 tokens of
+                    // 1,024 packed keys 34.2 us, 32.0 now; a 1,500-token prompt of two kv heads 40.4 / 38.1.)
                     if (who.y > 0) {
                         first = who.x;
                         parts = one_tile ? 2 * who.y : who.y;
-                        int n = 0;
-                        if (lane == 0) asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(n) : "l"(left) : "memory");
-                        finish = __shfl_sync(0xffffffffu, n, 0) == 1;
+                        finish = __shfl_sync(0xffffffffu, n_left, 0) == 1;
                         __syncwarp();
                     }
                     if (!finish) {
@@ -1069,11 +1076,7 @@ dense_attention_kernel(const __grid_constant__ DenseArgs a, const __grid_constan
                         if (who.y > 0) {
                             __syncwarp();
                             int n = 0;
-                            if (lane == 0) {
-                                __threadfence();
-                                n = atomicSub(left, 1);
-                                __threadfence();
-                            }
+                            if (lane == 0) asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], -1;" : "=r"(n) : "l"(left) : "memory");
                             finish = __shfl_sync(0xffffffffu, n, 0) == 1;
                             __syncwarp();
                         }
@@ -1088,9 +1091,13 @@ dense_attention_kernel(const __grid_constant__ DenseArgs a, const __grid_constan
                         return sl * kDenseBlock + (one_tile ? (p & 1) * kDenseRows + row : slot_row);
                     };
                     float M = m_own, den = 0.f;
-#pragma unroll 1
-                    for (int p = 0; p < parts; ++p)
-                        if (p != own) M = fmaxf(M, __ldcg(a.ws_m + at(p)));
+                    if (parts > 1) {                           // (asked for together: each is a round trip to L2)
+                        float m[2 * kDenseFoldParts];
+#pragma unroll
+                        for (int p = 0; p < 2 * kDenseFoldParts; ++p) m[p] = p < parts && p != own ? __ldcg(a.ws_m + at(p)) : -INFINITY;
+#pragma unroll
+                        for (int p = 0; p < 2 * kDenseFoldParts; ++p) M = fmaxf(M, m[p]);
+                    }
                     const size_t offset = dense_out_offset<PAGED>(a, id, d.h) + half * COLS;
 #pragma unroll 1
                     for (int c = 0; c < COLS; c += 32) {
