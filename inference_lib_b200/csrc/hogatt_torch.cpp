@@ -366,16 +366,22 @@ void fragment_append(const at::Tensor& keys, const at::Tensor& values, const at:
     const int64_t F = (int64_t)key_fragments.size();
     TORCH_CHECK_EQ((int64_t)value_fragments.size(), F);
     for (const int64_t f : write_to) TORCH_CHECK(f >= 0 && f < F, "fragment_append: write_to names fragment ", f, " of ", F);
+    const c10::Device device = keys.device();
+    const caffe2::TypeMeta dtype = keys.dtype();
+    std::vector<int32_t> to(write_to.begin(), write_to.end()), rows(F);
+    std::vector<void*> kptr(F), vptr(F);
     for (int64_t f = 0; f < F; ++f) {
         const at::Tensor &k = key_fragments[f], &v = value_fragments[f];
-        TORCH_CHECK(k.device() == keys.device() && v.device() == keys.device(), "fragment_append: fragments on another device");
-        TORCH_CHECK(k.scalar_type() == keys.scalar_type() && v.scalar_type() == keys.scalar_type(), "fragment_append: fragment dtype != keys' dtype");
-        TORCH_CHECK(k.is_contiguous() && v.is_contiguous() && k.dim() >= 3 && v.dim() >= 3, "fragment_append: fragments must be contiguous [Hkv,capacity,E]");
-        TORCH_CHECK_EQ(k.size(-1), E);
-        TORCH_CHECK_EQ(v.size(-1), Ev);
-        TORCH_CHECK_EQ(v.size(-2), k.size(-2));
-        TORCH_CHECK(k.size(-3) == Hkv && v.size(-3) == Hkv && k.numel() == Hkv * k.size(-2) * E && v.numel() == Hkv * k.size(-2) * Ev,
-                    "fragment_append: fragments must be [Hkv,capacity,E]");
+        const at::IntArrayRef ks = k.sizes(), vs = v.sizes();
+        const size_t kd = ks.size(), vd = vs.size();
+        TORCH_CHECK(k.device() == device && v.device() == device, "fragment_append: fragments on another device");
+        TORCH_CHECK(k.dtype() == dtype && v.dtype() == dtype, "fragment_append: fragment dtype != keys' dtype");
+        TORCH_CHECK(kd >= 3 && vd >= 3 && ks[kd - 1] == E && vs[vd - 1] == Ev && ks[kd - 2] == vs[vd - 2] && ks[kd - 3] == Hkv && vs[vd - 3] == Hkv &&
+                        k.numel() == Hkv * ks[kd - 2] * E && v.numel() == Hkv * ks[kd - 2] * Ev && k.is_contiguous() && v.is_contiguous(),
+                    "fragment_append: fragments must be contiguous [Hkv,capacity,E], not ", ks, " and ", vs);
+        kptr[f] = k.data_ptr();
+        vptr[f] = v.data_ptr();
+        rows[f] = (int32_t)ks[kd - 2];
     }
     for (const at::Tensor* t : {&lengths_in, (const at::Tensor*)&lengths_out})
         TORCH_CHECK(t->dim() == 1 && t->size(0) == F && t->is_contiguous() && t->scalar_type() == at::kInt,
@@ -408,13 +414,6 @@ void fragment_append(const at::Tensor& keys, const at::Tensor& values, const at:
     }
     p.new_rows = new_rows.has_value() ? new_rows->const_data_ptr<int>() : nullptr;
     p.take_leading = take_leading ? 1 : 0;
-    std::vector<int32_t> to(write_to.begin(), write_to.end()), rows(F);
-    std::vector<void*> kptr(F), vptr(F);
-    for (int64_t f = 0; f < F; ++f) {
-        kptr[f] = key_fragments[f].data_ptr();
-        vptr[f] = value_fragments[f].data_ptr();
-        rows[f] = (int32_t)key_fragments[f].size(-2);
-    }
     p.write_to = to.data();
     p.key_fragments = kptr.data();
     p.value_fragments = vptr.data();
