@@ -1196,6 +1196,12 @@ int launch_paged_dims(const PagedArgs& a, const PagedPlan& pl, int kernel, int d
     return HOGATT_ERR_UNSUPPORTED_HEAD_DIM;
 }
 
+template <class T>
+cudaError_t launch_append(const AppendArgs& a, dim3 grid, bool many, int vectorised, cudaStream_t stream) {
+    return many ? launch_kernel(append_kernel<T, kAppendCtas + 1>, grid, dim3(256), 0, stream, a, vectorised)
+                : launch_kernel(append_kernel<T, kAppendCtas>, grid, dim3(256), 0, stream, a, vectorised);
+}
+
 // ---- fixed scratch for hogatt_fused_launch_static ---------------------------------------------------
 // In host code `g_static_scratch` is only a handle for the symbol, not a device address; the address
 // the kernels can use comes from cudaGetSymbolAddress, looked up once per device.
@@ -1539,10 +1545,13 @@ int hogatt_append_launch(const hogatt_append* p, hogatt_stream_t stream) {
     const int64_t pieces = (int64_t)p->S * ((p->E + p->Ev) / (vectorised ? vec : 1));
     dim3 grid((unsigned)std::min<int64_t>((pieces + 255) / 256, 1 << 14), (unsigned)p->Hkv, (unsigned)p->W);
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+    int dev = 0, sms = 0, smem_optin = 0;
+    if (const int rc = current_device_info(&dev, &sms, &smem_optin)) return rc;
+    const bool many = (int64_t)grid.x * grid.y * grid.z > (int64_t)kAppendCtas * sms;
     switch (p->dtype) {
-        case HOGATT_F32: HOGATT_CUDA_OK(launch_kernel(append_kernel<float>, grid, dim3(256), 0, st, a, 0)); break;
-        case HOGATT_F16: HOGATT_CUDA_OK(launch_kernel(append_kernel<__half>, grid, dim3(256), 0, st, a, vectorised ? 1 : 0)); break;
-        default: HOGATT_CUDA_OK(launch_kernel(append_kernel<__nv_bfloat16>, grid, dim3(256), 0, st, a, vectorised ? 1 : 0)); break;
+        case HOGATT_F32: HOGATT_CUDA_OK(launch_append<float>(a, grid, many, 0, st)); break;
+        case HOGATT_F16: HOGATT_CUDA_OK(launch_append<__half>(a, grid, many, vectorised ? 1 : 0, st)); break;
+        default: HOGATT_CUDA_OK(launch_append<__nv_bfloat16>(a, grid, many, vectorised ? 1 : 0, st)); break;
     }
     return HOGATT_OK;
 }

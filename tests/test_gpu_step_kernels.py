@@ -80,3 +80,23 @@ def test_appends_in_a_row(dtype, E, S):
         assert torch.equal(ks[f][:, a:b].cpu(), want_k[f]) and torch.equal(vs[f][:, a:b].cpu(), want_v[f])
         for slab in (ks[f], vs[f]):
             assert (slab[:, :a] == 7).all() and (slab[:, b:] == 7).all()
+
+
+@pytest.mark.parametrize("dtype,E,rows", [(torch.bfloat16, 128, (592, 593, 2000)), (torch.float16, 64, (1184, 1185)), (torch.float32, 128, (74, 75))])
+def test_appends_of_a_prompts_rows(dtype, E, rows):
+    """Around four CTAs per SM (of 148): few rows' CTAs hold more registers."""
+    g = torch.Generator().manual_seed(E)
+    Hkv, inv = 8, 1.0 / (1e4 ** (torch.arange(0, E, 2, dtype=torch.float32) / E))
+    for S in rows:
+        k, v = (torch.randn(1, Hkv, S, E, generator=g).to(dtype) for _ in range(2))
+        cos, sin = oc.rotary_tables(torch.arange(3, 3 + S)[None].numpy(), inv.numpy())
+        kf, vf = (torch.full((Hkv, S + 9, E), 7.0, dtype=dtype, device=DEV) for _ in range(2))
+        lens = [torch.tensor([3], dtype=torch.int32, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)]
+        d = [t.to(DEV) for t in (k, v, cos, sin)]
+        assert _cabi.append(keys=d[0], values=d[1], cosines=d[2], sines=d[3], write_to=[0], key_fragments=[kf], value_fragments=[vf],
+                            lengths_in=lens[0], lengths_out=lens[1], stream=_stream()) == 0
+        torch.cuda.synchronize()
+        assert lens[1].tolist() == [3 + S]
+        assert torch.equal(kf[:, 3:3 + S].cpu(), oc.rotate_keys(k, cos, sin)[0]) and torch.equal(vf[:, 3:3 + S].cpu(), v[0])
+        for slab in (kf, vf):
+            assert (slab[:, :3] == 7).all() and (slab[:, 3 + S:] == 7).all()
