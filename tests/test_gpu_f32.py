@@ -40,3 +40,29 @@ def test_rows_past_the_true_length_are_not_touched():
     r = run_cabi(p, kernel=_cabi.KERNEL_FMA, keys=keys, values=values)
     assert r.rc == 0 and r.status == 0
     assert float((r.out.cpu() - ref).abs().max()) < 2e-5
+
+
+@pytest.mark.parametrize("E,rotary_dim", [(64, 64), (64, 32), (64, 12), (128, 128), (128, 40), (128, 2)])
+@pytest.mark.parametrize("G,shift", [(4, 0), (4, 1), (9, 1), (9, 2)])
+def test_rotation_of_the_queries(E, rotary_dim, G, shift):
+    """Part of a head, halves that are no whole 16-byte pieces, tables off the 16-byte boundary; 8 and 16 rows; the call of queries
+    that have been rotated before gives the same bits."""
+    p = wl.make_problem("f32", W=1, Hq=2 * G, Hkv=2, E=E, S=1, lengths=[70, 65], theta=1e4, dtype=torch.float32, seed=5, rotary_dim=rotary_dim)
+    ref, ref_rq = oracle.fused(p.queries, p.cos, p.sin, p.locations, p.keys, p.values, p.scale)
+    dev, d = torch.device("cuda:0"), p.to("cuda:0")
+    tables = []
+    for t in (d.cos, d.sin):
+        room = torch.empty(t.numel() + 4, device=dev)
+        room[shift:shift + t.numel()] = t.flatten()
+        tables.append(room[shift:shift + t.numel()].view(t.shape))
+    out, again = (torch.full((p.W, p.Hq, p.S, E), float("nan"), device=dev) for _ in range(2))
+    rq = torch.full(ref_rq.shape, float("nan"), device=dev)
+    for fused in (True, False):
+        bp = _cabi.bind(out=out if fused else again, queries=d.queries if fused else rq, locations=d.locations, keys=d.keys, values=d.values,
+                        scale=p.scale, fragment_lengths=d.fragment_lengths, cos=tables[0] if fused else None, sin=tables[1] if fused else None,
+                        rq=rq if fused else None)
+        _cabi.attach_workspace(bp, dev)
+        assert _cabi.launch(bp, torch.cuda.current_stream().cuda_stream) == 0
+        torch.cuda.synchronize()
+    assert torch.equal(rq.cpu(), ref_rq) and torch.equal(out, again)
+    assert float((out.cpu() - ref).abs().max()) < 2e-5
