@@ -300,10 +300,13 @@ int64_t tiles_upper_bound(const hogatt_problem* p, const Resolved& r) {
 }
 
 // Which tcgen05 kernel a call of at least 128 query rows per kv head runs on.  Blocks of two query tiles where they give every
-// CTA a step and do not fall apart into many partials each, unless the work is long enough to carry that (figures in
-// hogatt_dense_tile.cuh; two units cut into 74 parts each, 16,100 keys: 35 us against 27; one unit, 131,000 keys, 7 steps a
-// CTA: 52 against 44).  One tile per unit otherwise, and where the workspace is too small for the partials of the other (a
-// caller's fixed one).
+// CTA a step and do not fall apart into many partials each, unless the work is long enough to carry that.  One tile per unit
+// otherwise, and where the workspace is too small for the partials of the other (a caller's fixed one).  us per call on blocks / on
+// single tiles, where the line sends the call to single tiles: one unit (256 rows, one kv head) 16,000 keys 31.7 / 25.0, 64,000 keys
+// 37.1 / 31.2, 131,000 44.7 / 45.3; eight units 2,000 keys 23.6 / 27.0, 8,000 28.2 / 37.3, 32,000 48.5 / 65.2; 16 units 1,000 keys 24.9 /
+// 26.8, 16,000 47.1 / 64.5; to blocks: 24 units 1,000 keys 25.0 / 33.2; 32 units 500 keys 24.4 / 30.9; eight units 64,000 keys 72.6 /
+// 103.0.  (The line was drawn when the plan and the merge step of blocks took some 10 us more: from two units on, and some hundred
+// steps in all, it lies too high.)
 bool dense_pairs(const hogatt_problem* p, const Resolved& r, int grid) {
     if (r.kernel != HOGATT_KERNEL_DENSE || r.row_blocks < 2) return false;
     const int64_t units = (int64_t)((r.row_blocks + 1) / 2) * p->Hkv, steps = units * tiles_upper_bound(p, r);
@@ -516,8 +519,8 @@ int launch_fma_dims(const KernelArgs& args, int dev, int smem_optin, int grid, c
     return HOGATT_ERR_UNSUPPORTED_HEAD_DIM;
 }
 
-// fp32 with E == Ev == 64 or 128.  Up to 8 query rows per kv head take the instantiation of 8 rows, whose warps hold half as
-// many (it stays on the memory's side of the line where 16 rows reach it).
+// fp32 with E == Ev == 64 or 128.  Up to 8 query rows per kv head take the instantiation of 8 rows: half the products, and it stays
+// on the memory's side of the line where 16 rows reach it (7,402 keys of 8 kv heads: 24.7 us with 8 rows, 38.7 with 16).
 template <int HD, int R>
 int launch_f32(const KernelArgs& args, int dev, int smem_optin, int grid, cudaStream_t stream) {
     static std::atomic<size_t> granted[kMaxDevices];
@@ -1041,11 +1044,12 @@ bool paged_mma_disabled() {
 // 8-row swizzle groups (or hold whole tiles), the number of blocks known (a tensor map needs the extent).  AUTO takes it
 // where the prompt chunks of the batch -- the tokens beyond one per sequence, over as many keys as the block table has room
 // for -- would keep the mma.sync kernel (115 TFLOP/s: it reads every sequence once per 16 rows) busy for some 20 us: the
-// tcgen05 kernel takes up to 12 us more before and after.  The lengths are on the device; where the table has far more room than
-// the sequences have keys the rule guesses too high, and costs little.  Tables of 32,768 keys, 8 kv heads of 4 heads, us per call
-// on the tcgen05 / mma.sync kernel: a chunk of 512 tokens at 4,000 keys 46 / 245, at 512 keys 26 / 58; 128 tokens at 1,000 keys
-// 26 / 35, at 128 keys 17 / 19; 64 tokens at 64 keys 17 / 17; 40 at 40 16 / 16; 128 at 128 beside 64 single tokens at 300 keys 80 /
-// 67, at 4,000 keys 226 / 237; beside 200 at 1,000 keys 262 / 396.
+// tcgen05 kernel takes 15-18 us however short the call is.  The lengths are on the device; where the table has far more room than
+// the sequences have keys the rule guesses too high, and costs up to 7 us.  Tables of 32,768 keys, 8 kv heads of 4 heads, us per
+// call on the tcgen05 / mma.sync kernel: a chunk of 512 tokens at 4,000 keys 49 / 247, at 512 keys 27 / 60; 128 tokens at 1,000 keys
+// 26 / 36, at 128 keys 19 / 20; 64 tokens at 1,000 keys 23 / 26, at 64 keys 19 / 18; 40 at 2,000 keys 24 / 28, at 500 22 / 20, at 40
+// 18 / 17; 33 at 500 keys 22 / 15; left to the mma.sync kernel: 20 at 2,000 keys 25 / 18.  128 at 128 beside 64 single tokens at 300
+// keys 70 / 68, at 4,000 keys 215 / 237; beside 200 at 1,000 keys 240 / 396.
 bool paged_dense_wanted(const hogatt_paged_problem* p) {
     if (p->kernel != HOGATT_KERNEL_AUTO || p->cu_seqlens_q == nullptr || p->num_blocks <= 0) return false;
     if (dense_disabled() || paged_mma_disabled()) return false;

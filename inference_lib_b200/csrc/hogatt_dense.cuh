@@ -6,7 +6,7 @@
 // Decomposition.  Query rows are cut into tiles of 128 (the MMA's M).  A block is two tiles that read the same keys, a
 // unit is (block, kv head).  dense_plan_kernel finds, per tile and fragment, how many keys any of its rows sees; a
 // block walks only those, 128 keys per step -- of a causal prompt just over half (4,000 tokens: 543 us per call when
-// every block walked every key, 168 now) -- and the steps of all units are one list that a persistent grid of one
+// every block walked every key, 152 now) -- and the steps of all units are one list that a persistent grid of one
 // CTA per SM cuts into balanced contiguous ranges.  A unit that lies inside one range is normalised and stored by
 // its CTA; where units are cut into a few parts, the CTA that finishes last folds the partials of the others, else they are
 // left to dense_merge_kernel.

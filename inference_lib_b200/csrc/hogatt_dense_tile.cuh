@@ -1,8 +1,8 @@
 // tcgen05 attention for calls that do not fill the GPU with blocks of two query tiles (hogatt_dense.cuh): one 128-row tile per
 // unit, the same keys for every unit, tiles cut into balanced ranges like the mma.sync kernel's and merged by merge_kernel.
-// Half the work per unit, no plan kernel, no segment ring: 128 rows over one kv head and 16,100 keys take 21 us per call here and
-// 93 there, 1,024 rows over one kv head and 2,900 keys 25 and 42, 128 rows over 8 kv heads and 8,100 keys 31 and 61; with more
-// steps than CTAs the other kernel is up to twice as fast (512 causal tokens: 37 us here, 26 there).
+// Half the work per unit, no plan kernel, no segment ring.  us per call here / there: 128 rows over one kv head, 16,100 keys
+// 22.9 / 30.5, 131,000 keys 33.2 / 52.4; 128 rows over 8 kv heads, 4,000 keys 26.5 / 26.6; with more steps than CTAs the other
+// kernel is up to a third faster (512 causal tokens 37.8 / 25.9).
 //
 // Queries arrive already rotated; a 128-row tile of one fragment and kv head is one 5-D TMA box.  S = Q K^T into two tensor-memory
 // buffers, O += P V with P as the tensor-memory A operand, one issuing thread each.  Warp roles (352 threads): warps 0-7
