@@ -10,6 +10,7 @@
 #include <Python.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <c10/util/SmallVector.h>
 #include <torch/library.h>
 
 #include <algorithm>
@@ -368,8 +369,8 @@ void fragment_append(const at::Tensor& keys, const at::Tensor& values, const at:
     for (const int64_t f : write_to) TORCH_CHECK(f >= 0 && f < F, "fragment_append: write_to names fragment ", f, " of ", F);
     const c10::Device device = keys.device();
     const caffe2::TypeMeta dtype = keys.dtype();
-    std::vector<int32_t> to(write_to.begin(), write_to.end()), rows(F);
-    std::vector<void*> kptr(F), vptr(F);
+    c10::SmallVector<int32_t, 32> to(write_to.begin(), write_to.end()), rows(F);
+    c10::SmallVector<void*, 32> kptr(F), vptr(F);
     for (int64_t f = 0; f < F; ++f) {
         const at::Tensor &k = key_fragments[f], &v = value_fragments[f];
         const at::IntArrayRef ks = k.sizes(), vs = v.sizes();
